@@ -927,11 +927,15 @@ extern "C" cmn_status cmn_autotune(cmn_problem* p, int32_t precision, uint64_t n
       if (r > 0 && t < ms) ms = t;
     }
   };
-  out->candidates = 0;
-  out->ms_best = 1e30;
+  // the default shape is a candidate with the time it was measured at
   time_shape(occ, lanes_max, out->ms_default);
+  out->candidates = 1;
+  out->ms_best = out->ms_default;
+  out->blocks_per_sm = occ;
+  out->lanes_cap = lanes_max;
   for (int bps = 1; bps <= occ && e == cudaSuccess; ++bps) {
     for (int lanes = 1; lanes <= lanes_max && e == cudaSuccess; lanes <<= 1) {
+      if (bps == occ && lanes == lanes_max) continue;
       double ms;
       time_shape(bps, lanes, ms);
       ++out->candidates;
