@@ -95,6 +95,7 @@ static cudaError_t ensure_attributes()
   std::lock_guard<std::mutex> lock(g_attr_mu);
   if (dev < 31 && (g_attr_device_mask & (1 << dev))) return cudaSuccess;
   e = set_eval_kernel_attributes(max_dynamic_smem());
+  if (e == cudaSuccess) e = set_chain_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_batch_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess && dev < 31) g_attr_device_mask |= (1 << dev);
   return e;
@@ -117,6 +118,8 @@ cmn_problem::~cmn_problem()
   dfree(d_inc_seg);
   dfree(d_inc_off);
   dfree(d_inc_pcs);
+  dfree(d_chain_seg);
+  dfree(d_chain_term);
   if (cur != device) cudaSetDevice(cur);
 }
 
@@ -171,14 +174,16 @@ extern "C" cmn_status cmn_problem_create(const cmn_problem_desc* desc, cmn_probl
                        cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess && p->prog.inc_ok) {
-      auto up = [&](int32_t** d, const std::vector<int32_t>& h) {
+      auto up = [&](auto** d, const auto& h) {
         if (e == cudaSuccess) e = dalloc(d, std::max<size_t>(1, h.size()));
         if (e == cudaSuccess && !h.empty())
-          e = cudaMemcpy(*d, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
+          e = cudaMemcpy(*d, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice);
       };
       up(&p->d_inc_seg, p->prog.inc_seg);
       up(&p->d_inc_off, p->prog.inc_off);
       up(&p->d_inc_pcs, p->prog.inc_pcs);
+      up(&p->d_chain_seg, p->prog.chain_seg);
+      up(&p->d_chain_term, p->prog.chain_term);
     }
     if (e != cudaSuccess) {
       delete p;
@@ -586,6 +591,8 @@ extern "C" cmn_status cmn_bound(cmn_role* r, const double* box, const uint64_t* 
   a.slots = sp;
   a.max_slots = (int)r->slot_kinds.size();  // one parent: the stride of the slot table is unused
   a.n_children = r->n_regions;
+  a.chain = r->p->chain();
+  a.max_boxes = r->n_regions;
   a.out_lb = r->d_lb;
   a.out_flag = r->d_feas;
   a.sched = r->p->d_sched;
@@ -666,9 +673,12 @@ extern "C" cmn_status cmn_bound_children(cmn_role* r, const double* box, const u
   a.slots = sp;
   a.max_slots = (int)r->slot_kinds.size();
   a.n_children = r->n_regions;
+  a.chain = r->p->chain();
+  a.max_boxes = r->n_regions;
   a.sched = r->p->d_sched;
   a.g_max = r->p->prog.group_max;
   a.capacity = (uint64_t)r->grid * kEvalThreads;
+  a.out_flag = r->d_feas;  // scratch: the regions' feasibility
   a.agg_keys = r->d_agg;
   a.agg_m = r->n_regions / k;
   a.agg_k = k;
@@ -814,6 +824,8 @@ extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, co
   a.pstride = ps;
   a.pinfo = nullptr;
   a.n_children = n_boxes;
+  if (!fp32) a.chain = p->chain();
+  a.max_boxes = n_boxes;
   a.out_lb = dlb;
   a.out_ub = dub;
   a.out_flag = dfe;
@@ -1206,6 +1218,7 @@ extern "C" cmn_status cmn_solver_create(const cmn_problem* p, const cmn_solve_op
     b.prog32 = p->d_prog32;
     b.prog32p = p->d_prog32p;
     b.sched = p->d_sched;
+    b.chain = p->chain();
     b.kinds = p->d_kinds;
     b.root_lb = p->d_root_lb;
     b.root_ub = p->d_root_ub;

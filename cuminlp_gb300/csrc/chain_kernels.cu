@@ -1,0 +1,376 @@
+// chain_kernels.cu -- the FP64 evaluator of programs that are sets of sum
+// chains (every quadratic model), in two passes: the constraints, a tile of
+// boxes per block and a warp per chain; then the objective, lanes per box
+// (chain_core.cuh).
+//
+// What bounds it: FP64 instructions issue at 1/64 of the FP32 rate, and the
+// interpreter spends four of them per term on both bounds of every chain.
+// Here the constraints, nine tenths of a program's terms, are decided in
+// FP32, and FP64 work is left to the objective's lower bound and to the few
+// comparisons the FP32 error bound leaves open.  On the n = 64 MIQCQP (2^17
+// regions of one box) the interpreter took 18.5 ms, these passes 0.74 and
+// 0.84 ms: the first at 92 % of the shared-memory bandwidth (two 8-byte loads
+// per term and box), the second at 70 % of the FP64 pipe.
+#include <cfloat>
+#include <cstdint>
+
+#include "chain_core.cuh"
+#include "child_core.cuh"
+#include "launch.hpp"
+
+namespace cmn {
+
+namespace {
+
+constexpr int kTileWarps = 8;     // warps of a constraint tile: one per chain below that
+constexpr int kObjThreads = 128;  // threads of an objective block
+
+using V64 = ChildVars<double, double>;
+
+// The two-sided interpreter over one chain and its readers.
+template <bool kFused>
+__device__ __noinline__ void chain_general(const Instr* prog, int pc0, int pc1, const V64& vars, Verdict<double>& v)
+{
+  const Tile<double> t = {};
+  interval_range<double, V64, kFused>(prog, pc0, pc1, vars, t, v);
+}
+
+// A <= chain in FP64: its lower bound against the right side.
+template <bool kFused>
+__device__ __noinline__ bool chain_le_exact(const Instr* prog, const ChainSeg& s, const V64& vars)
+{
+  const double lo = chain_lo<kFused>(prog, s.pc0, s.pc1, vars);
+  if (lo == lo) return lo <= s.rhs;
+  Verdict<double> v = verdict_init<double>();
+  chain_general<kFused>(prog, s.pc0, s.pc2, vars, v);
+  return v.feasible;
+}
+
+// A constraint tile in shared memory: bounds cut to FP32 and their largest
+// magnitudes per variable, and the split variables of each box in FP64.
+struct TileSmem {
+  float2* x;     // [n_vars][boxes]
+  double* olo;   // [max_slots][boxes]
+  double* ohi;
+  float* hull;   // [n_vars]
+  int32_t* ovid;
+};
+
+__device__ __forceinline__ TileSmem tile_smem(unsigned char* raw, int n_vars, int ms, int boxes)
+{
+  TileSmem t;
+  t.x = reinterpret_cast<float2*>(raw);
+  t.olo = reinterpret_cast<double*>(t.x + (size_t)n_vars * boxes);
+  t.ohi = t.olo + (size_t)ms * boxes;
+  t.hull = reinterpret_cast<float*>(t.ohi + (size_t)ms * boxes);
+  t.ovid = reinterpret_cast<int32_t*>(t.hull + n_vars);
+  return t;
+}
+
+size_t tile_smem_bytes(int n_vars, int ms, int boxes)
+{
+  return ((size_t)n_vars * 8 + (size_t)ms * 20) * (size_t)boxes + (size_t)n_vars * 4;
+}
+
+__device__ __forceinline__ uint64_t box_count(const EvalArgs& a, bool list)
+{
+  return list ? *a.list_count : (a.n_children_dev ? *a.n_children_dev : a.n_children);
+}
+
+__device__ __forceinline__ float max_abs_group(float m, int boxes)
+{
+  for (int off = 1; off < boxes; off <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+  return m;
+}
+
+}  // namespace
+
+// The constraints of every box (all chains but an objective one).  kMode and
+// kFused as eval_children's; out_flag gets 0 / 1 (kMode 0 and 4), or
+// kChildNone, kChildDuplicate, kChildInfeasible or kChildEligible (1 and 3).
+// A tile has 2^log_boxes boxes, 32 >> log_boxes lanes on each.  Every warp of
+// a block walks the same tiles, so the barriers are uniform.
+template <int kMode, bool kFused>
+__global__ void __launch_bounds__(kTileWarps * 32, 4) chain_constraints_kernel(const EvalArgs a, int log_boxes)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned fail_s;  // boxes a constraint excludes
+  __shared__ unsigned bad_s;   // boxes outside the filter's range
+  __shared__ int next_s;       // next chain of the tile
+  const int boxes = 1 << log_boxes, L = 32 >> log_boxes;
+  const int ms = a.pinfo != nullptr ? a.max_slots : 0;
+  const TileSmem t = tile_smem(smem_raw, a.n_vars, ms, boxes);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int box = lane & (boxes - 1), sub = lane >> log_boxes;
+  if (a.done != nullptr && *a.done) return;
+  const uint64_t total = box_count(a, kMode == 3);
+  const uint64_t tiles = (total + (uint64_t)boxes - 1) >> log_boxes;
+  const int first = a.chain.seg[0].kind == kChainObjective ? 1 : 0;
+  for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    // this lane's box; lanes past the end shadow the last one
+    const uint64_t at = (tile << log_boxes) + box;
+    bool live = at < total;
+    const uint64_t idx = live ? at : total - 1;
+    const uint64_t g = kMode == 3 ? (uint64_t)a.list[idx] : idx;
+    uint64_t k, r;
+    child_of(a.log2C, g, k, r);
+    const bool writes = live && wid == 0 && sub == 0;
+    uint32_t count = 0;
+    const SlotPlan* sp = nullptr;
+    if (a.pinfo != nullptr) {
+      const ParentInfo pi = a.pinfo[k];
+      if ((kMode == 1 || kMode == 3) && (pi.fathom || r >= pi.nreg)) {
+        if (kMode == 1 && writes) a.out_flag[g] = kChildNone;
+        live = false;
+      } else {
+        count = pi.count;
+        sp = a.slots + k * (uint64_t)a.max_slots;
+      }
+    }
+    // (1) the tile: the parents' bounds, then the split variables
+    bool bad = false;
+    for (int v0 = wid * L; v0 < a.n_vars; v0 += W * L) {
+      const int v = v0 + sub;
+      float m = 0.0f;
+      if (v < a.n_vars) {
+        bool b = false;
+        const float lo = cut32(__ldg(a.plo + (uint64_t)v * a.pstride + k), b);
+        const float hi = cut32(__ldg(a.phi + (uint64_t)v * a.pstride + k), b);
+        t.x[v * boxes + box] = make_float2(lo, hi);
+        bad = bad || b;
+        m = b ? 0.0f : fmaxf(fabsf(lo), fabsf(hi));
+      }
+      m = max_abs_group(m, boxes);
+      if (v < a.n_vars && box == 0) t.hull[v] = m;
+    }
+    if (threadIdx.x == 0) {
+      fail_s = 0;
+      bad_s = 0;
+      next_s = first;
+    }
+    __syncthreads();
+    V64 cv;
+    cv.plo = a.plo + k;
+    cv.phi = a.phi + k;
+    cv.pstride = a.pstride;
+    cv.mask = 0;
+    cv.olo = t.olo + box;
+    cv.ohi = t.ohi + box;
+    cv.ovid = t.ovid + box;
+    cv.count = (int)count;
+    cv.stride = boxes;
+    bool dup = false;
+    for (uint32_t j = 0; j < count; ++j) {
+      const SlotPlan s = sp[j];
+      cv.mask |= 1ULL << (s.vid & 63);
+      const bool mine = (int)(j % (uint32_t)(W * L)) == wid * L + sub;
+      if (kMode == 1 || kMode == 3 || mine) {
+        const uint64_t part = slot_part(r, s);
+        if (part >= s.dom) dup = true;
+        if (mine) {
+          double lo, hi;
+          slot_bounds(s, a.plo[(uint64_t)s.vid * a.pstride + k], a.phi[(uint64_t)s.vid * a.pstride + k], part, lo, hi);
+          t.olo[j * boxes + box] = lo;
+          t.ohi[j * boxes + box] = hi;
+          t.ovid[j * boxes + box] = (int32_t)s.vid;
+          bool leads = true;  // a variable of two slots takes the first one's part
+          for (uint32_t q = 0; q < j; ++q) leads = leads && sp[q].vid != s.vid;
+          if (leads) t.x[s.vid * boxes + box] = make_float2(cut32(lo, bad), cut32(hi, bad));
+        }
+      }
+    }
+    if ((kMode == 1 || kMode == 3) && dup) {
+      if (live && wid == 0 && sub == 0) a.out_flag[g] = kChildDuplicate;
+      live = false;
+    }
+    if (bad) atomicOr(&bad_s, 1u << box);
+    const unsigned alive = __ballot_sync(0xffffffffu, live);  // the same in every warp
+    __syncthreads();
+    if (alive != 0u) {
+      const bool in_range = !((bad_s >> box) & 1u);
+      // (2) the chains, drawn from a ticket until every box is excluded
+      for (;;) {
+        int q = 0;
+        if (lane == 0) q = atomicAdd(&next_s, 1);
+        q = __shfl_sync(0xffffffffu, q, 0);
+        if (q >= a.chain.n_seg) break;
+        const ChainSeg& s = a.chain.seg[q];
+        bool ok = true, open = live && sub == 0;
+        if (s.kind == kChainLe && s.eps > 0.0f) {
+          const float err = s.eps * chain_magnitude(s, a.chain.term, t.hull);
+          float est = filter_chain(s, a.chain.term, t.x + box, (uint32_t)boxes, sub, L);
+          for (int off = boxes; off < 32; off <<= 1) est += __shfl_xor_sync(0xffffffffu, est, off);
+          if (in_range) {
+            ok = !(__fsub_rd(est, err) > s.rhs_up);
+            open = open && ok && !(__fadd_ru(est, err) <= s.rhs_dn);
+          }
+          if (open) ok = chain_le_exact<kFused>(a.prog, s, cv);
+        } else if (s.kind == kChainLe) {
+          if (open) ok = chain_le_exact<kFused>(a.prog, s, cv);
+        } else if (open) {
+          Verdict<double> v = verdict_init<double>();
+          chain_general<kFused>(a.prog, s.pc0, s.pc2, cv, v);
+          ok = v.feasible;
+        }
+        const unsigned no = __ballot_sync(0xffffffffu, live && sub == 0 && !ok);
+        if (lane == 0 && no) atomicOr(&fail_s, no);
+      }
+    }
+    __syncthreads();
+    if (live && wid == 0 && sub == 0) {
+      const bool feasible = !((fail_s >> box) & 1u);
+      if (kMode == 0 || kMode == 4) a.out_flag[g] = feasible ? 1 : 0;
+      else a.out_flag[g] = feasible ? kChildEligible : kChildInfeasible;
+    }
+    __syncthreads();  // the tile is restaged next
+  }
+}
+
+// The objective of every box the constraints left (kMode 0: of every box).
+// `flags`: the constraint pass ran, out_flag holds its verdicts; otherwise
+// no chain decides feasibility and the children's states are found here.
+// 2^lg lanes share a box when few boxes are live.
+template <int kMode, bool kFused, bool kHi>
+__global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const EvalArgs a, int flags)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int B = blockDim.x;
+  const int ms = a.pinfo != nullptr ? a.max_slots : 0;
+  double* olo = reinterpret_cast<double*>(smem_raw) + threadIdx.x;
+  double* ohi = olo + (size_t)ms * B;
+  int32_t* ovid = reinterpret_cast<int32_t*>(reinterpret_cast<double*>(smem_raw) + (size_t)2 * ms * B) + threadIdx.x;
+  if (a.done != nullptr && *a.done) return;
+  const uint64_t total = box_count(a, kMode == 3);
+  const double gub = a.gub ? *a.gub : DBL_MAX;
+  const ChainSeg s = a.chain.seg[0];
+  const bool pure = s.kind == kChainObjective;
+  const int lg = lanes_per_box(total, (uint64_t)gridDim.x * B, pure && !kHi ? 32 : 1);
+  const int G = 1 << lg;
+  const uint64_t per_block = (uint64_t)(B >> lg);
+  for (uint64_t base = (uint64_t)blockIdx.x * per_block; base < total; base += (uint64_t)gridDim.x * per_block) {
+    const uint64_t idx = base + (threadIdx.x >> lg);
+    const bool lead = (threadIdx.x & (G - 1)) == 0;
+    bool live = idx < total;
+    uint64_t g = 0, k = 0, r = 0;
+    V64 cv = {};
+    bool feasible = true;
+    if (live) {
+      g = kMode == 3 ? (uint64_t)a.list[idx] : idx;
+      child_of(a.log2C, g, k, r);
+      if (flags) {
+        const uint8_t f = a.out_flag[g];
+        if (kMode == 1 || kMode == 3) live = f == kChildEligible;
+        else if (kMode == 4 || kFused) live = f != 0;
+        feasible = f != 0;
+      } else if ((kMode == 1 || kMode == 3) && a.pinfo != nullptr) {
+        const ParentInfo pi = a.pinfo[k];
+        if (pi.fathom || r >= pi.nreg) {
+          if (kMode == 1 && lead) a.out_flag[g] = kChildNone;
+          live = false;
+        }
+      }
+    }
+    if (live) {
+      bool dup;
+      cv = child_vars<double, double>(a, a.plo, a.phi, k, r, olo, ohi, ovid, B, dup);
+      if (!flags && (kMode == 1 || kMode == 3) && dup) {
+        if (lead) a.out_flag[g] = kChildDuplicate;
+        live = false;
+      }
+    }
+    Verdict<double> v = verdict_init<double>();
+    bool general = !pure || kHi;
+    if (!general) {
+      if (lg > 0) v.obj.lo = chain_lo_group<kFused>(a.prog, s.pc0, s.pc1, cv, G, live);
+      else if (live) v.obj.lo = chain_lo<kFused>(a.prog, s.pc0, s.pc1, cv);
+      general = v.obj.lo != v.obj.lo;
+    }
+    if (general && live) chain_general<kFused>(a.prog, s.pc0, s.pc2, cv, v);
+    v.feasible = feasible;
+    if constexpr (kMode == 4) {
+      aggregate_fold(a, live && lead, r, v);
+    } else {
+      if (live && lead) write_verdict<double, kMode>(a, g, k, v, gub);
+    }
+  }
+}
+
+static uint64_t resident(uint64_t blocks, const void* kernel, int threads, size_t smem)
+{
+  int occ = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) occ = 1;
+  const uint64_t room = (uint64_t)sm_count() * (uint64_t)occ;
+  return blocks < 1 ? 1 : blocks < room ? blocks : room;
+}
+
+static size_t objective_smem(const EvalArgs& a)
+{
+  return (size_t)(a.pinfo != nullptr ? a.max_slots : 0) * 20 * kObjThreads;
+}
+
+template <int kMode, bool kFused, bool kHi>
+static cudaError_t launch_chain_t(const EvalArgs& a, cudaStream_t s)
+{
+  const int ms = a.pinfo != nullptr ? a.max_slots : 0;
+  const int chains = a.chain.n_seg - (a.chain.pure_objective ? 1 : 0);
+  if (chains > 0) {
+    // smaller tiles, more lanes per box, until the tiles fill the GPU
+    int lb = 5;
+    while (lb > 0 && (a.max_boxes >> lb) < (uint64_t)sm_count() * 2) --lb;
+    auto kernel = chain_constraints_kernel<kMode, kFused>;
+    const int threads = 32 * (chains < kTileWarps ? chains : kTileWarps);
+    const size_t smem = tile_smem_bytes(a.n_vars, ms, 1 << lb);
+    const uint64_t grid = resident((a.max_boxes + (1ull << lb) - 1) >> lb, (const void*)kernel, threads, smem);
+    kernel<<<(unsigned)grid, threads, smem, s>>>(a, lb);
+  }
+  auto kernel = chain_objective_kernel<kMode, kFused, kHi>;
+  const size_t smem = objective_smem(a);
+  const uint64_t grid = resident((a.max_boxes * 32 + kObjThreads - 1) / kObjThreads, (const void*)kernel, kObjThreads, smem);
+  kernel<<<(unsigned)grid, kObjThreads, smem, s>>>(a, chains > 0 ? 1 : 0);
+  return cudaGetLastError();
+}
+
+bool chain_fits(const EvalArgs& a)
+{
+  // the statics of the kernel take under 1 KiB beside the tile
+  return a.chain.n_seg > 0 &&
+         tile_smem_bytes(a.n_vars, a.pinfo != nullptr ? a.max_slots : 0, 32) + 1024 <= (size_t)max_dynamic_smem();
+}
+
+cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s)
+{
+  if (mode == 0) return a.out_ub != nullptr ? launch_chain_t<0, false, true>(a, s) : launch_chain_t<0, false, false>(a, s);
+  if (mode == 6) return launch_chain_t<0, true, false>(a, s);
+  if (mode == 1) return launch_chain_t<1, false, false>(a, s);
+  if (mode == 4) return launch_chain_t<4, false, true>(a, s);
+  return launch_chain_t<3, false, false>(a, s);
+}
+
+template <typename K>
+static cudaError_t allow(K kernel, int max_smem)
+{
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
+}
+
+template <int kMode, bool kFused, bool kHi>
+static cudaError_t allow_both(int max_smem)
+{
+  cudaError_t e = allow(chain_constraints_kernel<kMode, kFused>, max_smem);
+  return e == cudaSuccess ? allow(chain_objective_kernel<kMode, kFused, kHi>, max_smem) : e;
+}
+
+cudaError_t set_chain_kernel_attributes(int max_smem)
+{
+  cudaError_t e = allow_both<0, false, true>(max_smem);
+  if (e == cudaSuccess) e = allow_both<0, false, false>(max_smem);
+  if (e == cudaSuccess) e = allow_both<0, true, false>(max_smem);
+  if (e == cudaSuccess) e = allow_both<1, false, false>(max_smem);
+  if (e == cudaSuccess) e = allow_both<4, false, true>(max_smem);
+  if (e == cudaSuccess) e = allow_both<3, false, false>(max_smem);
+  return e;
+}
+
+}  // namespace cmn

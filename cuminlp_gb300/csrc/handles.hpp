@@ -23,10 +23,19 @@ struct cmn_problem {
   int32_t* d_inc_seg = nullptr;  // incremental child tables (Program::inc_*), null when none
   int32_t* d_inc_off = nullptr;
   int32_t* d_inc_pcs = nullptr;
+  cmn::ChainSeg* d_chain_seg = nullptr;  // sum chains (Program::chain_*), null when none
+  cmn::ChainTerm* d_chain_term = nullptr;
   // cmn_autotune's choice per precision (0 FP64, 1 FP32): blocks per SM
   // and lanes per box cap; 0 = not tuned
   int tuned_bps[2] = {0, 0};
   int tuned_lanes[2] = {0, 0};
+
+  cmn::ChainTab chain() const
+  {
+    if (!d_chain_seg) return cmn::ChainTab{};
+    return cmn::ChainTab{d_chain_seg, d_chain_term, (int32_t)prog.chain_seg.size(),
+                         prog.chain_seg[0].kind == cmn::kChainObjective ? 1 : 0};
+  }
 
   ~cmn_problem();
 };

@@ -155,6 +155,10 @@ struct EvalArgs {
   unsigned long long* agg_keys;
   uint64_t agg_m;
   uint64_t agg_k;
+  // FP64 passes: the program's sum chains, evaluated a warp per chain and 32
+  // boxes (chain_kernels.cu); n_seg 0: the interpreter
+  ChainTab chain;
+  uint64_t max_boxes;  // most boxes the launch can see (grid size)
 };
 
 struct SampleArgs {

@@ -39,6 +39,11 @@ int sample_screen_lg_min(int n_vars, int n_slots, bool has_sched, int threads);
 // 6: the lazy form's FP64 verdict of the staged parents (mode 0's outputs,
 // each term's coefficient and chain add fused into __fma_rd / __fma_ru)
 cudaError_t launch_eval(const EvalArgs& a, int mode, bool fp32, int grid, int threads, cudaStream_t s);
+// The FP64 modes over a program of sum chains (EvalArgs::chain):
+// chain_kernels.cu.  chain_fits: whether the launch takes that path.
+bool chain_fits(const EvalArgs& a);
+cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s);
+cudaError_t set_chain_kernel_attributes(int max_smem);
 cudaError_t launch_sample(const SampleArgs& a, int grid, int threads, cudaStream_t s);
 // the lazy form's incremental FP32 children: the common chain sums per
 // (segment, parent), then every child (EvalArgs::inc_* set, prog = FP32)

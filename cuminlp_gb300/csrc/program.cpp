@@ -286,6 +286,7 @@ class Compiler {
     out_.n_slots = max_slots_;
     build_schedule();
     build_incremental();
+    build_chains();
     out_.code32 = out_.code64;
     out_.code32p = out_.code64;
     for (size_t k = 0; k < out_.code64.size(); ++k) {
@@ -456,6 +457,92 @@ class Compiler {
     }
     out_.inc_off[lists.size()] = (int32_t)out_.inc_pcs.size();
     out_.inc_ok = true;
+  }
+
+  // Most that the FP32 filter of a chain of k terms can be off its FP64
+  // lower bound, per unit of summed term magnitude.  Per term: the two
+  // bounds cut to FP32 (2 u each, u = 2^-24), the product, the coefficient
+  // and its product (u each), 7 u.  The sum: two interleaved accumulators of
+  // k / 2 adds, joined, plus the constant: (k / 2 + 2) u.  The FP64 chain's
+  // own roundings (2^-52 each) and the comparison take the rest of the 13.
+  // The factor covers the products of these and the error of the summed
+  // magnitude itself (k / 2 u, k <= 8192).
+  static float chain_eps(int64_t k) { return (float)((double)(k / 2 + 13) * std::ldexp(1.0, -24) * 1.02); }
+
+  // Program::chain_*: the incremental segments as chains by reader.
+  void build_chains()
+  {
+    if (!out_.inc_ok) return;
+    const std::vector<Instr>& code = out_.code64;
+    std::vector<ChainSeg> segs;
+    for (int s = 0; s < out_.inc_segments; ++s) {
+      ChainSeg cs;
+      std::memset(&cs, 0, sizeof cs);
+      cs.kind = kChainGeneral;
+      cs.pc0 = out_.inc_seg[3 * s];
+      cs.pc1 = out_.inc_seg[3 * s + 1];
+      cs.pc2 = out_.inc_seg[3 * s + 2];
+      if (cs.pc1 > cs.pc0 && cs.pc2 == cs.pc1 + 1) {
+        const Instr& rd = code[cs.pc1];
+        const int op = rd.head & 7;
+        if ((rd.modes & 3) == kModeAcc && op == kOpObjective) cs.kind = kChainObjective;
+        if ((rd.modes & 3) == kModeAcc && op == kOpCheck && (rd.head >> 3) == CMN_CMP_LE) {
+          cs.kind = kChainLe;
+          cs.rhs = rd.c;
+          cs.rhs_dn = d2f_rd(rd.c);
+          cs.rhs_up = d2f_ru(rd.c);
+        }
+      }
+      if (cs.kind == kChainLe) add_filter(cs);
+      segs.push_back(cs);
+    }
+    auto rank = [&](const ChainSeg& s) {  // the objective's chain, general ones, <= chains
+      for (int pc = s.pc1; pc < s.pc2; ++pc)
+        if ((code[pc].head & 7) == kOpObjective) return -1;
+      return (int)s.kind;
+    };
+    std::stable_sort(segs.begin(), segs.end(), [&](const ChainSeg& a, const ChainSeg& b) {
+      const int ra = rank(a), rb = rank(b);
+      return ra != rb ? ra < rb : a.pc1 - a.pc0 > b.pc1 - b.pc0;
+    });
+    out_.chain_seg = segs;
+  }
+
+  // The FP32 filter's terms of a <= chain; leaves eps 0 (no filter) when a
+  // coefficient is outside the range its error bound covers.
+  void add_filter(ChainSeg& cs)
+  {
+    auto in_range = [](double c) { return std::fabs(c) >= std::ldexp(1.0, -40) && std::fabs(c) <= std::ldexp(1.0, 40); };
+    std::vector<ChainTerm> groups[6];
+    bool ok = cs.pc1 - cs.pc0 <= 8192;
+    auto put = [&](int g, double c, uint32_t a, uint32_t b) {
+      if (c == 0.0) return;
+      ok = ok && in_range(c);
+      groups[g + (c < 0.0 ? 1 : 0)].push_back(ChainTerm{a | (b << 16), d2f_rn(c)});
+    };
+    for (int pc = cs.pc0; pc < cs.pc1; ++pc) {
+      const Instr& in = out_.code64[pc];
+      const int sub = in.head >> 3;
+      if ((in.head & 7) == kOpLoadAcc) {
+        if ((in.modes & 3) == kModeVar) put(4, 1.0, in.a, in.a);
+        else if (in.c == 0.0 || in_range(in.c)) cs.c0 = d2f_rn(in.c);
+        else ok = false;
+        continue;
+      }
+      const double c = (sub & kTermHasC) ? in.c : 1.0;
+      const double sc = ((sub & kTermSub) && !(sub & kTermInit)) ? -c : c;
+      const int pk = sub & kTermPMask;
+      put(pk == kTermProd ? 0 : pk == kTermSqr ? 2 : 4, sc, in.a, pk == kTermProd ? in.b : in.a);
+    }
+    int64_t k = 0;
+    for (int g = 0; g < 6; ++g) {
+      cs.group[g] = (int32_t)out_.chain_term.size();
+      out_.chain_term.insert(out_.chain_term.end(), groups[g].begin(), groups[g].end());
+      if (out_.chain_term.size() & 1) out_.chain_term.push_back(ChainTerm{0, 0.0f});
+      k += (int64_t)groups[g].size() + 1;
+    }
+    cs.group[6] = (int32_t)out_.chain_term.size();
+    cs.eps = ok ? chain_eps(k) : 0.0f;
   }
 
   bool is_var(int64_t id) const { return p_.nodes[id].op == CMN_OP_VAR; }

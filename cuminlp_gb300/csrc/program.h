@@ -103,6 +103,43 @@ struct Instr {
 };
 static_assert(sizeof(Instr) == 16, "Instr layout");
 
+// ---- sum-chain programs (Program::chain_*) ----
+// One term of a chain's FP32 filter: c * x_a * x_b, c * sqr(x_a) or c * x_a.
+struct ChainTerm {
+  uint32_t ab;  // a in the low half, b in the high
+  float c;
+};
+
+enum ChainKind : int32_t {
+  kChainObjective = 0,  // read by the objective alone: one or both bounds
+  kChainGeneral = 1,    // any other reader: the two-sided interpreter
+  kChainLe = 2,         // read by one <= check alone: its lower bound
+};
+
+// One sum chain and its reader.
+struct ChainSeg {
+  int32_t kind;
+  int32_t pc0, pc1, pc2;  // chain instructions [pc0, pc1), readers [pc1, pc2)
+  // kChainLe: the filter's terms, by sign of the coefficient and product
+  // form -- [0,1) c > 0 x_a x_b, [1,2) c < 0 x_a x_b, [2,3) / [3,4) sqr,
+  // [4,5) / [5,6) linear; every group padded to an even length with c = 0
+  int32_t group[7];
+  float c0;              // constant start of the chain
+  float eps;             // FP32 error per unit of summed magnitude; 0: no filter
+  float rhs_dn, rhs_up;  // the right side rounded outward
+  int32_t pad;
+  double rhs;
+};
+
+// The chains of one program on the device: the one the objective reads
+// first, then the general ones, then the <= chains, longest first.
+struct ChainTab {
+  const ChainSeg* seg;
+  const ChainTerm* term;
+  int32_t n_seg;           // 0: the program is not a set of sum chains
+  int32_t pure_objective;  // the first one is kChainObjective
+};
+
 inline constexpr uint8_t make_head(uint8_t code, uint8_t sub)
 {
   return static_cast<uint8_t>(code | (sub << 3));

@@ -67,6 +67,10 @@ struct Program {
   // inc_pcs[inc_off[v * inc_segments + s] .. inc_off[v * inc_segments + s + 1])
   std::vector<int32_t> inc_off;
   std::vector<int32_t> inc_pcs;
+  // the same segments as chains with their readers, and the terms of the
+  // FP32 filter of the <= chains (ChainTab); empty unless inc_ok
+  std::vector<ChainSeg> chain_seg;
+  std::vector<ChainTerm> chain_term;
 };
 
 // Compiles the reachable DAG into the fused straight-line program.

@@ -175,6 +175,7 @@ struct SolverBufs {
   const Instr* prog32;
   const Instr* prog32p;  // FP32 point program (the lazy form's sample screen)
   const int32_t* sched;  // lane schedules of the program (null: none)
+  ChainTab chain;        // its sum chains (n_seg 0: none)
   const int32_t* kinds;
   const double* root_lb;
   const double* root_ub;

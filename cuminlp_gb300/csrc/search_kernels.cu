@@ -1442,6 +1442,8 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     pa.g_max = cfg.g_max;
     pa.capacity = cfg.eval_capacity;
     pa.error = &b.dev->error;
+    pa.chain = b.chain;
+    pa.max_boxes = cfg.e_max;
     e = launch_eval(pa, 6, false, eval_grid, kEvalThreads, side.stream);
     if (e != cudaSuccess) return e;
     mark(marks, 6, side.stream);
@@ -1479,6 +1481,8 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
   ea.sched = b.sched;
   ea.g_max = cfg.g_max;
   ea.capacity = cfg.eval_capacity;
+  ea.chain = b.chain;  // read by the FP64 passes
+  ea.max_boxes = max_children;
   cudaError_t e;
   if (cfg.precision == CMN_PRECISION_FP32_SCREEN) {
     ea.prog = b.prog32;

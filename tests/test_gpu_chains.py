@@ -1,0 +1,112 @@
+"""The evaluator of sum-chain programs (a tile of boxes per block, constraints
+decided in FP32 where its error bound allows) gives the oracle's verdicts bit
+for bit where it could go wrong: partial tiles, comparisons closer than the
+FP32 error, equality and shared-root readers, subtracted and constant chain
+terms, and bounds outside the FP32 filter's range."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle as O
+from cuminlp_gb300 import _abi as A
+from cuminlp_gb300 import generators as G
+from cuminlp_gb300.problem import Expr, Problem
+from cuminlp_gb300.solver import Bounder, DeviceProblem, eval_boxes
+from tests.conftest import bits_equal
+from tests.gpu_common import random_boxes
+from tests.test_gpu_solver import compare
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _built():
+    from cuminlp_gb300 import build
+    build.build_library()
+
+
+def mixed_problem() -> Problem:
+    """Chains of every reader and term form: <= and == checks, a constant and
+    a variable start, subtracted terms, terms without a coefficient, one root
+    read by the objective and a check, a product of a variable by itself."""
+    p = Problem()
+    x = [p.var(-3.0, 2.0), p.var(0.5, 4.0), p.var(-1.0, 1.0), p.int_var(0.0, 5.0), p.bin_var()]
+    obj = 2.0 * (x[0] * x[1]) - 3.0 * (x[2] * x[3]) + x[4] * x[0] - (x[1] * x[2])
+    p.set_objective(obj)
+    p.add_constraint(obj, A.CMP_LE, 4.0)
+    p.add_constraint(p.fixed(1.5) + x[0] * x[2] - 0.25 * x[3], A.CMP_LE, 1.0)
+    p.add_constraint(x[0] + 2.0 * x[1] - x[2], A.CMP_EQ, 1.0)
+    same = Expr(p.graph, p.graph.emit(A.OP_MUL, (x[2].id, x[2].id)))
+    p.add_constraint(-1.0 * same + 0.5 * (x[1] * x[1]) - 2.0 * x[4], A.CMP_LE, 2.0)
+    return p
+
+
+def near_problem(rhs_shift: float) -> Problem:
+    """One <= chain whose lower bound sits `rhs_shift` from the right side on
+    a whole lattice of boxes: 0 and one FP64 ulp are inside the FP32 error."""
+    p = Problem()
+    x = [p.var(-4.0, 4.0) for _ in range(6)]
+    acc = 1.25 * (x[0] * x[1])
+    for i in range(1, 5):
+        acc = acc + (0.5 + i) * (x[i] * x[i + 1])
+    p.set_objective(acc + 3.0 * x[0])
+    p.add_constraint(acc + 0.5 * (x[0] * x[0]), A.CMP_LE, -6.0 + rhs_shift)
+    return p
+
+
+def check(p: Problem, lo, hi):
+    g = eval_boxes(DeviceProblem(p), lo, hi)
+    o = O.OracleProblem(p).eval_boxes(lo, hi, A.PRECISION_FP64)
+    assert np.array_equal(g[2], o[2])
+    assert bits_equal(g[0], o[0]) and bits_equal(g[1], o[1])
+
+
+@pytest.mark.parametrize("count", [1, 31, 32, 33, 257, 4099])
+def test_partial_tiles(count):
+    rng = np.random.default_rng(count)
+    for p in (mixed_problem(), G.miqcqp_n32(1)):
+        check(p, *random_boxes(p, count, rng, 0.3))
+
+
+@pytest.mark.parametrize("shift", [0.0, 2.0 ** -50, -(2.0 ** -50), 2.0 ** -22, -(2.0 ** -22), 1.0])
+def test_comparisons_inside_the_fp32_error(shift):
+    # boxes on a quarter lattice: the chain's bound is exact, and -6 is one of
+    # its values
+    rng = np.random.default_rng(5)
+    lo = rng.integers(-8, 8, (6, 3000)) / 4.0
+    hi = lo + rng.integers(0, 3, lo.shape) / 4.0
+    p = near_problem(shift)
+    o = O.OracleProblem(p).eval_boxes(lo, hi, A.PRECISION_FP64)
+    assert 0 < np.sum(o[2]) < lo.shape[1]
+    check(p, lo, hi)
+
+
+@pytest.mark.parametrize("value", [0.0, -0.0, 1e-300, 1e-20, 5e-324, 1e13, 1e200, np.inf, -np.inf])
+def test_bounds_outside_the_filter_range(value):
+    rng = np.random.default_rng(3)
+    for p in (mixed_problem(), near_problem(0.25)):
+        lo, hi = random_boxes(p, 200, rng, 0.3)
+        at = rng.integers(0, lo.shape[0], 40), rng.integers(0, 200, 40)
+        lo[at] = np.minimum(value, hi[at])
+        both = rng.random(40) < 0.5
+        hi[at[0][both], at[1][both]] = np.maximum(value, lo[at[0][both], at[1][both]])
+        check(p, lo, hi)
+
+
+@pytest.mark.parametrize("bits", [1, 3, 6, 9])
+def test_role_regions(bits):
+    p = G.miqcqp_n32(2)
+    kinds, vids, widths, _ = O.bisection_choose(p.root_box(), p.var_kinds, bits)
+    n = int(np.prod(widths))
+    fe, lb = Bounder(DeviceProblem(p), kinds, n).bound(p.root_box(), vids, widths)
+    ofe, olb = O.OracleProblem(p).bound(p.root_box(), kinds, vids, widths, n)
+    assert np.array_equal(fe, ofe) and bits_equal(lb, olb)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "lazy"])
+@pytest.mark.parametrize("bits,parents", [(1, 3), (3, 33), (5, 20)])
+def test_solver_iterations(precision, bits, parents):
+    for p in (mixed_problem(), G.qcqp(G.QCQPSpec(n=9, m=3, n_int=2, int_lb=0, int_ub=6, rhs=(1.0, 3.0)), 77)):
+        compare(p, 9, bisection_budget=bits, batch_parents=parents, frontier_cap=500, precision=precision)
