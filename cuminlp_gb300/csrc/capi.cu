@@ -735,6 +735,9 @@ static cmn_status candidate_role(cmn_role* r, const double* box, const uint64_t*
   a.g_max = r->p->prog.group_max;
   a.capacity = (uint64_t)r->grid * kEvalThreads;
   a.lg_min = r->lg_min;
+  a.chain = r->p->chain();
+  for (int v = 0; v < a.n_vars; ++v)  // a box outside the filters' range takes the interpreter
+    if (!(std::fabs(box[2 * v]) <= kFilterMax) || !(std::fabs(box[2 * v + 1]) <= kFilterMax)) a.chain.points = 0;
   CK(launch_sample(a, r->grid, kEvalThreads, r->stream));
   Cand* best = r->d_block_best + r->grid;
   CK(launch_reduce_cand(r->d_block_best, r->grid, best, r->stream));

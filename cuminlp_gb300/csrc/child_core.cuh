@@ -1,5 +1,6 @@
 // child_core.cuh -- device code shared by the evaluators of children: which
-// parent and region a child is, its variables, and where its verdict goes.
+// parent and region a child is, its variables, where its verdict goes, and
+// the candidate reduction of the samplers.
 #pragma once
 
 #include <cfloat>
@@ -136,6 +137,36 @@ __device__ __forceinline__ void aggregate_fold(const EvalArgs& a, bool active, u
     atomicMin(a.agg_keys + c, kmin);
     atomicMax(a.agg_keys + a.agg_k + c, kmax);
   }
+}
+
+__device__ __forceinline__ void warp_min_cand(Cand& c)
+{
+  for (int off = 16; off > 0; off >>= 1) {
+    Cand o;
+    o.value = __shfl_down_sync(0xffffffffu, c.value, off);
+    o.k = __shfl_down_sync(0xffffffffu, c.k, off);
+    o.e = __shfl_down_sync(0xffffffffu, c.e, off);
+    o.pad = 0;
+    if (cand_less(o, c)) c = o;
+  }
+}
+
+// Block-wide min of one Cand per thread; result valid in thread 0.
+__device__ __forceinline__ Cand block_min_cand(Cand c)
+{
+  __shared__ Cand warp_best[32];
+  warp_min_cand(c);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) warp_best[wid] = c;
+  __syncthreads();
+  const int nw = (blockDim.x + 31) >> 5;
+  if (wid == 0) {
+    Cand x = lane < nw ? warp_best[lane] : Cand{INFINITY, 0xffffffffu, 0, ~0ULL};
+    warp_min_cand(x);
+    c = x;
+  }
+  __syncthreads();
+  return c;
 }
 
 }  // namespace cmn

@@ -517,36 +517,6 @@ __global__ void __launch_bounds__(kEvalThreads, CMN_EVAL_MIN_BLOCKS) eval_childr
   eval_children<double, kMode, double, true, kFused>(a, a.plo, a.phi);
 }
 
-__device__ __forceinline__ void warp_min_cand(Cand& c)
-{
-  for (int off = 16; off > 0; off >>= 1) {
-    Cand o;
-    o.value = __shfl_down_sync(0xffffffffu, c.value, off);
-    o.k = __shfl_down_sync(0xffffffffu, c.k, off);
-    o.e = __shfl_down_sync(0xffffffffu, c.e, off);
-    o.pad = 0;
-    if (cand_less(o, c)) c = o;
-  }
-}
-
-// Block-wide min of one Cand per thread; result valid in thread 0.
-__device__ __forceinline__ Cand block_min_cand(Cand c)
-{
-  __shared__ Cand warp_best[32];
-  warp_min_cand(c);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) warp_best[wid] = c;
-  __syncthreads();
-  const int nw = (blockDim.x + 31) >> 5;
-  if (wid == 0) {
-    Cand x = lane < nw ? warp_best[lane] : Cand{INFINITY, 0xffffffffu, 0, ~0ULL};
-    warp_min_cand(x);
-    c = x;
-  }
-  __syncthreads();
-  return c;
-}
-
 __device__ __forceinline__ bool admissible(const SampleArgs& a, const Tile<double>& t)
 {
   for (int v = 0; v < a.n_vars; ++v) {
@@ -1141,6 +1111,7 @@ int sample_screen_occupancy(size_t smem, int threads)
 
 cudaError_t launch_sample(const SampleArgs& a, int grid, int threads, cudaStream_t s)
 {
+  if (chain_sample_fits(a)) return launch_chain_sample(a, grid, s);
   const size_t smem = sample_smem_bytes(a.n_vars, a.n_slots, threads, a.lg_min);
   sample_children_kernel<<<grid, threads, smem, s>>>(a);
   return cudaGetLastError();

@@ -34,7 +34,7 @@ struct cmn_problem {
   {
     if (!d_chain_seg) return cmn::ChainTab{};
     return cmn::ChainTab{d_chain_seg, d_chain_term, (int32_t)prog.chain_seg.size(),
-                         prog.chain_seg[0].kind == cmn::kChainObjective ? 1 : 0};
+                         prog.chain_seg[0].kind == cmn::kChainObjective ? 1 : 0, prog.chain_points ? 1 : 0, 0};
   }
 
   ~cmn_problem();

@@ -195,6 +195,9 @@ struct SampleArgs {
   // lazy form: the sample screen writes `cbest` (prog = the FP32 point
   // program); the sampler then evaluates only each chunk's best in FP64
   Best32* cbest;
+  // the program's sum chains: points filtered in FP32 (chain_kernels.cu);
+  // n_seg 0: the interpreter
+  ChainTab chain;
 };
 
 }  // namespace cmn

@@ -44,6 +44,9 @@ cudaError_t launch_eval(const EvalArgs& a, int mode, bool fp32, int grid, int th
 bool chain_fits(const EvalArgs& a);
 cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s);
 cudaError_t set_chain_kernel_attributes(int max_smem);
+// the sampler over such a program (not the lazy form's chunk mode)
+bool chain_sample_fits(const SampleArgs& a);
+cudaError_t launch_chain_sample(const SampleArgs& a, int grid, cudaStream_t s);
 cudaError_t launch_sample(const SampleArgs& a, int grid, int threads, cudaStream_t s);
 // the lazy form's incremental FP32 children: the common chain sums per
 // (segment, parent), then every child (EvalArgs::inc_* set, prog = FP32)

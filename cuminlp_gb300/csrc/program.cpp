@@ -486,14 +486,15 @@ class Compiler {
         const Instr& rd = code[cs.pc1];
         const int op = rd.head & 7;
         if ((rd.modes & 3) == kModeAcc && op == kOpObjective) cs.kind = kChainObjective;
-        if ((rd.modes & 3) == kModeAcc && op == kOpCheck && (rd.head >> 3) == CMN_CMP_LE) {
-          cs.kind = kChainLe;
+        if ((rd.modes & 3) == kModeAcc && op == kOpCheck) {
+          if ((rd.head >> 3) == CMN_CMP_LE) cs.kind = kChainLe;
+          else cs.eq = 1;
           cs.rhs = rd.c;
           cs.rhs_dn = d2f_rd(rd.c);
           cs.rhs_up = d2f_ru(rd.c);
         }
       }
-      if (cs.kind == kChainLe) add_filter(cs);
+      if (cs.kind != kChainGeneral || cs.eq) add_filter(cs);
       segs.push_back(cs);
     }
     auto rank = [&](const ChainSeg& s) {  // the objective's chain, general ones, <= chains
@@ -506,9 +507,14 @@ class Compiler {
       return ra != rb ? ra < rb : a.pc1 - a.pc0 > b.pc1 - b.pc0;
     });
     out_.chain_seg = segs;
+    out_.chain_points = !segs.empty() && segs[0].kind == kChainObjective;
+    for (const ChainSeg& s : segs) out_.chain_points = out_.chain_points && s.eps > 0.0f;
+    for (size_t v = 0; v < p_.var_lb.size(); ++v)
+      out_.chain_points =
+          out_.chain_points && std::fabs(p_.var_lb[v]) <= kFilterMax && std::fabs(p_.var_ub[v]) <= kFilterMax;
   }
 
-  // The FP32 filter's terms of a <= chain; leaves eps 0 (no filter) when a
+  // The FP32 filter's terms of a chain; leaves eps 0 (no filter) when a
   // coefficient is outside the range its error bound covers.
   void add_filter(ChainSeg& cs)
   {

@@ -120,14 +120,14 @@ enum ChainKind : int32_t {
 struct ChainSeg {
   int32_t kind;
   int32_t pc0, pc1, pc2;  // chain instructions [pc0, pc1), readers [pc1, pc2)
-  // kChainLe: the filter's terms, by sign of the coefficient and product
+  // the filter's terms (kChainLe, kChainObjective, eq), by sign of the coefficient and product
   // form -- [0,1) c > 0 x_a x_b, [1,2) c < 0 x_a x_b, [2,3) / [3,4) sqr,
   // [4,5) / [5,6) linear; every group padded to an even length with c = 0
   int32_t group[7];
   float c0;              // constant start of the chain
   float eps;             // FP32 error per unit of summed magnitude; 0: no filter
   float rhs_dn, rhs_up;  // the right side rounded outward
-  int32_t pad;
+  int32_t eq;            // kChainGeneral read by one == check alone
   double rhs;
 };
 
@@ -138,7 +138,12 @@ struct ChainTab {
   const ChainTerm* term;
   int32_t n_seg;           // 0: the program is not a set of sum chains
   int32_t pure_objective;  // the first one is kChainObjective
+  int32_t points;          // points of the root box can be filtered in FP32
+  int32_t pad;
 };
+
+// Largest bound of a variable the FP32 filters take (cut32): 2^40.
+constexpr double kFilterMax = 1099511627776.0;
 
 inline constexpr uint8_t make_head(uint8_t code, uint8_t sub)
 {

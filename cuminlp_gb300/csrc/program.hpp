@@ -71,6 +71,7 @@ struct Program {
   // FP32 filter of the <= chains (ChainTab); empty unless inc_ok
   std::vector<ChainSeg> chain_seg;
   std::vector<ChainTerm> chain_term;
+  bool chain_points = false;  // every chain has a filter and the root box is in its range
 };
 
 // Compiles the reachable DAG into the fused straight-line program.

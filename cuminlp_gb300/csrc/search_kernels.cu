@@ -1591,6 +1591,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
   sa.g_max = cfg.g_max;
   sa.capacity = cfg.sample_capacity;
   sa.lg_min = cfg.sample_lg_min;
+  sa.chain = b.chain;
   if (cfg.precision == CMN_PRECISION_FP32_LAZY) {
     // FP32 screen of every sample, then each chunk's best in FP64
     SampleArgs qa = sa;

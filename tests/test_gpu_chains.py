@@ -13,7 +13,7 @@ import oracle as O
 from cuminlp_gb300 import _abi as A
 from cuminlp_gb300 import generators as G
 from cuminlp_gb300.problem import Expr, Problem
-from cuminlp_gb300.solver import Bounder, DeviceProblem, eval_boxes
+from cuminlp_gb300.solver import Bounder, DeviceProblem, Sampler, eval_boxes
 from tests.conftest import bits_equal
 from tests.gpu_common import random_boxes
 from tests.test_gpu_solver import compare
@@ -110,3 +110,41 @@ def test_role_regions(bits):
 def test_solver_iterations(precision, bits, parents):
     for p in (mixed_problem(), G.qcqp(G.QCQPSpec(n=9, m=3, n_int=2, int_lb=0, int_ub=6, rhs=(1.0, 3.0)), 77)):
         compare(p, 9, bisection_budget=bits, batch_parents=parents, frontier_cap=500, precision=precision)
+
+
+def flat_problem() -> Problem:
+    """An objective with few values: most points tie, so the FP32 bounds leave
+    many of a tile's points to FP64."""
+    p = Problem()
+    x = [p.int_var(0.0, 3.0), p.var(-2.0, 2.0), p.var(-1.0, 1.0)]
+    p.set_objective(x[0] + 2.0 * (x[0] * x[0]))
+    p.add_constraint(x[1] * x[1] + x[2] * x[2] + 0.5 * (x[1] * x[2]), A.CMP_LE, 3.0)
+    return p
+
+
+def equality_problem() -> Problem:
+    """An == chain that integer points meet exactly, beside a <= chain."""
+    p = Problem()
+    x = [p.int_var(-3.0, 4.0) for _ in range(4)] + [p.var(-2.0, 2.0)]
+    p.set_objective(x[0] * x[1] - 2.0 * (x[2] * x[4]) + x[3] * x[3])
+    p.add_constraint(2.0 * (x[0] * x[2]) + 1.0 * x[1], A.CMP_EQ, 3.0)
+    p.add_constraint(x[4] * x[4] + 0.5 * (x[0] * x[4]), A.CMP_LE, 2.0)
+    return p
+
+
+@pytest.mark.parametrize("bits,points", [(1, 1), (4, 3), (6, 1), (9, 2), (12, 1)])
+def test_sampled_candidates(bits, points):
+    for p in (G.miqcqp_n32(3), G.qcqp_n4(2), mixed_problem(), flat_problem(), equality_problem(),
+              G.qcqp(G.QCQPSpec(n=7, m=0), 5)):
+        kinds, vids, widths, _ = O.bisection_choose(p.root_box(), p.var_kinds, bits)
+        n = int(np.prod(widths))
+        c = Sampler(DeviceProblem(p), kinds, n, sample_points=points).sample(p.root_box(), vids, widths, 11)
+        found, value, point, index = O.OracleProblem(p).sample(p.root_box(), kinds, vids, widths, n, points, 11)
+        assert c.found == found and (not found or (c.value == value and bits_equal(c.point, point) and c.index == index))
+
+
+@pytest.mark.parametrize("bits,points", [(2, 1), (3, 2), (5, 1)])
+def test_solver_samples(bits, points):
+    # fathomed integer boxes (exact points, admissibility) among sampled ones
+    for p in (flat_problem(), equality_problem()):
+        compare(p, 8, bisection_budget=bits, batch_parents=40, frontier_cap=600, sample_points=points)
