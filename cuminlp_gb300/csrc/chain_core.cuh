@@ -178,6 +178,20 @@ __device__ __forceinline__ double term_lo(const Instr& cur, const V& vars)
   return neg ? emul_ru(cur.c, p) : emul_rd(cur.c, p);
 }
 
+// The upper bound's operand of a plain chain: the mirror of term_lo.
+template <typename V>
+__device__ __forceinline__ double term_hi(const Instr& cur, const V& vars)
+{
+  using A = Arith<double>;
+  const int sub = cur.head >> 3;
+  const bool has_c = (sub & kTermHasC) != 0;
+  const bool neg = (sub & kTermSub) != 0 && !(sub & kTermInit);
+  const bool cn = has_c && A::sgn(cur.c);
+  const double p = product_end(cur, sub, cn == neg, vars);
+  if (!has_c) return p;
+  return neg ? emul_rd(cur.c, p) : emul_ru(cur.c, p);
+}
+
 template <bool kFused>
 __device__ __forceinline__ double term_apply_lo(double acc, const Instr& cur, double p)
 {

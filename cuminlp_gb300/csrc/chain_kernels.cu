@@ -300,6 +300,299 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const E
   }
 }
 
+// ---- the objective of children, a warp per 32 consecutive ones ----
+// Siblings share most of their box: a term whose variables no sibling of the
+// warp narrows has one value for all of them, and one that reads a slot of
+// two parts has two.  Per chunk of 32 terms the warp's lanes form the
+// distinct (family, term, parts) values -- a family is the warp's children
+// of one parent --, leave them in shared memory, and every lane then adds
+// its own in program order.  FP64 work per term and child falls from about
+// 3.5 operations to the one add and a few hundredths; the chain of adds is
+// the reference's, so the bounds are too.
+constexpr int kFamSlots = 5;   // varying slots a family tabulates (32 children vary five bits)
+constexpr int kFamWidth = 4;   // widest slot it tabulates; wider ones are computed per child
+constexpr int kFamNone = 7;    // descriptor: the variable does not vary
+
+struct Family {
+  uint64_t k;
+  uint64_t mask;              // ChildVars::mask of its lead lane
+  uint64_t wide;              // variables (v & 63) computed per child
+  int32_t count;
+  int32_t lead;               // its first lane
+  int32_t nv;                 // tabulated slots
+  int32_t vid[kFamSlots];
+  int32_t slot[kFamSlots];
+  uint32_t widths;            // 4 bits each
+  uint8_t rep[kFamSlots][kFamWidth];  // a lane on each part
+};
+
+// A family's box with the variables of one term over given parts.
+struct FamVars {
+  V64 base;
+  int va, vb;  // -1: from base
+  Iv<double> a, b;
+  __device__ __forceinline__ Iv<double> var(int v) const
+  {
+    if (v == va) return a;
+    if (v == vb) return b;
+    return base.var(v);
+  }
+};
+
+// Most values a chunk needs: 32 terms of up to four each per family, two
+// where the families are pairs of children.
+static __host__ __device__ size_t family_values(int families) { return 128 * (size_t)(families < 8 ? families : 8); }
+// Bytes of a warp's tables: the values and their items, the descriptors, the
+// families, and the children's split variables.
+static __host__ __device__ size_t family_bytes(int families, int ms, bool hi)
+{
+  return (family_values(families) * (hi ? 18 : 10) + (size_t)families * (32 * 4 + sizeof(Family)) +
+          (size_t)ms * 32 * 20 + 15) & ~(size_t)15;
+}
+
+template <int kMode, bool kHi>
+__global__ void __launch_bounds__(kObjThreads, 5) chain_siblings_kernel(const EvalArgs a, int flags, int families)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, W = blockDim.x >> 5;
+  const int ms = a.max_slots;
+  const size_t nval = family_values(families);
+  unsigned char* base_p = smem_raw + family_bytes(families, ms, kHi) * wid;
+  double* vlo = reinterpret_cast<double*>(base_p);
+  double* vhi = vlo + (kHi ? nval : 0);
+  double* olo = vlo + (kHi ? 2 : 1) * nval + lane;
+  double* ohi = olo + (size_t)ms * 32;
+  Family* fam = reinterpret_cast<Family*>(ohi - lane + (size_t)ms * 32);
+  int32_t* ovid = reinterpret_cast<int32_t*>(fam + families) + lane;
+  uint32_t* desc = reinterpret_cast<uint32_t*>(ovid - lane + (size_t)ms * 32);
+  uint16_t* item = reinterpret_cast<uint16_t*>(desc + (size_t)families * 32);
+  if (a.done != nullptr && *a.done) return;
+  const uint64_t total = box_count(a, false);
+  const double gub = a.gub ? *a.gub : DBL_MAX;
+  const ChainSeg s = a.chain.seg[0];
+  const int flanes = 32 / families;  // lanes of a family
+  const int f = lane / flanes, lead = f * flanes;
+  const unsigned fmask = (flanes == 32 ? 0xffffffffu : ((1u << flanes) - 1u)) << lead;
+  const uint64_t tiles = (total + 31) >> 5;
+  for (uint64_t tile = (uint64_t)blockIdx.x * W + wid; tile < tiles; tile += (uint64_t)gridDim.x * W) {
+    const uint64_t at = (tile << 5) + lane;
+    bool live = at < total;
+    const uint64_t g = live ? at : total - 1;  // lanes past the end shadow the last child
+    uint64_t k, r;
+    child_of(a.log2C, g, k, r);
+    bool feasible = true;
+    const ParentInfo pi = a.pinfo[k];
+    if (flags && live) {
+      const uint8_t fl = a.out_flag[g];
+      if (kMode == 1) live = fl == kChildEligible;
+      else if (kMode == 4) live = fl != 0;
+      feasible = fl != 0;
+    } else if (live && kMode == 1 && (pi.fathom || r >= pi.nreg)) {
+      a.out_flag[g] = kChildNone;
+      live = false;
+    }
+    if (!__any_sync(0xffffffffu, live)) continue;
+    bool dup;
+    const V64 cv = child_vars<double, double>(a, a.plo, a.phi, k, r, olo, ohi, ovid, 32, dup);
+    if (kMode == 1 && !flags && dup) {
+      if (live) a.out_flag[g] = kChildDuplicate;
+      live = false;
+    }
+    // the family's varying slots; every lane of it finds the same ones
+    const SlotPlan* sp = a.slots + k * (uint64_t)a.max_slots;
+    uint32_t parts = 0, widths = 0;
+    int nv = 0;
+    uint64_t wide = 0;
+    if (lane == lead) {
+      fam[f].k = k;
+      fam[f].mask = cv.mask;
+      fam[f].count = cv.count;
+      fam[f].lead = lead;
+      // parts no child of the warp is on stand for the lead's
+      for (int e = 0; e < kFamSlots; ++e)
+        for (int q = 0; q < kFamWidth; ++q) fam[f].rep[e][q] = (uint8_t)lead;
+    }
+    __syncwarp();
+    const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)cv.count);
+    for (int j = 0; j < most; ++j) {
+      const bool has = j < cv.count;
+      uint64_t part = 0, width = 1;
+      int vid = -1;
+      bool first = has;
+      if (has) {
+        part = slot_part(r, sp[j]);
+        width = sp[j].width;
+        vid = (int)sp[j].vid;
+        for (int q = 0; q < j; ++q) first = first && ovid[q * 32] != vid;  // ChildVars reads the first slot
+      }
+      const uint64_t p0 = __shfl_sync(0xffffffffu, part, lead);
+      const bool varies = (__ballot_sync(0xffffffffu, first && part != p0) & fmask) != 0u;
+      if (varies) {
+        if (width <= kFamWidth && nv < kFamSlots) {
+          if (lane == lead) {
+            fam[f].vid[nv] = vid;
+            fam[f].slot[nv] = j;
+          }
+          fam[f].rep[nv][part] = (uint8_t)lane;  // any lane on that part will do
+          parts |= (uint32_t)part << (4 * nv);
+          widths |= (uint32_t)width << (4 * nv);
+          ++nv;
+        } else {
+          wide |= 1ULL << (vid & 63);
+        }
+      }
+    }
+    if (lane == lead) {
+      fam[f].nv = nv;
+      fam[f].widths = widths;
+      fam[f].wide = wide;
+    }
+    __syncwarp();
+    double lo = 0.0, hi = 0.0;
+    for (int base = s.pc0; base < s.pc1; base += 32) {
+      const int cnt = s.pc1 - base < 32 ? s.pc1 - base : 32;
+      // (1) lane = term: how many values each family needs, and where
+      int filled = 0;
+      bool any_wide = false;
+      Instr cur = {};
+      if (lane < cnt) cur = load_instr(a.prog, base + lane);
+      const int code = cur.head & 7, pk = (cur.head >> 3) & kTermPMask;
+      const bool reads_a = code == kOpTerm || (cur.modes & 3) == kModeVar;
+      const bool reads_b = code == kOpTerm && pk == kTermProd && cur.b != cur.a;
+      for (int q = 0; q < families; ++q) {
+        const Family& F = fam[q];
+        int ca = kFamNone, cb = kFamNone, wa = 1, wb = 1;
+        bool per_child = false;
+        if (lane < cnt) {
+          for (int e = 0; e < F.nv; ++e) {
+            const int w = (int)(F.widths >> (4 * e)) & 15;
+            if (reads_a && F.vid[e] == cur.a) ca = e, wa = w;
+            if (reads_b && F.vid[e] == cur.b) cb = e, wb = w;
+          }
+          per_child = (reads_a && ((F.wide >> (cur.a & 63)) & 1)) || (reads_b && ((F.wide >> (cur.b & 63)) & 1));
+        }
+        // a product of two four-part slots would outgrow the table
+        per_child = per_child || wa * wb > kFamWidth;
+        const int need = lane < cnt && !per_child ? wa * wb : 0;
+        int x = need;
+        for (int off = 1; off < 32; off <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, x, off);
+          if (lane >= off) x += y;
+        }
+        const int pos = filled + x - need;
+        if (lane < cnt)
+          desc[q * 32 + lane] = (uint32_t)pos | (uint32_t)ca << 16 | (uint32_t)cb << 20 | (uint32_t)wa << 24 | (per_child ? 1u << 31 : 0u);
+        for (int e = 0; e < need; ++e) item[pos + e] = (uint16_t)(q << 7 | lane << 2 | e);
+        filled += __shfl_sync(0xffffffffu, x, 31);
+        any_wide = any_wide || __any_sync(0xffffffffu, per_child);
+      }
+      __syncwarp();
+      // (2) lane = value
+      for (int it = lane; it < filled; it += 32) {
+        const uint32_t code_it = item[it];
+        const int q = (int)(code_it >> 7), j = (int)(code_it >> 2) & 31, combo = (int)code_it & 3;
+        const Family& F = fam[q];
+        const uint32_t d = desc[q * 32 + j];
+        const int ca = (int)(d >> 16) & 15, cb = (int)(d >> 20) & 15, wa = (int)(d >> 24) & 15;
+        const Instr ins = load_instr(a.prog, base + j);
+        FamVars fv;
+        fv.base.plo = a.plo + F.k;
+        fv.base.phi = a.phi + F.k;
+        fv.base.pstride = a.pstride;
+        fv.base.mask = F.mask;
+        fv.base.olo = olo - lane + F.lead;
+        fv.base.ohi = ohi - lane + F.lead;
+        fv.base.ovid = ovid - lane + F.lead;
+        fv.base.count = F.count;
+        fv.base.stride = 32;
+        fv.va = fv.vb = -1;
+        if (ca != kFamNone) {
+          const int rl = F.rep[ca][combo % wa] - lane, o = F.slot[ca] * 32 + rl;
+          fv.va = ins.a;
+          fv.a = Iv<double>{olo[o], ohi[o]};
+        }
+        if (cb != kFamNone) {
+          const int rl = F.rep[cb][combo / wa] - lane, o = F.slot[cb] * 32 + rl;
+          fv.vb = ins.b;
+          fv.b = Iv<double>{olo[o], ohi[o]};
+        }
+        const int sub = ins.head >> 3;
+        const bool neg = (sub & kTermSub) != 0 && !(sub & kTermInit);
+        if ((ins.head & 7) == kOpLoadAcc) {
+          const Iv<double> x = (ins.modes & 3) == kModeVar ? fv.var(ins.a) : Iv<double>{ins.c, ins.c};
+          vlo[it] = x.lo;
+          if (kHi) vhi[it] = x.hi;
+        } else {
+          const double l = term_lo<false>(ins, fv);
+          vlo[it] = neg ? -l : l;
+          if (kHi) {
+            const double h = term_hi(ins, fv);
+            vhi[it] = neg ? -h : h;
+          }
+        }
+      }
+      __syncwarp();
+      // (3) lane = child: its terms in order
+      const uint32_t* dl = desc + f * 32;
+      auto value_at = [&](uint32_t d) {
+        const uint32_t pa = (parts >> (4 * ((d >> 16) & 7))) & 15u, pb = (parts >> (4 * ((d >> 20) & 7))) & 15u;
+        return (d & 0xffffu) + pa + pb * ((d >> 24) & 15u);
+      };
+      auto add = [&](int j, double l, double h) {
+        const bool start = base + j == s.pc0;
+        lo = start ? l : __dadd_rd(lo, l);
+        if (kHi) hi = start ? h : __dadd_ru(hi, h);
+      };
+      if (!any_wide) {
+#pragma unroll 8
+        for (int j = 0; j < cnt; ++j) {
+          const uint32_t at_v = value_at(dl[j]);
+          add(j, vlo[at_v], kHi ? vhi[at_v] : 0.0);
+        }
+      } else {
+        for (int j = 0; j < cnt; ++j) {
+          const uint32_t d = dl[j];
+          double l, h = 0.0;
+          if (d >> 31) {
+            const Instr ins = load_instr(a.prog, base + j);
+            const int sub = ins.head >> 3;
+            const bool neg = (sub & kTermSub) != 0 && !(sub & kTermInit);
+            if ((ins.head & 7) == kOpLoadAcc) {
+              const Iv<double> x = cv.var(ins.a);
+              l = x.lo;
+              h = x.hi;
+            } else {
+              l = term_lo<false>(ins, cv);
+              l = neg ? -l : l;
+              if (kHi) {
+                h = term_hi(ins, cv);
+                h = neg ? -h : h;
+              }
+            }
+          } else {
+            const uint32_t at_v = value_at(d);
+            l = vlo[at_v];
+            if (kHi) h = vhi[at_v];
+          }
+          add(j, l, h);
+        }
+      }
+      __syncwarp();  // the tables are refilled next
+    }
+    Verdict<double> v = verdict_init<double>();
+    v.obj.lo = lo;
+    v.obj.hi = hi;
+    if (live && (lo != lo || (kHi && hi != hi))) chain_general<false>(a.prog, s.pc0, s.pc2, cv, v);
+    v.feasible = feasible;
+    if constexpr (kMode == 4) {
+      aggregate_fold(a, live, r, v);
+    } else {
+      if (live) write_verdict<double, kMode>(a, g, k, v, gub);
+    }
+    __syncwarp();  // the columns are rewritten next
+  }
+}
+
 // Point sampling and exact points (sample_children_kernel's results): every
 // point is drawn in FP64 and its constraints are summed in FP32; only a point
 // they do not exclude, and whose FP32 objective does not prove it worse than
@@ -535,6 +828,17 @@ static cudaError_t launch_chain_t(const EvalArgs& a, cudaStream_t s)
     const uint64_t grid = resident((a.max_boxes + (1ull << lb) - 1) >> lb, (const void*)kernel, threads, smem);
     kernel<<<(unsigned)grid, threads, smem, s>>>(a, lb);
   }
+  if constexpr (!kFused && kMode != 3) {
+    // children (of a role's box or of the solver's parents): siblings share
+    const int lc = a.log2C < 0 || a.log2C > 5 ? 5 : a.log2C;
+    const size_t fsmem = (kObjThreads / 32) * family_bytes(32 >> lc, ms, kHi);
+    if (a.pinfo != nullptr && lc > 0 && a.chain.pure_objective && fsmem + 1024 <= (size_t)max_dynamic_smem()) {
+      auto siblings = chain_siblings_kernel<kMode, kHi>;
+      const uint64_t grid = resident(((a.max_boxes + 31) / 32 + 3) / 4, (const void*)siblings, kObjThreads, fsmem);
+      siblings<<<(unsigned)grid, kObjThreads, fsmem, s>>>(a, chains > 0 ? 1 : 0, 32 >> lc);
+      return cudaGetLastError();
+    }
+  }
   auto kernel = chain_objective_kernel<kMode, kFused, kHi>;
   const size_t smem = objective_smem(a);
   const uint64_t grid = resident((a.max_boxes * 32 + kObjThreads - 1) / kObjThreads, (const void*)kernel, kObjThreads, smem);
@@ -595,6 +899,8 @@ template <int kMode, bool kFused, bool kHi>
 static cudaError_t allow_both(int max_smem)
 {
   cudaError_t e = allow(chain_constraints_kernel<kMode, kFused>, max_smem);
+  if constexpr (!kFused && kMode != 3)
+    if (e == cudaSuccess) e = allow(chain_siblings_kernel<kMode, kHi>, max_smem);
   return e == cudaSuccess ? allow(chain_objective_kernel<kMode, kFused, kHi>, max_smem) : e;
 }
 
