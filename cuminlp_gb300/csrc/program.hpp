@@ -71,6 +71,9 @@ struct Program {
   // FP32 filter of the <= chains (ChainTab); empty unless inc_ok
   std::vector<ChainSeg> chain_seg;
   std::vector<ChainTerm> chain_term;
+  std::vector<ChainTerm32> chain_term32;  // empty: the FP32 passes take the interpreter
+  std::vector<ChainTerm32> chain_var32;
+  std::vector<int32_t> chain_var_off;
   bool chain_points = false;  // every chain has a filter and the root box is in its range
 };
 

@@ -114,6 +114,7 @@ struct SolverCfg {
   int sample_lg_min;         // sampler point columns: one per 2^sample_lg_min lanes
   int inc;                   // lazy form: children by the incremental chain sums
   int inc_segments;
+  int inc_tile;              // in one pass over tiles of parents (lazy_children_kernel)
 };
 
 struct SolverBufs {

@@ -1507,7 +1507,10 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     ea.plo32 = b.plo32;
     ea.phi32 = b.phi32;
     ea.parent_lb = nullptr;  // folded in by lazy_fold_kernel
-    if (cfg.inc) {
+    if (cfg.inc_tile) {
+      ea.n_parents_dev = &b.dev->n_parents;
+      e = launch_lazy_children(ea, cfg.e_max, s);
+    } else if (cfg.inc) {
       ea.inc_segments = cfg.inc_segments;
       ea.n_parents_dev = &b.dev->n_parents;
       ea.inc_seg = b.inc_seg;
