@@ -97,6 +97,7 @@ static cudaError_t ensure_attributes()
   e = set_eval_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_chain_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_chain32_kernel_attributes(max_dynamic_smem());
+  if (e == cudaSuccess) e = set_chain_points_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_batch_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess && dev < 31) g_attr_device_mask |= (1 << dev);
   return e;
@@ -124,6 +125,7 @@ cmn_problem::~cmn_problem()
   dfree(d_chain_term32);
   dfree(d_chain_var32);
   dfree(d_chain_var_off);
+  dfree(d_chain_term_pt);
   if (cur != device) cudaSetDevice(cur);
 }
 
@@ -193,6 +195,7 @@ extern "C" cmn_status cmn_problem_create(const cmn_problem_desc* desc, cmn_probl
         up(&p->d_chain_var32, p->prog.chain_var32);
         up(&p->d_chain_var_off, p->prog.chain_var_off);
       }
+      if (!p->prog.chain_term_pt.empty()) up(&p->d_chain_term_pt, p->prog.chain_term_pt);
     }
     if (e != cudaSuccess) {
       delete p;

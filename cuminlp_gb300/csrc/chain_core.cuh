@@ -273,57 +273,4 @@ __device__ __forceinline__ double chain_lo_group(const Instr* __restrict__ prog,
   return acc;
 }
 
-// ---- points ----
-// This lane's share of one chain at the point x (one cut coordinate per
-// variable, `stride` apart) and of its terms' magnitudes.
-__device__ __forceinline__ void filter_point(const ChainSeg& s, const ChainTerm* __restrict__ term,
-                                             const float* __restrict__ x, uint32_t stride, int sub, int L, float& sum,
-                                             float& mag)
-{
-  float acc[2] = {sub == 0 ? s.c0 : 0.0f, 0.0f}, m[2] = {sub == 0 ? fabsf(s.c0) : 0.0f, 0.0f};
-  auto add = [&](int u, float t) {
-    acc[u] += t;
-    m[u] += fabsf(t);
-  };
-  filter_group(term, s.group[0], s.group[2], sub, L, [&](int u, uint32_t a, uint32_t b, float c) {
-    add(u, c * (x[a * stride] * x[b * stride]));
-  });
-  filter_group(term, s.group[2], s.group[4], sub, L, [&](int u, uint32_t a, uint32_t, float c) {
-    const float p = x[a * stride];
-    add(u, c * (p * p));
-  });
-  filter_group(term, s.group[4], s.group[6], sub, L, [&](int u, uint32_t a, uint32_t, float c) { add(u, c * x[a * stride]); });
-  sum = acc[0] + acc[1];
-  mag = m[0] + m[1];
-}
-
-// One term of the FP64 point program: [c *] (x_a [* x_b]), each operation
-// rounded to nearest, negated when it is subtracted.
-__device__ __forceinline__ double point_term(const Instr& cur, const double* __restrict__ x)
-{
-  const int sub = cur.head >> 3, pk = sub & kTermPMask;
-  double p = x[cur.a];
-  if (pk == kTermProd) p = __dmul_rn(p, x[cur.b]);
-  else if (pk == kTermSqr) p = __dmul_rn(p, p);
-  if (sub & kTermHasC) p = __dmul_rn(cur.c, p);
-  return (sub & kTermSub) && !(sub & kTermInit) ? -p : p;
-}
-
-// The chain's FP64 value at the point x by a whole warp: 32 terms at once,
-// then every lane adds them in order.
-__device__ __forceinline__ double point_chain_warp(const Instr* __restrict__ prog, int pc0, int pc1,
-                                                   const double* __restrict__ x)
-{
-  const int lane = threadIdx.x & 31;
-  const Instr first = load_instr(prog, pc0);
-  double acc = (first.head & 7) == kOpLoadAcc ? ((first.modes & 3) == kModeVar ? x[first.a] : first.c) : point_term(first, x);
-  for (int base = pc0 + 1; base < pc1; base += 32) {
-    const int pc = base + lane;
-    const double p = pc < pc1 ? point_term(load_instr(prog, pc), x) : 0.0;
-    const int cnt = pc1 - base < 32 ? pc1 - base : 32;
-    for (int j = 0; j < cnt; ++j) acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, p, j));
-  }
-  return acc;
-}
-
 }  // namespace cmn

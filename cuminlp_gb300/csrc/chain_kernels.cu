@@ -77,11 +77,6 @@ __device__ __forceinline__ uint64_t box_count(const EvalArgs& a, bool list)
   return list ? *a.list_count : (a.n_children_dev ? *a.n_children_dev : a.n_children);
 }
 
-__device__ __forceinline__ double key_value(uint64_t k)  // lb_key's inverse
-{
-  return __longlong_as_double((long long)((k >> 63) ? (k & 0x7fffffffffffffffULL) : ~k));
-}
-
 __device__ __forceinline__ float max_abs_group(float m, int boxes)
 {
   for (int off = 1; off < boxes; off <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
@@ -595,213 +590,6 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_siblings_kernel(const Ev
   }
 }
 
-// Point sampling and exact points (sample_children_kernel's results): every
-// point is drawn in FP64 and its constraints are summed in FP32; only a point
-// they do not exclude, and whose FP32 objective does not prove it worse than
-// the best point of this block (or, in the solver, than the incumbent), is
-// evaluated in FP64.  The best candidate is the same: what is left out is
-// infeasible or strictly worse than a candidate that was evaluated.
-//
-// A warp takes 2^log_pts points at a time, 32 >> log_pts lanes on each, then
-// evaluates the points left one by one with all its lanes, the FP32-best
-// first, so that one FP64 evaluation usually rules out the others.  Taken
-// where every chain has a filter and the boxes are within its range
-// (ChainTab::points): elsewhere too many points would be left.
-__global__ void __launch_bounds__(kObjThreads) chain_sample_kernel(const SampleArgs a, int log_pts)
-{
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned long long best_s;  // lb_key of the block's best value so far
-  const int pts = 1 << log_pts, L = 32 >> log_pts;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, W = blockDim.x >> 5;
-  const int pt = lane & (pts - 1), sub = lane >> log_pts;
-  const int n = a.n_vars;
-  double* x64 = reinterpret_cast<double*>(smem_raw) + (size_t)wid * n;
-  float* x32 = reinterpret_cast<float*>(reinterpret_cast<double*>(smem_raw) + (size_t)W * n) + (size_t)wid * n * pts;
-  if (a.done != nullptr && *a.done) {
-    if (threadIdx.x == 0) a.block_best[blockIdx.x] = Cand{INFINITY, 0xffffffffu, 0, ~0ULL};
-    return;
-  }
-  const uint64_t children = a.n_children_dev ? *a.n_children_dev : a.n_children;
-  const uint64_t per = a.exact ? 1 : a.S;
-  const uint64_t total = children * per;
-  const uint64_t salt_base = a.salt_base_dev ? *a.salt_base_dev : 0;
-  const double gub = a.gub ? *a.gub : DBL_MAX;
-  const bool solver = a.state != nullptr;
-  // a solver's candidate must be below the incumbent to count
-  if (threadIdx.x == 0) best_s = lb_key(solver ? gub : INFINITY);
-  __syncthreads();
-  Cand best = {INFINITY, 0xffffffffu, 0, ~0ULL};
-  unsigned long long rejected = 0;
-  const ChainSeg* seg = a.chain.seg;
-  const uint64_t warps = (uint64_t)gridDim.x * W;
-  for (uint64_t w0 = (uint64_t)blockIdx.x * W + wid; w0 << log_pts < total; w0 += warps) {
-    const uint64_t item = (w0 << log_pts) + pt;
-    bool live = item < total;
-    const uint64_t g = live ? item / per : 0, i = live ? item - g * per : 0;
-    uint64_t k = 0, r = 0;
-    child_of(a.log2C, g, k, r);
-    bool fathom = a.exact != 0;
-    uint32_t count = 0;
-    const SlotPlan* sp = nullptr;
-    if (a.pinfo != nullptr) {
-      const ParentInfo pi = a.pinfo[k];
-      fathom = fathom || pi.fathom;
-      count = pi.count;
-      sp = a.slots + k * (uint64_t)a.max_slots;
-      live = live && r < pi.nreg;
-    }
-    if (live && solver && !fathom) {
-      const uint8_t st = a.state[g];
-      live = a.sample_all ? (st != kChildNone) : (st == kChildEligible);
-    }
-    live = live && (!fathom || i == 0);
-    if (!__any_sync(0xffffffffu, live)) continue;
-    const uint64_t salt = a.salt_base_dev ? salt_base + k + 1 : a.salt;
-    auto coordinate = [&](int v, uint64_t kk, uint64_t rr, uint64_t ii, uint64_t ss, uint32_t cc, const SlotPlan* q,
-                          bool fa) {
-      double lo = a.plo[(uint64_t)v * a.pstride + kk], hi = a.phi[(uint64_t)v * a.pstride + kk];
-      for (uint32_t j = 0; j < cc; ++j)
-        if (q[j].vid == (uint32_t)v) {
-          slot_bounds(q[j], lo, hi, slot_part(rr, q[j]), lo, hi);
-          break;
-        }
-      return fa ? lo : sample_value(a.var_kinds[v] != 0, lo, hi, (uint64_t)v, ii, rr, ss);
-    };
-    // (1) the points, cut to FP32
-    bool bad = false;
-    for (int v = sub; v < n; v += L)
-      if (live) x32[v * pts + pt] = cut32(coordinate(v, k, r, i, salt, count, sp, fathom), bad);
-    for (int off = pts; off < 32; off <<= 1) bad = (__shfl_xor_sync(0xffffffffu, (int)bad, off) != 0) || bad;
-    __syncwarp();
-    // (2) the constraints, until no point is left
-    bool cand = live, proven = !bad;
-    for (int q = 0; q < a.chain.n_seg; ++q) {
-      const ChainSeg& s = seg[q];
-      if (s.kind == kChainObjective) continue;
-      if (!__any_sync(0xffffffffu, cand && !bad)) break;
-      float sum, mag;
-      filter_point(s, a.chain.term, x32 + pt, (uint32_t)pts, sub, L, sum, mag);
-      for (int off = pts; off < 32; off <<= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        mag += __shfl_xor_sync(0xffffffffu, mag, off);
-      }
-      const float err = s.eps * mag;
-      const float lo = __fsub_rd(sum, err), hi = __fadd_ru(sum, err);
-      if (bad) continue;
-      if (s.kind == kChainLe) {
-        cand = cand && !(lo > s.rhs_up);
-        proven = proven && hi <= s.rhs_dn;
-      } else {  // almost_equal's tolerance, at its largest over [lo, hi]
-        const float most = fmaxf(fmaxf(fabsf(lo), fabsf(hi)), fmaxf(fabsf(s.rhs_dn), fabsf(s.rhs_up)));
-        const float tol = fmaxf(1.001e-8f, 1.001e-6f * most);
-        cand = cand && !(__fsub_rd(lo, s.rhs_up) > tol || __fsub_rd(s.rhs_dn, hi) > tol);
-        proven = false;
-      }
-    }
-    // (3) the objective's lower end in FP32
-    float low = -INFINITY;
-    if (__any_sync(0xffffffffu, cand && !bad)) {
-      float sum, mag;
-      filter_point(seg[0], a.chain.term, x32 + pt, (uint32_t)pts, sub, L, sum, mag);
-      for (int off = pts; off < 32; off <<= 1) {
-        sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        mag += __shfl_xor_sync(0xffffffffu, mag, off);
-      }
-      low = __fsub_rd(sum, seg[0].eps * mag);
-      if (bad || !(low == low)) low = -INFINITY;
-    }
-    cand = cand && sub == 0;
-    const bool always = fathom && solver;  // inadmissible exact points are counted
-    // (4) the points left, in FP64: with the whole warp one by one, the
-    // smallest FP32 bound first; when the first of them leaves many (their
-    // bounds too close to tell apart), half as many at once as the tile has,
-    // in columns over the FP32 points, which are done with
-    const int cols = pts >> 1, lgc = 6 - log_pts;  // columns, log2 of the lanes on each
-    bool first = true;
-    for (;;) {
-      const double lim = key_value(*(volatile unsigned long long*)&best_s);
-      if (!always && (double)low > lim) cand = false;
-      const unsigned m = __ballot_sync(0xffffffffu, cand);
-      if (m == 0u) break;
-      const bool many = !first && cols > 1 && __popc(m) >= 6;
-      first = false;
-      int src, step, part;  // this lane's point, and its share of the work on it
-      if (many) {
-        part = lane & ((1 << lgc) - 1);
-        step = 1 << lgc;
-        unsigned rest = m;
-        for (int q = lane >> lgc; q > 0; --q) rest &= rest - 1u;
-        src = __ffs((int)rest) - 1;  // -1: no point for this column
-      } else {
-        part = lane;
-        step = 32;
-        float lo_min = cand ? low : INFINITY;
-        for (int off = 16; off > 0; off >>= 1) lo_min = fminf(lo_min, __shfl_xor_sync(0xffffffffu, lo_min, off));
-        const unsigned at = __ballot_sync(0xffffffffu, cand && low == lo_min);
-        src = __ffs((int)(at != 0u ? at : m)) - 1;
-      }
-      const int from = src < 0 ? lane : src;
-      const uint64_t k1 = __shfl_sync(0xffffffffu, k, from), r1 = __shfl_sync(0xffffffffu, r, from);
-      const uint64_t i1 = __shfl_sync(0xffffffffu, i, from), salt1 = __shfl_sync(0xffffffffu, salt, from);
-      const uint32_t c1 = __shfl_sync(0xffffffffu, count, from);
-      const bool f1 = __shfl_sync(0xffffffffu, (int)fathom, from) != 0;
-      const bool p1 = __shfl_sync(0xffffffffu, (int)proven, from) != 0;
-      const SlotPlan* sp1 = a.pinfo != nullptr ? a.slots + k1 * (uint64_t)a.max_slots : nullptr;
-      Tile<double> t = {};
-      t.lo = many ? reinterpret_cast<double*>(x32) + (lane >> lgc) : x64;
-      t.stride = many ? cols : 1;
-      __syncwarp();  // the columns' readers of the previous points are done
-      if (src >= 0)
-        for (int v = part; v < n; v += step) t.lo[v * t.stride] = coordinate(v, k1, r1, i1, salt1, c1, sp1, f1);
-      __syncwarp();
-      double value = INFINITY;
-      if (!many && p1) {
-        value = point_chain_warp(a.prog, seg[0].pc0, seg[0].pc1, x64);
-      } else {
-        PointVerdict pv = {INFINITY, true, false};
-        if (src >= 0) pv = run_point_lane(a.prog, a.sched, many ? lgc : 5, part, t);
-        pv = group_point_verdict(pv, step);
-        if (pv.feasible && pv.obj == pv.obj) value = pv.obj;
-      }
-      if (value != value) value = INFINITY;
-      if (src >= 0 && part == 0 && value < INFINITY) {
-        bool ok = true;
-        if (f1 && solver) {
-          for (int v = 0; v < n && ok; ++v) {
-            const double x = t.lo[v * t.stride];
-            if (!(x >= a.root_lb[v]) || !(x <= a.root_ub[v])) ok = false;
-            else if (a.var_kinds[v] != 0 && fabs(__dsub_rn(x, rint(x))) > 1e-6) ok = false;
-          }
-          if (!ok && value < gub) ++rejected;
-        }
-        if (ok) {
-          const Cand c = {value, (uint32_t)k1, 0, r1 * (f1 ? 1 : a.S) + i1};
-          if (cand_less(c, best)) best = c;
-          atomicMin(&best_s, (unsigned long long)lb_key(value));
-        }
-      }
-      // the points evaluated leave the list
-      unsigned done = 0;
-      if (many) {
-        unsigned rest = m;
-        for (int q = 0; q < cols && rest != 0u; ++q) rest &= rest - 1u;
-        done = m & ~rest;
-      } else {
-        done = 1u << src;
-      }
-      if ((done >> lane) & 1u) cand = false;
-      __syncwarp();
-    }
-    __syncwarp();  // the points are restaged next
-  }
-  best = block_min_cand(best);
-  if (threadIdx.x == 0) a.block_best[blockIdx.x] = best;
-  if (a.rejected != nullptr) {
-    for (int off = 16; off > 0; off >>= 1) rejected += __shfl_down_sync(0xffffffffu, rejected, off);
-    if (lane == 0 && rejected) atomicAdd(a.rejected, rejected);
-  }
-}
-
 static uint64_t resident(uint64_t blocks, const void* kernel, int threads, size_t smem)
 {
   int occ = 1;
@@ -864,30 +652,6 @@ cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s)
   return launch_chain_t<3, false, false>(a, s);
 }
 
-// Bytes of a warp's FP32 points; they shrink to fewer points of more lanes
-// until a block of four warps keeps within 32 KiB.
-constexpr size_t kPointBytes = 8 * 1024;
-
-static size_t sample_smem(int n, int log_pts) { return (size_t)(kObjThreads / 32) * n * (8 + ((size_t)4 << log_pts)); }
-
-bool chain_sample_fits(const SampleArgs& a)
-{
-  return a.chain.points && a.sched != nullptr && a.cbest == nullptr &&
-         sample_smem(a.n_vars, 0) + 2048 <= (size_t)max_dynamic_smem();
-}
-
-cudaError_t launch_chain_sample(const SampleArgs& a, int grid, cudaStream_t s)
-{
-  int lp = 5;
-  while (lp > 0 && ((size_t)a.n_vars * 4) << lp > kPointBytes) --lp;
-  if (a.n_children_dev == nullptr) {  // few points: more lanes on each
-    const uint64_t warps = (uint64_t)grid * (kObjThreads / 32), points = a.n_children * a.S;
-    while (lp > 0 && (points >> lp) < warps) --lp;
-  }
-  chain_sample_kernel<<<grid, kObjThreads, sample_smem(a.n_vars, lp), s>>>(a, lp);
-  return cudaGetLastError();
-}
-
 template <typename K>
 static cudaError_t allow(K kernel, int max_smem)
 {
@@ -914,7 +678,6 @@ cudaError_t set_chain_kernel_attributes(int max_smem)
   if (e == cudaSuccess) e = allow_both<1, false, false>(max_smem);
   if (e == cudaSuccess) e = allow_both<4, false, true>(max_smem);
   if (e == cudaSuccess) e = allow_both<3, false, false>(max_smem);
-  if (e == cudaSuccess) e = allow(chain_sample_kernel, max_smem);
   return e;
 }
 

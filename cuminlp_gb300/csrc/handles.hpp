@@ -28,6 +28,7 @@ struct cmn_problem {
   cmn::ChainTerm32* d_chain_term32 = nullptr;
   cmn::ChainTerm32* d_chain_var32 = nullptr;
   int32_t* d_chain_var_off = nullptr;
+  cmn::ChainTerm* d_chain_term_pt = nullptr;
   // cmn_autotune's choice per precision (0 FP64, 1 FP32): blocks per SM
   // and lanes per box cap; 0 = not tuned
   int tuned_bps[2] = {0, 0};
@@ -45,6 +46,7 @@ struct cmn_problem {
     t.term32 = d_chain_term32;
     t.var32 = d_chain_var32;
     t.var_off = d_chain_var_off;
+    t.term_pt = d_chain_term_pt;
     t.n_vars = (int32_t)host.n_vars();
     // no more warps than the terms over the longest chain, at most eight
     int64_t most = 1, all = 0;

@@ -54,6 +54,10 @@ cudaError_t set_chain32_kernel_attributes(int max_smem);
 // the sampler over such a program (not the lazy form's chunk mode)
 bool chain_sample_fits(const SampleArgs& a);
 cudaError_t launch_chain_sample(const SampleArgs& a, int grid, cudaStream_t s);
+// the lazy form's FP32 sample screen over such a program
+bool chain_screen_fits(const SampleArgs& a);
+cudaError_t launch_chain_screen(const SampleArgs& a, uint64_t max_children, cudaStream_t s);
+cudaError_t set_chain_points_attributes(int max_smem);
 cudaError_t launch_sample(const SampleArgs& a, int grid, int threads, cudaStream_t s);
 // the lazy form's incremental FP32 children: the common chain sums per
 // (segment, parent), then every child (EvalArgs::inc_* set, prog = FP32)

@@ -508,11 +508,40 @@ class Compiler {
     });
     out_.chain_seg = segs;
     build_chains32();
+    build_point_chains();
     out_.chain_points = !segs.empty() && segs[0].kind == kChainObjective;
     for (const ChainSeg& s : segs) out_.chain_points = out_.chain_points && s.eps > 0.0f;
     for (size_t v = 0; v < p_.var_lb.size(); ++v)
       out_.chain_points =
           out_.chain_points && std::fabs(p_.var_lb[v]) <= kFilterMax && std::fabs(p_.var_ub[v]) <= kFilterMax;
+  }
+
+  // Program::chain_term_pt: the chains' terms for FP32 points, for programs
+  // of one objective chain and single <= or == checks.
+  void build_point_chains()
+  {
+    const uint32_t one = (uint32_t)p_.var_lb.size();
+    if (one > 0xffffu || out_.chain_seg.empty() || out_.chain_seg[0].kind != kChainObjective) return;
+    for (const ChainSeg& s : out_.chain_seg)
+      if (s.kind == kChainGeneral && !s.eq) return;
+    for (ChainSeg& cs : out_.chain_seg) {
+      cs.pt = (int32_t)out_.chain_term_pt.size();
+      for (int pc = cs.pc0; pc < cs.pc1; ++pc) {
+        const Instr& in = out_.code64[pc];
+        const int sub = in.head >> 3, pk = sub & kTermPMask;
+        ChainTerm t = {one | (one << 16), 1.0f};
+        if ((in.head & 7) == kOpLoadAcc) {
+          if ((in.modes & 3) == kModeVar) t.ab = in.a | (one << 16);
+          else t.c = d2f_rn(in.c);
+        } else {
+          t.ab = in.a | ((pk == kTermProd ? (uint32_t)in.b : pk == kTermSqr ? (uint32_t)in.a : one) << 16);
+          if (sub & kTermHasC) t.c = d2f_rn(in.c);
+          if ((sub & kTermSub) && !(sub & kTermInit)) t.c = -t.c;
+        }
+        out_.chain_term_pt.push_back(t);
+      }
+      cs.pt_end = (int32_t)out_.chain_term_pt.size();
+    }
   }
 
   // Program::chain_term32 and chain_var32: the chains' terms with outward FP32

@@ -147,6 +147,7 @@ struct ChainSeg {
   int32_t eq;            // kChainGeneral read by one == check alone
   double rhs;
   int32_t t32, t32_end;  // the chain's terms in ChainTab::term32
+  int32_t pt, pt_end;    // and in ChainTab::term_pt
 };
 
 // The chains of one program on the device: the one the objective reads
@@ -164,6 +165,10 @@ struct ChainTab {
   const ChainTerm32* term32;
   const ChainTerm32* var32;
   const int32_t* var_off;
+  // FP32 points: the terms in program order as c * x_a * x_b, rounded to
+  // nearest, subtracted ones with -c, linear ones with the plane past the
+  // last variable as x_b (null: some chain has other readers)
+  const ChainTerm* term_pt;
   int32_t n_vars;
   int32_t warps32;  // warps of a tile that keep its chains' lengths balanced
 };

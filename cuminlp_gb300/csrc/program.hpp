@@ -74,6 +74,7 @@ struct Program {
   std::vector<ChainTerm32> chain_term32;  // empty: the FP32 passes take the interpreter
   std::vector<ChainTerm32> chain_var32;
   std::vector<int32_t> chain_var_off;
+  std::vector<ChainTerm> chain_term_pt;   // empty: points take the interpreter
   bool chain_points = false;  // every chain has a filter and the root box is in its range
 };
 

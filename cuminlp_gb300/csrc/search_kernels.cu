@@ -1601,7 +1601,8 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     qa.lg_min = cfg.screen_lg_min;
     qa.prog = b.prog32p;
     qa.cbest = b.cbest;
-    e = launch_sample_screen(qa, cfg.screen_grid, kEvalThreads, s);
+    e = chain_screen_fits(qa) ? launch_chain_screen(qa, max_children, s)
+                              : launch_sample_screen(qa, cfg.screen_grid, kEvalThreads, s);
     if (e != cudaSuccess) return e;
     sa.cbest = b.cbest;
   }
