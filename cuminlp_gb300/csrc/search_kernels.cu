@@ -1044,6 +1044,96 @@ __global__ void append_children_kernel(const SolverCfg cfg, const SolverBufs b)
     op(b.list[pos], pos);
 }
 
+// The same with G lanes per child, lane = variable: a box of the store is
+// contiguous, so a child's bounds go out in whole lines, where one thread per
+// child wrote 8 bytes of 32 lines at a time.  A group takes kAppendRun
+// children in a row and keeps the parent's bounds in registers while they
+// share it (the list is in parent order).  n = 64, 2^20 kept children (1.05 GB
+// of boxes): 1.18 ms with one thread per child.  From nine variables on; below
+// that a lane group would be mostly idle.
+constexpr int kAppendRun = 16;
+constexpr int kAppendVars = 2;  // variables a lane holds at a time
+
+template <int G>
+__global__ void __launch_bounds__(256) append_boxes_kernel(const SolverCfg cfg, const SolverBufs b)
+{
+  const SolverDev* d = b.dev;
+  if (d->done) return;
+  const uint64_t kept = d->kept, free_top = d->free_top;
+  const int n = cfg.n_vars;
+  const int gl = threadIdx.x & (G - 1);
+  const unsigned gmask = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << ((threadIdx.x & 31) & ~(G - 1));
+  const uint64_t groups = (uint64_t)gridDim.x * (blockDim.x / G);
+  const uint32_t par = d->parity;
+  const uint64_t pool = d->pool_size;
+  if (kept > free_top) {  // more children than free slots: never expected
+    if (threadIdx.x == 0 && blockIdx.x == 0) b.dev->error = 1;
+    return;
+  }
+  for (uint64_t run = (uint64_t)blockIdx.x * (blockDim.x / G) + threadIdx.x / G; run * kAppendRun < kept; run += groups) {
+    const uint64_t p0 = run * kAppendRun;
+    const int cnt = kept - p0 < kAppendRun ? (int)(kept - p0) : kAppendRun;
+    // lane = child: its store slot and the pool's entry
+    uint32_t g_of[kAppendRun / G > 0 ? kAppendRun / G : 1], s_of[kAppendRun / G > 0 ? kAppendRun / G : 1];
+#pragma unroll
+    for (int u = 0; u < (kAppendRun / G > 0 ? kAppendRun / G : 1); ++u) {
+      const int c = u * G + gl;
+      g_of[u] = s_of[u] = 0;
+      if (c < cnt) {
+        const uint64_t pos = p0 + c;
+        const uint32_t g = b.list[pos], s = b.free_slots[free_top - 1 - pos];
+        g_of[u] = g;
+        s_of[u] = s;
+        b.depth[s] = b.pdepth[g >> cfg.log2C] + 1;
+        parity_buf(b.lb, par)[pool + pos] = b.clb[g];
+        parity_buf(b.slot, par)[pool + pos] = s;
+        parity_buf(b.sel, par)[pool + pos] = kSelAlive;
+      }
+    }
+    // lane = variable: the boxes
+    for (int v0 = 0; v0 < n; v0 += G * kAppendVars) {
+      uint32_t cur = 0xffffffffu;
+      double lo[kAppendVars], hi[kAppendVars];
+      const SlotPlan* plan[kAppendVars];  // the slot that narrows the variable, if any
+      for (int c = 0; c < cnt; ++c) {
+        uint32_t g = g_of[0], s = s_of[0];
+#pragma unroll
+        for (int u = 1; u < (kAppendRun / G > 0 ? kAppendRun / G : 1); ++u)
+          if (c / G == u) g = g_of[u], s = s_of[u];
+        g = __shfl_sync(gmask, g, c & (G - 1), G);
+        s = __shfl_sync(gmask, s, c & (G - 1), G);
+        const uint32_t k = g >> cfg.log2C;
+        const uint64_t r = g & ((1u << cfg.log2C) - 1u);
+        if (k != cur) {
+          cur = k;
+          const uint32_t count = b.pinfo[k].count;
+          const SlotPlan* sp = b.slots + (uint64_t)k * cfg.max_slots;
+#pragma unroll
+          for (int u = 0; u < kAppendVars; ++u) {
+            const int v = v0 + u * G + gl;
+            plan[u] = nullptr;
+            if (v < n) {
+              lo[u] = b.plo[(uint64_t)v * cfg.e_max + k];
+              hi[u] = b.phi[(uint64_t)v * cfg.e_max + k];
+              for (uint32_t j = 0; j < count; ++j)
+                if (sp[j].vid == (uint32_t)v) plan[u] = sp + j;  // the last one, as the slots are applied in order
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kAppendVars; ++u) {
+          const int v = v0 + u * G + gl;
+          if (v >= n) continue;
+          double l = lo[u], h = hi[u];
+          if (plan[u] != nullptr) slot_bounds(*plan[u], lo[u], hi[u], slot_part(r, *plan[u]), l, h);
+          b.lo[(uint64_t)s * n + v] = l;
+          b.hi[(uint64_t)s * n + v] = h;
+        }
+      }
+    }
+  }
+}
+
 // pool entries [start, start + count) in position order, unpacked from the
 // store
 __global__ void frontier_gather_kernel(const SolverCfg cfg, const SolverBufs b, uint64_t start, uint64_t count,
@@ -1456,6 +1546,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     const int grid = (int)std::min<uint64_t>((cfg.e_max + 127) / 128, 2048);
     if (cfg.n_vars <= 8) branch_kernel<8><<<grid, 128, 0, s>>>(cfg, b);
     else if (cfg.n_vars <= 32) branch_kernel<32><<<grid, 128, 0, s>>>(cfg, b);
+    else if (cfg.n_vars <= 64) branch_kernel<64><<<grid, 128, 0, s>>>(cfg, b);
     else branch_kernel<0><<<grid, 128, 0, s>>>(cfg, b);
   }
   mark(marks, 1, s);
@@ -1629,7 +1720,9 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
   scatter(kept, ListChild{b}, max_children, s, b);
   {
     const int grid = (int)std::min<uint64_t>((max_children + 255) / 256, 4096);
-    append_children_kernel<<<grid, 256, 0, s>>>(cfg, b);
+    if (cfg.n_vars > 16) append_boxes_kernel<32><<<grid, 256, 0, s>>>(cfg, b);
+    else if (cfg.n_vars > 8) append_boxes_kernel<16><<<grid, 256, 0, s>>>(cfg, b);
+    else append_children_kernel<<<grid, 256, 0, s>>>(cfg, b);
   }
   size_kernel<<<1, 1, 0, s>>>(cfg, b);
 
