@@ -209,6 +209,7 @@ extern "C" cmn_status cmn_batch_create(const cmn_batch_config* config, cmn_batch
     c.max_cycle = (int64_t)o.max_cycle_size;
     c.enumerate_cap = (int64_t)o.enumerate_cap;
     c.seg_max = lazy ? (cf.max_segments > 0 ? cf.max_segments : (int)n_max + 1) : 0;
+    batch_tile_config(c, max_smem);
     const uint64_t K = c.K, nm = (uint64_t)n_max, G = K * child_stride;
 
     BatchBufs& b = s->b;
@@ -256,6 +257,13 @@ extern "C" cmn_status cmn_batch_create(const cmn_batch_config* config, cmn_batch
     A(&b.block_counts, (G + 511) / 512);
     A(&b.block_offsets, (G + 511) / 512);
     A(&b.child_base, K + 2);
+    A(&b.ptile, K + 1);
+    A(&b.ctile, K + 1);
+    A(&b.ltile, K + 1);
+    A(&b.stile, K + 1);
+    A(&b.qtile, K + 1);
+    A(&b.live, 4);
+    A(&b.sbest, K);
     uint32_t* order = nullptr;
     A(&order, K);
     b.order = order;
@@ -362,6 +370,8 @@ extern "C" cmn_status cmn_batch_add(cmn_batch* s, const cmn_problem* p, const cm
       d.inc_segments = p->prog.inc_segments;
     }
   }
+  d.chain = p->chain();
+  d.tile = batch_tile_takes(s->cfg, d.chain) ? 1 : 0;
   d.active = 1;
   d.iter_limit = opts->iter_limit;
   d.batch_iter_limit = opts->batch_iter_limit;

@@ -42,6 +42,13 @@ struct BatchCfg {
   uint64_t eval_capacity;    // threads the bound launches keep resident
   uint64_t sample_capacity;  // threads the sample launch keeps resident
   int seg_max;               // lazy form: sum-chain segments per instance program, at most
+  // instances whose program is a set of sum chains take the tile kernels
+  // (batch_chain_kernels.cu), where their shared memory fits
+  int tiles;                 // 1: it does
+  int sms;
+  int log_pts;               // points per warp of the tile samplers
+  int lazy_chains;           // LazyShape
+  int lazy_parts;
 };
 
 struct InstDesc {
@@ -68,7 +75,8 @@ struct InstDesc {
   const int32_t* inc_off;
   const int32_t* inc_pcs;
   int32_t inc_segments;
-  int32_t pad2_;
+  int32_t tile;  // 1: the instance takes the tile kernels
+  ChainTab chain;
 };
 
 struct InstState {
@@ -118,6 +126,18 @@ struct BatchBufs {
   uint32_t* block_counts;
   uint32_t* block_offsets;
   uint64_t* child_base;  // [K + 2]: exclusive prefix of live children by `order` position, then the lane cap
+  // the tile instances' work, as exclusive prefixes by `order` position
+  // ([K + 1]): tiles of parents and of children for the constraints (2^live[1]
+  // and 2^live[2] boxes each), tiles of 32 parents (lazy children), of 32
+  // children (objective) and of 2^log_pts children (points)
+  uint64_t* ptile;
+  uint64_t* ctile;
+  uint64_t* ltile;
+  uint64_t* stile;
+  uint64_t* qtile;
+  uint64_t* live;           // [0] live children of all instances, [1], [2] as above,
+                            // [3] most lanes any live instance can use per box
+  unsigned long long* sbest;  // [K] lb_key of the best point value known
   // [K]: the slots in the order the bound and sample launches walk their
   // children -- longest program first, so the launch's tail is short
   // programs (longest-processing-time-first balance)
@@ -135,6 +155,42 @@ struct BatchBufs {
   uint8_t* vlg;        // [K] log2 of the lanes per parent of each position
 };
 
+#ifdef __CUDACC__
+// Variable v of the staged parents of `slot`.
+__device__ __forceinline__ size_t splane(const BatchCfg& c, uint64_t slot, int v)
+{
+  return ((size_t)slot * c.n_max + v) * c.e_max;
+}
+
+// Largest `order` position whose prefix does not exceed i.
+__device__ __forceinline__ uint64_t position_of(const uint64_t* __restrict__ base, uint64_t K, uint64_t i)
+{
+  uint64_t lo = 0, hi = K;
+  while (hi - lo > 1) {
+    const uint64_t mid = (lo + hi) >> 1;
+    if (__ldg(base + mid) <= i) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+#endif
+
+// The tile kernels of an iteration (batch_chain_kernels.cu): constraints of
+// the staged parents (lazy form) or of the children, the lazy form's child
+// bounds, the children's objectives, and the points.
+struct BatchTileGrids {
+  int constraints = 0, children = 0, lazy = 0, objective = 0, points = 0;
+};
+// Sets cfg's tile fields; 0 tiles when the kernels' shared memory is short.
+void batch_tile_config(BatchCfg& cfg, int max_smem);
+BatchTileGrids batch_tile_grids(const BatchCfg& cfg);
+bool batch_tile_takes(const BatchCfg& cfg, const ChainTab& chain);
+cudaError_t batch_tile_parents(const BatchCfg& cfg, const BatchBufs& b, const BatchTileGrids& g, cudaStream_t s);
+cudaError_t batch_tile_lazy(const BatchCfg& cfg, const BatchBufs& b, const BatchTileGrids& g, cudaStream_t s);
+cudaError_t batch_tile_children(const BatchCfg& cfg, const BatchBufs& b, const BatchTileGrids& g, cudaStream_t s);
+cudaError_t batch_tile_points(const BatchCfg& cfg, const BatchBufs& b, const BatchTileGrids& g, cudaStream_t s);
+cudaError_t set_batch_tile_attributes(int max_smem);
+
 // Puts `slot`'s root box in its pool and resets its state.
 cudaError_t batch_init_slot(const BatchCfg& cfg, const BatchBufs& b, uint64_t slot, double gub0, cudaStream_t s);
 // Blocks of the grid-stride launches of an iteration.  `eval` serves the
@@ -146,6 +202,7 @@ struct BatchGrids {
   int inc_common = 1;
   int inc_parts = 1;
   int screen = 1;
+  BatchTileGrids tile;
 };
 BatchGrids batch_grids(const BatchCfg& cfg, int eval_grid);
 // Enqueues one iteration over every active instance (capturable).

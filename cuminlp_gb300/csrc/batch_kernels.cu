@@ -11,6 +11,7 @@
 #include <cstdint>
 
 #include "batch.hpp"
+#include "chain_tiles.cuh"
 #include "eval_core.cuh"
 #include "launch.hpp"
 #include "policy.cuh"
@@ -86,11 +87,6 @@ __device__ void bitonic_sort(uint64_t* keys, uint32_t* pos, uint32_t n)
 __device__ __forceinline__ size_t plane(const BatchCfg& c, uint64_t slot, int v)
 {
   return ((size_t)slot * c.n_max + v) * c.P;
-}
-
-__device__ __forceinline__ size_t splane(const BatchCfg& c, uint64_t slot, int v)
-{
-  return ((size_t)slot * c.n_max + v) * c.e_max;
 }
 
 // Stable in-place compaction of the marked entries among the first `n` of
@@ -237,6 +233,7 @@ __global__ void batch_begin_kernel(const BatchCfg c, const BatchBufs b)
   if (E > left) E = left;
   s.iterations += 1;
   s.n_parents = E;
+  b.sbest[slot] = lb_key(s.gub);  // a point must be below the incumbent to count
   s.salt_base = s.expansions;
   s.expansions += E;
   s.counters.iterations = s.iterations;
@@ -318,137 +315,144 @@ __global__ void batch_branch_kernel(const BatchCfg c, const BatchBufs b)
   }
 }
 
-// Exclusive prefix of the live children per slot (n_parents << B), slots
-// taken in `order`, into child_base[0..K]; child_base[K] is this
-// iteration's live child count and child_base[K + 1] the most lanes any
-// live instance can use per child.
+// Exclusive prefix over the block's 1024 threads of one value each; `total`
+// gets the sum.  Every thread calls it.
+__device__ __forceinline__ uint64_t block_prefix(uint64_t v, uint64_t& total)
+{
+  __shared__ uint64_t wsum[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint64_t x = v;
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint64_t y = __shfl_up_sync(0xffffffffu, x, off);
+    if (lane >= off) x += y;
+  }
+  if (lane == 31) wsum[wid] = x;
+  __syncthreads();
+  if (wid == 0) {
+    uint64_t w = wsum[lane];
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, w, off);
+      if (lane >= off) w += y;
+    }
+    wsum[lane] = w;
+  }
+  __syncthreads();
+  const uint64_t before = (wid > 0 ? wsum[wid - 1] : 0) + x - v;
+  total = wsum[31];
+  __syncthreads();
+  return before;
+}
+
+// Lays out this iteration's work by `order` position: exclusive prefixes,
+// their totals at [K].
+//
+// child_base: the live children (n_parents << B) of the instances that take
+// the interpreter; child_base[K + 1] is the most lanes any of them can use
+// per child.  ptile, ctile, ltile, stile, qtile: the tile instances' tiles
+// (batch.hpp); the constraints' tiles shrink until there are two for every SM.
 //
 // The lazy form's verdict takes its parents in warp runs: a run is one
 // warp over 32 >> lg parents of one instance, 2^lg lanes per parent.  lg
 // is chosen per instance: the capacity's lanes when few parents are live,
 // and more for a long program, until a run is at most half of a warp's
 // fair share of the verdict's work (the parents' program lengths over the
-// grid's warps), within the lanes the instance's schedule has.  vrun gets
-// the runs' exclusive prefix by `order` position and their total, vlg each
+// grid's warps), within the lanes the instance's schedule has; a tile
+// instance's objective chain takes the capacity's lanes.  vrun gets the
+// runs' exclusive prefix by `order` position and their total, vlg each
 // position's lg, and the run ticket is reset.
 __global__ void __launch_bounds__(1024) batch_live_kernel(const BatchCfg c, const BatchBufs b)
 {
-  __shared__ uint64_t wsum[32], wrun[32];
-  __shared__ uint64_t carry, rcarry;
-  __shared__ int gmax;
-  __shared__ unsigned long long work, parents;
+  __shared__ int gmax, gmax_all;
+  __shared__ unsigned long long work, parents, tile_parents;
   if (threadIdx.x == 0) {
-    carry = 0;
-    rcarry = 0;
     gmax = 1;
+    gmax_all = 1;
     work = 0;
     parents = 0;
+    tile_parents = 0;
   }
   __syncthreads();
   const bool runs = b.vrun != nullptr;
-  int my_gmax = 1;
-  unsigned long long my_work = 0, my_par = 0;
+  int my_gmax = 1, my_all = 1;
+  unsigned long long my_work = 0, my_par = 0, my_tile = 0;
   for (uint64_t i = threadIdx.x; i < c.K; i += 1024) {
     const uint64_t np = b.st[i].n_parents;
-    if (np > 0 && b.desc[i].g_max > my_gmax) my_gmax = b.desc[i].g_max;
-    my_work += np * (uint64_t)b.desc[i].prog_len;
+    const InstDesc& d = b.desc[i];
+    if (np > 0 && d.g_max > my_all) my_all = d.g_max;
+    if (np > 0 && !d.tile && d.g_max > my_gmax) my_gmax = d.g_max;
+    if (!d.tile) my_work += np * (uint64_t)d.prog_len;
+    else my_tile += np;
     my_par += np;
   }
   atomicMax(&gmax, my_gmax);
-  if (runs) {
-    atomicAdd(&work, my_work);
-    atomicAdd(&parents, my_par);
-  }
+  atomicMax(&gmax_all, my_all);
+  atomicAdd(&work, my_work);
+  atomicAdd(&parents, my_par);
+  atomicAdd(&tile_parents, my_tile);
   __syncthreads();
-  int lg_cap = 0;
-  unsigned long long half_share = 0;
-  if (runs) {
-    lg_cap = lanes_per_box(parents, c.eval_capacity, min(gmax, c.g_max));
-    const unsigned long long warps = c.eval_capacity >> 5 > 0 ? c.eval_capacity >> 5 : 1;
-    half_share = work / (64ULL * warps);  // (work / 32 lanes / warps) / 2
-    if (half_share < 64) half_share = 64;
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto log_boxes = [&](unsigned long long boxes) {
+    int lb = 5;
+    while (lb > 0 && (boxes >> lb) < 2ULL * (unsigned)c.sms) --lb;
+    return lb;
+  };
+  const int lbp = log_boxes(tile_parents), lbc = log_boxes(tile_parents << c.log2C);
+  const int lg_cap = lanes_per_box(parents, c.eval_capacity, min(gmax, c.g_max));
+  const int lg_chain = lanes_per_box(parents, c.eval_capacity, 32);
+  const unsigned long long warps = c.eval_capacity >> 5 > 0 ? c.eval_capacity >> 5 : 1;
+  unsigned long long half_share = work / (64ULL * warps);  // (work / 32 lanes / warps) / 2
+  if (half_share < 64) half_share = 64;
+  uint64_t* const out[7] = {b.child_base, b.vrun, b.ptile, b.ctile, b.ltile, b.stile, b.qtile};
+  uint64_t carry[7] = {};
   for (uint64_t base = 0; base < c.K; base += 1024) {
     const uint64_t i = base + threadIdx.x;
-    uint64_t v = 0, u = 0;
+    uint64_t v[7] = {};
     int lgi = 0;
     if (i < c.K) {
       const uint32_t slot = b.order[i];
-      const uint64_t np = b.st[slot].n_parents;
-      v = np << c.log2C;
-      if (runs && np > 0) {
-        const InstDesc& d = b.desc[slot];
+      const uint64_t np = b.st[slot].n_parents, nc = np << c.log2C;
+      const InstDesc& d = b.desc[slot];
+      if (np > 0 && d.tile) {
+        lgi = lg_chain;
+        v[2] = (np + (1ULL << lbp) - 1) >> lbp;
+        v[3] = (nc + (1ULL << lbc) - 1) >> lbc;
+        v[4] = (np + 31) >> 5;
+        v[5] = (nc + 31) >> 5;
+        v[6] = (nc + (1ULL << c.log_pts) - 1) >> c.log_pts;
+      } else if (np > 0) {
+        v[0] = nc;
         int lim = 0;
         while (lim < 5 && (2 << lim) <= d.g_max) ++lim;
         int l = 0;
         while (l < lim && ((unsigned long long)d.prog_len >> l) > half_share) ++l;
         lgi = max(l, min(lg_cap, lim));
-        u = ((np << lgi) + 31) >> 5;
       }
+      v[1] = ((np << lgi) + 31) >> 5;
     }
-    uint64_t x = v, y = u;
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint64_t xa = __shfl_up_sync(0xffffffffu, x, off);
-      const uint64_t ya = __shfl_up_sync(0xffffffffu, y, off);
-      if (lane >= off) {
-        x += xa;
-        y += ya;
-      }
+    for (int q = 0; q < 7; ++q) {
+      if (out[q] == nullptr) continue;
+      uint64_t total;
+      const uint64_t at = block_prefix(v[q], total);
+      if (i < c.K) out[q][i] = carry[q] + at;
+      carry[q] += total;
     }
-    if (lane == 31) {
-      wsum[wid] = x;
-      wrun[wid] = y;
-    }
-    __syncthreads();
-    if (wid == 0) {
-      uint64_t w = wsum[lane], z = wrun[lane];
-      for (int off = 1; off < 32; off <<= 1) {
-        const uint64_t wa = __shfl_up_sync(0xffffffffu, w, off);
-        const uint64_t za = __shfl_up_sync(0xffffffffu, z, off);
-        if (lane >= off) {
-          w += wa;
-          z += za;
-        }
-      }
-      wsum[lane] = w;
-      wrun[lane] = z;
-    }
-    __syncthreads();
-    const uint64_t cy = carry, ry = rcarry;
-    if (i < c.K) {
-      b.child_base[i] = cy + (wid > 0 ? wsum[wid - 1] : 0) + x - v;
-      if (runs) {
-        b.vrun[i] = ry + (wid > 0 ? wrun[wid - 1] : 0) + y - u;
-        b.vlg[i] = (uint8_t)lgi;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      carry = cy + wsum[31];
-      rcarry = ry + wrun[31];
-    }
-    __syncthreads();
+    if (runs && i < c.K) b.vlg[i] = (uint8_t)lgi;
   }
   if (threadIdx.x == 0) {
-    b.child_base[c.K] = carry;
+    for (int q = 0; q < 7; ++q)
+      if (out[q] != nullptr) out[q][c.K] = carry[q];
     b.child_base[c.K + 1] = (uint64_t)min(gmax, c.g_max);
-    if (runs) {
-      b.vrun[c.K] = rcarry;
-      b.vrun[c.K + 1] = 0;
-    }
+    b.live[0] = parents << c.log2C;
+    b.live[1] = (uint64_t)lbp;
+    b.live[2] = (uint64_t)lbc;
+    b.live[3] = (uint64_t)min(gmax_all, c.g_max);
+    if (runs) b.vrun[c.K + 1] = 0;
   }
 }
 
 // Live child i -> its global index slot * child_stride + local.
 __device__ __forceinline__ uint64_t live_child(const BatchCfg& c, const BatchBufs& b, uint64_t i)
 {
-  uint64_t lo = 0, hi = c.K;  // largest position with child_base[pos] <= i
-  while (hi - lo > 1) {
-    const uint64_t mid = (lo + hi) >> 1;
-    if (__ldg(b.child_base + mid) <= i) lo = mid;
-    else hi = mid;
-  }
+  const uint64_t lo = position_of(b.child_base, c.K, i);
   return (uint64_t)__ldg(b.order + lo) * c.child_stride + (i - __ldg(b.child_base + lo));
 }
 
@@ -546,21 +550,39 @@ __global__ void __launch_bounds__(kEvalThreads) batch_verdict_kernel(const Batch
     if (wl == 0) w = atomicAdd(ticket, 1ULL);
     w = __shfl_sync(0xffffffffu, w, 0);
     if (w >= runs) break;
-    uint64_t pos = 0, hi = c.K;  // largest position with vrun[pos] <= w: it has runs
-    while (hi - pos > 1) {
-      const uint64_t mid = (pos + hi) >> 1;
-      if (b.vrun[mid] <= w) pos = mid;
-      else hi = mid;
-    }
+    const uint64_t pos = position_of(b.vrun, c.K, w);
     const uint64_t slot = b.order[pos];
     const int lg = b.vlg[pos];
     const int G = 1 << lg;
     const int lane = wl & (G - 1);
     const uint64_t k = ((w - b.vrun[pos]) << (5 - lg)) + (uint64_t)(wl >> lg);
-    const bool live = k < b.st[slot].n_parents;
+    bool live = k < b.st[slot].n_parents;
+    const InstDesc& d = b.desc[slot];
+    if (d.tile) {
+      // the constraints are decided (batch_constraints_kernel): the objective
+      // of the boxes they leave
+      live = live && b.pfeas[slot * c.e_max + k] != 0;
+      if (!__any_sync(0xffffffffu, live)) continue;
+      V64 cv = {};
+      cv.plo = b.plo + splane(c, slot, 0) + k;
+      cv.phi = b.phi + splane(c, slot, 0) + k;
+      cv.pstride = c.e_max;
+      const ChainSeg& s = d.chain.seg[0];
+      double lo = 0.0;
+      if (lg > 0) lo = chain_lo_group<true>(d.prog64, s.pc0, s.pc1, cv, G, live);
+      else if (live) lo = chain_lo<true>(d.prog64, s.pc0, s.pc1, cv);
+      if (live && lane == 0) {
+        if (lo != lo) {
+          Verdict<double> v = verdict_init<double>();
+          chain_general<true>(d.prog64, s.pc0, s.pc2, cv, v);
+          lo = v.obj.lo;
+        }
+        b.plb[slot * c.e_max + k] = lo;
+      }
+      continue;
+    }
     Verdict<double> v = verdict_init<double>();
     if (live) {
-      const InstDesc& d = b.desc[slot];
       ChildVars<double, double> cv = {};
       cv.plo = b.plo + splane(c, slot, 0) + k;
       cv.phi = b.phi + splane(c, slot, 0) + k;
@@ -609,7 +631,7 @@ __global__ void batch_drop_kernel(const BatchCfg c, const BatchBufs b)
 // the incremental tables (inc_common_kernel per instance).
 __global__ void __launch_bounds__(kEvalThreads) batch_inc_common_kernel(const BatchCfg c, const BatchBufs b)
 {
-  const uint64_t total = c.K * (uint64_t)c.seg_max * c.e_max;
+  const uint64_t total = b.child_base[c.K] > 0 ? c.K * (uint64_t)c.seg_max * c.e_max : 0;  // none: all in tiles
   for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t k = idx % c.e_max, rest = idx / c.e_max;
@@ -617,7 +639,7 @@ __global__ void __launch_bounds__(kEvalThreads) batch_inc_common_kernel(const Ba
     const uint64_t slot = rest / (uint64_t)c.seg_max;
     if (k >= b.st[slot].n_parents) continue;
     const InstDesc& d = b.desc[slot];
-    if (s >= d.inc_segments) continue;
+    if (d.tile || s >= d.inc_segments) continue;
     const ParentInfo pi = b.pinfo[slot * c.e_max + k];
     if (pi.nreg == 0 || pi.fathom) continue;  // no bounded children
     const SlotPlan* sp = b.slots + (slot * c.e_max + k) * c.max_slots;
@@ -653,7 +675,7 @@ __global__ void __launch_bounds__(kEvalThreads) batch_inc_common_kernel(const Ba
 __global__ void __launch_bounds__(kEvalThreads) batch_inc_parts_kernel(const BatchCfg c, const BatchBufs b)
 {
   const uint64_t C = 1ULL << c.log2C;
-  const uint64_t total = c.K * C * c.e_max;
+  const uint64_t total = b.child_base[c.K] > 0 ? c.K * C * c.e_max : 0;
   for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t k = idx % c.e_max, rest = idx / c.e_max;
@@ -661,7 +683,7 @@ __global__ void __launch_bounds__(kEvalThreads) batch_inc_parts_kernel(const Bat
     if (k >= b.st[slot].n_parents) continue;
     const InstDesc& d = b.desc[slot];
     const int S = d.inc_segments;
-    if (S == 0) continue;
+    if (d.tile || S == 0) continue;
     const ParentInfo pi = b.pinfo[slot * c.e_max + k];
     if (pi.fathom || pi.nreg == 0) continue;
     const SlotPlan* sp = b.slots + (slot * c.e_max + k) * c.max_slots;
@@ -825,7 +847,7 @@ __global__ void __launch_bounds__(kEvalThreads) batch_chunk_kernel(const BatchCf
   t.tid = threadIdx.x;  // every lane stages its group's point in its own column
   const uint64_t per_slot = (c.child_stride + 31) >> 5;
   const uint64_t items = c.K * per_slot;
-  const int lg = lanes_per_box((b.child_base[c.K] + 31) >> 5, c.sample_capacity, (int)b.child_base[c.K + 1]);
+  const int lg = lanes_per_box((b.live[0] + 31) >> 5, c.sample_capacity, (int)b.live[3]);
   const int lane = threadIdx.x & 31;
   const uint64_t per_warp = 32u >> lg;
   const uint64_t warps = (uint64_t)gridDim.x * (uint64_t)(B >> 5);
@@ -962,7 +984,7 @@ __global__ void __launch_bounds__(kEvalThreads, 4) batch_eval_kernel(const Batch
     planes_hi = b.phi;
   }
   const uint64_t total = kMode == 3 ? *b.list_count : b.child_base[c.K];
-  const int lg = lanes_per_box(total, c.eval_capacity, (int)b.child_base[c.K + 1]);
+  const int lg = lanes_per_box(total, c.eval_capacity, (int)(kMode == 3 ? b.live[3] : b.child_base[c.K + 1]));
   const int G = 1 << lg;
   const int lane = threadIdx.x & (G - 1);
   const uint64_t per_block = (uint64_t)(B >> lg);
@@ -1531,6 +1553,7 @@ BatchGrids batch_grids(const BatchCfg& c, int eval_grid)
   g.eval = eval_grid;
   g.inc_common = resident_grid(batch_inc_common_kernel, 0, c.K * (uint64_t)c.seg_max * c.e_max);
   g.inc_parts = resident_grid(batch_inc_parts_kernel, 0, c.K * (c.e_max << c.log2C));
+  g.tile = batch_tile_grids(c);
   g.screen = resident_grid(batch_screen_kernel, batch_screen_smem(c), c.K * c.child_stride);
   return g;
 }
@@ -1554,9 +1577,13 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
     // bounds with each parent's certified bound folded in, and the band's
     // FP64 pass (the single-instance solver runs the verdict beside the
     // bounds; the states and counters are the same)
+    cudaError_t e = batch_tile_parents(c, b, grids.tile, s);
+    if (e != cudaSuccess) return e;
     batch_verdict_kernel<<<eval_grid, kEvalThreads, batch_verdict_smem(c), s>>>(c, b);
     const uint64_t np2 = c.K * c.e_max;
     batch_drop_kernel<<<(int)((np2 + 255) / 256), 256, 0, s>>>(c, b);
+    e = batch_tile_lazy(c, b, grids.tile, s);
+    if (e != cudaSuccess) return e;
     batch_inc_common_kernel<<<grids.inc_common, kEvalThreads, 0, s>>>(c, b);
     batch_inc_parts_kernel<<<grids.inc_parts, kEvalThreads, 0, s>>>(c, b);
     batch_eval_kernel<float, 5><<<eval_grid, kEvalThreads, batch_eval_smem(c, true), s>>>(c, b);
@@ -1566,6 +1593,8 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
     batch_list_scatter_kernel<<<lg, 512, 0, s>>>(c, b);
     batch_eval_kernel<double, 3><<<eval_grid, kEvalThreads, batch_eval_smem(c, false), s>>>(c, b);
     mark(marks, 2, s);
+    e = batch_tile_points(c, b, grids.tile, s);
+    if (e != cudaSuccess) return e;
     batch_screen_kernel<<<grids.screen, kEvalThreads, batch_screen_smem(c), s>>>(c, b);
     batch_chunk_kernel<<<eval_grid, kEvalThreads, batch_sample_smem(c), s>>>(c, b);
     mark(marks, 3, s);
@@ -1581,9 +1610,13 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
     batch_list_scatter_kernel<<<lg, 512, 0, s>>>(c, b);
     batch_eval_kernel<double, 3><<<eval_grid, kEvalThreads, batch_eval_smem(c, false), s>>>(c, b);
   } else {
+    const cudaError_t e = batch_tile_children(c, b, grids.tile, s);
+    if (e != cudaSuccess) return e;
     batch_eval_kernel<double, 1><<<eval_grid, kEvalThreads, batch_eval_smem(c, false), s>>>(c, b);
   }
   mark(marks, 2, s);
+  const cudaError_t ep = batch_tile_points(c, b, grids.tile, s);
+  if (ep != cudaSuccess) return ep;
   batch_sample_kernel<<<eval_grid, kEvalThreads, batch_sample_smem(c), s>>>(c, b);
   mark(marks, 3, s);
   batch_finish_kernel<<<(int)c.K, kMiThreads, sort_smem_bytes(), s>>>(c, b);

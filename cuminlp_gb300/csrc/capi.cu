@@ -99,6 +99,7 @@ static cudaError_t ensure_attributes()
   if (e == cudaSuccess) e = set_chain32_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_chain_points_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_batch_kernel_attributes(max_dynamic_smem());
+  if (e == cudaSuccess) e = set_batch_tile_attributes(max_dynamic_smem());
   if (e == cudaSuccess && dev < 31) g_attr_device_mask |= (1 << dev);
   return e;
 }
