@@ -222,7 +222,12 @@ extern "C" cmn_status cmn_batch_create(const cmn_batch_config* config, cmn_batch
     A(&b.lo, K * nm * c.P);
     A(&b.hi, K * nm * c.P);
     A(&b.lb, K * c.P);
+    A(&b.idx, K * c.P);
     A(&b.depth, K * c.P);
+    A(&b.free_slots, K * c.P);
+    A(&b.pslot, K * c.e_max);
+    A(&b.klist, G);
+    A(&b.kslot, G);
     A(&b.plo, K * nm * c.e_max);
     A(&b.phi, K * nm * c.e_max);
     if (fp32 || lazy) {
@@ -571,26 +576,33 @@ extern "C" cmn_status cmn_batch_frontier(cmn_batch* s, uint64_t slot, double* bo
   if (m == 0) return CMN_OK;
   const BatchCfg& c = s->cfg;
   const int n = s->h_desc[slot].n_vars;
-  const size_t base = (size_t)slot * c.n_max * c.P;
+  // the pool's store slots, then the boxes and depths they name
+  std::vector<uint32_t> idx(m);
+  BCK(cudaMemcpyAsync(idx.data(), s->b.idx + (size_t)slot * c.P, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
+  BCK(cudaStreamSynchronize(s->stream));
+  const uint64_t top = m == 0 ? 0 : *std::max_element(idx.begin(), idx.end()) + 1;
   if (boxes) {
-    std::vector<double> lo((size_t)n * m), hi((size_t)n * m);
-    BCK(cudaMemcpy2DAsync(lo.data(), m * sizeof(double), s->b.lo + base, c.P * sizeof(double), m * sizeof(double), n,
-                          cudaMemcpyDeviceToHost, s->stream));
-    BCK(cudaMemcpy2DAsync(hi.data(), m * sizeof(double), s->b.hi + base, c.P * sizeof(double), m * sizeof(double), n,
-                          cudaMemcpyDeviceToHost, s->stream));
+    const size_t base = (size_t)slot * c.P * c.n_max;
+    std::vector<double> lo(top * c.n_max), hi(top * c.n_max);
+    BCK(cudaMemcpyAsync(lo.data(), s->b.lo + base, lo.size() * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    BCK(cudaMemcpyAsync(hi.data(), s->b.hi + base, hi.size() * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     BCK(cudaStreamSynchronize(s->stream));
     for (uint64_t i = 0; i < m; ++i)
       for (int v = 0; v < n; ++v) {
-        boxes[2 * (i * n + v)] = lo[(size_t)v * m + i];
-        boxes[2 * (i * n + v) + 1] = hi[(size_t)v * m + i];
+        boxes[2 * (i * n + v)] = lo[(size_t)idx[i] * c.n_max + v];
+        boxes[2 * (i * n + v) + 1] = hi[(size_t)idx[i] * c.n_max + v];
       }
   }
   if (lower_bounds)
     BCK(cudaMemcpyAsync(lower_bounds, s->b.lb + (size_t)slot * c.P, m * sizeof(double), cudaMemcpyDeviceToHost,
                         s->stream));
-  if (depths)
-    BCK(cudaMemcpyAsync(depths, s->b.depth + (size_t)slot * c.P, m * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+  if (depths) {
+    std::vector<uint32_t> dep(top);
+    BCK(cudaMemcpyAsync(dep.data(), s->b.depth + (size_t)slot * c.P, top * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                         s->stream));
+    BCK(cudaStreamSynchronize(s->stream));
+    for (uint64_t i = 0; i < m; ++i) depths[i] = dep[idx[i]];
+  }
   BCK(cudaStreamSynchronize(s->stream));
   return CMN_OK;
 }

@@ -20,7 +20,7 @@
 namespace cmn {
 
 constexpr int kMiThreads = 1024;   // threads of a per-instance block
-constexpr int kMiSortMax = 8192;   // largest pool a block sorts in shared memory
+constexpr int kMiSortMax = 8192;   // largest pool a block holds (eight entries a thread)
 
 struct BatchCfg {
   int n_max;        // variables per instance, at most
@@ -90,6 +90,8 @@ struct InstState {
   uint64_t expansions;
   uint64_t iterations;
   uint64_t remaining;
+  uint64_t free_top;  // free store slots
+  uint64_t kept;      // children the last iteration kept
   uint64_t viable;
   uint64_t dropped_min_key;
   uint32_t done;
@@ -103,10 +105,15 @@ struct InstState {
 struct BatchBufs {
   InstDesc* desc;
   InstState* st;
-  double* lo;  // [K][n_max][P]
+  double* lo;  // [K][P][n_max]: the box store, a box contiguous
   double* hi;
-  double* lb;  // [K][P]
-  uint32_t* depth;
+  double* lb;  // [K][P] the pool in position order: lower bound,
+  uint32_t* idx;         // [K][P] and store slot
+  uint32_t* depth;       // [K][P] by store slot
+  uint32_t* free_slots;  // [K][P] stack of free store slots (InstState::free_top)
+  uint32_t* pslot;       // [K][e_max] store slots of the selected parents, in order
+  uint32_t* klist;       // [K][child_stride] the kept children, in order,
+  uint32_t* kslot;       // and their store slots
   double* plo;  // [K][n_max][e_max]
   double* phi;
   float* plo32;  // FP32 screen only: the same planes rounded outward

@@ -1,11 +1,18 @@
 // batch_kernels.cu -- the multi-instance iteration (see batch.hpp).
 //
-// Per iteration: begin (thread per instance) -> select + gather + in-place
-// compaction (block per instance, pool sorted in shared memory) -> branch
-// (thread per parent) -> bound (one launch over all instances' children;
-// FP64, or FP32 screen + FP64 certify) -> sample (one launch) -> finish
-// (block per instance: ArgMin, incumbent and witness, prune, append kept
-// children, evict above the cap, pool minimum, adaptive screen).
+// Per iteration: begin (thread per instance) -> select (block per instance:
+// radix select, the pool closed over the parents) -> stage the parents'
+// boxes -> branch (thread per parent) -> bound (one launch over all
+// instances' children; FP64, or FP32 screen + FP64 certify) -> sample (one
+// launch) -> finish (block per instance: ArgMin, incumbent and witness,
+// prune, pool entries of the kept children, evict above the cap, pool
+// minimum, adaptive screen) -> append the kept children's boxes.
+//
+// The pool holds a box's lower bound and its slot in the instance's box
+// store, so the per-instance blocks move 12 bytes an entry; whole boxes move
+// only in the two grid-wide copies.  With boxes moved plane by plane and the
+// selections by a bitonic sort, the two per-instance kernels took 250 and
+// 500 us an iteration at n <= 48 and 8192 entries, on one SM per instance.
 #include <algorithm>
 #include <cfloat>
 #include <cstdint>
@@ -34,144 +41,186 @@ __device__ __forceinline__ double key_to_lb_b(uint64_t k)
   return __longlong_as_double((long long)u);
 }
 
-__device__ __forceinline__ uint64_t next_pow2(uint64_t x)
-{
-  uint64_t p = 1;
-  while (p < x) p <<= 1;
-  return p;
-}
+// Items a thread of a per-instance block holds: item u of thread t is
+// u * kMiThreads + t, so a warp reads whole lines.
+__device__ __forceinline__ uint32_t mi_item(int u) { return (uint32_t)u * kMiThreads + threadIdx.x; }
 
-// exclusive rank of `f` among the block's threads (1024 threads)
-__device__ __forceinline__ int block_rank(bool f, int& total)
+// Ranks in item order of the flagged items of the block (for every item: the
+// flagged items before it); returns their count.  Every thread calls it.
+__device__ __forceinline__ uint32_t mi_ranks(const bool (&f)[kMaxPerThread], uint32_t (&rank)[kMaxPerThread])
 {
-  __shared__ int warp_tot[kMiThreads / 32];
+  constexpr int kMiWarps = kMiThreads / 32;
+  constexpr int kPer = kMaxPerThread * kMiWarps / 32;
+  __shared__ uint32_t tab[kMaxPerThread * kMiWarps];
+  __shared__ uint32_t all;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const unsigned ball = __ballot_sync(0xffffffffu, f);
-  if (lane == 0) warp_tot[wid] = __popc(ball);
-  __syncthreads();
-  int before = 0;
-  total = 0;
-  for (int w = 0; w < kMiThreads / 32; ++w) {
-    if (w < wid) before += warp_tot[w];
-    total += warp_tot[w];
+  unsigned ball[kMaxPerThread];
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u) {
+    ball[u] = __ballot_sync(0xffffffffu, f[u]);
+    if (lane == 0) tab[u * kMiWarps + wid] = __popc(ball[u]);
   }
   __syncthreads();
-  return before + __popc(ball & ((1u << lane) - 1u));
-}
-
-// ascending bitonic sort of (key, pos) pairs, n a power of two
-__device__ void bitonic_sort(uint64_t* keys, uint32_t* pos, uint32_t n)
-{
-  for (uint32_t k = 2; k <= n; k <<= 1) {
-    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint32_t ixj = i ^ j;
-        if (ixj > i) {
-          const bool asc = (i & k) == 0;
-          const uint64_t ka = keys[i], kb = keys[ixj];
-          const uint32_t pa = pos[i], pb = pos[ixj];
-          const bool b_less = kb < ka || (kb == ka && pb < pa);
-          if (asc ? b_less : !b_less) {
-            keys[i] = kb;
-            keys[ixj] = ka;
-            pos[i] = pb;
-            pos[ixj] = pa;
-          }
-        }
-      }
-      __syncthreads();
+  if (wid == 0) {
+    uint32_t v[kPer], sum = 0;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      v[e] = tab[lane * kPer + e];
+      sum += v[e];
     }
-  }
-}
-
-__device__ __forceinline__ size_t plane(const BatchCfg& c, uint64_t slot, int v)
-{
-  return ((size_t)slot * c.n_max + v) * c.P;
-}
-
-// Stable in-place compaction of the marked entries among the first `n` of
-// `slot`'s pool (marks in `keep`, new positions built in `newpos`).
-__device__ void compact_pool(const BatchCfg& c, const BatchBufs& b, uint64_t slot, uint32_t n, int n_vars,
-                             const uint8_t* keep, uint32_t* newpos, uint32_t* running)
-{
-  if (threadIdx.x == 0) *running = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < n; base += kMiThreads) {
-    const uint32_t i = base + threadIdx.x;
-    const bool f = i < n && keep[i];
-    int total;
-    const int r = block_rank(f, total);
-    if (f) newpos[i] = *running + (uint32_t)r;
-    __syncthreads();
-    if (threadIdx.x == 0) *running += (uint32_t)total;
-    __syncthreads();
-  }
-  double val[kMaxPerThread];
-  for (int v = -1; v < 2 * n_vars; ++v) {
-    // v = -1: lower bounds; then lo / hi planes
-    double* arr = v < 0 ? b.lb + (size_t)slot * c.P : (v & 1 ? b.hi : b.lo) + plane(c, slot, v >> 1);
-#pragma unroll
-    for (int j = 0; j < kMaxPerThread; ++j) {
-      const uint32_t i = threadIdx.x + j * kMiThreads;
-      if (i < n && keep[i]) val[j] = arr[i];
+    uint32_t x = sum;
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+      if (lane >= off) x += y;
     }
-    __syncthreads();
+    uint32_t run = x - sum;
 #pragma unroll
-    for (int j = 0; j < kMaxPerThread; ++j) {
-      const uint32_t i = threadIdx.x + j * kMiThreads;
-      if (i < n && keep[i]) arr[newpos[i]] = val[j];
+    for (int e = 0; e < kPer; ++e) {
+      tab[lane * kPer + e] = run;
+      run += v[e];
     }
-    __syncthreads();
-  }
-  uint32_t dv[kMaxPerThread];
-  uint32_t* dep = b.depth + (size_t)slot * c.P;
-#pragma unroll
-  for (int j = 0; j < kMaxPerThread; ++j) {
-    const uint32_t i = threadIdx.x + j * kMiThreads;
-    if (i < n && keep[i]) dv[j] = dep[i];
+    if (lane == 31) all = x;
   }
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < kMaxPerThread; ++j) {
-    const uint32_t i = threadIdx.x + j * kMiThreads;
-    if (i < n && keep[i]) dep[newpos[i]] = dv[j];
-  }
+  for (int u = 0; u < kMaxPerThread; ++u)
+    rank[u] = tab[u * kMiWarps + wid] + __popc(ball[u] & ((1u << lane) - 1u));
+  const uint32_t total = all;
   __syncthreads();
+  return total;
 }
 
-struct SortSmem {
-  uint64_t* keys;
-  uint32_t* pos;
-  uint8_t* flag;
-};
-
-__device__ __forceinline__ SortSmem sort_smem(unsigned char* raw)
+// Marks the k smallest (key, position) of the block's n items, keys in
+// registers: a radix select over the bits below the common leading ones,
+// kMiBits at a time, ties in the last bucket by position.  Every thread
+// calls it.
+constexpr int kMiBits = 10;
+__device__ __forceinline__ void mi_select(const uint64_t (&key)[kMaxPerThread], uint32_t n, uint32_t k,
+                                          bool (&take)[kMaxPerThread])
 {
-  SortSmem s;
-  s.keys = reinterpret_cast<uint64_t*>(raw);
-  s.pos = reinterpret_cast<uint32_t*>(s.keys + kMiSortMax);
-  s.flag = reinterpret_cast<uint8_t*>(s.pos + kMiSortMax);
-  return s;
-}
-
-// Marks the `k` smallest (key, position) entries among the first `n`.
-__device__ void mark_smallest(const double* lb, uint32_t n, uint32_t k, const SortSmem& s)
-{
+  __shared__ uint32_t hist[1 << kMiBits];
+  __shared__ uint32_t wsum[kMiThreads / 32];
+  __shared__ unsigned long long min_s, max_s;
+  __shared__ uint32_t pick_d, pick_before, pick_cnt;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (k >= n) {
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) s.flag[i] = 1;
-    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kMaxPerThread; ++u) take[u] = mi_item(u) < n;
     return;
   }
-  const uint32_t n2 = (uint32_t)next_pow2(n);
-  for (uint32_t i = threadIdx.x; i < n2; i += blockDim.x) {
-    s.keys[i] = i < n ? lb_key(lb[i]) : ~0ULL;
-    s.pos[i] = i < n ? i : 0xffffffffu;
-    if (i < n) s.flag[i] = 0;
+  if (threadIdx.x == 0) {
+    min_s = ~0ULL;
+    max_s = 0;
   }
   __syncthreads();
-  bitonic_sort(s.keys, s.pos, n2);
-  for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) s.flag[s.pos[i]] = 1;
+  unsigned long long lo = ~0ULL, hi = 0;
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u)
+    if (mi_item(u) < n) {
+      lo = key[u] < lo ? key[u] : lo;
+      hi = key[u] > hi ? key[u] : hi;
+    }
+  for (int off = 16; off > 0; off >>= 1) {
+    const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo, off), b = __shfl_xor_sync(0xffffffffu, hi, off);
+    lo = a < lo ? a : lo;
+    hi = b > hi ? b : hi;
+  }
+  if (lane == 0) {
+    atomicMin(&min_s, lo);
+    atomicMax(&max_s, hi);
+  }
   __syncthreads();
+  lo = min_s;
+  hi = max_s;
+  int left = lo == hi ? 0 : 64 - __clzll((long long)(lo ^ hi));  // bits still open
+  uint64_t mask = left == 64 ? 0 : ~0ULL << left, prefix = lo & mask;
+  bool settled = false;  // the bucket is taken whole
+  while (left > 0 && !settled) {
+    const int bits = left < kMiBits ? left : kMiBits, shift = left - bits;
+    for (int i = threadIdx.x; i < (1 << kMiBits); i += kMiThreads) hist[i] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kMaxPerThread; ++u)
+      if (mi_item(u) < n && (key[u] & mask) == prefix) atomicAdd(&hist[(key[u] >> shift) & ((1u << bits) - 1u)], 1u);
+    __syncthreads();
+    // one bin per thread
+    const uint32_t c = hist[threadIdx.x];
+    uint32_t x = c;
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+      if (lane >= off) x += y;
+    }
+    if (lane == 31) wsum[wid] = x;
+    __syncthreads();
+    if (wid == 0) {
+      uint32_t w = wsum[lane];
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, w, off);
+        if (lane >= off) w += y;
+      }
+      wsum[lane] = w;
+    }
+    __syncthreads();
+    const uint32_t before = x - c + (wid > 0 ? wsum[wid - 1] : 0);
+    if (before < k && k <= before + c) {  // exactly one bin holds the k-th
+      pick_d = threadIdx.x;
+      pick_before = before;
+      pick_cnt = c;
+    }
+    __syncthreads();
+    k -= pick_before;
+    prefix |= (uint64_t)pick_d << shift;
+    mask |= (uint64_t)((1u << bits) - 1u) << shift;
+    left = shift;
+    settled = pick_cnt == k;
+    __syncthreads();
+  }
+  bool eq[kMaxPerThread];
+  uint32_t rank[kMaxPerThread];
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u) eq[u] = mi_item(u) < n && (key[u] & mask) == prefix;
+  if (!settled) mi_ranks(eq, rank);
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u)
+    take[u] = mi_item(u) < n && (eq[u] ? settled || rank[u] < k : (key[u] & mask) < prefix);
+}
+
+__device__ __forceinline__ size_t box_at(const BatchCfg& c, uint64_t slot, uint64_t store)
+{
+  return ((size_t)slot * c.P + store) * c.n_max;
+}
+
+// Keeps the flagged pool entries in order, and pushes the others' store slots
+// on the free stack in position order.  Every thread of the block calls it;
+// returns the entries kept.
+__device__ __forceinline__ uint32_t keep_entries(const BatchCfg& c, const BatchBufs& b, uint64_t slot, uint32_t n,
+                                                 const bool (&keep)[kMaxPerThread], uint32_t free_top)
+{
+  double* lb = b.lb + (size_t)slot * c.P;
+  uint32_t* idx = b.idx + (size_t)slot * c.P;
+  uint32_t* fr = b.free_slots + (size_t)slot * c.P;
+  double l[kMaxPerThread];
+  uint32_t s[kMaxPerThread], rank[kMaxPerThread];
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u)
+    if (mi_item(u) < n) {
+      l[u] = lb[mi_item(u)];
+      s[u] = idx[mi_item(u)];
+    }
+  const uint32_t kept = mi_ranks(keep, rank);  // its barriers order the reads before the writes
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u) {
+    const uint32_t i = mi_item(u);
+    if (i >= n) continue;
+    if (keep[u]) {
+      lb[rank[u]] = l[u];
+      idx[rank[u]] = s[u];
+    } else {
+      fr[free_top + (i - rank[u])] = s[u];
+    }
+  }
+  __syncthreads();
+  return kept;
 }
 
 }  // namespace
@@ -181,12 +230,14 @@ __global__ void batch_init_slot_kernel(const BatchCfg c, const BatchBufs b, uint
 {
   const InstDesc d = b.desc[slot];
   for (int v = threadIdx.x; v < c.n_max; v += blockDim.x) {
-    if (v < d.n_vars) {
-      b.lo[plane(c, slot, v)] = d.root_lb[v];
-      b.hi[plane(c, slot, v)] = d.root_ub[v];
+    if (v < d.n_vars) {  // the root box in store slot 0
+      b.lo[box_at(c, slot, 0) + v] = d.root_lb[v];
+      b.hi[box_at(c, slot, 0) + v] = d.root_ub[v];
     }
     b.best_point[slot * c.n_max + v] = __longlong_as_double(0x7ff8000000000000LL);
   }
+  // every other store slot is free; pops take the low slots first
+  for (uint64_t i = threadIdx.x; i + 1 < c.P; i += blockDim.x) b.free_slots[slot * c.P + i] = (uint32_t)(c.P - 1 - i);
   if (threadIdx.x == 0) {
     InstState* s = &b.st[slot];
     memset(s, 0, sizeof(InstState));
@@ -200,7 +251,9 @@ __global__ void batch_init_slot_kernel(const BatchCfg c, const BatchBufs b, uint
     s->use_screen = 1;
     s->counters.peak_frontier = 1;
     b.lb[slot * c.P] = -DBL_MAX;
+    b.idx[slot * c.P] = 0;
     b.depth[slot * c.P] = 0;
+    s->free_top = c.P - 1;
   }
 }
 
@@ -240,56 +293,131 @@ __global__ void batch_begin_kernel(const BatchCfg c, const BatchBufs b)
   s.counters.expansions = s.expansions;
 }
 
-// select the E best parents, stage them, compact the rest in place
+// Selects the E best parents, lists their store slots in pool order, and
+// closes the pool over them.  The boxes stay where they are: the pool holds
+// each box's store slot, so an entry moves 12 bytes, not the whole box.
 __global__ void __launch_bounds__(kMiThreads) batch_select_kernel(const BatchCfg c, const BatchBufs b)
 {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ uint32_t running;
   const uint64_t slot = blockIdx.x;
   InstState* st = &b.st[slot];
   const uint32_t E = (uint32_t)st->n_parents;
   if (E == 0) return;
-  const uint32_t L = (uint32_t)st->pool_size;
-  const int n = b.desc[slot].n_vars;
-  const SortSmem s = sort_smem(smem_raw);
-  mark_smallest(b.lb + (size_t)slot * c.P, L, E, s);
-  // gather the selected parents in pool order
-  if (threadIdx.x == 0) running = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < L; base += kMiThreads) {
-    const uint32_t i = base + threadIdx.x;
-    const bool f = i < L && s.flag[i];
-    int total;
-    const int r = block_rank(f, total);
-    if (f) {
-      const uint32_t k = running + (uint32_t)r;
-      for (int v = 0; v < n; ++v) {
-        const double lo = b.lo[plane(c, slot, v) + i], hi = b.hi[plane(c, slot, v) + i];
-        b.plo[splane(c, slot, v) + k] = lo;
-        b.phi[splane(c, slot, v) + k] = hi;
-        if (b.plo32 != nullptr) {
-          b.plo32[splane(c, slot, v) + k] = __double2float_rd(lo);
-          b.phi32[splane(c, slot, v) + k] = __double2float_ru(hi);
-        }
-      }
-      b.pdepth[slot * c.e_max + k] = b.depth[(size_t)slot * c.P + i];
+  const uint32_t L = (uint32_t)st->pool_size, free_top = (uint32_t)st->free_top;
+  const double* lb = b.lb + (size_t)slot * c.P;
+  const uint32_t* idx = b.idx + (size_t)slot * c.P;
+  uint64_t key[kMaxPerThread];
+  bool take[kMaxPerThread];
+  uint32_t s[kMaxPerThread], rank[kMaxPerThread];
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u) {
+    key[u] = ~0ULL;
+    s[u] = 0;
+    if (mi_item(u) < L) {
+      key[u] = lb_key(lb[mi_item(u)]);
+      s[u] = idx[mi_item(u)];
     }
-    __syncthreads();
-    if (threadIdx.x == 0) running += (uint32_t)total;
-    __syncthreads();
   }
-  // the unselected entries keep their order at the front of the pool
-  for (uint32_t i = threadIdx.x; i < L; i += blockDim.x) s.flag[i] = !s.flag[i];
-  __syncthreads();
-  compact_pool(c, b, slot, L, n, s.flag, s.pos, &running);
+  mi_select(key, L, E, take);
+  mi_ranks(take, rank);
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u) {
+    if (take[u]) {
+      b.pslot[slot * c.e_max + rank[u]] = s[u];
+      b.pdepth[slot * c.e_max + rank[u]] = b.depth[(size_t)slot * c.P + s[u]];
+    }
+    take[u] = mi_item(u) < L && !take[u];
+  }
+  keep_entries(c, b, slot, L, take, free_top);
   if (threadIdx.x == 0) {
     st->remaining = L - E;
     st->pool_size = L - E;
+    st->free_top = free_top + E;
   }
 }
 
+// The selected parents' boxes into the staging planes, lane = parent.
+__global__ void __launch_bounds__(256) batch_stage_kernel(const BatchCfg c, const BatchBufs b)
+{
+  const uint64_t total = c.K * c.e_max;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t slot = i / c.e_max, k = i - slot * c.e_max;
+    if (k >= b.st[slot].n_parents) continue;
+    const int n = b.desc[slot].n_vars;
+    const size_t at = box_at(c, slot, b.pslot[i]);
+    const double* __restrict__ lo = b.lo + at;
+    const double* __restrict__ hi = b.hi + at;
+    double* __restrict__ plo = b.plo;
+    double* __restrict__ phi = b.phi;
+#pragma unroll 4
+    for (int v = 0; v < n; ++v) {
+      const double l = lo[v], h = hi[v];
+      const size_t to = splane(c, slot, v) + k;
+      plo[to] = l;
+      phi[to] = h;
+      if (b.plo32 != nullptr) {
+        b.plo32[to] = __double2float_rd(l);
+        b.phi32[to] = __double2float_ru(h);
+      }
+    }
+  }
+}
+
+// The kept children's boxes into their store slots (batch_finish_kernel lists
+// them), a warp per child, lane = variable.
+__global__ void __launch_bounds__(256) batch_append_kernel(const BatchCfg c, const BatchBufs b)
+{
+  const int lane = threadIdx.x & 31;
+  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const uint64_t per = c.child_stride;
+  for (uint64_t w = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < c.K * ((per + 15) / 16); w += warps) {
+    const uint64_t slot = w / ((per + 15) / 16), p0 = (w - slot * ((per + 15) / 16)) * 16;
+    const uint64_t kept = b.st[slot].n_parents > 0 ? b.st[slot].kept : 0;
+    if (p0 >= kept) continue;
+    const int n = b.desc[slot].n_vars;
+    const int cnt = kept - p0 < 16 ? (int)(kept - p0) : 16;
+    uint32_t mine = 0, to = 0;
+    if (lane < cnt) {
+      mine = b.klist[slot * per + p0 + lane];
+      to = b.kslot[slot * per + p0 + lane];
+    }
+    for (int v = lane; v < n + 31 - (n + 31) % 32; v += 32) {  // every lane takes the shuffles
+      uint32_t cur = 0xffffffffu;
+      double lo = 0.0, hi = 0.0;
+      const SlotPlan* plan = nullptr;
+      for (int q = 0; q < cnt; ++q) {
+        const uint32_t local = __shfl_sync(0xffffffffu, mine, q), store = __shfl_sync(0xffffffffu, to, q);
+        const uint32_t k = local >> c.log2C;
+        if (v >= n) continue;
+        if (k != cur) {
+          cur = k;
+          lo = b.plo[splane(c, slot, v) + k];
+          hi = b.phi[splane(c, slot, v) + k];
+          plan = nullptr;
+          const size_t pk = slot * c.e_max + k;
+          const uint32_t count = b.pinfo[pk].count;
+          for (uint32_t j = 0; j < count; ++j)
+            if (b.slots[pk * c.max_slots + j].vid == (uint32_t)v) {
+              plan = b.slots + pk * c.max_slots + j;
+              break;
+            }
+        }
+        double l = lo, h = hi;
+        if (plan != nullptr) slot_bounds(*plan, lo, hi, slot_part(local & ((1u << c.log2C) - 1u), *plan), l, h);
+        b.lo[box_at(c, slot, store) + v] = l;
+        b.hi[box_at(c, slot, store) + v] = h;
+      }
+    }
+  }
+}
+
+// kLocal: the policy's scratch in local memory (n_max <= kLocal; 0: in the
+// global arrays), as branch_kernel.
+template <int kLocal>
 __global__ void batch_branch_kernel(const BatchCfg c, const BatchBufs b)
 {
+  EnumCand ec_local[kLocal > 0 ? kLocal : 1];
+  BisCand bc_local[kLocal > 0 ? kLocal : 1];
+  uint64_t heap_local[kLocal > 0 ? kLocal : 1];
   const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= c.K * c.e_max) return;
   const uint64_t slot = idx / c.e_max, k = idx % c.e_max;
@@ -297,9 +425,9 @@ __global__ void batch_branch_kernel(const BatchCfg c, const BatchBufs b)
   if (k >= st->n_parents) return;
   const InstDesc d = b.desc[slot];
   const size_t pk = slot * c.e_max + k;
-  EnumCand* ec = reinterpret_cast<EnumCand*>(b.enum_scratch) + pk * c.n_max;
-  BisCand* bc = reinterpret_cast<BisCand*>(b.bis_scratch) + pk * c.n_max;
-  uint64_t* heap = b.heap_scratch + pk * c.n_max;
+  EnumCand* ec = kLocal > 0 ? ec_local : reinterpret_cast<EnumCand*>(b.enum_scratch) + pk * c.n_max;
+  BisCand* bc = kLocal > 0 ? bc_local : reinterpret_cast<BisCand*>(b.bis_scratch) + pk * c.n_max;
+  uint64_t* heap = kLocal > 0 ? heap_local : b.heap_scratch + pk * c.n_max;
   SlotPlan* sp = b.slots + pk * c.max_slots;
   const PolicyParams pp = {c.log2C, c.max_cycle, c.enumerate_cap, c.relative};
   const ParentInfo pi =
@@ -1184,8 +1312,6 @@ __global__ void __launch_bounds__(kEvalThreads) batch_sample_kernel(const BatchC
 // per instance: incumbent, prune, append kept children, evict, statistics
 __global__ void __launch_bounds__(kMiThreads) batch_finish_kernel(const BatchCfg c, const BatchBufs b)
 {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ uint32_t running;
   __shared__ Cand best_s;
   __shared__ unsigned long long cnt[10];
   __shared__ unsigned long long min_key_s;
@@ -1255,14 +1381,19 @@ __global__ void __launch_bounds__(kMiThreads) batch_finish_kernel(const BatchCfg
   __syncthreads();
   const double gub = st->gub;
 
-  // (2) verdict counts and (3) append kept children after the remaining pool
+  // (2) verdict counts and (3) the kept children behind the remaining pool:
+  // their pool entries, and a list for batch_append_kernel to write the boxes
   const uint32_t remaining = (uint32_t)st->remaining;
-  if (threadIdx.x == 0) running = 0;
-  __syncthreads();
-  unsigned long long l_dup = 0, l_inf = 0, l_dom = 0, l_kept = 0, l_smp = 0, l_valid = 0, l_excl = 0, l_cert = 0;
-  for (uint32_t cb = 0; cb < nch; cb += kMiThreads) {
-    const uint32_t local = cb + threadIdx.x;
-    bool keep = false;
+  uint32_t free_top = (uint32_t)st->free_top;
+  double* lb = b.lb + (size_t)slot * c.P;
+  uint32_t* idx = b.idx + (size_t)slot * c.P;
+  unsigned long long l_dup = 0, l_inf = 0, l_dom = 0, l_smp = 0, l_valid = 0, l_excl = 0, l_cert = 0;
+  bool keep[kMaxPerThread];
+  uint32_t rank[kMaxPerThread];
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u) {
+    const uint32_t local = mi_item(u);
+    keep[u] = false;
     if (local < nch) {
       const uint8_t raw = b.cstate[cbase + local];
       const uint64_t k = local >> c.log2C, r = local & ((1ULL << c.log2C) - 1ULL);
@@ -1279,80 +1410,75 @@ __global__ void __launch_bounds__(kMiThreads) batch_finish_kernel(const BatchCfg
           if (s8 == kChildDuplicate) ++l_dup;
           else if (s8 == kChildInfeasible) ++l_inf;
           else if (s8 == kChildDominated || s8 == kChildScreened || b.clb[cbase + local] > gub) ++l_dom;
-          else {
-            ++l_kept;
-            keep = true;
-          }
+          else keep[u] = true;
         }
       }
     }
-    int total;
-    const int rank = block_rank(keep, total);
-    if (keep) {
-      const uint32_t at = remaining + running + (uint32_t)rank;
-      const uint64_t k = local >> c.log2C, r = local & ((1ULL << c.log2C) - 1ULL);
-      const size_t pk = slot * c.e_max + k;
-      const ParentInfo pi = b.pinfo[pk];
-      const SlotPlan* sp = b.slots + pk * c.max_slots;
-      for (int v = 0; v < n; ++v) {
-        double hi;
-        const double lo = child_bound(c, b, slot, k, r, v, sp, pi.count, hi);
-        b.lo[plane(c, slot, v) + at] = lo;
-        b.hi[plane(c, slot, v) + at] = hi;
-      }
-      b.lb[(size_t)slot * c.P + at] = b.clb[cbase + local];
-      b.depth[(size_t)slot * c.P + at] = b.pdepth[pk] + 1;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) running += (uint32_t)total;
-    __syncthreads();
   }
-  atomicAdd(&cnt[0], l_dup);
-  atomicAdd(&cnt[1], l_inf);
-  atomicAdd(&cnt[2], l_dom);
-  atomicAdd(&cnt[3], l_kept);
-  atomicAdd(&cnt[4], l_smp);
-  atomicAdd(&cnt[5], l_valid);
-  atomicAdd(&cnt[6], l_excl);
-  atomicAdd(&cnt[7], l_cert);
+  const uint32_t kept = mi_ranks(keep, rank);
+#pragma unroll
+  for (int u = 0; u < kMaxPerThread; ++u) {
+    if (!keep[u]) continue;
+    const uint32_t local = mi_item(u);
+    const uint32_t store = b.free_slots[(size_t)slot * c.P + free_top - 1 - rank[u]];
+    lb[remaining + rank[u]] = b.clb[cbase + local];
+    idx[remaining + rank[u]] = store;
+    b.depth[(size_t)slot * c.P + store] = b.pdepth[slot * c.e_max + (local >> c.log2C)] + 1;
+    b.klist[cbase + rank[u]] = local;
+    b.kslot[cbase + rank[u]] = store;
+  }
+  free_top -= kept;
+  {
+    unsigned long long v[7] = {l_dup, l_inf, l_dom, l_smp, l_valid, l_excl, l_cert};
+    const int at[7] = {0, 1, 2, 4, 5, 6, 7};
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+      const unsigned w = __reduce_add_sync(0xffffffffu, (unsigned)v[q]);
+      if ((threadIdx.x & 31) == 0 && w) atomicAdd(&cnt[at[q]], (unsigned long long)w);
+    }
+    if (threadIdx.x == 0) cnt[3] = kept;
+  }
   __syncthreads();
-  const uint32_t new_size = remaining + (uint32_t)cnt[3];
+  const uint32_t new_size = remaining + kept;
 
   // (4) above the cap: keep the `cap` best, fold the rest into the floor
   uint32_t final_size = new_size;
   if (new_size > c.cap) {
-    const SortSmem s = sort_smem(smem_raw);
-    const double* lbp = b.lb + (size_t)slot * c.P;
-    mark_smallest(lbp, new_size, (uint32_t)c.cap, s);
-    unsigned long long via = 0, dom = 0;
+    uint64_t key[kMaxPerThread];
+    bool stay[kMaxPerThread];
+#pragma unroll
+    for (int u = 0; u < kMaxPerThread; ++u) key[u] = mi_item(u) < new_size ? lb_key(lb[mi_item(u)]) : ~0ULL;
+    mi_select(key, new_size, (uint32_t)c.cap, stay);
+    unsigned via = 0, dom = 0;
     uint64_t mk = ~0ULL;
-    for (uint32_t i = threadIdx.x; i < new_size; i += blockDim.x) {
-      if (s.flag[i]) continue;
-      const double x = lbp[i];
-      if (x <= gub) {
+#pragma unroll
+    for (int u = 0; u < kMaxPerThread; ++u) {
+      if (mi_item(u) >= new_size || stay[u]) continue;
+      if (lb[mi_item(u)] <= gub) {
         ++via;
-        const uint64_t kk = lb_key(x);
-        mk = kk < mk ? kk : mk;
+        mk = key[u] < mk ? key[u] : mk;
       } else {
         ++dom;
       }
     }
-    atomicAdd(&cnt[8], via);
-    atomicAdd(&cnt[9], dom);
+    via = __reduce_add_sync(0xffffffffu, via);
+    dom = __reduce_add_sync(0xffffffffu, dom);
+    if ((threadIdx.x & 31) == 0) {
+      if (via) atomicAdd(&cnt[8], (unsigned long long)via);
+      if (dom) atomicAdd(&cnt[9], (unsigned long long)dom);
+    }
     if (mk != ~0ULL) atomicMin(&min_key_s, (unsigned long long)mk);
-    __syncthreads();
-    compact_pool(c, b, slot, new_size, n, s.flag, s.pos, &running);
-    final_size = (uint32_t)c.cap;
+    final_size = keep_entries(c, b, slot, new_size, stay, free_top);
+    free_top += new_size - final_size;
   }
 
   // (5) pool minimum and viable count
-  uint64_t mk = ~0ULL;
-  unsigned long long viable = 0;
-  const double* lbp = b.lb + (size_t)slot * c.P;
+  unsigned long long mk = ~0ULL;
+  unsigned viable = 0;
   for (uint32_t i = threadIdx.x; i < final_size; i += blockDim.x) {
-    const uint64_t kk = lb_key(lbp[i]);
+    const uint64_t kk = lb_key(lb[i]);
     mk = kk < mk ? kk : mk;
-    if (lbp[i] <= gub) ++viable;
+    if (lb[i] <= gub) ++viable;
   }
   __shared__ unsigned long long pool_min_s, viable_s;
   if (threadIdx.x == 0) {
@@ -1360,8 +1486,15 @@ __global__ void __launch_bounds__(kMiThreads) batch_finish_kernel(const BatchCfg
     viable_s = 0;
   }
   __syncthreads();
-  atomicMin(&pool_min_s, (unsigned long long)mk);
-  atomicAdd(&viable_s, viable);
+  viable = __reduce_add_sync(0xffffffffu, viable);
+  for (int off = 16; off > 0; off >>= 1) {
+    const unsigned long long o = __shfl_xor_sync(0xffffffffu, mk, off);
+    mk = o < mk ? o : mk;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(&pool_min_s, mk);
+    if (viable) atomicAdd(&viable_s, (unsigned long long)viable);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     cmn_counters& ct = st->counters;
@@ -1388,6 +1521,8 @@ __global__ void __launch_bounds__(kMiThreads) batch_finish_kernel(const BatchCfg
     if (min_key_s < st->dropped_min_key) st->dropped_min_key = min_key_s;
     if (st->dropped_min_key != ~0ULL) st->dropped_lb_min = key_to_lb_b(st->dropped_min_key);
     st->pool_size = final_size;
+    st->free_top = free_top;
+    st->kept = kept;
     st->pool_min_key = pool_min_s;
     st->viable = viable_s;
     if (final_size > ct.peak_frontier) ct.peak_frontier = final_size;
@@ -1500,17 +1635,10 @@ int batch_sample_occupancy(const BatchCfg& c)
   return n;
 }
 
-static size_t sort_smem_bytes() { return (size_t)kMiSortMax * (8 + 4 + 1); }
-
 cudaError_t set_batch_kernel_attributes(int max_smem)
 {
   const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, batch_select_kernel);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(batch_select_kernel, at, max_smem - (int)fa.sharedSizeBytes);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, batch_finish_kernel);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(batch_finish_kernel, at, max_smem - (int)fa.sharedSizeBytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(batch_eval_kernel<double, 1>, at, max_smem);
+  cudaError_t e = cudaFuncSetAttribute(batch_eval_kernel<double, 1>, at, max_smem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(batch_eval_kernel<float, 2>, at, max_smem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(batch_eval_kernel<double, 3>, at, max_smem);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(batch_sample_kernel, at, max_smem);
@@ -1558,6 +1686,14 @@ BatchGrids batch_grids(const BatchCfg& c, int eval_grid)
   return g;
 }
 
+// per instance: incumbent, prune, pool; then the kept children's boxes
+static void finish(const BatchCfg& c, const BatchBufs& b, cudaStream_t s)
+{
+  batch_finish_kernel<<<(int)c.K, kMiThreads, 0, s>>>(c, b);
+  const uint64_t warps = c.K * ((c.child_stride + 15) / 16);
+  batch_append_kernel<<<(int)std::min<uint64_t>((warps + 7) / 8, 8192), 256, 0, s>>>(c, b);
+}
+
 cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGrids& grids, cudaStream_t s,
                             const cudaEvent_t* marks)
 {
@@ -1565,9 +1701,13 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
   mark(marks, 0, s);
   const int kb = (int)((c.K + 255) / 256);
   batch_begin_kernel<<<kb, 256, 0, s>>>(c, b);
-  batch_select_kernel<<<(int)c.K, kMiThreads, sort_smem_bytes(), s>>>(c, b);
+  batch_select_kernel<<<(int)c.K, kMiThreads, 0, s>>>(c, b);
   const uint64_t np = c.K * c.e_max;
-  batch_branch_kernel<<<(int)((np + 127) / 128), 128, 0, s>>>(c, b);
+  batch_stage_kernel<<<(int)std::min<uint64_t>((np + 255) / 256, 8192), 256, 0, s>>>(c, b);
+  const int bg = (int)((np + 127) / 128);
+  if (c.n_max <= 32) batch_branch_kernel<32><<<bg, 128, 0, s>>>(c, b);
+  else if (c.n_max <= 64) batch_branch_kernel<64><<<bg, 128, 0, s>>>(c, b);
+  else batch_branch_kernel<0><<<bg, 128, 0, s>>>(c, b);
   batch_live_kernel<<<1, 1024, 0, s>>>(c, b);
   mark(marks, 1, s);
   const bool fp32 = c.precision == CMN_PRECISION_FP32_SCREEN;
@@ -1598,7 +1738,7 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
     batch_screen_kernel<<<grids.screen, kEvalThreads, batch_screen_smem(c), s>>>(c, b);
     batch_chunk_kernel<<<eval_grid, kEvalThreads, batch_sample_smem(c), s>>>(c, b);
     mark(marks, 3, s);
-    batch_finish_kernel<<<(int)c.K, kMiThreads, sort_smem_bytes(), s>>>(c, b);
+    finish(c, b, s);
     mark(marks, 4, s);
     return cudaGetLastError();
   }
@@ -1619,7 +1759,7 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
   if (ep != cudaSuccess) return ep;
   batch_sample_kernel<<<eval_grid, kEvalThreads, batch_sample_smem(c), s>>>(c, b);
   mark(marks, 3, s);
-  batch_finish_kernel<<<(int)c.K, kMiThreads, sort_smem_bytes(), s>>>(c, b);
+  finish(c, b, s);
   mark(marks, 4, s);
   return cudaGetLastError();
 }
