@@ -186,7 +186,7 @@ __device__ __forceinline__ uint64_t position_of(const uint64_t* __restrict__ bas
 // the staged parents (lazy form) or of the children, the lazy form's child
 // bounds, the children's objectives, and the points.
 struct BatchTileGrids {
-  int constraints = 0, children = 0, lazy = 0, objective = 0, points = 0;
+  int constraints = 0, children = 0, lazy = 0, objective = 0, points = 0, picks = 0;
 };
 // Sets cfg's tile fields; 0 tiles when the kernels' shared memory is short.
 void batch_tile_config(BatchCfg& cfg, int max_smem);

@@ -197,6 +197,43 @@ __global__ void __launch_bounds__(kPointThreads) batch_points_kernel(const Batch
   }
 }
 
+// The lazy form's picks, one per chunk of 32 children, in FP64 (cval, ce; the
+// chunk's other children +inf): a warp per 32 chunks of an instance.
+__global__ void __launch_bounds__(kPointThreads) batch_picks_kernel(const BatchCfg c, const BatchBufs b)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint8_t list_s[kPointThreads];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, W = blockDim.x >> 5;
+  double* x64 = reinterpret_cast<double*>(smem_raw) + (size_t)wid * c.n_max;
+  float* x32 = reinterpret_cast<float*>(smem_raw + (size_t)W * c.n_max * 8 + wid * point_bytes(c.n_max, c.log_pts));
+  const int pts = 1 << c.log_pts;
+  const uint64_t per_slot = (((c.child_stride + 31) >> 5) + pts - 1) >> c.log_pts;
+  for (uint64_t w = (uint64_t)blockIdx.x * W + wid; w < c.K * per_slot; w += (uint64_t)gridDim.x * W) {
+    const uint64_t pos = w / per_slot, slot = b.order[pos];
+    const uint64_t total = b.st[slot].n_parents << c.log2C, chunk = ((w - pos * per_slot) << c.log_pts) + lane;
+    if (((w - pos * per_slot) << (c.log_pts + 5)) >= total || !b.desc[slot].tile || !b.desc[slot].chain.points) continue;
+    SampleArgs a;
+    point_args(c, b, slot, a);
+    const uint64_t cbase = slot * c.child_stride;
+    PointOf p = {};
+    bool cand = lane < pts && (chunk << 5) < total;
+    if (cand) {
+      const uint64_t g1 = total < (chunk << 5) + 32 ? total : (chunk << 5) + 32;
+      for (uint64_t g = chunk << 5; g < g1; ++g) b.cval[cbase + g] = INFINITY;
+      cand = chunk_point(a, chunk, total, b.st[slot].salt_base, p);
+    }
+    __syncwarp();
+    unsigned long long rejected = 0;
+    sample_tile(a, x64, x32, list_s + wid * 32, c.log_pts, p, cand, b.sbest + slot, b.st[slot].gub, rejected,
+                [&](const PointOf& o, double value) {
+                  const uint64_t at = cbase + (o.k << c.log2C) + o.r;
+                  b.cval[at] = value;
+                  b.ce[at] = o.r * (o.fathom ? 1 : c.S) + o.i;
+                });
+    if (rejected) atomicAdd((unsigned long long*)&b.st[slot].counters.witness_rejected, rejected);
+  }
+}
+
 // ---- host ----
 static size_t constraints_smem(const BatchCfg& c) { return tile_smem_bytes(c.n_max, c.max_slots, 32); }
 static int families_of(const BatchCfg& c) { return 32 >> (c.log2C < 5 ? c.log2C : 5); }
@@ -210,6 +247,7 @@ static size_t points_smem(const BatchCfg& c, bool screen)
   return (size_t)(kPointThreads / 32) *
          (screen ? point_bytes(c.n_max + 1, c.log_pts) : (size_t)c.n_max * 8 + point_bytes(c.n_max, c.log_pts));
 }
+static size_t picks_smem(const BatchCfg& c) { return points_smem(c, false); }
 
 void batch_tile_config(BatchCfg& c, int max_smem)
 {
@@ -217,7 +255,8 @@ void batch_tile_config(BatchCfg& c, int max_smem)
   const bool lazy = c.precision == CMN_PRECISION_FP32_LAZY;
   c.sms = sm_count();
   c.log_pts = log_points(c.n_max + 1);
-  c.tiles = c.precision != CMN_PRECISION_FP32_SCREEN && constraints_smem(c) <= room && points_smem(c, lazy) <= room;
+  c.tiles = c.precision != CMN_PRECISION_FP32_SCREEN && constraints_smem(c) <= room && points_smem(c, true) <= room &&
+            picks_smem(c) <= room;
   if (lazy) {
     c.lazy_parts = (1 << c.log2C) + 1;
     c.lazy_chains = c.max_slots <= kLazySlots ? c.seg_max : 0;
@@ -253,6 +292,7 @@ BatchTileGrids batch_tile_grids(const BatchCfg& c)
     g.constraints = resident(batch_constraints_kernel<0, true>, kTileWarps * 32, constraints_smem(c));
     g.lazy = resident(batch_lazy_kernel, kLazyThreads, lazy_bytes(c));
     g.points = resident(batch_points_kernel<true>, kPointThreads, points_smem(c, true));
+    g.picks = resident(batch_picks_kernel, kPointThreads, picks_smem(c));
   } else {
     g.children = resident(batch_constraints_kernel<1, false>, kTileWarps * 32, constraints_smem(c));
     g.objective = resident(batch_siblings_kernel, kObjThreads, siblings_smem(c));
@@ -286,10 +326,14 @@ cudaError_t batch_tile_children(const BatchCfg& c, const BatchBufs& b, const Bat
 cudaError_t batch_tile_points(const BatchCfg& c, const BatchBufs& b, const BatchTileGrids& g, cudaStream_t s)
 {
   if (!c.tiles) return cudaSuccess;
-  if (c.precision == CMN_PRECISION_FP32_LAZY)
+  if (c.precision == CMN_PRECISION_FP32_LAZY) {
     batch_points_kernel<true><<<g.points, kPointThreads, points_smem(c, true), s>>>(c, b);
-  else
+    const uint64_t warps = c.K * ((((c.child_stride + 31) >> 5) + (1u << c.log_pts) - 1) >> c.log_pts);
+    const int grid = (int)std::min<uint64_t>((warps + 3) / 4, (uint64_t)g.picks);
+    batch_picks_kernel<<<grid, kPointThreads, picks_smem(c), s>>>(c, b);
+  } else {
     batch_points_kernel<false><<<g.points, kPointThreads, points_smem(c, false), s>>>(c, b);
+  }
   return cudaGetLastError();
 }
 
@@ -310,6 +354,7 @@ cudaError_t set_batch_tile_attributes(int max_smem)
   if (e == cudaSuccess) e = allow(batch_lazy_kernel, max_smem);
   if (e == cudaSuccess) e = allow(batch_points_kernel<true>, max_smem);
   if (e == cudaSuccess) e = allow(batch_points_kernel<false>, max_smem);
+  if (e == cudaSuccess) e = allow(batch_picks_kernel, max_smem);
   return e;
 }
 

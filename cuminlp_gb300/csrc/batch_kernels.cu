@@ -696,9 +696,7 @@ __global__ void __launch_bounds__(kEvalThreads) batch_verdict_kernel(const Batch
       cv.phi = b.phi + splane(c, slot, 0) + k;
       cv.pstride = c.e_max;
       const ChainSeg& s = d.chain.seg[0];
-      double lo = 0.0;
-      if (lg > 0) lo = chain_lo_group<true>(d.prog64, s.pc0, s.pc1, cv, G, live);
-      else if (live) lo = chain_lo<true>(d.prog64, s.pc0, s.pc1, cv);
+      double lo = chain_lo_group<true>(d.prog64, s.pc0, s.pc1, cv, lg, live);
       if (live && lane == 0) {
         if (lo != lo) {
           Verdict<double> v = verdict_init<double>();
@@ -991,7 +989,7 @@ __global__ void __launch_bounds__(kEvalThreads) batch_chunk_kernel(const BatchCf
       const uint64_t ch = idx % per_slot;
       const uint64_t nch = b.st[slot].n_parents << c.log2C;
       const uint64_t g0 = ch << 5;
-      if (g0 < nch) {
+      if (g0 < nch && !(b.desc[slot].tile && b.desc[slot].chain.points)) {  // those: batch_picks_kernel
         const uint64_t g1 = nch < g0 + 32 ? nch : g0 + 32;
         const uint64_t cbase = slot * c.child_stride;
         float bv = INFINITY;

@@ -228,13 +228,15 @@ __device__ __forceinline__ double chain_lo(const Instr* __restrict__ prog, int p
   return acc;
 }
 
-// The same chain by a group of G lanes on one box (G a power of two): the
-// lanes form G terms at once, then every lane adds them in order.  Every
-// lane of the warp calls it; a lane without a box passes active = false.
-template <bool kFused, typename V>
-__device__ __forceinline__ double chain_lo_group(const Instr* __restrict__ prog, int pc0, int pc1, const V& vars, int G,
-                                                 bool active)
+// The same chain by a group of G = 2^kLg lanes on one box: the lanes form G
+// terms at once, then every lane adds them in order.  Every lane of the warp
+// calls it; a lane without a box passes active = false.  A term past the end
+// is +0 times 1, which adds nothing in this rounding; a term that is not
+// fused is its value times 1, the same sum.
+template <int kLg, bool kFused, typename V>
+__device__ __noinline__ double chain_lo_lanes(const Instr* __restrict__ prog, int pc0, int pc1, const V& vars, bool active)
 {
+  constexpr int G = 1 << kLg;
   const int gl = threadIdx.x & (G - 1);
   double acc = 0.0;
   const Instr first = load_instr(prog, pc0);
@@ -245,32 +247,36 @@ __device__ __forceinline__ double chain_lo_group(const Instr* __restrict__ prog,
   for (int base = pc0 + 1; base < pc1; base += G) {
     const int pc = base + gl;
     double p = 0.0, c = 1.0;
-    int fused = 0;
     if (active && pc < pc1) {
       const Instr cur = load_instr(prog, pc);
       const int sub = cur.head >> 3;
       const bool neg = (sub & kTermSub) != 0;
       p = term_lo<kFused>(cur, vars);
-      if (fused_term<double, kFused>(sub)) {
-        fused = 1;
-        c = neg ? -cur.c : cur.c;
-      } else if (neg) {
-        p = -p;
-      }
+      if (fused_term<double, kFused>(sub)) c = neg ? -cur.c : cur.c;
+      else if (neg) p = -p;
     }
-    const int cnt = pc1 - base < G ? pc1 - base : G;
-    for (int j = 0; j < cnt; ++j) {
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
       const double pj = __shfl_sync(0xffffffffu, p, j, G);
-      if (kFused) {
-        const double cj = __shfl_sync(0xffffffffu, c, j, G);
-        const int fj = __shfl_sync(0xffffffffu, fused, j, G);
-        acc = fj ? __fma_rd(cj, pj, acc) : __dadd_rd(acc, pj);
-      } else {
-        acc = __dadd_rd(acc, pj);
-      }
+      if (kFused) acc = __fma_rd(__shfl_sync(0xffffffffu, c, j, G), pj, acc);
+      else acc = __dadd_rd(acc, pj);
     }
   }
   return acc;
+}
+
+template <bool kFused, typename V>
+__device__ __forceinline__ double chain_lo_group(const Instr* __restrict__ prog, int pc0, int pc1, const V& vars, int lg,
+                                                 bool active)
+{
+  switch (lg) {
+    case 1: return chain_lo_lanes<1, kFused>(prog, pc0, pc1, vars, active);
+    case 2: return chain_lo_lanes<2, kFused>(prog, pc0, pc1, vars, active);
+    case 3: return chain_lo_lanes<3, kFused>(prog, pc0, pc1, vars, active);
+    case 4: return chain_lo_lanes<4, kFused>(prog, pc0, pc1, vars, active);
+    case 5: return chain_lo_lanes<5, kFused>(prog, pc0, pc1, vars, active);
+    default: return active ? chain_lo<kFused>(prog, pc0, pc1, vars) : 0.0;
+  }
 }
 
 }  // namespace cmn

@@ -75,8 +75,7 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const E
     Verdict<double> v = verdict_init<double>();
     bool general = !pure || kHi;
     if (!general) {
-      if (lg > 0) v.obj.lo = chain_lo_group<kFused>(a.prog, s.pc0, s.pc1, cv, G, live);
-      else if (live) v.obj.lo = chain_lo<kFused>(a.prog, s.pc0, s.pc1, cv);
+      v.obj.lo = chain_lo_group<kFused>(a.prog, s.pc0, s.pc1, cv, lg, live);
       general = v.obj.lo != v.obj.lo;
     }
     if (general && live) chain_general<kFused>(a.prog, s.pc0, s.pc2, cv, v);

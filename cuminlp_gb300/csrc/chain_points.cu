@@ -20,6 +20,8 @@ namespace cmn {
 // usually rules out the others.  Taken
 // where every chain has a filter and the boxes are within its range
 // (ChainTab::points): elsewhere too many points would be left.
+// kChunks: the points are the lazy form's picks, one per chunk of children.
+template <bool kChunks>
 __global__ void __launch_bounds__(kPointThreads) chain_sample_kernel(const SampleArgs a, int log_pts)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -37,7 +39,7 @@ __global__ void __launch_bounds__(kPointThreads) chain_sample_kernel(const Sampl
   }
   const uint64_t children = a.n_children_dev ? *a.n_children_dev : a.n_children;
   const uint64_t per = a.exact ? 1 : a.S;
-  const uint64_t total = children * per;
+  const uint64_t total = kChunks ? (children + (1ULL << kChunkLog2) - 1) >> kChunkLog2 : children * per;
   const uint64_t salt_base = a.salt_base_dev ? *a.salt_base_dev : 0;
   const double gub = a.gub ? *a.gub : DBL_MAX;
   const bool solver = a.state != nullptr;
@@ -52,7 +54,9 @@ __global__ void __launch_bounds__(kPointThreads) chain_sample_kernel(const Sampl
     const uint64_t item = (w0 << log_pts) + lane;
     PointOf p = {};
     bool cand = lane < pts && item < total;
-    if (cand) {
+    if (kChunks) {
+      cand = cand && chunk_point(a, item, children, salt_base, p);
+    } else if (cand) {
       const uint64_t g = item / per;
       p.i = item - g * per;
       cand = point_child(a, g, salt_base, p) && (!p.fathom || p.i == 0);
@@ -89,7 +93,7 @@ static size_t screen_smem(int n, int log_pts) { return (size_t)(kPointThreads / 
 
 bool chain_sample_fits(const SampleArgs& a)
 {
-  return a.chain.points && a.sched != nullptr && a.cbest == nullptr &&
+  return a.chain.points && a.sched != nullptr &&
          sample_smem(a.n_vars, 0) + 2048 <= (size_t)max_dynamic_smem();
 }
 
@@ -100,7 +104,8 @@ cudaError_t launch_chain_sample(const SampleArgs& a, int grid, cudaStream_t s)
     const uint64_t warps = (uint64_t)grid * (kPointThreads / 32), points = a.n_children * a.S;
     while (lp > 0 && (points >> lp) < warps) --lp;
   }
-  chain_sample_kernel<<<grid, kPointThreads, sample_smem(a.n_vars, lp), s>>>(a, lp);
+  if (a.cbest != nullptr) chain_sample_kernel<true><<<grid, kPointThreads, sample_smem(a.n_vars, lp), s>>>(a, lp);
+  else chain_sample_kernel<false><<<grid, kPointThreads, sample_smem(a.n_vars, lp), s>>>(a, lp);
   return cudaGetLastError();
 }
 
@@ -133,7 +138,8 @@ static cudaError_t allow(K kernel, int max_smem)
 
 cudaError_t set_chain_points_attributes(int max_smem)
 {
-  cudaError_t e = allow(chain_sample_kernel, max_smem);
+  cudaError_t e = allow(chain_sample_kernel<false>, max_smem);
+  if (e == cudaSuccess) e = allow(chain_sample_kernel<true>, max_smem);
   return e == cudaSuccess ? allow(chain_screen_kernel, max_smem) : e;
 }
 

@@ -51,7 +51,7 @@ cudaError_t launch_chain32(const EvalArgs& a, int mode, cudaStream_t s);
 bool lazy_children_fits(const ChainTab& t, int n_vars, int max_slots, int log2C);
 cudaError_t launch_lazy_children(const EvalArgs& a, uint64_t max_parents, cudaStream_t s);
 cudaError_t set_chain32_kernel_attributes(int max_smem);
-// the sampler over such a program (not the lazy form's chunk mode)
+// the sampler over such a program
 bool chain_sample_fits(const SampleArgs& a);
 cudaError_t launch_chain_sample(const SampleArgs& a, int grid, cudaStream_t s);
 // the lazy form's FP32 sample screen over such a program

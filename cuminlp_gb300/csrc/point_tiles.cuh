@@ -168,9 +168,9 @@ __device__ __forceinline__ double point_chain_warp(const Instr* __restrict__ pro
   double acc = (first.head & 7) == kOpLoadAcc ? ((first.modes & 3) == kModeVar ? x[first.a] : first.c) : point_term(first, x);
   for (int base = pc0 + 1; base < pc1; base += 32) {
     const int pc = base + lane;
-    const double p = pc < pc1 ? point_term(load_instr(prog, pc), x) : 0.0;
-    const int cnt = pc1 - base < 32 ? pc1 - base : 32;
-    for (int j = 0; j < cnt; ++j) acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, p, j));
+    const double p = pc < pc1 ? point_term(load_instr(prog, pc), x) : -0.0;  // -0 adds nothing
+#pragma unroll
+    for (int j = 0; j < 32; ++j) acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, p, j));
   }
   return acc;
 }
@@ -355,6 +355,29 @@ __device__ __forceinline__ void sample_tile(const SampleArgs& a, double* x64, fl
     __syncwarp();
   }
   __syncwarp();  // the points are restaged next
+}
+
+// The lazy form's chunk of children [32c, 32c + 32): the child and sample
+// with the smallest FP32 value (ties: the first child, then the first
+// sample).  False when no point of the chunk is feasible in FP32.
+__device__ __forceinline__ bool chunk_point(const SampleArgs& a, uint64_t c, uint64_t total, uint64_t salt_base, PointOf& p)
+{
+  float best = INFINITY;
+  uint64_t g = 0, i = 0;
+  const uint64_t g0 = c << kChunkLog2;
+  const uint64_t g1 = total < g0 + (1ULL << kChunkLog2) ? total : g0 + (1ULL << kChunkLog2);
+  for (uint64_t x = g0; x < g1; ++x) {
+    const Best32 b = a.cbest[x];
+    if (b.value < best) {
+      best = b.value;
+      g = x;
+      i = b.i;
+    }
+  }
+  if (!(best < INFINITY)) return false;
+  point_child(a, g, salt_base, p);
+  p.i = i;
+  return true;
 }
 
 // The lazy form's sample screen (sample_screen_kernel's results): every
