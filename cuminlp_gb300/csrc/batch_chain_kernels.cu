@@ -198,7 +198,11 @@ __global__ void __launch_bounds__(kPointThreads) batch_points_kernel(const Batch
 }
 
 // The lazy form's picks, one per chunk of 32 children, in FP64 (cval, ce; the
-// chunk's other children +inf): a warp per 32 chunks of an instance.
+// chunk's other children +inf): a warp per 2^kLogPicks
+// chunks of an instance (few, so that the picks that need FP64, one after the
+// other in a warp, spread over the SMs).
+constexpr int kLogPicks = 3;
+
 __global__ void __launch_bounds__(kPointThreads) batch_picks_kernel(const BatchCfg c, const BatchBufs b)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -206,12 +210,12 @@ __global__ void __launch_bounds__(kPointThreads) batch_picks_kernel(const BatchC
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, W = blockDim.x >> 5;
   double* x64 = reinterpret_cast<double*>(smem_raw) + (size_t)wid * c.n_max;
   float* x32 = reinterpret_cast<float*>(smem_raw + (size_t)W * c.n_max * 8 + wid * point_bytes(c.n_max, c.log_pts));
-  const int pts = 1 << c.log_pts;
-  const uint64_t per_slot = (((c.child_stride + 31) >> 5) + pts - 1) >> c.log_pts;
+  const int log_pts = c.log_pts < kLogPicks ? c.log_pts : kLogPicks, pts = 1 << log_pts;
+  const uint64_t per_slot = (((c.child_stride + 31) >> 5) + pts - 1) >> log_pts;
   for (uint64_t w = (uint64_t)blockIdx.x * W + wid; w < c.K * per_slot; w += (uint64_t)gridDim.x * W) {
     const uint64_t pos = w / per_slot, slot = b.order[pos];
-    const uint64_t total = b.st[slot].n_parents << c.log2C, chunk = ((w - pos * per_slot) << c.log_pts) + lane;
-    if (((w - pos * per_slot) << (c.log_pts + 5)) >= total || !b.desc[slot].tile || !b.desc[slot].chain.points) continue;
+    const uint64_t total = b.st[slot].n_parents << c.log2C, chunk = ((w - pos * per_slot) << log_pts) + lane;
+    if (((w - pos * per_slot) << (log_pts + 5)) >= total || !b.desc[slot].tile || !b.desc[slot].chain.points) continue;
     SampleArgs a;
     point_args(c, b, slot, a);
     const uint64_t cbase = slot * c.child_stride;
@@ -224,7 +228,7 @@ __global__ void __launch_bounds__(kPointThreads) batch_picks_kernel(const BatchC
     }
     __syncwarp();
     unsigned long long rejected = 0;
-    sample_tile(a, x64, x32, list_s + wid * 32, c.log_pts, p, cand, b.sbest + slot, b.st[slot].gub, rejected,
+    sample_tile(a, x64, x32, list_s + wid * 32, log_pts, p, cand, b.sbest + slot, b.st[slot].gub, rejected,
                 [&](const PointOf& o, double value) {
                   const uint64_t at = cbase + (o.k << c.log2C) + o.r;
                   b.cval[at] = value;
@@ -328,7 +332,8 @@ cudaError_t batch_tile_points(const BatchCfg& c, const BatchBufs& b, const Batch
   if (!c.tiles) return cudaSuccess;
   if (c.precision == CMN_PRECISION_FP32_LAZY) {
     batch_points_kernel<true><<<g.points, kPointThreads, points_smem(c, true), s>>>(c, b);
-    const uint64_t warps = c.K * ((((c.child_stride + 31) >> 5) + (1u << c.log_pts) - 1) >> c.log_pts);
+    const int lp = std::min(c.log_pts, kLogPicks);
+    const uint64_t warps = c.K * ((((c.child_stride + 31) >> 5) + (1u << lp) - 1) >> lp);
     const int grid = (int)std::min<uint64_t>((warps + 3) / 4, (uint64_t)g.picks);
     batch_picks_kernel<<<grid, kPointThreads, picks_smem(c), s>>>(c, b);
   } else {

@@ -84,8 +84,28 @@ __device__ __forceinline__ float chain32(const ChainTerm32* __restrict__ term, i
 {
   const uint4* __restrict__ w = reinterpret_cast<const uint4*>(term);
   float acc = 0.0f;
-#pragma unroll 2
-  for (int q = t0; q < t1; ++q) {
+  int q = t0;
+  // four plain terms at a time: their loads and products before the first add
+  for (; q + 4 <= t1; q += 4) {
+    uint4 t[4];
+    uint32_t special = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      t[u] = __ldg(w + q + u);
+      special |= t[u].y;
+    }
+    if ((special & (kT32Sub | kT32Raw | kT32Const)) == 0u) {
+      float e[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) e[u] = term_end<kUp>(t[u], x[(t[u].x & 0xffffu) * 32], x[(t[u].x >> 16) * 32]) + 0.0f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc = kUp ? __fadd_ru(acc, e[u]) : __fadd_rd(acc, e[u]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc = term_add<kUp>(acc, t[u], x[(t[u].x & 0xffffu) * 32], x[(t[u].x >> 16) * 32]);
+    }
+  }
+  for (; q < t1; ++q) {
     const uint4 t = __ldg(w + q);
     acc = term_add<kUp>(acc, t, x[(t.x & 0xffffu) * 32], x[(t.x >> 16) * 32]);
   }

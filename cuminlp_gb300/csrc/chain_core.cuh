@@ -244,23 +244,31 @@ __device__ __noinline__ double chain_lo_lanes(const Instr* __restrict__ prog, in
     if ((first.head & 7) == kOpLoadAcc) acc = (first.modes & 3) == kModeVar ? vars.var(first.a).lo : first.c;
     else acc = term_lo<kFused>(first, vars);  // initialising TERM
   }
+  // the next G terms are formed while the last ones are added
+  auto form = [&](int pc, double& p, double& c) {
+    p = 0.0;
+    c = 1.0;
+    if (!active || pc >= pc1) return;
+    const Instr cur = load_instr(prog, pc);
+    const int sub = cur.head >> 3;
+    const bool neg = (sub & kTermSub) != 0;
+    p = term_lo<kFused>(cur, vars);
+    if (fused_term<double, kFused>(sub)) c = neg ? -cur.c : cur.c;
+    else if (neg) p = -p;
+  };
+  double p, c;
+  form(pc0 + 1 + gl, p, c);
   for (int base = pc0 + 1; base < pc1; base += G) {
-    const int pc = base + gl;
-    double p = 0.0, c = 1.0;
-    if (active && pc < pc1) {
-      const Instr cur = load_instr(prog, pc);
-      const int sub = cur.head >> 3;
-      const bool neg = (sub & kTermSub) != 0;
-      p = term_lo<kFused>(cur, vars);
-      if (fused_term<double, kFused>(sub)) c = neg ? -cur.c : cur.c;
-      else if (neg) p = -p;
-    }
+    double pn, cn;
+    form(base + G + gl, pn, cn);
 #pragma unroll
     for (int j = 0; j < G; ++j) {
       const double pj = __shfl_sync(0xffffffffu, p, j, G);
       if (kFused) acc = __fma_rd(__shfl_sync(0xffffffffu, c, j, G), pj, acc);
       else acc = __dadd_rd(acc, pj);
     }
+    p = pn;
+    c = cn;
   }
   return acc;
 }

@@ -166,11 +166,14 @@ __device__ __forceinline__ double point_chain_warp(const Instr* __restrict__ pro
   const int lane = threadIdx.x & 31;
   const Instr first = load_instr(prog, pc0);
   double acc = (first.head & 7) == kOpLoadAcc ? ((first.modes & 3) == kModeVar ? x[first.a] : first.c) : point_term(first, x);
+  // -0 adds nothing; the next 32 terms are formed while the last are added
+  auto form = [&](int pc) { return pc < pc1 ? point_term(load_instr(prog, pc), x) : -0.0; };
+  double p = form(pc0 + 1 + lane);
   for (int base = pc0 + 1; base < pc1; base += 32) {
-    const int pc = base + lane;
-    const double p = pc < pc1 ? point_term(load_instr(prog, pc), x) : -0.0;  // -0 adds nothing
+    const double pn = form(base + 32 + lane);
 #pragma unroll
     for (int j = 0; j < 32; ++j) acc = __dadd_rn(acc, __shfl_sync(0xffffffffu, p, j));
+    p = pn;
   }
   return acc;
 }
