@@ -753,9 +753,8 @@ static cmn_status candidate_role(cmn_role* r, const double* box, const uint64_t*
     if (!(std::fabs(box[2 * v]) <= kFilterMax) || !(std::fabs(box[2 * v + 1]) <= kFilterMax)) a.chain.points = 0;
   CK(launch_sample(a, r->grid, kEvalThreads, r->stream));
   Cand* best = r->d_block_best + r->grid;
-  CK(launch_reduce_cand(r->d_block_best, r->grid, best, r->stream));
-  CK(launch_witness(best, plo, phi, 1, pi, sp, 64, r->p->d_kinds, a.n_vars, r->S, salt, nullptr, exact, nullptr,
-                    r->d_point, r->stream));
+  const WitnessArgs w = {plo, phi, 1, pi, sp, 64, r->p->d_kinds, a.n_vars, r->S, salt, nullptr, exact, r->d_point};
+  CK(launch_candidate(r->d_block_best, r->grid, best, w, Incumbent{}, r->stream));
   CK(cudaMemcpyAsync(r->h_cand, best, sizeof(Cand), cudaMemcpyDeviceToHost, r->stream));
   CK(cudaMemcpyAsync(r->h_point, r->d_point, a.n_vars * sizeof(double), cudaMemcpyDeviceToHost, r->stream));
   CK(cudaStreamSynchronize(r->stream));

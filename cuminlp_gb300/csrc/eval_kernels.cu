@@ -876,45 +876,57 @@ __global__ void __launch_bounds__(kEvalThreads) sample_screen_kernel(const Sampl
   }
 }
 
-// Final ArgMin over the per-block candidates (one block).
-__global__ void reduce_cand_kernel(const Cand* __restrict__ block_best, int n, Cand* __restrict__ out)
+// One block: the ArgMin over the per-block candidates, the solver's incumbent
+// update (Incumbent::gub set), and the witness: the point the sampler (or the
+// exact grid) drew for the candidate's parent and element.  As three kernels
+// these cost an iteration of a small solve three launches of 2-7 us each.
+__global__ void __launch_bounds__(256) candidate_kernel(const Cand* __restrict__ block_best, int n, Cand* __restrict__ out,
+                                                        const WitnessArgs w, const Incumbent inc)
 {
+  __shared__ Cand best_s;
+  __shared__ int write_s;
+  if (inc.done != nullptr && *inc.done) return;
   Cand best = {INFINITY, 0xffffffffu, 0, ~0ULL};
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const Cand c = block_best[i];
     if (cand_less(c, best)) best = c;
   }
   best = block_min_cand(best);
-  if (threadIdx.x == 0) *out = best;
-}
-
-// Witness of a candidate: the point the sampler (or the exact grid) drew
-// for (parent k, element e).  One thread per variable.
-__global__ void witness_kernel(const Cand* __restrict__ cand, const double* __restrict__ plo,
-                               const double* __restrict__ phi, uint64_t pstride, const ParentInfo* __restrict__ pinfo,
-                               const SlotPlan* __restrict__ slots, int max_slots, const int32_t* __restrict__ kinds,
-                               int n_vars, uint64_t S, uint64_t salt, const uint64_t* __restrict__ salt_base_dev,
-                               int exact, const uint32_t* __restrict__ write_flag, double* __restrict__ out)
-{
-  if (write_flag != nullptr && *write_flag == 0) return;
-  const Cand c = *cand;
+  if (threadIdx.x == 0) {
+    *out = best;
+    best_s = best;
+    write_s = 1;
+    if (inc.gub != nullptr) {
+      const bool improved = best.value < DBL_MAX && best.value < *inc.gub;
+      *inc.improved = improved ? 1u : 0u;
+      if (improved) {
+        *inc.gub = best.value;
+        *inc.best = best;
+        *inc.have_best = 1;
+      }
+      write_s = improved ? 1 : 0;
+    }
+  }
+  __syncthreads();
+  if (!write_s) return;
+  const Cand c = best_s;
   const bool found = c.value < DBL_MAX;
   const uint64_t k = c.k;
-  bool fathom = exact != 0;
-  if (pinfo && found) fathom = fathom || pinfo[k].fathom;
-  const uint64_t SS = fathom ? 1 : S;
+  bool fathom = w.exact != 0;
+  if (w.pinfo && found) fathom = fathom || w.pinfo[k].fathom;
+  const uint64_t SS = fathom ? 1 : w.S;
   const uint64_t r = found ? c.e / SS : 0, i = found ? c.e % SS : 0;
-  const uint64_t sl = salt_base_dev ? *salt_base_dev + k + 1 : salt;
-  for (int v = threadIdx.x + blockIdx.x * blockDim.x; v < n_vars; v += blockDim.x * gridDim.x) {
+  const uint64_t sl = w.salt_base_dev ? *w.salt_base_dev + k + 1 : w.salt;
+  for (int v = threadIdx.x; v < w.n_vars; v += blockDim.x) {
     if (!found) {
-      out[v] = __longlong_as_double(0x7ff8000000000000LL);
+      w.point[v] = __longlong_as_double(0x7ff8000000000000LL);
       continue;
     }
-    double lo = plo[(uint64_t)v * pstride + k];
-    double hi = phi[(uint64_t)v * pstride + k];
-    if (pinfo) {
-      const SlotPlan* sp = slots + k * (uint64_t)max_slots;
-      const uint32_t count = pinfo[k].count;
+    double lo = w.plo[(uint64_t)v * w.pstride + k];
+    double hi = w.phi[(uint64_t)v * w.pstride + k];
+    if (w.pinfo) {
+      const SlotPlan* sp = w.slots + k * (uint64_t)w.max_slots;
+      const uint32_t count = w.pinfo[k].count;
       for (uint32_t j = 0; j < count; ++j) {
         if (sp[j].vid == (uint32_t)v) {
           const uint64_t part = slot_part(r, sp[j]);
@@ -923,7 +935,7 @@ __global__ void witness_kernel(const Cand* __restrict__ cand, const double* __re
         }
       }
     }
-    out[v] = fathom ? lo : sample_value(kinds[v] != 0, lo, hi, (uint64_t)v, i, r, sl);
+    w.point[v] = fathom ? lo : sample_value(w.kinds[v] != 0, lo, hi, (uint64_t)v, i, r, sl);
   }
 }
 
@@ -1118,21 +1130,10 @@ cudaError_t launch_sample(const SampleArgs& a, int grid, int threads, cudaStream
   return cudaGetLastError();
 }
 
-cudaError_t launch_reduce_cand(const Cand* block_best, int n, Cand* out, cudaStream_t s)
+cudaError_t launch_candidate(const Cand* block_best, int n, Cand* out, const WitnessArgs& w, const Incumbent& inc,
+                             cudaStream_t s)
 {
-  reduce_cand_kernel<<<1, 1024, 0, s>>>(block_best, n, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_witness(const Cand* cand, const double* plo, const double* phi, uint64_t pstride,
-                           const ParentInfo* pinfo, const SlotPlan* slots, int max_slots, const int32_t* kinds,
-                           int n_vars, uint64_t S, uint64_t salt, const uint64_t* salt_base_dev, int exact,
-                           const uint32_t* write_flag, double* out, cudaStream_t s)
-{
-  const int threads = 128;
-  const int grid = (n_vars + threads - 1) / threads;
-  witness_kernel<<<grid, threads, 0, s>>>(cand, plo, phi, pstride, pinfo, slots, max_slots, kinds, n_vars, S, salt,
-                                          salt_base_dev, exact, write_flag, out);
+  candidate_kernel<<<1, 256, 0, s>>>(block_best, n, out, w, inc);
   return cudaGetLastError();
 }
 

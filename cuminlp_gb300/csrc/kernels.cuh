@@ -200,4 +200,31 @@ struct SampleArgs {
   ChainTab chain;
 };
 
+// What a candidate's point is drawn from (candidate_kernel).
+struct WitnessArgs {
+  const double* plo;  // parent planes, as SampleArgs
+  const double* phi;
+  uint64_t pstride;
+  const ParentInfo* pinfo;
+  const SlotPlan* slots;
+  int max_slots;
+  const int32_t* kinds;
+  int n_vars;
+  uint64_t S;
+  uint64_t salt;  // as SampleArgs
+  const uint64_t* salt_base_dev;
+  int exact;
+  double* point;
+};
+
+// The solver's incumbent: the witness is written only when the candidate
+// improves it (gub null: always).
+struct Incumbent {
+  const uint32_t* done;
+  double* gub;
+  Cand* best;
+  uint32_t* have_best;
+  uint32_t* improved;
+};
+
 }  // namespace cmn

@@ -67,11 +67,8 @@ size_t inc_child_smem_bytes(int max_slots, int threads);
 // the lazy form's FP32 sample screen (SampleArgs::cbest out, prog = the
 // FP32 point program)
 cudaError_t launch_sample_screen(const SampleArgs& a, int grid, int threads, cudaStream_t s);
-cudaError_t launch_reduce_cand(const Cand* block_best, int n, Cand* out, cudaStream_t s);
-cudaError_t launch_witness(const Cand* cand, const double* plo, const double* phi, uint64_t pstride,
-                           const ParentInfo* pinfo, const SlotPlan* slots, int max_slots, const int32_t* kinds,
-                           int n_vars, uint64_t S, uint64_t salt, const uint64_t* salt_base_dev, int exact,
-                           const uint32_t* write_flag, double* out, cudaStream_t s);
+cudaError_t launch_candidate(const Cand* block_best, int n, Cand* out, const WitnessArgs& w, const Incumbent& inc,
+                             cudaStream_t s);
 
 // Largest dynamic shared memory a block may use on this device.
 int max_dynamic_smem();

@@ -172,10 +172,13 @@ extern "C" cmn_status cmn_sample_noalloc(const cmn_problem* p, const uint8_t* sl
   a.g_max = p->prog.group_max;
   a.capacity = (uint64_t)grid * threads;
   a.lg_min = lg_min;
+  a.chain = p->chain();
+  for (int64_t v = 0; v < n; ++v)  // as the sampler role: a box outside the filters' range takes the interpreter
+    if (!(std::fabs(box[2 * v]) <= kFilterMax) || !(std::fabs(box[2 * v + 1]) <= kFilterMax)) a.chain.points = 0;
   NA_CK(launch_sample(a, grid, threads, s));
-  NA_CK(launch_reduce_cand(d_blocks, grid, d_result, s));
-  NA_CK(launch_witness(d_result, d_box, d_box + 1, 2, &d_slots->info, d_slots->slots, 64, p->d_kinds, (int)n,
-                       sample_points, salt, nullptr, 0, nullptr, d_point, s));
+  const WitnessArgs w = {d_box, d_box + 1, 2, &d_slots->info, d_slots->slots, 64, p->d_kinds, (int)n, sample_points,
+                         salt, nullptr, 0, d_point};
+  NA_CK(launch_candidate(d_blocks, grid, d_result, w, Incumbent{}, s));
   Cand result;
   NA_CK(cudaMemcpyAsync(&result, d_result, sizeof(Cand), cudaMemcpyDeviceToHost, s));
   NA_CK(cudaMemcpyAsync(point, d_point, 8 * (size_t)n, cudaMemcpyDeviceToHost, s));

@@ -17,7 +17,7 @@ constexpr int kScanBlock = 512;  // threads per block of the compaction kernels
 constexpr int kScanItems = 8;    // items per thread
 constexpr int kScanTile = kScanBlock * kScanItems;
 constexpr int kHistUnroll = 8;   // entries per lane in flight in the radix histogram
-constexpr int kPickThreads = kRadixBins / 2;  // two bins per thread
+constexpr int kHistThreads = 256;  // threads of a radix histogram block
 
 constexpr uint8_t kSelAlive = 0;
 constexpr uint8_t kSelParent = 1;
@@ -83,6 +83,7 @@ struct SolverDev {
   uint32_t have_best;
   uint32_t improved;
   uint32_t error;
+  uint32_t ticket;         // blocks of the running histogram pass that are done
   Cand best;
   cmn_counters counters;
 };

@@ -157,7 +157,7 @@ __device__ __forceinline__ bool target_live(const RadixState& r)
   return r.active && !r.settled && r.bits_left != 0;
 }
 
-__global__ void radix_init_kernel(const SolverCfg cfg, const SolverBufs b, int which)
+__device__ void radix_init(const SolverCfg& cfg, const SolverBufs& b, int which)
 {
   SolverDev* d = b.dev;
   for (int t = 0; t < n_targets(which); ++t) {
@@ -192,12 +192,76 @@ __global__ void radix_init_kernel(const SolverCfg cfg, const SolverBufs b, int w
   }
 }
 
+__global__ void radix_init_kernel(const SolverCfg cfg, const SolverBufs b, int which) { radix_init(cfg, b, which); }
+
+// Picks the digit whose bin holds the k-th entry: a scan over the bins by one
+// block of kHistThreads. When the entries up to and including that bin are
+// exactly k, the bin is taken whole and the search stops.
+__device__ void radix_pick(const SolverBufs& b, RadixState* rs)
+{
+  constexpr int kPer = kRadixBins / kHistThreads;
+  __shared__ uint64_t warp_sum[kHistThreads / 32];
+  __shared__ int pick_d;
+  __shared__ uint64_t pick_cum, pick_cnt;
+  const int bits = rs->bits_left < (uint32_t)kRadixBits ? (int)rs->bits_left : kRadixBits;
+  const int shift = (int)rs->bits_left - bits;
+  const int nb = 1 << bits;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  uint32_t c[kPer];
+  uint64_t x = 0;
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    c[e] = t * kPer + e < nb ? __ldcg(&rs->hist[t * kPer + e]) : 0u;
+    x += c[e];
+  }
+  const uint64_t own = x;
+  if (t == 0) pick_d = -1;
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint64_t y = __shfl_up_sync(0xffffffffu, x, off);
+    if (lane >= off) x += y;
+  }
+  if (lane == 31) warp_sum[wid] = x;
+  __syncthreads();
+  uint64_t run = x - own;
+  for (int w = 0; w < wid; ++w) run += warp_sum[w];
+  const uint64_t k = rs->k;
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    if (run < k && k <= run + c[e]) {  // exactly one bin holds the k-th entry
+      pick_d = t * kPer + e;
+      pick_cum = run;
+      pick_cnt = c[e];
+    }
+    run += c[e];
+    if (t * kPer + e < nb) rs->hist[t * kPer + e] = 0;
+  }
+  __syncthreads();
+  if (t == 0) {
+    if (pick_d < 0) {  // fewer entries in the bucket than its rank: never expected
+      b.dev->error = 1;
+      rs->settled = 1;
+      rs->rank = 0;
+    } else {
+      rs->less += pick_cum;
+      rs->k = k - pick_cum;
+      rs->prefix |= (uint64_t)pick_d << shift;
+      rs->mask |= ((uint64_t)(nb - 1)) << shift;
+      rs->bits_left = (uint32_t)shift;
+      if (pick_cum + pick_cnt == k) {
+        rs->settled = 1;
+        rs->rank = 0;
+      }
+    }
+  }
+  __syncthreads();
+}
+
 // One digit's histogram per live target over the entries inside its
 // bucket, in one read of the keys. Each thread counts a run of equal bins
 // in registers and adds it to the block's shared histogram only when the
 // bin changes: converging lower bounds share most leading digits, so a pass
 // makes few shared-memory atomics instead of one per entry on one address.
-__global__ void radix_hist_kernel(const SolverCfg cfg, const SolverBufs b, int which)
+__global__ void __launch_bounds__(kHistThreads) radix_hist_kernel(const SolverCfg cfg, const SolverBufs b, int which)
 {
   __shared__ uint32_t h[2][kRadixBins];
   const int T = n_targets(which);
@@ -220,7 +284,6 @@ __global__ void radix_hist_kernel(const SolverCfg cfg, const SolverBufs b, int w
   const bool same = go[0] && go[1] && prefix[0] == prefix[1] && mask[0] == mask[1] && shift[0] == shift[1];
   const bool count1 = go[1] && !same;
   const uint64_t n = rs_n(b.dev, which);
-  if ((uint64_t)blockIdx.x * blockDim.x >= n) return;
   for (int t = 0; t < 2; ++t)
     for (int i = threadIdx.x; i < kRadixBins; i += blockDim.x) h[t][i] = 0;
   __syncthreads();
@@ -268,77 +331,19 @@ __global__ void radix_hist_kernel(const SolverCfg cfg, const SolverBufs b, int w
     for (int i = threadIdx.x; i < nb[t]; i += blockDim.x)
       if (src[i]) atomicAdd(&b.radix[t].hist[i], src[i]);
   }
+  // the last block to add its counts picks the digits: every block takes one
+  // ticket, and none waits
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&b.dev->ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int t = 0; t < T; ++t)
+    if (go[t]) radix_pick(b, b.radix + t);
+  if (threadIdx.x == 0) b.dev->ticket = 0;
   (void)cfg;
-}
-
-// Picks the digit whose bin holds the k-th entry: a block scan over the
-// bins (two per thread); block t serves target t. When the entries up to
-// and including that bin are exactly k, the bin is taken whole and the
-// search stops.
-__global__ void __launch_bounds__(kPickThreads) radix_pick_kernel(const SolverBufs b)
-{
-  __shared__ uint64_t warp_sum[kPickThreads / 32];
-  __shared__ int pick_d;
-  __shared__ uint64_t pick_cum, pick_cnt;
-  RadixState* rs = b.radix + blockIdx.x;
-  if (!target_live(*rs)) return;
-  const int bits = rs->bits_left < (uint32_t)kRadixBits ? (int)rs->bits_left : kRadixBits;
-  const int shift = (int)rs->bits_left - bits;
-  const int nb = 1 << bits;
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  const int b0 = 2 * t;
-  const uint32_t c0 = b0 < nb ? rs->hist[b0] : 0u;
-  const uint32_t c1 = b0 + 1 < nb ? rs->hist[b0 + 1] : 0u;
-  if (t == 0) pick_d = -1;
-  uint64_t x = (uint64_t)c0 + c1;
-  for (int off = 1; off < 32; off <<= 1) {
-    const uint64_t y = __shfl_up_sync(0xffffffffu, x, off);
-    if (lane >= off) x += y;
-  }
-  if (lane == 31) warp_sum[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    uint64_t s = lane < kPickThreads / 32 ? warp_sum[lane] : 0;
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint64_t y = __shfl_up_sync(0xffffffffu, s, off);
-      if (lane >= off) s += y;
-    }
-    if (lane < kPickThreads / 32) warp_sum[lane] = s;  // inclusive
-  }
-  __syncthreads();
-  const uint64_t incl = x + (wid > 0 ? warp_sum[wid - 1] : 0);
-  const uint64_t excl = incl - c0 - c1;
-  const uint64_t k = rs->k;
-  if (excl < k && k <= incl) {  // exactly one thread holds the k-th entry
-    if (excl + c0 >= k) {
-      pick_d = b0;
-      pick_cum = excl;
-      pick_cnt = c0;
-    } else {
-      pick_d = b0 + 1;
-      pick_cum = excl + c0;
-      pick_cnt = c1;
-    }
-  }
-  __syncthreads();
-  if (b0 < nb) rs->hist[b0] = 0;
-  if (b0 + 1 < nb) rs->hist[b0 + 1] = 0;
-  if (t != 0) return;
-  if (pick_d < 0) {  // fewer entries in the bucket than its rank: never expected
-    b.dev->error = 1;
-    rs->settled = 1;
-    rs->rank = 0;
-    return;
-  }
-  rs->less += pick_cum;
-  rs->k = k - pick_cum;
-  rs->prefix |= (uint64_t)pick_d << shift;
-  rs->mask |= ((uint64_t)(nb - 1)) << shift;
-  rs->bits_left = (uint32_t)shift;
-  if (pick_cum + pick_cnt == k) {
-    rs->settled = 1;
-    rs->rank = 0;
-  }
 }
 
 // ---------------------------------------------------------------------
@@ -528,16 +533,25 @@ __device__ __forceinline__ uint64_t block_min(uint64_t m)
   return acc;
 }
 
-// Exclusive scan of the tile counts of `*n_items` items (one block of 1024
-// threads); writes the total to *total_out when given.
-__global__ void __launch_bounds__(1024) scan_kernel(const uint32_t* __restrict__ counts,
-                                                    uint32_t* __restrict__ offsets,
+// Exclusive scan of the tile counts of `*n_items` items (a block of 1024
+// threads each); writes the total to *total_out when given.
+struct ScanArgs {
+  const uint32_t* counts;
+  uint32_t* offsets;
+  uint64_t* total_out;
+  const uint32_t* active;
+};
+
+__global__ void __launch_bounds__(1024) scan_kernel(const ScanArgs first, const ScanArgs second,
                                                     const uint64_t* __restrict__ n_items,
-                                                    uint64_t* __restrict__ total_out,
-                                                    const uint32_t* __restrict__ active,
                                                     const uint32_t* __restrict__ skip,
                                                     const uint32_t* __restrict__ done)
 {
+  const ScanArgs& a = blockIdx.x == 0 ? first : second;
+  const uint32_t* __restrict__ counts = a.counts;
+  uint32_t* __restrict__ offsets = a.offsets;
+  uint64_t* const total_out = a.total_out;
+  const uint32_t* const active = a.active;
   __shared__ uint64_t warp_sum[32];
   if (*done || (skip && *skip)) return;
   if (active && !*active) {
@@ -1022,12 +1036,31 @@ __global__ void __launch_bounds__(kScanBlock, 2) copy_pool_kernel(const SolverCf
   }
 }
 
-// stages the next iteration's parents listed by the pool move
+__device__ void finish_pool(const SolverCfg& cfg, const SolverBufs& b)
+{
+  SolverDev* d = b.dev;
+  // the survivors were moved to the other buffer: exactly the cap when
+  // evicting, otherwise every alive entry
+  const uint64_t expect = d->evict ? cfg.cap : d->new_size;
+  if (d->survivors != expect) d->error = 1;
+  d->free_top += d->extent - d->survivors;  // the parents' and the evicted slots
+  if (d->free_top + d->survivors != cfg.pstride) d->error = 1;
+  if (d->pre_count != d->pre_k) d->error = 1;
+  d->pre_valid = d->pre_k > 0 ? 1u : 0u;
+  d->pool_size = d->survivors;
+  d->parity = 1 - d->parity;
+  if (d->dropped_min_key != ~0ULL) d->dropped_lb_min = key_to_lb(d->dropped_min_key);
+  if (d->pool_size > d->counters.peak_frontier) d->counters.peak_frontier = d->pool_size;
+}
+
+// Stages the next iteration's parents listed by the pool move; one thread
+// closes the iteration (it writes nothing the staging reads).
 __global__ void stage_next_kernel(const SolverCfg cfg, const SolverBufs b)
 {
   const SolverDev* d = b.dev;
   if (d->done) return;
   const uint64_t n = d->pre_count < cfg.e_max ? d->pre_count : cfg.e_max;
+  if (blockIdx.x == 0 && threadIdx.x == 0) finish_pool(cfg, b);
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
     stage_parent(cfg, b, b.pslot[k], k);
 }
@@ -1270,67 +1303,70 @@ __global__ void lazy_fold_kernel(const SolverCfg cfg, const SolverBufs b)
 // ---------------------------------------------------------------------
 // incumbent, prune accounting, pool finish
 // ---------------------------------------------------------------------
-__global__ void incumbent_kernel(const SolverBufs b, const Cand* __restrict__ best)
+// One tile of children: counts of their verdicts (search/driver.hpp:319-350),
+// of the evaluations the form counts per valid child, the key range of the
+// children the pool takes, and the tile's kept children for the compaction.
+__global__ void __launch_bounds__(kScanBlock) prune_count_kernel(const SolverCfg cfg, const SolverBufs b)
 {
-  SolverDev* d = b.dev;
-  if (d->done) return;
-  const Cand c = *best;
-  d->improved = 0;
-  if (c.value < DBL_MAX && c.value < d->gub) {
-    d->gub = c.value;
-    d->best = c;
-    d->have_best = 1;
-    d->improved = 1;
-  }
-}
-
-// counts of this iteration's child verdicts (search/driver.hpp:319-350)
-__global__ void prune_count_kernel(const SolverCfg cfg, const SolverBufs b)
-{
+  const uint64_t t0 = tile_first();
   SolverDev* d = b.dev;
   if (d->done) return;
   const uint64_t n = d->n_children;
-  const double gub = d->gub;
-  unsigned long long dup = 0, inf = 0, dom = 0, kept = 0, sampled = 0;
-  uint64_t mkey = ~0ULL, xkey = 0;  // key range of the children the pool takes
-  for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
+  if ((uint64_t)blockIdx.x * kScanTile >= n) return;
+  const uint64_t gub = dbits(d->gub);
+  uint32_t dup = 0, inf = 0, dom = 0, kept = 0, sampled = 0, valid = 0, entries = 0;
+  uint64_t mkey = ~0ULL, xkey = 0;
+#pragma unroll
+  for (int j = 0; j < kScanItems; ++j) {
+    const uint64_t g = tile_item(t0, j);
+    if (g >= n) continue;
     const uint8_t s = b.cstate[g];
     if (s == kChildNone) continue;
     if (cfg.sample_all || s == kChildEligible) ++sampled;
-    if (s == kChildDuplicate) ++dup;
-    else if (s == kChildInfeasible) ++inf;
-    else if (s == kChildDominated || bits_lt(dbits(gub), dbits(b.clb[g]))) ++dom;
-    else ++kept;
+    if (s == kChildDuplicate) {
+      ++dup;
+      continue;
+    }
+    ++valid;
+    if (s == kChildInfeasible) {
+      ++inf;
+      continue;
+    }
+    const uint64_t lb = dbits(b.clb[g]);
+    const bool keep = s != kChildDominated && !bits_lt(gub, lb);
+    if (keep) ++kept;
+    else ++dom;
+    if (keep && s == kChildEligible) ++entries;  // KeptChild
     if (s == kChildEligible) {  // a superset of the kept children
-      const uint64_t k = lb_key(b.clb[g]);
+      const uint64_t k = bits_key(lb);
       mkey = k < mkey ? k : mkey;
       xkey = k > xkey ? k : xkey;
     }
   }
-  unsigned long long c[5] = {dup, inf, dom, kept, sampled};
+  const int mine = tile_count((int)entries);
+  unsigned long long c[6] = {dup, inf, dom, kept, sampled, valid};
   block_sum(c);
   mkey = block_min(mkey);
   xkey = block_max(xkey);
-  if (threadIdx.x == 0) {
-    if (mkey != ~0ULL) atomicMin((unsigned long long*)&d->child_min_key, (unsigned long long)mkey);
-    if (xkey != 0) atomicMax((unsigned long long*)&d->child_max_key, (unsigned long long)xkey);
-    if (c[0]) atomicAdd((unsigned long long*)&d->counters.pruned_duplicate, c[0]);
-    if (c[1]) atomicAdd((unsigned long long*)&d->counters.pruned_infeasible, c[1]);
-    if (c[2]) atomicAdd((unsigned long long*)&d->counters.pruned_dominated, c[2]);
-    if (c[3]) atomicAdd((unsigned long long*)&d->counters.enqueued, c[3]);
-    if (c[4]) atomicAdd((unsigned long long*)&d->counters.sampled, c[4] * cfg.S);
-  }
+  if (threadIdx.x != 0) return;
+  b.block_counts[blockIdx.x] = (uint32_t)mine;
+  if (mkey != ~0ULL) atomicMin((unsigned long long*)&d->child_min_key, (unsigned long long)mkey);
+  if (xkey != 0) atomicMax((unsigned long long*)&d->child_max_key, (unsigned long long)xkey);
+  if (c[0]) atomicAdd((unsigned long long*)&d->counters.pruned_duplicate, c[0]);
+  if (c[1]) atomicAdd((unsigned long long*)&d->counters.pruned_infeasible, c[1]);
+  if (c[2]) atomicAdd((unsigned long long*)&d->counters.pruned_dominated, c[2]);
+  if (c[3]) atomicAdd((unsigned long long*)&d->counters.enqueued, c[3]);
+  if (c[4]) atomicAdd((unsigned long long*)&d->counters.sampled, c[4] * cfg.S);
+  if (c[5] && cfg.precision == CMN_PRECISION_FP64) atomicAdd((unsigned long long*)&d->counters.certified_fp64, c[5]);
+  if (c[5] && cfg.precision == CMN_PRECISION_FP32_LAZY) atomicAdd((unsigned long long*)&d->counters.screened_fp32, c[5]);
 }
 
-// FP64 evaluations of this iteration: every non-duplicate child in FP64
-// mode, the certify list in the screened mode.
+// The screen's tallies: children bounded, and excluded by the verdicts.
 __global__ void eval_count_kernel(const SolverCfg cfg, const SolverBufs b)
 {
   SolverDev* d = b.dev;
   if (d->done) return;
   const uint64_t n = d->n_children;
-  const bool fp32 = cfg.precision == CMN_PRECISION_FP32_SCREEN;
-  const bool lazy = cfg.precision == CMN_PRECISION_FP32_LAZY;
   unsigned long long valid = 0, excluded = 0;
   for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (uint64_t)gridDim.x * blockDim.x) {
     const uint8_t s = b.cstate[g];
@@ -1343,9 +1379,9 @@ __global__ void eval_count_kernel(const SolverCfg cfg, const SolverBufs b)
   if (threadIdx.x == 0) {
     if (c[0]) atomicAdd((unsigned long long*)&d->iter_valid, c[0]);
     if (c[1]) atomicAdd((unsigned long long*)&d->iter_excluded, c[1]);
-    if (c[0] && ((fp32 && d->use_screen) || lazy)) atomicAdd((unsigned long long*)&d->counters.screened_fp32, c[0]);
-    if (c[0] && !fp32 && !lazy) atomicAdd((unsigned long long*)&d->counters.certified_fp64, c[0]);
+    if (c[0] && d->use_screen) atomicAdd((unsigned long long*)&d->counters.screened_fp32, c[0]);
   }
+  (void)cfg;
 }
 
 // The screen stays on while it excludes at least a quarter of the children
@@ -1358,19 +1394,14 @@ __global__ void screen_policy_kernel(const SolverCfg cfg, const SolverBufs b)
   const uint64_t v = d->iter_valid;
   const uint64_t x = d->use_screen ? v - d->certify_count : d->iter_excluded;
   if (v > 0) d->use_screen = (x * 4 >= v) ? 1 : 0;
-}
-
-__global__ void certify_count_kernel(const SolverBufs b)
-{
-  SolverDev* d = b.dev;
-  if (d->done) return;
   d->counters.certified_fp64 += d->certify_count;
 }
 
-__global__ void size_kernel(const SolverCfg cfg, const SolverBufs b)
+__device__ void size_pool(const SolverCfg& cfg, const SolverBufs& b)
 {
   SolverDev* d = b.dev;
-  if (d->done) return;
+  // lazy form: the band's FP64 pass
+  if (cfg.precision == CMN_PRECISION_FP32_LAZY) d->counters.certified_fp64 += d->certify_count;
   d->remaining = d->pool_size - d->n_parents;
   d->new_size = d->remaining + d->kept;
   d->extent = d->pool_size + d->kept;
@@ -1388,22 +1419,12 @@ __global__ void size_kernel(const SolverCfg cfg, const SolverBufs b)
   d->pool_max_key = 0;
 }
 
-__global__ void finish_kernel(const SolverCfg cfg, const SolverBufs b)
+// Sizes of the rebuilt pool, and the start of its select (one block).
+__global__ void size_kernel(const SolverCfg cfg, const SolverBufs b)
 {
-  SolverDev* d = b.dev;
-  if (d->done) return;
-  // the survivors were moved to the other buffer: exactly the cap when
-  // evicting, otherwise every alive entry
-  const uint64_t expect = d->evict ? cfg.cap : d->new_size;
-  if (d->survivors != expect) d->error = 1;
-  d->free_top += d->extent - d->survivors;  // the parents' and the evicted slots
-  if (d->free_top + d->survivors != cfg.pstride) d->error = 1;
-  if (d->pre_count != d->pre_k) d->error = 1;
-  d->pre_valid = d->pre_k > 0 ? 1u : 0u;
-  d->pool_size = d->survivors;
-  d->parity = 1 - d->parity;
-  if (d->dropped_min_key != ~0ULL) d->dropped_lb_min = key_to_lb(d->dropped_min_key);
-  if (d->pool_size > d->counters.peak_frontier) d->counters.peak_frontier = d->pool_size;
+  if (threadIdx.x == 0 && !b.dev->done) size_pool(cfg, b);
+  __syncthreads();
+  radix_init(cfg, b, 1);
 }
 
 __global__ void pool_min_kernel(const SolverBufs b, uint64_t* viable_out)
@@ -1442,7 +1463,8 @@ static int tiles(uint64_t max_items) { return (int)((max_items + kScanTile - 1) 
 static void scan(const SolverBufs& b, const uint32_t* counts, uint32_t* offsets, const uint64_t* n_items_dev,
                  uint64_t* total_dev, const uint32_t* active, const uint32_t* skip, cudaStream_t s)
 {
-  scan_kernel<<<1, 1024, 0, s>>>(counts, offsets, n_items_dev, total_dev, active, skip, &b.dev->done);
+  const ScanArgs a = {counts, offsets, total_dev, active};
+  scan_kernel<<<1, 1024, 0, s>>>(a, a, n_items_dev, skip, &b.dev->done);
 }
 
 template <class P>
@@ -1463,25 +1485,25 @@ static void scatter(const P& pred, const Op& op, uint64_t max_items, cudaStream_
 // staged them); which = 1: the cap and the next iteration's parents
 static void radix_select(const SolverCfg& cfg, const SolverBufs& b, int which, uint64_t max_items, cudaStream_t s)
 {
-  const int T = which == 0 ? 1 : 2;
   const uint32_t* skip = which == 0 ? &b.dev->skip_select : nullptr;
-  radix_init_kernel<<<1, 256, 0, s>>>(cfg, b, which);
-  const int grid = (int)std::min<uint64_t>((max_items + 255) / 256, 4096);
+  if (which == 0) radix_init_kernel<<<1, 256, 0, s>>>(cfg, b, which);  // which = 1: size_kernel
+  const int grid = (int)std::min<uint64_t>((max_items + kHistThreads * kHistUnroll - 1) / (kHistThreads * kHistUnroll),
+                                           (uint64_t)sm_count() * 8);
   // digits of up to 11 bits from below the keys' common leading bits;
   // the passes after the buckets settle or the bits run out return at once
-  for (int p = 0; p < (64 + kRadixBits - 1) / kRadixBits; ++p) {
-    radix_hist_kernel<<<grid, 256, 0, s>>>(cfg, b, which);
-    radix_pick_kernel<<<T, kPickThreads, 0, s>>>(b);
-  }
+  for (int p = 0; p < (64 + kRadixBits - 1) / kRadixBits; ++p) radix_hist_kernel<<<grid, kHistThreads, 0, s>>>(cfg, b, which);
   // ranks among entries inside the threshold buckets, then the marks with
   // the tile counts of the entries the next compactions move
   const uint64_t* n_dev = which == 0 ? &b.dev->pool_size : &b.dev->extent;
+  const int scans = which == 0 ? 1 : 2;
   eq_count_kernel<<<tiles(max_items), kScanBlock, 0, s>>>(cfg, b, which);
-  scan(b, b.block_counts, b.block_offsets, n_dev, nullptr, &b.radix[0].rank, skip, s);
-  if (which == 1) scan(b, b.block_counts2, b.block_offsets2, n_dev, nullptr, &b.radix[1].rank, nullptr, s);
+  scan_kernel<<<scans, 1024, 0, s>>>(ScanArgs{b.block_counts, b.block_offsets, nullptr, &b.radix[0].rank},
+                                     ScanArgs{b.block_counts2, b.block_offsets2, nullptr, &b.radix[1].rank}, n_dev, skip,
+                                     &b.dev->done);
   mark_kernel<<<tiles(max_items), kScanBlock, 0, s>>>(cfg, b, which);
-  scan(b, b.block_counts, b.block_offsets, n_dev, which == 0 ? nullptr : &b.dev->survivors, nullptr, skip, s);
-  if (which == 1) scan(b, b.block_counts2, b.block_offsets2, n_dev, &b.dev->pre_count, nullptr, nullptr, s);
+  scan_kernel<<<scans, 1024, 0, s>>>(
+      ScanArgs{b.block_counts, b.block_offsets, which == 0 ? nullptr : &b.dev->survivors, nullptr},
+      ScanArgs{b.block_counts2, b.block_offsets2, &b.dev->pre_count, nullptr}, n_dev, skip, &b.dev->done);
 }
 
 static void mark(const cudaEvent_t* marks, int i, cudaStream_t s)
@@ -1644,15 +1666,10 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     e = launch_eval(ea, 1, false, eval_grid, kEvalThreads, s);
     if (e != cudaSuccess) return e;
   }
-  {
+  if (cfg.precision == CMN_PRECISION_FP32_SCREEN) {
     const int grid = (int)std::min<uint64_t>((max_children + 255) / 256, 1024);
     eval_count_kernel<<<grid, 256, 0, s>>>(cfg, b);
-    if (cfg.precision == CMN_PRECISION_FP32_SCREEN) {
-      certify_count_kernel<<<1, 1, 0, s>>>(b);
-      screen_policy_kernel<<<1, 1, 0, s>>>(cfg, b);
-    } else if (cfg.precision == CMN_PRECISION_FP32_LAZY) {
-      certify_count_kernel<<<1, 1, 0, s>>>(b);
-    }
+    screen_policy_kernel<<<1, 1, 0, s>>>(cfg, b);
   }
   mark(marks, 2, s);
 
@@ -1700,23 +1717,19 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
   e = launch_sample(sa, sample_grid, kEvalThreads, s);
   if (e != cudaSuccess) return e;
   Cand* best = b.block_best + b.n_block_best - 1;  // last entry holds the result
-  e = launch_reduce_cand(b.block_best, sample_grid, best, s);
-  if (e != cudaSuccess) return e;
-  incumbent_kernel<<<1, 1, 0, s>>>(b, best);
-  e = launch_witness(best, b.plo, b.phi, cfg.e_max, b.pinfo, b.slots, cfg.max_slots, b.kinds, cfg.n_vars, cfg.S, 0,
-                     &b.dev->salt_base, 0, &b.dev->improved, b.best_point, s);
+  const WitnessArgs w = {b.plo, b.phi, cfg.e_max, b.pinfo, b.slots, cfg.max_slots, b.kinds, cfg.n_vars, cfg.S, 0,
+                         &b.dev->salt_base, 0, b.best_point};
+  e = launch_candidate(b.block_best, sample_grid, best, w,
+                       Incumbent{&b.dev->done, &b.dev->gub, &b.dev->best, &b.dev->have_best, &b.dev->improved}, s);
   if (e != cudaSuccess) return e;
   mark(marks, 3, s);
 
   // (5) prune with the new incumbent and rebuild the pool
-  {
-    const int grid = (int)std::min<uint64_t>((max_children + 255) / 256, 1024);
-    prune_count_kernel<<<grid, 256, 0, s>>>(cfg, b);
-  }
+  prune_count_kernel<<<tiles(max_children), kScanBlock, 0, s>>>(cfg, b);
   // the kept children go behind the pool in the current buffer; the
   // parents stay there as holes until the one compaction below
   KeptChild kept{b};
-  compact(kept, max_children, &b.dev->n_children, &b.dev->kept, b, s);
+  scan(b, b.block_counts, b.block_offsets, &b.dev->n_children, &b.dev->kept, nullptr, nullptr, s);
   scatter(kept, ListChild{b}, max_children, s, b);
   {
     const int grid = (int)std::min<uint64_t>((max_children + 255) / 256, 4096);
@@ -1724,7 +1737,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     else if (cfg.n_vars > 8) append_boxes_kernel<16><<<grid, 256, 0, s>>>(cfg, b);
     else append_children_kernel<<<grid, 256, 0, s>>>(cfg, b);
   }
-  size_kernel<<<1, 1, 0, s>>>(cfg, b);
+  size_kernel<<<1, 256, 0, s>>>(cfg, b);
 
   // (6) over the cap: keep the `cap` best alive entries, fold the rest into
   // the floor; then move every alive entry to the other buffer in order
@@ -1734,7 +1747,6 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     const int grid = (int)std::min<uint64_t>((cfg.e_max + 255) / 256, 1024);
     stage_next_kernel<<<grid, 256, 0, s>>>(cfg, b);
   }
-  finish_kernel<<<1, 1, 0, s>>>(cfg, b);
   mark(marks, 4, s);
   return cudaGetLastError();
 }
