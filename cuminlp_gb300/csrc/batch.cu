@@ -87,7 +87,7 @@ struct cmn_batch {
   std::vector<uint8_t> busy;
   std::vector<Clock::time_point> t_add;
   std::vector<double> elapsed_ms;  // add -> first step that saw it stopped
-  std::vector<void*> allocs;
+  void* slab = nullptr;  // every device array
   uint64_t alloc_bytes = 0;
   bool fresh = false;  // h_st matches the device: nothing enqueued since pull()
   int eval_grid = 1;
@@ -104,23 +104,10 @@ struct cmn_batch {
       if (ev) cudaEventDestroy(ev);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
-    for (void* a : allocs) cudaFree(a);
+    if (slab) cudaFree(slab);
     if (h_st) cudaFreeHost(h_st);
     if (stream) cudaStreamDestroy(stream);
     if (cur != device) cudaSetDevice(cur);
-  }
-
-  template <typename T>
-  cudaError_t alloc(T** ptr, size_t n)
-  {
-    *ptr = nullptr;
-    const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(ptr), bytes);
-    if (e == cudaSuccess) {
-      allocs.push_back(*ptr);
-      alloc_bytes += bytes;
-    }
-    return e;
   }
 
   cmn_status pull()
@@ -214,8 +201,10 @@ extern "C" cmn_status cmn_batch_create(const cmn_batch_config* config, cmn_batch
 
     BatchBufs& b = s->b;
     cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+    Slab slab;
     auto A = [&](auto** ptr, size_t count) {
-      if (e == cudaSuccess) e = s->alloc(ptr, count);
+      slab.add(ptr, count);
+      s->alloc_bytes += std::max<size_t>(count, 1) * sizeof(**ptr);
     };
     A(&b.desc, K);
     A(&b.st, K);
@@ -248,11 +237,10 @@ extern "C" cmn_status cmn_batch_create(const cmn_batch_config* config, cmn_batch
     A(&b.slots, K * c.e_max * (uint64_t)c.max_slots);
     EnumCand* ec = nullptr;
     BisCand* bc = nullptr;
-    A(&ec, K * c.e_max * nm);
-    A(&bc, K * c.e_max * nm);
-    b.enum_scratch = ec;
-    b.bis_scratch = bc;
-    A(&b.heap_scratch, K * c.e_max * nm);
+    const uint64_t policy = n_max > kPolicyLocal ? K * c.e_max * nm : 0;  // local memory below
+    A(&ec, policy);
+    A(&bc, policy);
+    A(&b.heap_scratch, policy);
     A(&b.clb, G);
     A(&b.cstate, G);
     A(&b.cval, G);
@@ -271,8 +259,11 @@ extern "C" cmn_status cmn_batch_create(const cmn_batch_config* config, cmn_batch
     A(&b.sbest, K);
     uint32_t* order = nullptr;
     A(&order, K);
-    b.order = order;
     A(&b.best_point, K * nm);
+    if (e == cudaSuccess) e = slab.alloc(&s->slab);
+    b.order = order;
+    b.enum_scratch = ec;
+    b.bis_scratch = bc;
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&s->h_st), sizeof(InstState) * K);
     if (e != cudaSuccess) {
       delete s;

@@ -25,10 +25,10 @@ __device__ __forceinline__ void slot_args(const BatchCfg& c, const BatchBufs& b,
 {
   const InstDesc& d = b.desc[slot];
   const InstState& st = b.st[slot];
+  a = {};  // what is not set below is off
   a.prog = d.prog64;
   a.prog_len = d.prog_len;
   a.n_vars = d.n_vars;
-  a.n_slots = 0;
   a.log2C = c.log2C;
   a.plo = b.plo + splane(c, slot, 0);
   a.phi = b.phi + splane(c, slot, 0);
@@ -39,15 +39,9 @@ __device__ __forceinline__ void slot_args(const BatchCfg& c, const BatchBufs& b,
   a.slots = b.slots + slot * c.e_max * c.max_slots;
   a.max_slots = c.max_slots;
   a.n_children = st.n_parents << c.log2C;
-  a.n_children_dev = nullptr;
   a.n_parents_dev = &st.n_parents;
-  a.list = nullptr;
-  a.list_count = nullptr;
   a.gub = &st.gub;
-  a.done = nullptr;
-  a.parent_lb = nullptr;
   a.out_lb = b.clb + slot * c.child_stride;
-  a.out_ub = nullptr;
   a.out_flag = b.cstate + slot * c.child_stride;
   a.chain = d.chain;
 }
@@ -56,10 +50,10 @@ __device__ __forceinline__ void point_args(const BatchCfg& c, const BatchBufs& b
 {
   const InstDesc& d = b.desc[slot];
   const InstState& st = b.st[slot];
+  a = {};  // what is not set below is off
   a.prog = d.prog64;
   a.prog_len = d.prog_len;
   a.n_vars = d.n_vars;
-  a.n_slots = 0;
   a.log2C = c.log2C;
   a.plo = b.plo + splane(c, slot, 0);
   a.phi = b.phi + splane(c, slot, 0);
@@ -71,9 +65,7 @@ __device__ __forceinline__ void point_args(const BatchCfg& c, const BatchBufs& b
   a.root_lb = d.root_lb;
   a.root_ub = d.root_ub;
   a.S = c.S;
-  a.salt = 0;
   a.salt_base_dev = &st.salt_base;
-  a.exact = 0;
   a.sample_all = c.sample_all;
   a.state = b.cstate + slot * c.child_stride;
   a.sched = d.sched;

@@ -1704,7 +1704,7 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
   batch_stage_kernel<<<(int)std::min<uint64_t>((np + 255) / 256, 8192), 256, 0, s>>>(c, b);
   const int bg = (int)((np + 127) / 128);
   if (c.n_max <= 32) batch_branch_kernel<32><<<bg, 128, 0, s>>>(c, b);
-  else if (c.n_max <= 64) batch_branch_kernel<64><<<bg, 128, 0, s>>>(c, b);
+  else if (c.n_max <= kPolicyLocal) batch_branch_kernel<kPolicyLocal><<<bg, 128, 0, s>>>(c, b);
   else batch_branch_kernel<0><<<bg, 128, 0, s>>>(c, b);
   batch_live_kernel<<<1, 1024, 0, s>>>(c, b);
   mark(marks, 1, s);

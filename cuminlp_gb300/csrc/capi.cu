@@ -111,22 +111,8 @@ cmn_problem::~cmn_problem()
 {
   int cur = 0;
   if (cudaGetDevice(&cur) == cudaSuccess && cur != device) cudaSetDevice(device);
-  dfree(d_prog64);
-  dfree(d_prog32);
-  dfree(d_prog32p);
-  dfree(d_kinds);
-  dfree(d_root_lb);
-  dfree(d_root_ub);
-  dfree(d_sched);
-  dfree(d_inc_seg);
-  dfree(d_inc_off);
-  dfree(d_inc_pcs);
-  dfree(d_chain_seg);
-  dfree(d_chain_term);
-  dfree(d_chain_term32);
-  dfree(d_chain_var32);
-  dfree(d_chain_var_off);
-  dfree(d_chain_term_pt);
+  dfree(d_tables);
+  dfree(d_ws);
   if (cur != device) cudaSetDevice(cur);
 }
 
@@ -156,36 +142,21 @@ extern "C" cmn_status cmn_problem_create(const cmn_problem_desc* desc, cmn_probl
       delete p;
       return fail(CMN_CUDA_ERROR, "no CUDA device");
     }
-    const size_t L = p->prog.code64.size();
-    const int64_t n = p->host.n_vars();
-    cudaError_t e = dalloc(&p->d_prog64, L);
-    if (e == cudaSuccess) e = dalloc(&p->d_prog32, L);
-    if (e == cudaSuccess) e = dalloc(&p->d_prog32p, L);
-    if (e == cudaSuccess) e = dalloc(&p->d_kinds, (size_t)n);
-    if (e == cudaSuccess) e = dalloc(&p->d_root_lb, (size_t)n);
-    if (e == cudaSuccess) e = dalloc(&p->d_root_ub, (size_t)n);
-    if (e == cudaSuccess && L) e = cudaMemcpy(p->d_prog64, p->prog.code64.data(), L * sizeof(Instr), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && L) e = cudaMemcpy(p->d_prog32, p->prog.code32.data(), L * sizeof(Instr), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && L)
-      e = cudaMemcpy(p->d_prog32p, p->prog.code32p.data(), L * sizeof(Instr), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-      e = cudaMemcpy(p->d_kinds, p->host.var_kinds.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-      e = cudaMemcpy(p->d_root_lb, p->host.var_lb.data(), n * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-      e = cudaMemcpy(p->d_root_ub, p->host.var_ub.data(), n * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !p->prog.sched.empty()) {
-      e = dalloc(&p->d_sched, p->prog.sched.size());
-      if (e == cudaSuccess)
-        e = cudaMemcpy(p->d_sched, p->prog.sched.data(), p->prog.sched.size() * sizeof(int32_t),
-                       cudaMemcpyHostToDevice);
-    }
-    if (e == cudaSuccess && p->prog.inc_ok) {
-      auto up = [&](auto** d, const auto& h) {
-        if (e == cudaSuccess) e = dalloc(d, std::max<size_t>(1, h.size()));
-        if (e == cudaSuccess && !h.empty())
-          e = cudaMemcpy(*d, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice);
-      };
+    // every table at its place in one host image, one allocation, one copy
+    Slab slab;
+    std::vector<std::pair<const void*, size_t>> src;
+    auto up = [&](auto** d, const auto& h) {
+      slab.add(d, h.size());
+      src.push_back({h.data(), h.size() * sizeof(h[0])});
+    };
+    up(&p->d_prog64, p->prog.code64);
+    up(&p->d_prog32, p->prog.code32);
+    up(&p->d_prog32p, p->prog.code32p);
+    up(&p->d_kinds, p->host.var_kinds);
+    up(&p->d_root_lb, p->host.var_lb);
+    up(&p->d_root_ub, p->host.var_ub);
+    if (!p->prog.sched.empty()) up(&p->d_sched, p->prog.sched);
+    if (p->prog.inc_ok) {
       up(&p->d_inc_seg, p->prog.inc_seg);
       up(&p->d_inc_off, p->prog.inc_off);
       up(&p->d_inc_pcs, p->prog.inc_pcs);
@@ -197,6 +168,16 @@ extern "C" cmn_status cmn_problem_create(const cmn_problem_desc* desc, cmn_probl
         up(&p->d_chain_var_off, p->prog.chain_var_off);
       }
       if (!p->prog.chain_term_pt.empty()) up(&p->d_chain_term_pt, p->prog.chain_term_pt);
+    }
+    cudaError_t e = slab.alloc(&p->d_tables);
+    if (e == cudaSuccess) {
+      std::vector<unsigned char> image(slab.bytes());
+      size_t at = 0;
+      for (const auto& t : src) {
+        if (t.second > 0) std::memcpy(image.data() + at, t.first, t.second);
+        at += (std::max<size_t>(t.second, 1) + 255) & ~(size_t)255;
+      }
+      e = cudaMemcpy(p->d_tables, image.data(), image.size(), cudaMemcpyHostToDevice);
     }
     if (e != cudaSuccess) {
       delete p;
@@ -387,11 +368,11 @@ struct cmn_role {
   uint8_t* d_feas = nullptr;
   double* d_lb = nullptr;
   Cand* d_block_best = nullptr;
-  double* d_point = nullptr;
   uint8_t* h_feas = nullptr;
   double* h_lb = nullptr;
   double* h_point = nullptr;
   Cand* h_cand = nullptr;
+  bool direct = false;  // the kernels write their results to the pinned buffers
   // aggregate bounds: 2k fold keys on the device and host, k results
   unsigned long long* d_agg = nullptr;
   unsigned long long* h_agg = nullptr;
@@ -407,12 +388,9 @@ struct cmn_role {
     if (h_agg) cudaFreeHost(h_agg);
     if (h_agg_out) cudaFreeHost(h_agg_out);
     dfree(d_stage);
-    dfree(d_feas);
     dfree(d_lb);
     dfree(d_block_best);
-    dfree(d_point);
     if (h_stage) cudaFreeHost(h_stage);
-    if (h_feas) cudaFreeHost(h_feas);
     if (h_lb) cudaFreeHost(h_lb);
     if (h_point) cudaFreeHost(h_point);
     if (h_cand) cudaFreeHost(h_cand);
@@ -420,6 +398,11 @@ struct cmn_role {
     if (p && cur != p->device) cudaSetDevice(cur);
   }
 };
+
+// Up to this many regions the verdicts go straight to pinned host memory, as
+// a candidate does: a device-to-host copy is a launch of its own, and a small
+// call is made of launches.
+constexpr uint64_t kDirectRegions = 1u << 14;
 
 static bool is_enum_kind(uint8_t k) { return k == CMN_SLOT_INTEGER_ENUMERATE || k == CMN_SLOT_BINARY_ENUMERATE; }
 
@@ -512,13 +495,14 @@ extern "C" cmn_status cmn_role_build(const cmn_problem* p, int32_t role, const u
         1, eval_kernel_occupancy(0, false, eval_smem_bytes(p->prog.n_slots, (int)slot_count, false, threads), threads));
     r->grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(blocks_needed, (uint64_t)sm_count() * occ));
     if (role == CMN_ROLE_BOUNDER) {
-      if (e == cudaSuccess) e = dalloc(&r->d_feas, n_regions);
-      if (e == cudaSuccess) e = dalloc(&r->d_lb, n_regions);
-      if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&r->h_feas), n_regions);
-      if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&r->h_lb), n_regions * sizeof(double));
+      // bounds, then feasibility, in one buffer on either side: one copy back
+      r->direct = n_regions <= kDirectRegions;
+      if (e == cudaSuccess) e = dalloc(&r->d_lb, n_regions + (n_regions + 7) / 8);
+      if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&r->h_lb), n_regions * 9);
+      r->d_feas = reinterpret_cast<uint8_t*>(r->d_lb + n_regions);
+      r->h_feas = reinterpret_cast<uint8_t*>(r->h_lb + n_regions);
     } else {
       if (e == cudaSuccess) e = dalloc(&r->d_block_best, (size_t)r->grid + 1);
-      if (e == cudaSuccess) e = dalloc(&r->d_point, (size_t)n);
       if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&r->h_point), n * sizeof(double));
       if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&r->h_cand), sizeof(Cand));
     }
@@ -621,9 +605,13 @@ extern "C" cmn_status cmn_bound(cmn_role* r, const double* box, const uint64_t* 
   a.sched = r->p->d_sched;
   a.g_max = r->p->prog.group_max;
   a.capacity = (uint64_t)r->grid * r->threads;
+  if (r->direct) {
+    a.out_lb = r->h_lb;
+    a.out_flag = r->h_feas;
+    a.flags = r->d_feas;
+  }
   CK(launch_eval(a, 0, false, r->grid, r->threads, r->stream));
-  CK(cudaMemcpyAsync(r->h_feas, r->d_feas, r->n_regions, cudaMemcpyDeviceToHost, r->stream));
-  CK(cudaMemcpyAsync(r->h_lb, r->d_lb, r->n_regions * sizeof(double), cudaMemcpyDeviceToHost, r->stream));
+  if (!r->direct) CK(cudaMemcpyAsync(r->h_lb, r->d_lb, r->n_regions * 9, cudaMemcpyDeviceToHost, r->stream));
   CK(cudaStreamSynchronize(r->stream));
   if (feasible) *feasible = r->h_feas;
   if (obj_lb) *obj_lb = r->h_lb;
@@ -762,11 +750,9 @@ static cmn_status candidate_role(cmn_role* r, const double* box, const uint64_t*
   for (int v = 0; v < a.n_vars; ++v)  // a box outside the filters' range takes the interpreter
     if (!(std::fabs(box[2 * v]) <= kFilterMax) || !(std::fabs(box[2 * v + 1]) <= kFilterMax)) a.chain.points = 0;
   CK(launch_sample(a, r->grid, kEvalThreads, r->stream));
-  Cand* best = r->d_block_best + r->grid;
-  const WitnessArgs w = {plo, phi, 1, pi, sp, 64, r->p->d_kinds, a.n_vars, r->S, salt, nullptr, exact, r->d_point};
-  CK(launch_candidate(r->d_block_best, r->grid, best, w, Incumbent{}, r->stream));
-  CK(cudaMemcpyAsync(r->h_cand, best, sizeof(Cand), cudaMemcpyDeviceToHost, r->stream));
-  CK(cudaMemcpyAsync(r->h_point, r->d_point, a.n_vars * sizeof(double), cudaMemcpyDeviceToHost, r->stream));
+  // the candidate and its point go straight to the pinned buffers
+  const WitnessArgs w = {plo, phi, 1, pi, sp, 64, r->p->d_kinds, a.n_vars, r->S, salt, nullptr, exact, r->h_point};
+  CK(launch_candidate(r->d_block_best, r->grid, r->h_cand, w, Incumbent{}, r->stream));
   CK(cudaStreamSynchronize(r->stream));
   const Cand c = *r->h_cand;
   out->found = c.value < DBL_MAX ? 1 : 0;
@@ -822,16 +808,35 @@ extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, co
   double* tmp = nullptr;
   uint8_t* tmpf = nullptr;
   uint64_t ps = stride;
+  std::unique_lock<std::mutex> ws(p->ws_mu, std::defer_lock);
+  unsigned char* own = nullptr;  // a staging buffer of this call alone
+  struct Release {
+    unsigned char*& p;
+    ~Release() { dfree(p); }
+  } release{own};
   if (!device_pointers) {
     ps = n_boxes;
     const size_t planes = (size_t)n * n_boxes;
-    CK(dalloc(&tmp, 2 * planes + 2 * n_boxes));
-    CK(dalloc(&tmpf, n_boxes));
-    for (int64_t v = 0; v < n; ++v) {
-      CK(cudaMemcpyAsync(tmp + v * n_boxes, lo + v * stride, n_boxes * sizeof(double), cudaMemcpyHostToDevice, s));
-      CK(cudaMemcpyAsync(tmp + planes + v * n_boxes, hi + v * stride, n_boxes * sizeof(double), cudaMemcpyHostToDevice,
-                         s));
+    const size_t bytes = (2 * planes + 2 * n_boxes) * sizeof(double) + n_boxes;
+    // the problem's kept workspace, unless the call is large or another
+    // thread is in it
+    if (bytes <= kEvalWorkspace && ws.try_lock()) {
+      if (p->ws_bytes < bytes) {
+        dfree(p->d_ws);
+        p->d_ws = nullptr;
+        p->ws_bytes = 0;
+        CK(dalloc(&p->d_ws, bytes));
+        p->ws_bytes = bytes;
+      }
+      tmp = reinterpret_cast<double*>(p->d_ws);
+    } else {
+      CK(dalloc(&own, bytes));
+      tmp = reinterpret_cast<double*>(own);
     }
+    tmpf = reinterpret_cast<uint8_t*>(tmp + 2 * planes + 2 * n_boxes);
+    const size_t row = n_boxes * sizeof(double);
+    CK(cudaMemcpy2DAsync(tmp, row, lo, stride * sizeof(double), row, (size_t)n, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpy2DAsync(tmp + planes, row, hi, stride * sizeof(double), row, (size_t)n, cudaMemcpyHostToDevice, s));
     dlo = tmp;
     dhi = tmp + planes;
     dlb = tmp + 2 * planes;
@@ -864,8 +869,6 @@ extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, co
   a.capacity = (uint64_t)sm_count() * occ * threads;
   cudaError_t e = launch_eval(a, 0, fp32, grid, threads, s);
   if (e != cudaSuccess) {
-    dfree(tmp);
-    dfree(tmpf);
     return fail(CMN_CUDA_ERROR, std::string("eval launch: ") + cudaGetErrorString(e));
   }
   if (!device_pointers) {
@@ -873,8 +876,6 @@ extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, co
     if (obj_ub) CK(cudaMemcpyAsync(obj_ub, dub, n_boxes * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(feasible, dfe, n_boxes, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    dfree(tmp);
-    dfree(tmpf);
   }
   return CMN_OK;
 }
@@ -1031,7 +1032,7 @@ struct cmn_solver {
   SolverDev* h_dev = nullptr;  // pinned mirror
   uint64_t* d_viable = nullptr;
   uint64_t* h_viable = nullptr;
-  std::vector<void*> allocs;
+  void* slab = nullptr;  // every device array
   int eval_grid = 1, sample_grid = 1;
   double elapsed_ms = 0;
   uint64_t launched = 0;
@@ -1054,19 +1055,11 @@ struct cmn_solver {
     if (graph) cudaGraphDestroy(graph);
     if (exec_steady) cudaGraphExecDestroy(exec_steady);
     if (graph_steady) cudaGraphDestroy(graph_steady);
-    for (void* a : allocs) cudaFree(a);
+    if (slab) cudaFree(slab);
     if (h_dev) cudaFreeHost(h_dev);
     if (h_viable) cudaFreeHost(h_viable);
     if (stream) cudaStreamDestroy(stream);
     if (p && cur != p->device) cudaSetDevice(cur);
-  }
-
-  template <typename T>
-  cudaError_t alloc(T** ptr, size_t n)
-  {
-    cudaError_t e = dalloc(ptr, n);
-    if (e == cudaSuccess) allocs.push_back(*ptr);
-    return e;
   }
 };
 
@@ -1173,9 +1166,8 @@ extern "C" cmn_status cmn_solver_create(const cmn_problem* p, const cmn_solve_op
 
     SolverBufs& b = s->b;
     cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
-    auto A = [&](auto** ptr, size_t count) {
-      if (e == cudaSuccess) e = s->alloc(ptr, count);
-    };
+    Slab slab;
+    auto A = [&](auto** ptr, size_t count) { slab.add(ptr, count); };
     A(&b.dev, 1);
     A(&b.radix, 2);
     for (int q = 0; q < 2; ++q) {
@@ -1214,11 +1206,11 @@ extern "C" cmn_status cmn_solver_create(const cmn_problem* p, const cmn_solve_op
     A(&b.slots, cfg.e_max * (size_t)cfg.max_slots);
     unsigned char* es = nullptr;
     unsigned char* bs = nullptr;
-    A(&es, cfg.e_max * (size_t)n * sizeof(EnumCand));
-    A(&bs, cfg.e_max * (size_t)n * sizeof(BisCand));
-    b.enum_scratch = es;
-    b.bis_scratch = bs;
-    A(&b.heap_scratch, cfg.e_max * (size_t)n);
+    // the branching policy keeps its scratch in local memory up to 64 variables
+    const size_t policy = n > kPolicyLocal ? cfg.e_max * (size_t)n : 0;
+    A(&es, policy * sizeof(EnumCand));
+    A(&bs, policy * sizeof(BisCand));
+    A(&b.heap_scratch, policy);
     A(&b.clb, maxc);
     A(&b.cstate, maxc);
     if (lazy) A(&b.cbest, maxc);
@@ -1232,6 +1224,9 @@ extern "C" cmn_status cmn_solver_create(const cmn_problem* p, const cmn_solve_op
     A(&b.block_best, (size_t)b.n_block_best);
     A(&b.best_point, (size_t)n);
     A(&s->d_viable, 1);
+    if (e == cudaSuccess) e = slab.alloc(&s->slab);
+    b.enum_scratch = es;
+    b.bis_scratch = bs;
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&s->h_dev), sizeof(SolverDev));
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&s->h_viable), sizeof(uint64_t));
     if (e != cudaSuccess) {

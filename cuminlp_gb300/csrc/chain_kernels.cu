@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const E
       g = kMode == 3 ? (uint64_t)a.list[idx] : idx;
       child_of(a.log2C, g, k, r);
       if (flags) {
-        const uint8_t f = a.out_flag[g];
+        const uint8_t f = kMode == 0 && a.flags != nullptr ? a.flags[g] : a.out_flag[g];
         if (kMode == 1 || kMode == 3) live = f == kChildEligible;
         else if (kMode == 4 || kFused) live = f != 0;
         feasible = f != 0;

@@ -217,7 +217,8 @@ __device__ void constraints_tile(const EvalArgs& a, unsigned char* smem, TileSha
   __syncthreads();
   if (live && wid == 0 && sub == 0) {
     const bool feasible = !((sh.fail >> box) & 1u);
-    if (kMode == 0 || kMode == 4) a.out_flag[g] = feasible ? 1 : 0;
+    if (kMode == 0 && a.flags != nullptr) a.flags[g] = feasible ? 1 : 0;
+    else if (kMode == 0 || kMode == 4) a.out_flag[g] = feasible ? 1 : 0;
     else a.out_flag[g] = feasible ? kChildEligible : kChildInfeasible;
   }
   __syncthreads();  // the tile is restaged next
@@ -302,7 +303,7 @@ __device__ void siblings_tile(const EvalArgs& a, unsigned char* smem, int flags,
   bool feasible = true;
   const ParentInfo pi = a.pinfo[k];
   if (flags && live) {
-    const uint8_t fl = a.out_flag[g];
+    const uint8_t fl = kMode == 0 && a.flags != nullptr ? a.flags[g] : a.out_flag[g];
     if (kMode == 1) live = fl == kChildEligible;
     else if (kMode == 4) live = fl != 0;
     feasible = fl != 0;

@@ -3,7 +3,10 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "../../include/cuminlp_gb300.h"
 #include "program.hpp"
@@ -29,6 +32,13 @@ struct cmn_problem {
   cmn::ChainTerm32* d_chain_var32 = nullptr;
   int32_t* d_chain_var_off = nullptr;
   cmn::ChainTerm* d_chain_term_pt = nullptr;
+  // one allocation holds every table above
+  void* d_tables = nullptr;
+  // host-buffer calls of cmn_eval_boxes stage through this, up to
+  // kEvalWorkspace bytes; a second call at the same time takes its own
+  mutable std::mutex ws_mu;
+  mutable unsigned char* d_ws = nullptr;
+  mutable size_t ws_bytes = 0;
   // cmn_autotune's choice per precision (0 FP64, 1 FP32): blocks per SM
   // and lanes per box cap; 0 = not tuned
   int tuned_bps[2] = {0, 0};
@@ -64,6 +74,34 @@ struct cmn_problem {
 };
 
 namespace cmn {
+
+constexpr size_t kEvalWorkspace = 64u << 20;
+
+// Collects arrays and gives them places in one device allocation: a solver
+// has some forty, and each cudaMalloc / cudaFree of its own took 30-80 us.
+class Slab {
+ public:
+  template <typename T>
+  void add(T** ptr, size_t n)
+  {
+    const size_t bytes = (n > 0 ? n : 1) * sizeof(T);
+    parts_.push_back({reinterpret_cast<void**>(ptr), total_});
+    total_ += (bytes + 255) & ~(size_t)255;
+  }
+  size_t bytes() const { return total_; }
+  cudaError_t alloc(void** base)
+  {
+    *base = nullptr;
+    cudaError_t e = cudaMalloc(base, total_ > 0 ? total_ : 256);
+    if (e == cudaSuccess)
+      for (auto& p : parts_) *p.first = static_cast<unsigned char*>(*base) + p.second;
+    return e;
+  }
+
+ private:
+  std::vector<std::pair<void**, size_t>> parts_;
+  size_t total_ = 0;
+};
 
 // Records `msg` as this thread's cmn_last_error() and returns `st`.
 cmn_status set_error(cmn_status st, const std::string& msg);

@@ -146,6 +146,9 @@ struct EvalArgs {
   double* out_lb;
   double* out_ub;
   uint8_t* out_flag;  // role/raw: feasible; solver: ChildState
+  // kMode 0: where the constraint pass leaves its verdicts for the objective
+  // pass when out_flag is host memory; null: in out_flag
+  uint8_t* flags;
   uint32_t* error;    // solver: set when a staged program tile never arrived
   // byte offset in dynamic shared memory of the staged program tiles (FP64
   // passes with one lane per box); 0: the program is read from global memory

@@ -29,6 +29,10 @@ namespace cmn {
 #define CMN_POLICY_D2U(x) ((unsigned long long)(x))
 #endif
 
+// Most variables whose policy scratch (88 bytes each) a device thread keeps in
+// local memory.
+constexpr int kPolicyLocal = 64;
+
 struct EnumCand {
   uint64_t vid, domain, bits;
   uint32_t kind, pad;

@@ -1568,7 +1568,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     const int grid = (int)std::min<uint64_t>((cfg.e_max + 127) / 128, 2048);
     if (cfg.n_vars <= 8) branch_kernel<8><<<grid, 128, 0, s>>>(cfg, b);
     else if (cfg.n_vars <= 32) branch_kernel<32><<<grid, 128, 0, s>>>(cfg, b);
-    else if (cfg.n_vars <= 64) branch_kernel<64><<<grid, 128, 0, s>>>(cfg, b);
+    else if (cfg.n_vars <= kPolicyLocal) branch_kernel<kPolicyLocal><<<grid, 128, 0, s>>>(cfg, b);
     else branch_kernel<0><<<grid, 128, 0, s>>>(cfg, b);
   }
   mark(marks, 1, s);
