@@ -29,7 +29,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-O2", "-Xcompiler", "-frounding-math",
     "--expt-relaxed-constexpr", "-DNDEBUG",
 ]
-SOURCES = ["program.cpp", "eval_kernels.cu", "chain_kernels.cu", "chain32_kernels.cu", "chain_points.cu", "search_kernels.cu", "batch_kernels.cu", "batch_chain_kernels.cu", "capi.cu", "batch.cu",
+SOURCES = ["program.cpp", "eval_kernels.cu", "chain_kernels.cu", "chain32_kernels.cu", "chain_points.cu", "level_kernels.cu", "search_kernels.cu", "batch_kernels.cu", "batch_chain_kernels.cu", "capi.cu", "batch.cu",
            "server.cpp", "noalloc.cu", "emu_check.cu"]
 
 

@@ -98,6 +98,7 @@ static cudaError_t ensure_attributes()
   if (e == cudaSuccess) e = set_chain_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_chain32_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_chain_points_attributes(max_dynamic_smem());
+  if (e == cudaSuccess) e = set_level_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_batch_kernel_attributes(max_dynamic_smem());
   if (e == cudaSuccess) e = set_batch_tile_attributes(max_dynamic_smem());
   if (e == cudaSuccess && dev < 31) g_attr_device_mask |= (1 << dev);
@@ -168,6 +169,12 @@ extern "C" cmn_status cmn_problem_create(const cmn_problem_desc* desc, cmn_probl
         up(&p->d_chain_var_off, p->prog.chain_var_off);
       }
       if (!p->prog.chain_term_pt.empty()) up(&p->d_chain_term_pt, p->prog.chain_term_pt);
+    }
+    if (!p->prog.level_off.empty()) {
+      up(&p->d_prog64l, p->prog.code64l);
+      up(&p->d_prog32l, p->prog.code32l);
+      up(&p->d_level_off, p->prog.level_off);
+      up(&p->d_level_run, p->prog.level_run);
     }
     cudaError_t e = slab.alloc(&p->d_tables);
     if (e == cudaSuccess) {
@@ -599,6 +606,7 @@ extern "C" cmn_status cmn_bound(cmn_role* r, const double* box, const uint64_t* 
   a.max_slots = (int)r->slot_kinds.size();  // one parent: the stride of the slot table is unused
   a.n_children = r->n_regions;
   a.chain = r->p->chain();
+  a.level = r->p->levels();
   a.max_boxes = r->n_regions;
   a.out_lb = r->d_lb;
   a.out_flag = r->d_feas;
@@ -855,6 +863,7 @@ extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, co
   a.pinfo = nullptr;
   a.n_children = n_boxes;
   a.chain = p->chain();
+  a.level = p->levels();
   a.max_boxes = n_boxes;
   a.out_lb = dlb;
   a.out_ub = dub;

@@ -1082,6 +1082,7 @@ size_t inc_child_smem_bytes(int max_slots, int threads)
 
 cudaError_t launch_eval(const EvalArgs& a, int mode, bool fp32, int grid, int threads, cudaStream_t s)
 {
+  if (mode == 0 && level_fits(a, fp32)) return launch_level(a, fp32, s);
   if (fp32) {
     if (chain32_fits(a, mode)) return launch_chain32(a, mode, s);
     if (mode == 0) return launch_eval_t<float, 0>(a, grid, threads, s);

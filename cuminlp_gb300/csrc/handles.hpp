@@ -32,6 +32,10 @@ struct cmn_problem {
   cmn::ChainTerm32* d_chain_var32 = nullptr;
   int32_t* d_chain_var_off = nullptr;
   cmn::ChainTerm* d_chain_term_pt = nullptr;
+  cmn::Instr* d_prog64l = nullptr;  // the program in levels (Program::level_*), null when none
+  cmn::Instr* d_prog32l = nullptr;
+  int32_t* d_level_off = nullptr;
+  int32_t* d_level_run = nullptr;
   // one allocation holds every table above
   void* d_tables = nullptr;
   // host-buffer calls of cmn_eval_boxes stage through this, up to
@@ -67,6 +71,19 @@ struct cmn_problem {
     }
     const int64_t w = (all + most - 1) / most;
     t.warps32 = (int32_t)(w < 1 ? 1 : w > 8 ? 8 : w);
+    return t;
+  }
+
+  cmn::LevelTab levels() const
+  {
+    cmn::LevelTab t{};
+    if (!d_level_off) return t;
+    t.prog64 = d_prog64l;
+    t.prog32 = d_prog32l;
+    t.off = d_level_off;
+    t.run = d_level_run;
+    t.levels = (int32_t)(prog.level_off.size() - 1) / cmn::kLevelWarps;
+    t.slots = prog.level_slots;
     return t;
   }
 

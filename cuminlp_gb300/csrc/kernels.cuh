@@ -162,6 +162,7 @@ struct EvalArgs {
   // boxes (chain_kernels.cu); n_seg 0: the interpreter
   ChainTab chain;
   uint64_t max_boxes;  // most boxes the launch can see (grid size)
+  LevelTab level;      // kMode 0: the program in levels, for few boxes
 };
 
 struct SampleArgs {

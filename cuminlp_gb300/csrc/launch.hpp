@@ -44,6 +44,10 @@ cudaError_t launch_eval(const EvalArgs& a, int mode, bool fp32, int grid, int th
 bool chain_fits(const EvalArgs& a);
 cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s);
 cudaError_t set_chain_kernel_attributes(int max_smem);
+// mode 0 over few boxes of a program in levels (level_kernels.cu)
+bool level_fits(const EvalArgs& a, bool fp32);
+cudaError_t launch_level(const EvalArgs& a, bool fp32, cudaStream_t s);
+cudaError_t set_level_kernel_attributes(int max_smem);
 // FP32 modes 0 (boxes) and 2 (screen) over such a program, and the lazy
 // form's child bounds (chain32_kernels.cu)
 bool chain32_fits(const EvalArgs& a, int mode);

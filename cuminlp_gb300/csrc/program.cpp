@@ -2,6 +2,7 @@
 #include "program.hpp"
 
 #include <algorithm>
+#include <array>
 #include <cfloat>
 #include <cmath>
 #include <cstring>
@@ -287,6 +288,7 @@ class Compiler {
     build_schedule();
     build_incremental();
     build_chains();
+    build_levels();
     out_.code32 = out_.code64;
     out_.code32p = out_.code64;
     for (size_t k = 0; k < out_.code64.size(); ++k) {
@@ -306,6 +308,15 @@ class Compiler {
         q.c32.clo = d2f_rn(c);
         q.c32.chi = q.c32.clo;
       }
+    }
+    out_.code32l = out_.code64l;
+    for (size_t k = 0; k < out_.code64l.size(); ++k) {  // the same constants, the levels' slots
+      const Instr l = out_.code64l[k];
+      Instr& s = out_.code32l[k];
+      s = out_.code32[k];
+      s.dst = l.dst;
+      s.a = l.a;
+      s.b = l.b;
     }
   }
 
@@ -457,6 +468,129 @@ class Compiler {
     }
     out_.inc_off[lists.size()] = (int32_t)out_.inc_pcs.size();
     out_.inc_ok = true;
+  }
+
+  // Program::level_*.
+  void build_levels()
+  {
+    const std::vector<Instr>& code = out_.code64;
+    const int len = (int)code.size();
+    if (out_.n_slots == 0 || len < 4 * kLevelWarps) return;
+    auto is = [&](int pc, int op) { return (code[pc].head & 7) == op; };
+    auto resets = [&](int pc) { return is(pc, kOpLoadAcc) || (is(pc, kOpTerm) && ((code[pc].head >> 3) & kTermInit)); };
+    // which operand fields an instruction reads, and whether it reads the accumulator
+    auto slots_of = [&](int pc, int (&s)[2]) {
+      const Instr& in = code[pc];
+      const int ma = in.modes & 3, mb = (in.modes >> 2) & 3;
+      s[0] = s[1] = -1;
+      if (is(pc, kOpTerm) || is(pc, kOpStoreAcc) || is(pc, kOpConstToSlot)) return;
+      if (ma == kModeSlot) s[0] = in.a;
+      if (is(pc, kOpGeneric) && mb == kModeSlot) s[1] = in.b;
+    };
+    auto reads_acc = [&](int pc) {
+      const Instr& in = code[pc];
+      const int sub = in.head >> 3;
+      if (is(pc, kOpStoreAcc)) return true;
+      if (is(pc, kOpTerm)) return !(sub & kTermInit);
+      if (is(pc, kOpConstToSlot)) return false;
+      if ((in.modes & 3) == kModeAcc) return true;
+      // a unary node's second operand points at the accumulator unread
+      const bool binary = is(pc, kOpGeneric) && (sub == kGAdd || sub == kGSub || sub == kGMul || sub == kGDiv ||
+                                                 sub == kGPow || sub == kGMin || sub == kGMax);
+      return binary && ((in.modes >> 2) & 3) == kModeAcc;
+    };
+    auto writes = [&](int pc) { return is(pc, kOpGeneric) || is(pc, kOpStoreAcc) || is(pc, kOpConstToSlot); };
+    // runs: from an accumulator reset to its last reader, else one instruction
+    std::vector<std::pair<int, int>> runs;
+    for (int pc = 0; pc < len;) {
+      int end = pc + 1;
+      if (resets(pc)) {
+        for (int q = pc + 1; q < len && !resets(q); ++q)
+          if (reads_acc(q)) end = q + 1;
+      } else if (reads_acc(pc)) {
+        return;  // an accumulator read outside its chain's run: never emitted
+      }
+      runs.push_back({pc, end});
+      pc = end;
+    }
+    // levels: one past the runs that wrote the slots a run reads
+    const int R = (int)runs.size();
+    std::vector<int> writer(out_.n_slots, -1), level(R, 0);
+    std::vector<std::vector<int>> values(R);           // instructions of a run that write slots
+    std::vector<std::array<int, 2>> from(len, {-1, -1});  // instruction that wrote each operand
+    std::vector<int> run_of(len, 0), def(out_.n_slots, -1);
+    int levels = 0;
+    for (int r = 0; r < R; ++r) {
+      for (int pc = runs[r].first; pc < runs[r].second; ++pc) {
+        run_of[pc] = r;
+        int s[2];
+        slots_of(pc, s);
+        for (int e = 0; e < 2; ++e) {
+          if (s[e] < 0) continue;
+          const int d = def[s[e]];
+          if (d < 0) return;  // a slot read before it is written: never emitted
+          from[pc][e] = d;
+          if (run_of[d] != r) level[r] = std::max(level[r], level[run_of[d]] + 1);
+        }
+        if (writes(pc)) def[code[pc].dst] = pc;
+      }
+      levels = std::max(levels, level[r] + 1);
+    }
+    // warps: longest run first, to the warp with the least of the level
+    std::vector<std::vector<std::vector<int>>> lists(levels, std::vector<std::vector<int>>(kLevelWarps));
+    std::vector<int> order(R);
+    for (int r = 0; r < R; ++r) order[r] = r;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+      return runs[a].second - runs[a].first > runs[b].second - runs[b].first;
+    });
+    std::vector<std::array<int, kLevelWarps>> load(levels);
+    for (auto& l : load) l.fill(0);
+    for (int r : order) {
+      int w = 0;
+      for (int q = 1; q < kLevelWarps; ++q)
+        if (load[level[r]][q] < load[level[r]][w]) w = q;
+      lists[level[r]][w].push_back(r);
+      load[level[r]][w] += runs[r].second - runs[r].first;
+    }
+    int64_t span = 0;
+    for (const auto& l : load) span += *std::max_element(l.begin(), l.end());
+    if (span * 2 > len) return;  // too sequential for the barriers to pay
+    // slots: a value keeps its own from its level to the last one that reads it
+    std::vector<int> last(len, -1), slot(len, -1), free_list;
+    for (int pc = 0; pc < len; ++pc)
+      for (int e = 0; e < 2; ++e)
+        if (from[pc][e] >= 0) last[from[pc][e]] = std::max(last[from[pc][e]], level[run_of[pc]]);
+    std::vector<std::vector<int>> dies(levels);
+    int next = 0;
+    for (int l = 0; l < levels; ++l) {
+      for (int w = 0; w < kLevelWarps; ++w)
+        for (int r : lists[l][w])
+          for (int pc = runs[r].first; pc < runs[r].second; ++pc)
+            if (writes(pc)) {
+              if (free_list.empty()) free_list.push_back(next++);
+              slot[pc] = free_list.back();
+              free_list.pop_back();
+              dies[std::max(last[pc], l)].push_back(slot[pc]);
+            }
+      free_list.insert(free_list.end(), dies[l].begin(), dies[l].end());
+    }
+    out_.level_slots = next;
+    out_.code64l = code;
+    for (int pc = 0; pc < len; ++pc) {
+      Instr& in = out_.code64l[pc];
+      if (writes(pc)) in.dst = (uint16_t)slot[pc];
+      if (from[pc][0] >= 0) in.a = (uint16_t)slot[from[pc][0]];
+      if (from[pc][1] >= 0) in.b = (uint16_t)slot[from[pc][1]];
+    }
+    for (int l = 0; l < levels; ++l)
+      for (int w = 0; w < kLevelWarps; ++w) {
+        out_.level_off.push_back((int32_t)out_.level_run.size() / 2);
+        for (int r : lists[l][w]) {
+          out_.level_run.push_back(runs[r].first);
+          out_.level_run.push_back(runs[r].second);
+        }
+      }
+    out_.level_off.push_back((int32_t)out_.level_run.size() / 2);
   }
 
   // Most that the FP32 filter of a chain of k terms can be off its FP64

@@ -173,6 +173,17 @@ struct ChainTab {
   int32_t warps32;  // warps of a tile that keep its chains' lengths balanced
 };
 
+// A program laid out in levels (Program::level_*), on the device.
+struct LevelTab {
+  const Instr* prog64;
+  const Instr* prog32;
+  const int32_t* off;
+  const int32_t* run;
+  int32_t levels;  // 0: none
+  int32_t slots;
+};
+constexpr int kLevelWarps = 8;
+
 // Largest bound of a variable the FP32 filters take (cut32): 2^40.
 constexpr double kFilterMax = 1099511627776.0;
 

@@ -75,6 +75,16 @@ struct Program {
   std::vector<ChainTerm32> chain_var32;
   std::vector<int32_t> chain_var_off;
   std::vector<ChainTerm> chain_term_pt;   // empty: points take the interpreter
+  // A program with shared slots, laid out for kLevelWarps warps that share a
+  // tile of boxes: contiguous runs of instructions (a sum chain with its
+  // readers, or one node) in levels of runs that do not read each other's
+  // slots.  level_off[l * kLevelWarps + w] is warp w's first run of level l,
+  // run 2j and 2j + 1 of level_run the j-th run's instructions; code64l /
+  // code32l are the program with slots of its own (a slot is not reused
+  // within the level that last reads it).  Empty when it does not pay.
+  std::vector<int32_t> level_off, level_run;
+  std::vector<Instr> code64l, code32l;
+  int level_slots = 0;
   bool chain_points = false;  // every chain has a filter and the root box is in its range
 };
 
