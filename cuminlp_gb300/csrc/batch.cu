@@ -93,15 +93,12 @@ struct cmn_batch {
   int eval_grid = 1;
   BatchGrids grids;
   uint64_t kernels_per_iter = 0;
-  cudaEvent_t marks[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 
   ~cmn_batch()
   {
     int cur = 0;
     if (cudaGetDevice(&cur) == cudaSuccess && cur != device) cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
-    for (cudaEvent_t ev : marks)
-      if (ev) cudaEventDestroy(ev);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     if (slab) cudaFree(slab);
@@ -256,6 +253,7 @@ extern "C" cmn_status cmn_batch_create(const cmn_batch_config* config, cmn_batch
     A(&b.stile, K + 1);
     A(&b.qtile, K + 1);
     A(&b.live, 4);
+    slab.add(&b.stamps, 5);
     A(&b.sbest, K);
     uint32_t* order = nullptr;
     A(&order, K);
@@ -280,6 +278,7 @@ extern "C" cmn_status cmn_batch_create(const cmn_batch_config* config, cmn_batch
     std::memset(s->h_st, 0, sizeof(InstState) * K);
     for (uint64_t i = 0; i < K; ++i) s->h_st[i].done = 1;
     e = cudaMemsetAsync(b.desc, 0, sizeof(InstDesc) * K, s->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(b.stamps, 0, 5 * sizeof(uint64_t), s->stream);
     if (e == cudaSuccess) e = s->upload_order();
     if (e == cudaSuccess) e = cudaMemcpyAsync(b.st, s->h_st, sizeof(InstState) * K, cudaMemcpyHostToDevice, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
@@ -290,10 +289,9 @@ extern "C" cmn_status cmn_batch_create(const cmn_batch_config* config, cmn_batch
     c.eval_capacity = (uint64_t)s->eval_grid * kEvalThreads;
     c.sample_capacity = c.eval_capacity;
     s->grids = batch_grids(c, s->eval_grid);
-    for (int i = 0; i < 5 && e == cudaSuccess; ++i) e = cudaEventCreate(&s->marks[i]);
     if (e == cudaSuccess) e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      cudaError_t e2 = batch_iteration(c, b, s->grids, s->stream, s->marks);
+      cudaError_t e2 = batch_iteration(c, b, s->grids, s->stream);
       e = cudaStreamEndCapture(s->stream, &s->graph);
       if (e2 != cudaSuccess) e = e2;
     }
@@ -472,14 +470,13 @@ extern "C" cmn_status cmn_batch_phase_ms(cmn_batch* s, double* ms5)
 {
   if (!s || !ms5) return fail(CMN_INVALID_CONFIGURATION, "null argument");
   BCK(cudaSetDevice(s->device));
-  BCK(cudaEventSynchronize(s->marks[4]));
-  float t = 0;
-  for (int i = 0; i < 4; ++i) {
-    BCK(cudaEventElapsedTime(&t, s->marks[i], s->marks[i + 1]));
-    ms5[i] = t;
-  }
-  BCK(cudaEventElapsedTime(&t, s->marks[0], s->marks[4]));
-  ms5[4] = t;
+  uint64_t t[5];
+  BCK(cudaMemcpyAsync(t, s->b.stamps, sizeof t, cudaMemcpyDeviceToHost, s->stream));
+  BCK(cudaStreamSynchronize(s->stream));
+  if (t[0] == 0) return fail(CMN_CUDA_ERROR, "no iteration has run");
+  auto ms = [&](int from, int to) { return t[to] > t[from] ? (double)(t[to] - t[from]) * 1e-6 : 0.0; };
+  for (int i = 0; i < 4; ++i) ms5[i] = ms(i, i + 1);
+  ms5[4] = ms(0, 4);
   return CMN_OK;
 }
 

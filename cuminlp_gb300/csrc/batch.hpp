@@ -144,6 +144,7 @@ struct BatchBufs {
   uint64_t* qtile;
   uint64_t* live;           // [0] live children of all instances, [1], [2] as above,
                             // [3] most lanes any live instance can use per box
+  uint64_t* stamps;         // [5] phase boundaries of the last iteration
   unsigned long long* sbest;  // [K] lb_key of the best point value known
   // [K]: the slots in the order the bound and sample launches walk their
   // children -- longest program first, so the launch's tail is short
@@ -213,10 +214,9 @@ struct BatchGrids {
 };
 BatchGrids batch_grids(const BatchCfg& cfg, int eval_grid);
 // Enqueues one iteration over every active instance (capturable).
-// `marks` (5 events or null) are recorded at the phase boundaries: start,
+// The kernels write BatchBufs::stamps (ns) at the phase boundaries: start,
 // after select + branch, after bound, after sample, after finish.
-cudaError_t batch_iteration(const BatchCfg& cfg, const BatchBufs& b, const BatchGrids& grids, cudaStream_t s,
-                            const cudaEvent_t* marks);
+cudaError_t batch_iteration(const BatchCfg& cfg, const BatchBufs& b, const BatchGrids& grids, cudaStream_t s);
 size_t batch_eval_smem(const BatchCfg& cfg, bool fp32);
 size_t batch_sample_smem(const BatchCfg& cfg);
 // resident blocks per SM of the bound (fp32: screen) and sample kernels

@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kPointThreads) batch_points_kernel(const Batch
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, W = blockDim.x >> 5;
   uint8_t* list = list_s + wid * 32;
   const int pts = 1 << c.log_pts;
+  stamp_first(b.stamps + 2);
   const uint64_t tiles = b.qtile[c.K];
   for (uint64_t tile = (uint64_t)blockIdx.x * W + wid; tile < tiles; tile += (uint64_t)gridDim.x * W) {
     const uint64_t pos = position_of(b.qtile, c.K, tile), slot = b.order[pos];

@@ -260,6 +260,10 @@ __global__ void batch_init_slot_kernel(const BatchCfg c, const BatchBufs b, uint
 __global__ void batch_begin_kernel(const BatchCfg c, const BatchBufs b)
 {
   const uint64_t slot = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (slot == 0) {
+    const uint64_t t = now_ns();
+    for (int i = 0; i < 5; ++i) b.stamps[i] = t;
+  }
   if (slot >= c.K) return;
   InstState& s = b.st[slot];
   const InstDesc& d = b.desc[slot];
@@ -368,11 +372,13 @@ __global__ void __launch_bounds__(256) batch_append_kernel(const BatchCfg c, con
 {
   const int lane = threadIdx.x & 31;
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  bool worked = false;
   const uint64_t per = c.child_stride;
   for (uint64_t w = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < c.K * ((per + 15) / 16); w += warps) {
     const uint64_t slot = w / ((per + 15) / 16), p0 = (w - slot * ((per + 15) / 16)) * 16;
     const uint64_t kept = b.st[slot].n_parents > 0 ? b.st[slot].kept : 0;
     if (p0 >= kept) continue;
+    worked = true;
     const int n = b.desc[slot].n_vars;
     const int cnt = kept - p0 < 16 ? (int)(kept - p0) : 16;
     uint32_t mine = 0, to = 0;
@@ -408,6 +414,7 @@ __global__ void __launch_bounds__(256) batch_append_kernel(const BatchCfg c, con
       }
     }
   }
+  if (lane == 0) stamp_last(b.stamps + 4, worked);
 }
 
 // kLocal: the policy's scratch in local memory (n_max <= kLocal; 0: in the
@@ -574,6 +581,7 @@ __global__ void __launch_bounds__(1024) batch_live_kernel(const BatchCfg c, cons
     b.live[2] = (uint64_t)lbc;
     b.live[3] = (uint64_t)min(gmax_all, c.g_max);
     if (runs) b.vrun[c.K + 1] = 0;
+    stamp_last(b.stamps + 1, true);
   }
 }
 
@@ -896,6 +904,7 @@ __global__ void __launch_bounds__(kEvalThreads) batch_screen_kernel(const BatchC
   t.shi = t.slo;
   t.stride = B;
   t.tid = threadIdx.x;
+  if (!c.tiles) stamp_first(b.stamps + 2);  // else batch_points_kernel does
   const uint64_t total = b.child_base[c.K];
   for (uint64_t idx = (uint64_t)blockIdx.x * B + threadIdx.x; idx < total; idx += (uint64_t)gridDim.x * B) {
     const uint64_t g = live_child(c, b, idx);
@@ -1225,6 +1234,7 @@ __global__ void __launch_bounds__(kEvalThreads) batch_sample_kernel(const BatchC
   t.shi = t.slo;
   t.stride = B;
   t.tid = threadIdx.x;
+  if (!c.tiles) stamp_first(b.stamps + 2);  // else batch_points_kernel does
   const uint64_t total = b.child_base[c.K];
   const int lg = lanes_per_box(total, c.sample_capacity, (int)b.child_base[c.K + 1]);
   const int G = 1 << lg;
@@ -1314,6 +1324,7 @@ __global__ void __launch_bounds__(kMiThreads) batch_finish_kernel(const BatchCfg
   __shared__ unsigned long long cnt[10];
   __shared__ unsigned long long min_key_s;
   const uint64_t slot = blockIdx.x;
+  stamp_first(b.stamps + 3);
   InstState* st = &b.st[slot];
   const uint32_t E = (uint32_t)st->n_parents;
   if (E == 0) return;
@@ -1653,11 +1664,6 @@ cudaError_t batch_init_slot(const BatchCfg& c, const BatchBufs& b, uint64_t slot
   return cudaGetLastError();
 }
 
-static void mark(const cudaEvent_t* marks, int i, cudaStream_t s)
-{
-  if (marks) cudaEventRecordWithFlags(marks[i], s, cudaEventRecordExternal);
-}
-
 // Blocks for a grid-stride launch of `kernel` over `items` threads' worth
 // of work: as many as stay resident on every SM, no more than the items
 // need.
@@ -1692,11 +1698,9 @@ static void finish(const BatchCfg& c, const BatchBufs& b, cudaStream_t s)
   batch_append_kernel<<<(int)std::min<uint64_t>((warps + 7) / 8, 8192), 256, 0, s>>>(c, b);
 }
 
-cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGrids& grids, cudaStream_t s,
-                            const cudaEvent_t* marks)
+cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGrids& grids, cudaStream_t s)
 {
   const int eval_grid = grids.eval;
-  mark(marks, 0, s);
   const int kb = (int)((c.K + 255) / 256);
   batch_begin_kernel<<<kb, 256, 0, s>>>(c, b);
   batch_select_kernel<<<(int)c.K, kMiThreads, 0, s>>>(c, b);
@@ -1707,7 +1711,6 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
   else if (c.n_max <= kPolicyLocal) batch_branch_kernel<kPolicyLocal><<<bg, 128, 0, s>>>(c, b);
   else batch_branch_kernel<0><<<bg, 128, 0, s>>>(c, b);
   batch_live_kernel<<<1, 1024, 0, s>>>(c, b);
-  mark(marks, 1, s);
   const bool fp32 = c.precision == CMN_PRECISION_FP32_SCREEN;
   const bool lazy = c.precision == CMN_PRECISION_FP32_LAZY;
   if (lazy) {
@@ -1730,14 +1733,11 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
     batch_list_scan_kernel<<<1, 1024, 0, s>>>(c, b);
     batch_list_scatter_kernel<<<lg, 512, 0, s>>>(c, b);
     batch_eval_kernel<double, 3><<<eval_grid, kEvalThreads, batch_eval_smem(c, false), s>>>(c, b);
-    mark(marks, 2, s);
     e = batch_tile_points(c, b, grids.tile, s);
     if (e != cudaSuccess) return e;
     batch_screen_kernel<<<grids.screen, kEvalThreads, batch_screen_smem(c), s>>>(c, b);
     batch_chunk_kernel<<<eval_grid, kEvalThreads, batch_sample_smem(c), s>>>(c, b);
-    mark(marks, 3, s);
     finish(c, b, s);
-    mark(marks, 4, s);
     return cudaGetLastError();
   }
   if (fp32) {
@@ -1752,13 +1752,10 @@ cudaError_t batch_iteration(const BatchCfg& c, const BatchBufs& b, const BatchGr
     if (e != cudaSuccess) return e;
     batch_eval_kernel<double, 1><<<eval_grid, kEvalThreads, batch_eval_smem(c, false), s>>>(c, b);
   }
-  mark(marks, 2, s);
   const cudaError_t ep = batch_tile_points(c, b, grids.tile, s);
   if (ep != cudaSuccess) return ep;
   batch_sample_kernel<<<eval_grid, kEvalThreads, batch_sample_smem(c), s>>>(c, b);
-  mark(marks, 3, s);
   finish(c, b, s);
-  mark(marks, 4, s);
   return cudaGetLastError();
 }
 

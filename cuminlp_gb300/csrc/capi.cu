@@ -1046,7 +1046,6 @@ struct cmn_solver {
   double elapsed_ms = 0;
   uint64_t launched = 0;
   uint64_t kernels_per_iter = 0;
-  cudaEvent_t marks[kPhaseMarks] = {};
   SideStream side;
 
   ~cmn_solver()
@@ -1055,8 +1054,6 @@ struct cmn_solver {
     if (p && cudaGetDevice(&cur) == cudaSuccess && cur != p->device) cudaSetDevice(p->device);
     if (stream) cudaStreamSynchronize(stream);
     if (side.stream) cudaStreamSynchronize(side.stream);
-    for (cudaEvent_t ev : marks)
-      if (ev) cudaEventDestroy(ev);
     if (side.fork) cudaEventDestroy(side.fork);
     if (side.join) cudaEventDestroy(side.join);
     if (side.stream) cudaStreamDestroy(side.stream);
@@ -1256,7 +1253,6 @@ extern "C" cmn_status cmn_solver_create(const cmn_problem* p, const cmn_solve_op
     e = solver_init(cfg, b, p->d_root_lb, p->d_root_ub, gub0, s->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b.best_point, 0xff, (size_t)n * sizeof(double), s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-    for (int i = 0; i < kPhaseMarks && e == cudaSuccess; ++i) e = cudaEventCreate(&s->marks[i]);
     // the side stream carries the lazy form's FP64 verdict, the longest of
     // the work it runs beside: its blocks go first
     int prio_low = 0, prio_high = 0;
@@ -1269,8 +1265,7 @@ extern "C" cmn_status cmn_solver_create(const cmn_problem* p, const cmn_solve_op
       cudaGraph_t* g = steady ? &s->graph_steady : &s->graph;
       e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
       if (e == cudaSuccess) {
-        cudaError_t e2 =
-            solver_iteration(cfg, b, s->eval_grid, s->sample_grid, s->stream, s->side, s->marks, steady == 0);
+        cudaError_t e2 = solver_iteration(cfg, b, s->eval_grid, s->sample_grid, s->stream, s->side, steady == 0);
         e = cudaStreamEndCapture(s->stream, g);
         if (e2 != cudaSuccess) e = e2;
       }
@@ -1475,17 +1470,19 @@ extern "C" cmn_status cmn_solver_outcome(cmn_solver* s, cmn_outcome* out)
   return CMN_OK;
 }
 
+static double stamp_ms(const uint64_t* t, int from, int to)
+{
+  return t[to] > t[from] ? (double)(t[to] - t[from]) * 1e-6 : 0.0;
+}
+
 extern "C" cmn_status cmn_solver_phase_ms(cmn_solver* s, double* ms5)
 {
   if (!s || !ms5) return fail(CMN_INVALID_CONFIGURATION, "null argument");
-  CK(cudaEventSynchronize(s->marks[4]));
-  float t = 0;
-  for (int i = 0; i < 4; ++i) {
-    CK(cudaEventElapsedTime(&t, s->marks[i], s->marks[i + 1]));
-    ms5[i] = t;
-  }
-  CK(cudaEventElapsedTime(&t, s->marks[0], s->marks[4]));
-  ms5[4] = t;
+  if (s->launched == 0) return fail(CMN_CUDA_ERROR, "no iteration has run");
+  const cmn_status st = pull_state(s);
+  if (st != CMN_OK) return st;
+  for (int i = 0; i < 4; ++i) ms5[i] = stamp_ms(s->h_dev->stamps, i, i + 1);
+  ms5[4] = stamp_ms(s->h_dev->stamps, 0, 4);
   return CMN_OK;
 }
 
@@ -1494,12 +1491,11 @@ extern "C" cmn_status cmn_solver_lazy_ms(cmn_solver* s, double* ms2)
   if (!s || !ms2) return fail(CMN_INVALID_CONFIGURATION, "null argument");
   if (s->cfg.precision != CMN_PRECISION_FP32_LAZY)
     return fail(CMN_INVALID_CONFIGURATION, "the solver does not run the lazy form");
-  CK(cudaEventSynchronize(s->marks[4]));
-  float t = 0;
-  CK(cudaEventElapsedTime(&t, s->marks[5], s->marks[6]));
-  ms2[0] = t;
-  CK(cudaEventElapsedTime(&t, s->marks[1], s->marks[7]));
-  ms2[1] = t;
+  if (s->launched == 0) return fail(CMN_CUDA_ERROR, "no iteration has run");
+  const cmn_status st = pull_state(s);
+  if (st != CMN_OK) return st;
+  ms2[0] = stamp_ms(s->h_dev->stamps, 5, 6);
+  ms2[1] = stamp_ms(s->h_dev->stamps, 1, 7);
   return CMN_OK;
 }
 

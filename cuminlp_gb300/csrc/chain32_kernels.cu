@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(kLazyThreads, 2) lazy_children_kernel(const Ev
   if (a.done != nullptr && *a.done) return;
   const uint64_t E = *a.n_parents_dev, tiles = (E + 31) >> 5;
   for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) lazy_tile(a, h, smem_raw, sh, tile, E);
+  if (threadIdx.x == 0) stamp_last(a.t_last, blockIdx.x < tiles);
 }
 
 // ---- launchers ----

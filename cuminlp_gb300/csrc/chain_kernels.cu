@@ -14,6 +14,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) chain_constraints_kernel(c
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ TileShared sh;
   if (a.done != nullptr && *a.done) return;
+  if constexpr (kFused) stamp_first(a.t_first);
   const uint64_t total = box_count(a, kMode == 3);
   const uint64_t tiles = (total + (1ULL << log_boxes) - 1) >> log_boxes;
   for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x)
@@ -34,6 +35,8 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const E
   double* ohi = olo + (size_t)ms * B;
   int32_t* ovid = reinterpret_cast<int32_t*>(reinterpret_cast<double*>(smem_raw) + (size_t)2 * ms * B) + threadIdx.x;
   if (a.done != nullptr && *a.done) return;
+  if constexpr (kFused)
+    if (!flags) stamp_first(a.t_first);
   const uint64_t total = box_count(a, kMode == 3);
   const double gub = a.gub ? *a.gub : DBL_MAX;
   const ChainSeg s = a.chain.seg[0];
@@ -86,6 +89,8 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const E
       if (live && lead) write_verdict<double, kMode>(a, g, k, v, gub);
     }
   }
+  if constexpr (kFused)
+    if ((threadIdx.x & 31) == 0) stamp_last(a.t_last, (uint64_t)blockIdx.x * per_block < total);
 }
 
 template <int kMode, bool kHi>

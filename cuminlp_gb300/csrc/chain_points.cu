@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(kPointThreads) chain_sample_kernel(const Sampl
     if (threadIdx.x == 0) a.block_best[blockIdx.x] = Cand{INFINITY, 0xffffffffu, 0, ~0ULL};
     return;
   }
+  stamp_first(a.t_first);
   const uint64_t children = a.n_children_dev ? *a.n_children_dev : a.n_children;
   const uint64_t per = a.exact ? 1 : a.S;
   const uint64_t total = kChunks ? (children + (1ULL << kChunkLog2) - 1) >> kChunkLog2 : children * per;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(kPointThreads) chain_screen_kernel(const Sampl
   const int wid = threadIdx.x >> 5, W = blockDim.x >> 5;
   float* x = reinterpret_cast<float*>(smem_raw + wid * point_bytes(a.n_vars + 1, log_pts));
   if (a.done != nullptr && *a.done) return;
+  stamp_first(a.t_first);
   const uint64_t total = a.n_children_dev ? *a.n_children_dev : a.n_children;
   const uint64_t salt_base = a.salt_base_dev ? *a.salt_base_dev : 0;
   for (uint64_t w0 = (uint64_t)blockIdx.x * W + wid; w0 << log_pts < total; w0 += (uint64_t)gridDim.x * W)

@@ -8,6 +8,7 @@
 
 #include "eval_core.cuh"
 #include "kernels.cuh"
+#include "stamps.cuh"
 
 namespace cmn {
 

@@ -495,6 +495,7 @@ __global__ void __launch_bounds__(kEvalThreads, CMN_EVAL_MIN_BLOCKS) eval_childr
     }
     write_verdict<float, 5>(a, g, k, v, gub);
   }
+  if ((threadIdx.x & 31) == 0) stamp_last(a.t_last, (uint64_t)blockIdx.x * B < total);
 }
 
 template <typename T, int kMode, bool kFused = false>
@@ -503,10 +504,13 @@ __global__ void __launch_bounds__(kEvalThreads, CMN_EVAL_MIN_BLOCKS) eval_childr
   if constexpr (sizeof(T) == 4) {
     if (a.plo32 != nullptr) {
       eval_children<T, kMode, float>(a, a.plo32, a.phi32);
+      if (kMode == 5 && threadIdx.x == 0) stamp_last(a.t_last, true);
       return;
     }
   }
+  if constexpr (kFused) stamp_first(a.t_first);
   eval_children<T, kMode, double, false, kFused>(a, a.plo, a.phi);
+  if ((kMode == 5 || kFused) && threadIdx.x == 0) stamp_last(a.t_last, true);
 }
 
 // The FP64 one-lane passes with their program staged in shared memory
@@ -514,7 +518,10 @@ __global__ void __launch_bounds__(kEvalThreads, CMN_EVAL_MIN_BLOCKS) eval_childr
 template <int kMode, bool kFused = false>
 __global__ void __launch_bounds__(kEvalThreads, CMN_EVAL_MIN_BLOCKS) eval_children_staged_kernel(const EvalArgs a)
 {
+  if constexpr (kFused) stamp_first(a.t_first);
   eval_children<double, kMode, double, true, kFused>(a, a.plo, a.phi);
+  if constexpr (kFused)
+    if (threadIdx.x == 0) stamp_last(a.t_last, true);
 }
 
 __device__ __forceinline__ bool admissible(const SampleArgs& a, const Tile<double>& t)
@@ -681,6 +688,7 @@ __global__ void __launch_bounds__(kEvalThreads) sample_children_kernel(const Sam
     if (threadIdx.x == 0) a.block_best[blockIdx.x] = Cand{INFINITY, 0xffffffffu, 0, ~0ULL};
     return;
   }
+  stamp_first(a.t_first);
   const uint64_t total = a.n_children_dev ? *a.n_children_dev : a.n_children;
   const uint64_t salt_base = a.salt_base_dev ? *a.salt_base_dev : 0;
   const double gub = a.gub ? *a.gub : DBL_MAX;
@@ -793,6 +801,7 @@ __global__ void __launch_bounds__(kEvalThreads) sample_screen_kernel(const Sampl
   t.stride = cols;
   t.tid = threadIdx.x >> lg;
   if (a.done != nullptr && *a.done) return;
+  stamp_first(a.t_first);
   const uint64_t total = a.n_children_dev ? *a.n_children_dev : a.n_children;
   const uint64_t salt_base = a.salt_base_dev ? *a.salt_base_dev : 0;
   const uint64_t per_block = (uint64_t)cols;
@@ -893,6 +902,7 @@ __global__ void __launch_bounds__(256) candidate_kernel(const Cand* __restrict__
   }
   best = block_min_cand(best);
   if (threadIdx.x == 0) {
+    stamp_last(inc.t_last, true);
     *out = best;
     best_s = best;
     write_s = 1;

@@ -163,6 +163,9 @@ struct EvalArgs {
   ChainTab chain;
   uint64_t max_boxes;  // most boxes the launch can see (grid size)
   LevelTab level;      // kMode 0: the program in levels, for few boxes
+  // solver: when the first block started, when the last one ended (or null)
+  uint64_t* t_first;
+  uint64_t* t_last;
 };
 
 struct SampleArgs {
@@ -202,6 +205,7 @@ struct SampleArgs {
   // the program's sum chains: points filtered in FP32 (chain_kernels.cu);
   // n_seg 0: the interpreter
   ChainTab chain;
+  uint64_t* t_first;  // as EvalArgs
 };
 
 // What a candidate's point is drawn from (candidate_kernel).
@@ -229,6 +233,7 @@ struct Incumbent {
   Cand* best;
   uint32_t* have_best;
   uint32_t* improved;
+  uint64_t* t_last;  // as EvalArgs
 };
 
 }  // namespace cmn

@@ -86,6 +86,7 @@ struct SolverDev {
   uint32_t ticket;         // blocks of the running histogram pass that are done
   Cand best;
   cmn_counters counters;
+  uint64_t stamps[8];      // phase boundaries of the last iteration (ns); solver_iteration
 };
 
 // Static configuration baked into the captured iteration.
@@ -197,16 +198,15 @@ struct SideStream {
 };
 
 // Enqueues one batched iteration (all kernels) on `s`; capturable.
-// `marks` (kPhaseMarks events or null) are recorded as event nodes: 0-4 at
-// the phase boundaries (start, after branching, after bounding, after
-// sampling, end); in the lazy form 5 and 6 around the FP64 verdict on the
-// side stream and 7 after the FP32 child bounds.
+// The kernels write SolverDev::stamps: 0-4 at the phase boundaries (start,
+// after branching, after bounding, after sampling, end); in the lazy form 5
+// and 6 around the FP64 verdict on the side stream and 7 after the FP32 child
+// bounds.
 // `with_select`: the iteration selects and stages its own parents (the first
 // iteration); otherwise the previous iteration staged them, and the
 // iteration flags a device error if it did not.
-constexpr int kPhaseMarks = 8;
 cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval_grid, int sample_grid,
-                             cudaStream_t s, const SideStream& side, const cudaEvent_t* marks, bool with_select);
+                             cudaStream_t s, const SideStream& side, bool with_select);
 // Fills min key / viable count of the current pool (after the run).
 cudaError_t solver_pool_stats(const SolverCfg& cfg, const SolverBufs& b, uint64_t* viable_dev, cudaStream_t s);
 // Copies pool entries [start, start + count) in position order: boxes as

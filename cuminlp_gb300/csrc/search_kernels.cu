@@ -16,6 +16,7 @@
 #include "launch.hpp"
 #include "policy.cuh"
 #include "search.hpp"
+#include "stamps.cuh"
 
 namespace cmn {
 
@@ -95,6 +96,8 @@ __global__ void begin_kernel(const SolverCfg cfg, const SolverBufs b, int requir
   uint64_t E = L < cfg.e_max ? L : cfg.e_max;
   const uint64_t left = cfg.iter_limit - d->expansions;
   if (E > left) E = left;
+  const uint64_t t = now_ns();
+  for (int i = 0; i < 8; ++i) d->stamps[i] = t;
   // the previous iteration staged the E best entries of this pool already
   d->skip_select = (d->pre_valid && d->pre_k == E) ? 1u : 0u;
   if (require_staged && !d->skip_select) d->error = 1;
@@ -1063,6 +1066,7 @@ __global__ void stage_next_kernel(const SolverCfg cfg, const SolverBufs b)
   if (blockIdx.x == 0 && threadIdx.x == 0) finish_pool(cfg, b);
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
     stage_parent(cfg, b, b.pslot[k], k);
+  if (threadIdx.x == 0) stamp_last(b.dev->stamps + 4, (uint64_t)blockIdx.x * blockDim.x < n);
 }
 
 // appends the kept children listed (in order) by the compaction, one thread
@@ -1222,6 +1226,7 @@ __global__ void branch_kernel(const SolverCfg cfg, const SolverBufs b)
       bounded += pi.nreg;
     }
   }
+  if (threadIdx.x == 0) stamp_last(b.dev->stamps + 1, (uint64_t)blockIdx.x * blockDim.x < E);
   if (lazy) return;  // every thread of the block takes this branch
   unsigned long long c[3] = {fathomed, fathomed_points, bounded};
   block_sum(c);
@@ -1506,18 +1511,12 @@ static void radix_select(const SolverCfg& cfg, const SolverBufs& b, int which, u
       ScanArgs{b.block_counts2, b.block_offsets2, &b.dev->pre_count, nullptr}, n_dev, skip, &b.dev->done);
 }
 
-static void mark(const cudaEvent_t* marks, int i, cudaStream_t s)
-{
-  if (marks) cudaEventRecordWithFlags(marks[i], s, cudaEventRecordExternal);
-}
-
 cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval_grid, int sample_grid,
-                             cudaStream_t s, const SideStream& side, const cudaEvent_t* marks, bool with_select)
+                             cudaStream_t s, const SideStream& side, bool with_select)
 {
   const bool lazy = cfg.precision == CMN_PRECISION_FP32_LAZY;
   const uint64_t max_children = cfg.e_max << cfg.log2C;
   const uint64_t max_pool = cfg.pstride;
-  mark(marks, 0, s);
   begin_kernel<<<1, 1, 0, s>>>(cfg, b, with_select ? 0 : 1);
 
   // (1) select the E best parents and stage them (after the first
@@ -1536,7 +1535,6 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     cudaError_t e = cudaEventRecord(side.fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(side.stream, side.fork, 0);
     if (e != cudaSuccess) return e;
-    mark(marks, 5, side.stream);
     EvalArgs pa = {};
     pa.prog = b.prog64;
     pa.prog_len = cfg.prog_len;
@@ -1556,9 +1554,10 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     pa.error = &b.dev->error;
     pa.chain = b.chain;
     pa.max_boxes = cfg.e_max;
+    pa.t_first = b.dev->stamps + 5;
+    pa.t_last = b.dev->stamps + 6;
     e = launch_eval(pa, 6, false, eval_grid, kEvalThreads, side.stream);
     if (e != cudaSuccess) return e;
-    mark(marks, 6, side.stream);
     e = cudaEventRecord(side.join, side.stream);
     if (e != cudaSuccess) return e;
   }
@@ -1571,7 +1570,6 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     else if (cfg.n_vars <= kPolicyLocal) branch_kernel<kPolicyLocal><<<grid, 128, 0, s>>>(cfg, b);
     else branch_kernel<0><<<grid, 128, 0, s>>>(cfg, b);
   }
-  mark(marks, 1, s);
 
   // (3) bound every child: FP64, or FP32 screen + FP64 certify
   EvalArgs ea = {};
@@ -1620,6 +1618,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     ea.plo32 = b.plo32;
     ea.phi32 = b.phi32;
     ea.parent_lb = nullptr;  // folded in by lazy_fold_kernel
+    ea.t_last = b.dev->stamps + 7;
     if (cfg.inc_tile) {
       ea.n_parents_dev = &b.dev->n_parents;
       e = launch_lazy_children(ea, cfg.e_max, s);
@@ -1636,7 +1635,6 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
       e = launch_eval(ea, 5, true, eval_grid, kEvalThreads, s);
     }
     if (e != cudaSuccess) return e;
-    mark(marks, 7, s);
     // join the parents' FP64 verdict: drop the boxes it excludes, fold the
     // certified bounds into their children
     e = cudaStreamWaitEvent(s, side.join, 0);
@@ -1656,6 +1654,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     ca.plo32 = nullptr;
     ca.phi32 = nullptr;
     ca.parent_lb = b.plb;
+    ca.t_last = nullptr;
     ca.inc_segments = 0;
     ca.list = b.list;
     ca.list_count = &b.dev->certify_count;
@@ -1671,7 +1670,6 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     eval_count_kernel<<<grid, 256, 0, s>>>(cfg, b);
     screen_policy_kernel<<<1, 1, 0, s>>>(cfg, b);
   }
-  mark(marks, 2, s);
 
   // (4) sample, ArgMin, incumbent update and witness
   SampleArgs sa = {};
@@ -1703,6 +1701,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
   sa.capacity = cfg.sample_capacity;
   sa.lg_min = cfg.sample_lg_min;
   sa.chain = b.chain;
+  sa.t_first = b.dev->stamps + 2;
   if (cfg.precision == CMN_PRECISION_FP32_LAZY) {
     // FP32 screen of every sample, then each chunk's best in FP64
     SampleArgs qa = sa;
@@ -1713,6 +1712,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
                               : launch_sample_screen(qa, cfg.screen_grid, kEvalThreads, s);
     if (e != cudaSuccess) return e;
     sa.cbest = b.cbest;
+    sa.t_first = nullptr;
   }
   e = launch_sample(sa, sample_grid, kEvalThreads, s);
   if (e != cudaSuccess) return e;
@@ -1720,9 +1720,8 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
   const WitnessArgs w = {b.plo, b.phi, cfg.e_max, b.pinfo, b.slots, cfg.max_slots, b.kinds, cfg.n_vars, cfg.S, 0,
                          &b.dev->salt_base, 0, b.best_point};
   e = launch_candidate(b.block_best, sample_grid, best, w,
-                       Incumbent{&b.dev->done, &b.dev->gub, &b.dev->best, &b.dev->have_best, &b.dev->improved}, s);
+                       Incumbent{&b.dev->done, &b.dev->gub, &b.dev->best, &b.dev->have_best, &b.dev->improved, b.dev->stamps + 3}, s);
   if (e != cudaSuccess) return e;
-  mark(marks, 3, s);
 
   // (5) prune with the new incumbent and rebuild the pool
   prune_count_kernel<<<tiles(max_children), kScanBlock, 0, s>>>(cfg, b);
@@ -1747,7 +1746,6 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     const int grid = (int)std::min<uint64_t>((cfg.e_max + 255) / 256, 1024);
     stage_next_kernel<<<grid, 256, 0, s>>>(cfg, b);
   }
-  mark(marks, 4, s);
   return cudaGetLastError();
 }
 

@@ -341,7 +341,7 @@ class Solver:
 
     def phase_ms(self) -> list[float]:
         """[select+branch, bound, sample, prune+rebuild, whole] device ms of the
-        last iteration, from events recorded inside its graph."""
+        last iteration that expanded boxes, written by its kernels."""
         ms = (C.c_double * 5)()
         check(lib().cmn_solver_phase_ms(self.handle, ms))
         return list(ms)

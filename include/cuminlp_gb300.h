@@ -461,8 +461,8 @@ cmn_status cmn_solver_frontier(cmn_solver* solver, double* boxes,
                                double* lower_bounds, uint32_t* depths,
                                uint64_t room, uint64_t* count);
 
-/* Phase timings of the most recent iteration, from CUDA events recorded
- * inside the captured iteration: [0] select+branch, [1] bound (FP64
+/* Phase timings of the most recent iteration that expanded boxes, written
+ * by its kernels (device clock): [0] select+branch, [1] bound (FP64
  * evaluation, or FP32 screen + FP64 certify; in the lazy form the FP32
  * child bounds, the wait for the parents' FP64 verdict that runs beside
  * them, and the fold), [2] sample + incumbent, [3] prune + pool rebuild,
