@@ -1032,12 +1032,8 @@ struct cmn_solver {
   SolverCfg cfg{};
   SolverBufs b{};
   cudaStream_t stream = nullptr;
-  // the first iteration selects its parents; every later one finds them
-  // staged by its predecessor and runs the graph without the select
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  cudaGraph_t graph_steady = nullptr;
-  cudaGraphExec_t exec_steady = nullptr;
   SolverDev* h_dev = nullptr;  // pinned mirror
   uint64_t* d_viable = nullptr;
   uint64_t* h_viable = nullptr;
@@ -1059,8 +1055,6 @@ struct cmn_solver {
     if (side.stream) cudaStreamDestroy(side.stream);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
-    if (exec_steady) cudaGraphExecDestroy(exec_steady);
-    if (graph_steady) cudaGraphDestroy(graph_steady);
     if (slab) cudaFree(slab);
     if (h_dev) cudaFreeHost(h_dev);
     if (h_viable) cudaFreeHost(h_viable);
@@ -1260,22 +1254,18 @@ extern "C" cmn_status cmn_solver_create(const cmn_problem* p, const cmn_solve_op
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->side.stream, cudaStreamNonBlocking, prio_high);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->side.fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->side.join, cudaEventDisableTiming);
-    // capture one iteration, with and without the parent select
-    for (int steady = 0; steady < 2 && e == cudaSuccess; ++steady) {
-      cudaGraph_t* g = steady ? &s->graph_steady : &s->graph;
-      e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
-      if (e == cudaSuccess) {
-        cudaError_t e2 = solver_iteration(cfg, b, s->eval_grid, s->sample_grid, s->stream, s->side, steady == 0);
-        e = cudaStreamEndCapture(s->stream, g);
-        if (e2 != cudaSuccess) e = e2;
-      }
-      if (e == cudaSuccess) e = cudaGraphInstantiate(steady ? &s->exec_steady : &s->exec, *g, 0);
+    if (e == cudaSuccess) e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      cudaError_t e2 = solver_iteration(cfg, b, s->eval_grid, s->sample_grid, s->stream, s->side);
+      e = cudaStreamEndCapture(s->stream, &s->graph);
+      if (e2 != cudaSuccess) e = e2;
     }
-    if (e == cudaSuccess) {  // kernels of a steady iteration
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&s->exec, s->graph, 0);
+    if (e == cudaSuccess) {  // kernels of an iteration
       size_t nn = 0;
-      e = cudaGraphGetNodes(s->graph_steady, nullptr, &nn);
+      e = cudaGraphGetNodes(s->graph, nullptr, &nn);
       std::vector<cudaGraphNode_t> nodes(nn);
-      if (e == cudaSuccess && nn) e = cudaGraphGetNodes(s->graph_steady, nodes.data(), &nn);
+      if (e == cudaSuccess && nn) e = cudaGraphGetNodes(s->graph, nodes.data(), &nn);
       for (size_t i = 0; i < nn && e == cudaSuccess; ++i) {
         cudaGraphNodeType t;
         e = cudaGraphNodeGetType(nodes[i], &t);
@@ -1316,7 +1306,7 @@ extern "C" cmn_status cmn_solver_step(cmn_solver* s, uint64_t max_iterations)
   while (!s->h_dev->done && (max_iterations == 0 || done_iters < max_iterations)) {
     uint64_t k = burst;
     if (max_iterations) k = std::min<uint64_t>(k, max_iterations - done_iters);
-    for (uint64_t i = 0; i < k; ++i) CK(cudaGraphLaunch(s->launched + i == 0 ? s->exec : s->exec_steady, s->stream));
+    for (uint64_t i = 0; i < k; ++i) CK(cudaGraphLaunch(s->exec, s->stream));
     done_iters += k;
     s->launched += k;
     st = pull_state(s);

@@ -17,7 +17,6 @@ constexpr int kScanBlock = 512;  // threads per block of the compaction kernels
 constexpr int kScanItems = 8;    // items per thread
 constexpr int kScanTile = kScanBlock * kScanItems;
 constexpr int kHistUnroll = 8;   // entries per lane in flight in the radix histogram
-constexpr int kHistThreads = 256;  // threads of a radix histogram block
 
 constexpr uint8_t kSelAlive = 0;
 constexpr uint8_t kSelParent = 1;
@@ -69,7 +68,7 @@ struct SolverDev {
   uint64_t pre_k;
   uint64_t pre_count;
   uint32_t pre_valid;      // the staged parents are the next iteration's
-  uint32_t skip_select;    // this iteration's parents were staged already
+  uint32_t barrier;        // barriers of the rebuild passed (any launch)
   uint64_t certify_count;
   uint64_t evict;          // 1 when the rebuilt pool exceeds the cap
   uint64_t dropped_min_key;
@@ -83,7 +82,7 @@ struct SolverDev {
   uint32_t have_best;
   uint32_t improved;
   uint32_t error;
-  uint32_t ticket;         // blocks of the running histogram pass that are done
+  uint32_t ticket;         // blocks of the rebuild that reached its next barrier
   Cand best;
   cmn_counters counters;
   uint64_t stamps[8];      // phase boundaries of the last iteration (ns); solver_iteration
@@ -202,11 +201,9 @@ struct SideStream {
 // after branching, after bounding, after sampling, end); in the lazy form 5
 // and 6 around the FP64 verdict on the side stream and 7 after the FP32 child
 // bounds.
-// `with_select`: the iteration selects and stages its own parents (the first
-// iteration); otherwise the previous iteration staged them, and the
-// iteration flags a device error if it did not.
+// The parents were staged by the previous iteration, or by solver_init.
 cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval_grid, int sample_grid,
-                             cudaStream_t s, const SideStream& side, bool with_select);
+                             cudaStream_t s, const SideStream& side);
 // Fills min key / viable count of the current pool (after the run).
 cudaError_t solver_pool_stats(const SolverCfg& cfg, const SolverBufs& b, uint64_t* viable_dev, cudaStream_t s);
 // Copies pool entries [start, start + count) in position order: boxes as

@@ -39,8 +39,17 @@ __global__ void init_kernel(const SolverCfg cfg, const SolverBufs b, const doubl
 {
   const int t = threadIdx.x + blockIdx.x * blockDim.x;
   for (int v = t; v < cfg.n_vars; v += blockDim.x * gridDim.x) {  // the root box in store slot 0
-    b.lo[v] = root_lb[v];
-    b.hi[v] = root_ub[v];
+    const double lo = root_lb[v], hi = root_ub[v];
+    b.lo[v] = lo;
+    b.hi[v] = hi;
+    // and staged: the first iteration's parent
+    const uint64_t at = (uint64_t)v * cfg.e_max;
+    b.plo[at] = lo;
+    b.phi[at] = hi;
+    if (b.plo32 != nullptr) {
+      b.plo32[at] = __double2float_rd(lo);
+      b.phi32[at] = __double2float_ru(hi);
+    }
   }
   if (t == 0) {
     SolverDev* d = b.dev;
@@ -52,6 +61,10 @@ __global__ void init_kernel(const SolverCfg cfg, const SolverBufs b, const doubl
     b.lb[0][0] = -DBL_MAX;
     b.slot[0][0] = 0;
     b.depth[0] = 0;
+    b.sel[0][0] = kSelParent;
+    b.pdepth[0] = 0;
+    d->pre_valid = 1;
+    d->pre_k = 1;
     d->free_top = cfg.pstride - 1;
     d->pool_size = 1;
     d->pool_min_key = lb_key(-DBL_MAX);
@@ -72,7 +85,7 @@ __global__ void free_init_kernel(const SolverCfg cfg, const SolverBufs b)
 
 // Top of the loop of search/driver.hpp:221-233: convergence of the least
 // pending lower bound, the expansion budget, and this iteration's size.
-__global__ void begin_kernel(const SolverCfg cfg, const SolverBufs b, int require_staged)
+__global__ void begin_kernel(const SolverCfg cfg, const SolverBufs b)
 {
   SolverDev* d = b.dev;
   d->improved = 0;  // an iteration after the stop must not rewrite the witness
@@ -98,9 +111,9 @@ __global__ void begin_kernel(const SolverCfg cfg, const SolverBufs b, int requir
   if (E > left) E = left;
   const uint64_t t = now_ns();
   for (int i = 0; i < 8; ++i) d->stamps[i] = t;
-  // the previous iteration staged the E best entries of this pool already
-  d->skip_select = (d->pre_valid && d->pre_k == E) ? 1u : 0u;
-  if (require_staged && !d->skip_select) d->error = 1;
+  // the previous iteration's rebuild (the first one: init_kernel) staged the E
+  // best entries of this pool
+  if (!d->pre_valid || d->pre_k != E) d->error = 1;
   d->pre_valid = 0;
   d->pre_k = 0;
   d->pre_count = 0;
@@ -128,11 +141,9 @@ __global__ void begin_kernel(const SolverCfg cfg, const SolverBufs b, int requir
 // ---------------------------------------------------------------------
 // radix select of the k-th smallest lower-bound key
 // ---------------------------------------------------------------------
-// which = 0: the current pool (n = pool_size; one target, k = n_parents),
-//            the first iteration only
-// which = 1: the current buffer after the children were appended behind
-//            the pool (n = extent), alive entries only; target 0 the cap
-//            (when evicting), target 1 the next iteration's parents
+// over the current buffer after the children were appended behind the pool
+// (n = extent), alive entries only: target 0 the cap (when evicting), target 1
+// the next iteration's parents
 
 // one of the two pool buffers without indexing the parameter arrays by a
 // runtime value (which would copy them to local memory)
@@ -145,42 +156,21 @@ __device__ __forceinline__ T* parity_buf(T* const (&a)[2], uint32_t p)
 __device__ __forceinline__ const double* pool_lb(const SolverBufs& b) { return parity_buf(b.lb, b.dev->parity); }
 __device__ __forceinline__ uint8_t* pool_sel(const SolverBufs& b) { return parity_buf(b.sel, b.dev->parity); }
 
-__device__ __forceinline__ uint64_t rs_n(const SolverDev* d, int which)
-{
-  return which == 0 ? d->pool_size : d->extent;
-}
-
-// Number of select targets of a pass: which = 0 selects this iteration's
-// parents; which = 1 selects the entries that stay under the cap (target 0)
-// and, among them, the next iteration's parents (target 1).
-__device__ __forceinline__ int n_targets(int which) { return which == 0 ? 1 : 2; }
-
 __device__ __forceinline__ bool target_live(const RadixState& r)
 {
   return r.active && !r.settled && r.bits_left != 0;
 }
 
-__device__ void radix_init(const SolverCfg& cfg, const SolverBufs& b, int which)
+__device__ void radix_init(const SolverCfg& cfg, const SolverBufs& b)
 {
-  SolverDev* d = b.dev;
-  for (int t = 0; t < n_targets(which); ++t) {
+  const SolverDev* d = b.dev;
+  for (int t = 0; t < 2; ++t) {
     RadixState* rs = b.radix + t;
-    uint64_t k;
-    bool active;
-    if (which == 0) {
-      k = d->n_parents;
-      active = !d->done && !d->skip_select && k < d->pool_size;
-    } else if (t == 0) {
-      k = cfg.cap;
-      active = !d->done && d->evict && k < d->new_size;
-    } else {
-      k = d->pre_k;
-      active = !d->done && k > 0 && k < d->new_size;
-    }
+    const uint64_t k = t == 0 ? cfg.cap : d->pre_k;
+    const bool active = (t == 0 ? d->evict != 0 : k > 0) && k < d->new_size;
     for (int i = threadIdx.x; i < kRadixBins; i += blockDim.x) rs->hist[i] = 0;
     if (threadIdx.x == 0) {
-      const uint64_t lo = which == 0 ? d->pool_min_key : d->evict_lo_key;
-      const uint64_t hi = which == 0 ? d->pool_max_key : d->evict_hi_key;
+      const uint64_t lo = d->evict_lo_key, hi = d->evict_hi_key;
       const int common = lo <= hi ? ((lo ^ hi) == 0 ? 64 : __clzll((long long)(lo ^ hi))) : 0;
       const uint64_t top = common == 0 ? 0 : (~0ULL << (64 - common));
       rs->prefix = lo & top;
@@ -195,15 +185,13 @@ __device__ void radix_init(const SolverCfg& cfg, const SolverBufs& b, int which)
   }
 }
 
-__global__ void radix_init_kernel(const SolverCfg cfg, const SolverBufs b, int which) { radix_init(cfg, b, which); }
-
 // Picks the digit whose bin holds the k-th entry: a scan over the bins by one
-// block of kHistThreads. When the entries up to and including that bin are
+// block of kScanBlock threads. When the entries up to and including that bin are
 // exactly k, the bin is taken whole and the search stops.
 __device__ void radix_pick(const SolverBufs& b, RadixState* rs)
 {
-  constexpr int kPer = kRadixBins / kHistThreads;
-  __shared__ uint64_t warp_sum[kHistThreads / 32];
+  constexpr int kPer = kRadixBins / kScanBlock;
+  __shared__ uint64_t warp_sum[kScanBlock / 32];
   __shared__ int pick_d;
   __shared__ uint64_t pick_cum, pick_cnt;
   const int bits = rs->bits_left < (uint32_t)kRadixBits ? (int)rs->bits_left : kRadixBits;
@@ -260,18 +248,17 @@ __device__ void radix_pick(const SolverBufs& b, RadixState* rs)
 }
 
 // One digit's histogram per live target over the entries inside its
-// bucket, in one read of the keys. Each thread counts a run of equal bins
-// in registers and adds it to the block's shared histogram only when the
-// bin changes: converging lower bounds share most leading digits, so a pass
-// makes few shared-memory atomics instead of one per entry on one address.
-__global__ void __launch_bounds__(kHistThreads) radix_hist_kernel(const SolverCfg cfg, const SolverBufs b, int which)
+// bucket, in one read of the keys; false when no target is live. Each thread
+// counts a run of equal bins in registers and adds it to the block's shared
+// histogram only when the bin changes: converging lower bounds share most
+// leading digits, so a pass makes few shared-memory atomics instead of one per
+// entry on one address.
+__device__ __forceinline__ bool radix_hist(const SolverBufs& b, uint64_t n, uint32_t parity, bool (&go)[2])
 {
   __shared__ uint32_t h[2][kRadixBins];
-  const int T = n_targets(which);
-  bool go[2] = {false, false};
   int shift[2] = {0, 0}, nb[2] = {1, 1};
   uint64_t prefix[2] = {0, 0}, mask[2] = {0, 0};
-  for (int t = 0; t < T; ++t) {
+  for (int t = 0; t < 2; ++t) {
     const RadixState& r = b.radix[t];
     go[t] = target_live(r);
     if (!go[t]) continue;
@@ -281,17 +268,16 @@ __global__ void __launch_bounds__(kHistThreads) radix_hist_kernel(const SolverCf
     prefix[t] = r.prefix;
     mask[t] = r.mask;
   }
-  if (!go[0] && !go[1]) return;
+  if (!go[0] && !go[1]) return false;
   // while both targets sit in the same bucket (the first pass of a rebuild)
   // their histograms are the same: count once, add to both
   const bool same = go[0] && go[1] && prefix[0] == prefix[1] && mask[0] == mask[1] && shift[0] == shift[1];
   const bool count1 = go[1] && !same;
-  const uint64_t n = rs_n(b.dev, which);
   for (int t = 0; t < 2; ++t)
     for (int i = threadIdx.x; i < kRadixBins; i += blockDim.x) h[t][i] = 0;
   __syncthreads();
-  const uint64_t* __restrict__ lb = reinterpret_cast<const uint64_t*>(pool_lb(b));
-  const uint8_t* __restrict__ sel = which == 1 ? pool_sel(b) : nullptr;
+  const uint64_t* __restrict__ lb = reinterpret_cast<const uint64_t*>(parity_buf(b.lb, parity));
+  const uint8_t* sel = parity_buf(b.sel, parity);
   const int lane = threadIdx.x & 31;
   // each warp takes chunks of 32 x kHistUnroll consecutive entries and
   // issues all their loads before it bins them
@@ -306,7 +292,7 @@ __global__ void __launch_bounds__(kHistThreads) radix_hist_kernel(const SolverCf
       const uint64_t i = c * kChunk + (uint64_t)u * 32 + lane;
       in[u] = i < n;
       x[u] = in[u] ? lb[i] : 0;
-      if (sel != nullptr && in[u]) in[u] = sel[i] == kSelAlive;
+      if (in[u]) in[u] = sel[i] == kSelAlive;
     }
 #pragma unroll
     for (int u = 0; u < kHistUnroll; ++u) {
@@ -328,25 +314,13 @@ __global__ void __launch_bounds__(kHistThreads) radix_hist_kernel(const SolverCf
   for (int t = 0; t < 2; ++t)
     if (run[t]) atomicAdd(&h[t][run_bin[t]], run[t]);
   __syncthreads();
-  for (int t = 0; t < T; ++t) {
+  for (int t = 0; t < 2; ++t) {
     if (!go[t]) continue;
     const uint32_t* src = (t == 1 && same) ? h[0] : h[t];
     for (int i = threadIdx.x; i < nb[t]; i += blockDim.x)
       if (src[i]) atomicAdd(&b.radix[t].hist[i], src[i]);
   }
-  // the last block to add its counts picks the digits: every block takes one
-  // ticket, and none waits
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&b.dev->ticket, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int t = 0; t < T; ++t)
-    if (go[t]) radix_pick(b, b.radix + t);
-  if (threadIdx.x == 0) b.dev->ticket = 0;
-  (void)cfg;
+  return true;
 }
 
 // ---------------------------------------------------------------------
@@ -355,9 +329,10 @@ __global__ void __launch_bounds__(kHistThreads) radix_hist_kernel(const SolverCf
 // so every pass reads whole cache lines and keeps kScanItems loads in flight
 // per thread.
 // ---------------------------------------------------------------------
-// first item of this thread in its block's tile, read once per kernel (the
-// special registers are slow to re-read)
-__device__ __forceinline__ uint64_t tile_first() { return (uint64_t)blockIdx.x * kScanTile + threadIdx.x; }
+// first item of this thread in a tile (by default its block's), read once per
+// kernel (the special registers are slow to re-read)
+__device__ __forceinline__ uint64_t tile_first(uint64_t tile) { return tile * kScanTile + threadIdx.x; }
+__device__ __forceinline__ uint64_t tile_first() { return tile_first(blockIdx.x); }
 
 __device__ __forceinline__ uint64_t tile_item(uint64_t t0, int j) { return t0 + (uint64_t)j * kScanBlock; }
 
@@ -406,13 +381,14 @@ __device__ __forceinline__ int tile_ranks(const bool (&f)[kScanItems], int (&ran
   return tile_total;
 }
 
-// tile_ranks of two flag sets with one pair of barriers
+// tile_ranks of two flag sets with one pair of barriers; their counts in `total`
 __device__ __forceinline__ void tile_ranks2(const bool (&f)[kScanItems], const bool (&g)[kScanItems],
-                                            int (&rf)[kScanItems], int (&rg)[kScanItems])
+                                            int (&rf)[kScanItems], int (&rg)[kScanItems], int (&total)[2])
 {
   constexpr int kWarps = kScanBlock / 32;
   constexpr int kPer = kScanItems * kWarps / 32;
   __shared__ int tab[2][kScanItems * kWarps];
+  __shared__ int tile_total[2];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   unsigned bf[kScanItems], bg[kScanItems];
 #pragma unroll
@@ -444,8 +420,11 @@ __device__ __forceinline__ void tile_ranks2(const bool (&f)[kScanItems], const b
       t[lane * kPer + e] = run;
       run += v[e];
     }
+    if (lane == 31) tile_total[wid] = x;
   }
   __syncthreads();
+  total[0] = tile_total[0];
+  total[1] = tile_total[1];
   const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
   for (int j = 0; j < kScanItems; ++j) {
@@ -536,31 +515,14 @@ __device__ __forceinline__ uint64_t block_min(uint64_t m)
   return acc;
 }
 
-// Exclusive scan of the tile counts of `*n_items` items (a block of 1024
-// threads each); writes the total to *total_out when given.
-struct ScanArgs {
-  const uint32_t* counts;
-  uint32_t* offsets;
-  uint64_t* total_out;
-  const uint32_t* active;
-};
-
-__global__ void __launch_bounds__(1024) scan_kernel(const ScanArgs first, const ScanArgs second,
-                                                    const uint64_t* __restrict__ n_items,
-                                                    const uint32_t* __restrict__ skip,
+// Exclusive scan of the tile counts of `*n_items` items (one block of 1024
+// threads); writes the total to *total_out.
+__global__ void __launch_bounds__(1024) scan_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets,
+                                                    const uint64_t* __restrict__ n_items, uint64_t* total_out,
                                                     const uint32_t* __restrict__ done)
 {
-  const ScanArgs& a = blockIdx.x == 0 ? first : second;
-  const uint32_t* __restrict__ counts = a.counts;
-  uint32_t* __restrict__ offsets = a.offsets;
-  uint64_t* const total_out = a.total_out;
-  const uint32_t* const active = a.active;
   __shared__ uint64_t warp_sum[32];
-  if (*done || (skip && *skip)) return;
-  if (active && !*active) {
-    if (threadIdx.x == 0 && total_out) *total_out = 0;
-    return;
-  }
+  if (*done) return;
   const uint64_t n = *n_items;
   const uint64_t nblocks = (n + kScanTile - 1) / kScanTile;
   // each thread sums a run of consecutive counts, the block scans the sums
@@ -589,7 +551,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(const ScanArgs first, const 
   }
   __syncthreads();
   uint64_t run = x - sum + (wid > 0 ? warp_sum[wid - 1] : 0);
-  if (threadIdx.x == blockDim.x - 1 && total_out) *total_out = run + sum;
+  if (threadIdx.x == blockDim.x - 1) *total_out = run + sum;
   for (uint64_t i = b0; i < b1; ++i) {
     offsets[i] = (uint32_t)run;
     run += src[i];
@@ -634,37 +596,6 @@ __global__ void __launch_bounds__(kScanBlock) count_kernel(const P pred, uint32_
   if (threadIdx.x == 0) counts[blockIdx.x] = (uint32_t)c;
 }
 
-// Tile counts of the alive entries inside each ranked target's threshold
-// bucket (target 0 into block_counts, target 1 into block_counts2).
-__global__ void __launch_bounds__(kScanBlock) eq_count_kernel(const SolverCfg cfg, const SolverBufs b, int which)
-{
-  const uint64_t t0 = tile_first();
-  const SolverDev* d = b.dev;
-  const RadixState* rs = b.radix;
-  const bool r0 = rs[0].rank != 0, r1 = which == 1 && rs[1].rank != 0;
-  if (d->done || (!r0 && !r1)) return;
-  const uint64_t n = rs_n(d, which);
-  if ((uint64_t)blockIdx.x * kScanTile >= n) return;
-  const uint64_t* __restrict__ lb = reinterpret_cast<const uint64_t*>(pool_lb(b));
-  const uint8_t* __restrict__ sel = pool_sel(b);
-  int c0 = 0, c1 = 0;
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    const uint64_t i = tile_item(t0, j);
-    if (i >= n || (which == 1 && sel[i] != kSelAlive)) continue;
-    const uint64_t key = bits_key(lb[i]);
-    c0 += (r0 && (key & rs[0].mask) == rs[0].prefix) ? 1 : 0;
-    c1 += (r1 && (key & rs[1].mask) == rs[1].prefix) ? 1 : 0;
-  }
-  c0 = tile_count<0>(c0);
-  c1 = tile_count<1>(c1);
-  if (threadIdx.x == 0) {
-    if (r0) b.block_counts[blockIdx.x] = (uint32_t)c0;
-    if (r1) b.block_counts2[blockIdx.x] = (uint32_t)c1;
-  }
-  (void)cfg;
-}
-
 // The select decision of one target for one entry (`key` already masked).
 struct TargetView {
   bool active, settled, ranked;
@@ -680,120 +611,6 @@ struct TargetView {
     return (key & mask) < prefix;
   }
 };
-
-// Marks the k smallest (key, position) entries of each target: all keys
-// below the threshold bucket, and the first `k` entries inside it in
-// position order (all of them once the bucket is settled).
-//   which = 0: marks this iteration's parents kSelParent and the others
-//              kSelAlive, and writes the tile counts of the parents;
-//   which = 1: marks alive entries outside the cap kSelEvicted (leaving the
-//              parents' holes as they are) and folds them into the dropped
-//              floor (search/budget.hpp:190-209); marks the next iteration's
-//              parents among those that stay kSelNextParent; writes the tile
-//              counts of the entries that stay and of the next parents.
-__global__ void __launch_bounds__(kScanBlock, 2) mark_kernel(const SolverCfg cfg, const SolverBufs b, int which)
-{
-  const uint64_t t0 = tile_first();
-  SolverDev* d = b.dev;
-  if (which == 0 && d->skip_select) return;
-  // the control words and the tile's entries are loaded together: a tile is
-  // short, so a chain of dependent loads would set its duration
-  const uint32_t done = d->done, skip = d->skip_select;
-  const uint64_t n = rs_n(d, which);
-  const uint64_t pre_k = d->pre_k;
-  const uint64_t* __restrict__ lb = reinterpret_cast<const uint64_t*>(pool_lb(b));
-  uint8_t* __restrict__ sel = pool_sel(b);
-  uint64_t x[kScanItems];  // raw bits of the lower bounds
-  uint8_t sv[kScanItems];
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    const uint64_t i = tile_item(t0, j);
-    const bool inb = i < cfg.pstride;
-    x[j] = inb ? lb[i] : 0;
-    sv[j] = (which == 1 && inb) ? sel[i] : kSelAlive;
-  }
-  if (done || (which == 0 && skip)) return;
-  if ((uint64_t)blockIdx.x * kScanTile >= n) return;
-  const TargetView A(b.radix[0]);
-  const bool pre = which == 1 && pre_k > 0;
-  const TargetView B(b.radix[which == 1 ? 1 : 0]);
-  const uint64_t gub = dbits(d->gub);
-  bool alive[kScanItems], eqA[kScanItems], eqB[kScanItems];
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    alive[j] = tile_item(t0, j) < n && sv[j] == kSelAlive;
-    const uint64_t key = bits_key(x[j]);
-    eqA[j] = A.active && alive[j] && (key & A.mask) == A.prefix;
-    eqB[j] = pre && B.active && alive[j] && (key & B.mask) == B.prefix;
-  }
-  int rankA[kScanItems] = {}, rankB[kScanItems] = {};
-  uint64_t baseA = 0, baseB = 0;
-  if (A.ranked) {  // the same for the whole grid
-    tile_ranks<0>(eqA, rankA);
-    baseA = b.block_offsets[blockIdx.x];
-  }
-  if (pre && B.ranked) {
-    tile_ranks<1>(eqB, rankB);
-    baseB = b.block_offsets2[blockIdx.x];
-  }
-  int outA = 0, outB = 0;
-  uint32_t viable = 0, dominated = 0;
-  uint64_t mkey = ~0ULL;
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    if (!alive[j]) continue;
-    const uint64_t key = bits_key(x[j]);
-    const bool ta = A.take(key, eqA[j], baseA + (uint64_t)rankA[j]);
-    const bool tb = pre && ta && B.take(key, eqB[j], baseB + (uint64_t)rankB[j]);
-    const uint64_t i = tile_item(t0, j);
-    if (which == 0) {
-      sel[i] = ta ? kSelParent : kSelAlive;
-    } else if (!ta) {
-      sel[i] = kSelEvicted;
-      if (bits_le(x[j], gub)) {
-        ++viable;
-        mkey = key < mkey ? key : mkey;
-      } else {
-        ++dominated;
-      }
-    } else if (tb) {
-      sel[i] = kSelNextParent;
-    }
-    outA += ta ? 1 : 0;
-    outB += tb ? 1 : 0;
-  }
-  // the tile's counts and the eviction tallies, with one barrier
-  struct Part {
-    uint32_t a, b, viable, dominated;
-    uint64_t mkey;
-  };
-  __shared__ Part part[kScanBlock / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  {
-    const uint32_t pa = __reduce_add_sync(0xffffffffu, (uint32_t)outA);
-    const uint32_t pb = __reduce_add_sync(0xffffffffu, (uint32_t)outB);
-    const uint32_t pv = __reduce_add_sync(0xffffffffu, viable);
-    const uint32_t pd = __reduce_add_sync(0xffffffffu, dominated);
-    const uint64_t pm = warp_min_u64(mkey);
-    if (lane == 0) part[wid] = Part{pa, pb, pv, pd, pm};
-  }
-  __syncthreads();
-  if (wid != 0) return;
-  const bool has = lane < kScanBlock / 32;
-  const uint32_t ta = __reduce_add_sync(0xffffffffu, has ? part[lane].a : 0u);
-  const uint32_t tb = __reduce_add_sync(0xffffffffu, has ? part[lane].b : 0u);
-  const uint32_t tv = __reduce_add_sync(0xffffffffu, has ? part[lane].viable : 0u);
-  const uint32_t td = __reduce_add_sync(0xffffffffu, has ? part[lane].dominated : 0u);
-  const uint64_t tm = warp_min_u64(has ? part[lane].mkey : ~0ULL);
-  if (lane != 0) return;
-  b.block_counts[blockIdx.x] = ta;
-  if (which == 1) b.block_counts2[blockIdx.x] = tb;
-  if (which == 1 && A.active) {
-    if (tv) atomicAdd((unsigned long long*)&d->counters.dropped_viable, (unsigned long long)tv);
-    if (td) atomicAdd((unsigned long long*)&d->counters.dropped_dominated, (unsigned long long)td);
-    if (tm != ~0ULL) atomicMin((unsigned long long*)&d->dropped_min_key, (unsigned long long)tm);
-  }
-}
 
 // stage the box in store slot `s` as parent `pos` of the staging planes
 __device__ __forceinline__ void stage_parent(const SolverCfg& cfg, const SolverBufs& b, uint64_t s, uint64_t pos)
@@ -915,158 +732,6 @@ __global__ void __launch_bounds__(kScanBlock) scatter_kernel(const P pred, const
 #pragma unroll
   for (int j = 0; j < kScanItems; ++j)
     if (f[j]) op(tile_item(t0, j), base + (uint64_t)rank[j]);
-}
-
-// Stages this iteration's parents (kSelParent entries of the pool, in
-// position order) from the store into the parent planes, unless the
-// previous iteration staged them.
-__global__ void __launch_bounds__(kScanBlock) gather_parents_kernel(const SolverCfg cfg, const SolverBufs b,
-                                                                    const uint32_t* __restrict__ offsets)
-{
-  const uint64_t t0 = tile_first();
-  const SolverDev* d = b.dev;
-  if (d->done || d->skip_select) return;
-  const uint64_t n = d->pool_size;
-  const uint64_t base = offsets[blockIdx.x];
-  const uint8_t* __restrict__ sel = pool_sel(b);
-  uint8_t sv[kScanItems];
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    const uint64_t i = tile_item(t0, j);
-    sv[j] = i < cfg.pstride ? sel[i] : kSelAlive;
-  }
-  if ((uint64_t)blockIdx.x * kScanTile >= n) return;
-  bool f[kScanItems];
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) f[j] = tile_item(t0, j) < n && sv[j] == kSelParent;
-  int rank[kScanItems];
-  tile_ranks(f, rank);
-  const uint32_t* slot = parity_buf(b.slot, d->parity);
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j)
-    if (f[j]) stage_parent(cfg, b, slot[tile_item(t0, j)], base + (uint64_t)rank[j]);
-}
-
-// Moves the entries that stay, in order, to the other buffer (lower bound,
-// store slot and mark), folds their keys into the pool's key range, lists
-// the store slots of the next iteration's parents among them in order, and
-// pushes the store slots of the others (this iteration's parents and the
-// evicted) onto the free stack in position order.
-__global__ void __launch_bounds__(kScanBlock, 2) copy_pool_kernel(const SolverCfg cfg, const SolverBufs b)
-{
-  const uint64_t t0 = tile_first();
-  SolverDev* d = b.dev;
-  // control words, the tile's entries and its offsets are loaded together
-  const uint32_t done = d->done;
-  const uint64_t n = d->extent;
-  const uint64_t free_base = d->free_top;
-  const uint32_t p = d->parity, q = 1 - p;
-  const uint64_t* __restrict__ slb = reinterpret_cast<const uint64_t*>(parity_buf(b.lb, p));
-  const uint32_t* __restrict__ sslot = parity_buf(b.slot, p);
-  const uint8_t* __restrict__ ssel = parity_buf(b.sel, p);
-  uint64_t* __restrict__ dlb = reinterpret_cast<uint64_t*>(parity_buf(b.lb, q));
-  uint32_t* __restrict__ dslot = parity_buf(b.slot, q);
-  uint8_t* __restrict__ dsel = parity_buf(b.sel, q);
-  const uint64_t base = b.block_offsets[blockIdx.x];
-  const uint64_t pbase = b.block_offsets2[blockIdx.x];
-  bool f[kScanItems], g[kScanItems], in[kScanItems];
-  uint64_t x[kScanItems];  // raw bits of the lower bounds
-  uint32_t sl[kScanItems];
-  uint8_t sv[kScanItems];
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    const uint64_t i = tile_item(t0, j);
-    const bool inb = i < cfg.pstride;
-    sv[j] = inb ? ssel[i] : kSelParent;
-    x[j] = inb ? slb[i] : 0;
-    sl[j] = inb ? sslot[i] : 0u;
-  }
-  if (done) return;
-  if ((uint64_t)blockIdx.x * kScanTile >= n) return;
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    in[j] = tile_item(t0, j) < n;
-    f[j] = in[j] && (sv[j] == kSelAlive || sv[j] == kSelNextParent);
-    g[j] = in[j] && sv[j] == kSelNextParent;
-  }
-  // the key range of the entries that stay, per warp before the barriers
-  // of the ranks, for thread 0 after them
-  __shared__ uint64_t part_min[kScanBlock / 32], part_max[kScanBlock / 32];
-  {
-    uint64_t mkey = ~0ULL, xkey = 0;
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j)
-      if (f[j]) {
-        const uint64_t k = bits_key(x[j]);
-        mkey = k < mkey ? k : mkey;
-        xkey = k > xkey ? k : xkey;
-      }
-    mkey = warp_min_u64(mkey);
-    xkey = warp_max_u64(xkey);
-    if ((threadIdx.x & 31) == 0) {
-      part_min[threadIdx.x >> 5] = mkey;
-      part_max[threadIdx.x >> 5] = xkey;
-    }
-  }
-  int rank[kScanItems], prank[kScanItems];  // stayers / next parents before each item
-  tile_ranks2(f, g, rank, prank);
-  if (threadIdx.x == 0) {
-    uint64_t mkey = ~0ULL, xkey = 0;
-    for (int w = 0; w < kScanBlock / 32; ++w) {
-      mkey = part_min[w] < mkey ? part_min[w] : mkey;
-      xkey = part_max[w] > xkey ? part_max[w] : xkey;
-    }
-    if (mkey != ~0ULL) atomicMin((unsigned long long*)&d->pool_min_key, (unsigned long long)mkey);
-    if (xkey != 0) atomicMax((unsigned long long*)&d->pool_max_key, (unsigned long long)xkey);
-  }
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    if (!in[j]) continue;
-    const uint64_t i = tile_item(t0, j);
-    const uint64_t stay_before = base + (uint64_t)rank[j];
-    if (f[j]) {
-      dlb[stay_before] = x[j];
-      dslot[stay_before] = sl[j];
-      dsel[stay_before] = g[j] ? kSelParent : kSelAlive;
-      if (g[j]) {
-        const uint64_t pos = pbase + (uint64_t)prank[j];
-        if (pos < cfg.e_max) b.pslot[pos] = sl[j];
-        else d->error = 1;
-      }
-    } else {
-      b.free_slots[free_base + (i - stay_before)] = sl[j];
-    }
-  }
-}
-
-__device__ void finish_pool(const SolverCfg& cfg, const SolverBufs& b)
-{
-  SolverDev* d = b.dev;
-  // the survivors were moved to the other buffer: exactly the cap when
-  // evicting, otherwise every alive entry
-  const uint64_t expect = d->evict ? cfg.cap : d->new_size;
-  if (d->survivors != expect) d->error = 1;
-  d->free_top += d->extent - d->survivors;  // the parents' and the evicted slots
-  if (d->free_top + d->survivors != cfg.pstride) d->error = 1;
-  if (d->pre_count != d->pre_k) d->error = 1;
-  d->pre_valid = d->pre_k > 0 ? 1u : 0u;
-  d->pool_size = d->survivors;
-  d->parity = 1 - d->parity;
-  if (d->dropped_min_key != ~0ULL) d->dropped_lb_min = key_to_lb(d->dropped_min_key);
-  if (d->pool_size > d->counters.peak_frontier) d->counters.peak_frontier = d->pool_size;
-}
-
-// Stages the next iteration's parents listed by the pool move; one thread
-// closes the iteration (it writes nothing the staging reads).
-__global__ void stage_next_kernel(const SolverCfg cfg, const SolverBufs b)
-{
-  const SolverDev* d = b.dev;
-  if (d->done) return;
-  const uint64_t n = d->pre_count < cfg.e_max ? d->pre_count : cfg.e_max;
-  if (blockIdx.x == 0 && threadIdx.x == 0) finish_pool(cfg, b);
-  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
-    stage_parent(cfg, b, b.pslot[k], k);
-  if (threadIdx.x == 0) stamp_last(b.dev->stamps + 4, (uint64_t)blockIdx.x * blockDim.x < n);
 }
 
 // appends the kept children listed (in order) by the compaction, one thread
@@ -1424,12 +1089,323 @@ __device__ void size_pool(const SolverCfg& cfg, const SolverBufs& b)
   d->pool_max_key = 0;
 }
 
-// Sizes of the rebuilt pool, and the start of its select (one block).
-__global__ void size_kernel(const SolverCfg cfg, const SolverBufs b)
+__device__ void finish_pool(const SolverCfg& cfg, const SolverBufs& b)
 {
-  if (threadIdx.x == 0 && !b.dev->done) size_pool(cfg, b);
+  SolverDev* d = b.dev;
+  // the survivors were moved to the other buffer: exactly the cap when
+  // evicting, otherwise every alive entry
+  const uint64_t expect = d->evict ? cfg.cap : d->new_size;
+  if (d->survivors != expect) d->error = 1;
+  d->free_top += d->extent - d->survivors;  // the parents' and the evicted slots
+  if (d->free_top + d->survivors != cfg.pstride) d->error = 1;
+  if (d->pre_count != d->pre_k) d->error = 1;
+  d->pre_valid = d->pre_k > 0 ? 1u : 0u;
+  d->pool_size = d->survivors;
+  d->parity = 1 - d->parity;
+  if (d->dropped_min_key != ~0ULL) d->dropped_lb_min = key_to_lb(d->dropped_min_key);
+  if (d->pool_size > d->counters.peak_frontier) d->counters.peak_frontier = d->pool_size;
+}
+
+// ---------------------------------------------------------------------
+// the pool's rebuild, one launch
+// ---------------------------------------------------------------------
+// A barrier of the launch's blocks: every block takes a ticket, the last one
+// runs `last` and opens it.  The launch is cooperative, so every block is
+// resident and the others wait no longer than a pass takes; the wait has a
+// limit (about a second) all the same, after which the device error is set and
+// false returned.
+constexpr uint32_t kBarrierSpins = 1u << 21;
+template <class F>
+__device__ __forceinline__ bool grid_barrier(SolverDev* d, F last)
+{
+  __shared__ int last_s, ok_s;
   __syncthreads();
-  radix_init(cfg, b, 1);
+  uint32_t gen = 0;
+  if (threadIdx.x == 0) {
+    gen = *(volatile uint32_t*)&d->barrier;
+    __threadfence();
+    last_s = atomicAdd(&d->ticket, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (last_s) {
+    last();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      d->ticket = 0;
+      __threadfence();
+      atomicAdd(&d->barrier, 1u);
+      ok_s = 1;
+    }
+  } else if (threadIdx.x == 0) {
+    int ok = 0;
+    for (uint32_t i = 0; i < kBarrierSpins && !ok; ++i) ok = *(volatile uint32_t*)&d->barrier != gen;
+    if (!ok) d->error = 1;
+    __threadfence();
+    ok_s = ok;
+  }
+  __syncthreads();
+  return ok_s != 0;
+}
+
+// Sums of two per-block counts over the blocks before this one, and over all.
+__device__ __forceinline__ void blocks_before(const uint32_t* c0, const uint32_t* c1, uint64_t (&before)[2],
+                                              uint64_t (&all)[2])
+{
+  __shared__ unsigned long long acc[4];
+  __syncthreads();
+  if (threadIdx.x < 4) acc[threadIdx.x] = 0;
+  __syncthreads();
+  unsigned long long v[4] = {};
+  for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+    const uint32_t a = __ldcg(c0 + i), c = __ldcg(c1 + i);
+    v[2] += a;
+    v[3] += c;
+    if (i < blockIdx.x) {
+      v[0] += a;
+      v[1] += c;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    for (int off = 16; off > 0; off >>= 1) v[e] += __shfl_down_sync(0xffffffffu, v[e], off);
+    if ((threadIdx.x & 31) == 0 && v[e]) atomicAdd(&acc[e], v[e]);
+  }
+  __syncthreads();
+  before[0] = acc[0];
+  before[1] = acc[1];
+  all[0] = acc[2];
+  all[1] = acc[3];
+}
+
+// Alive entries of tile `tile` inside each ranked target's threshold bucket.
+__device__ __forceinline__ void eq_count(const SolverBufs& b, uint64_t tile, uint64_t n, uint32_t p,
+                                         const TargetView& A, const TargetView& B, int (&c)[2])
+{
+  const uint64_t t0 = tile_first(tile);
+  const uint64_t* __restrict__ lb = reinterpret_cast<const uint64_t*>(parity_buf(b.lb, p));
+  const uint8_t* sel = parity_buf(b.sel, p);
+#pragma unroll
+  for (int j = 0; j < kScanItems; ++j) {
+    const uint64_t i = tile_item(t0, j);
+    if (i >= n || sel[i] != kSelAlive) continue;
+    const uint64_t key = bits_key(lb[i]);
+    c[0] += (A.ranked && (key & A.mask) == A.prefix) ? 1 : 0;
+    c[1] += (B.ranked && (key & B.mask) == B.prefix) ? 1 : 0;
+  }
+}
+
+// Marks the k smallest (key, position) entries of each target among a tile's
+// alive ones: all keys below the threshold bucket, and the entries inside it
+// by rank (`base`: those before the tile, advanced past it).  An entry outside
+// the cap becomes kSelEvicted and is folded into the dropped floor
+// (search/budget.hpp:190-209); a parent of the next iteration among those that
+// stay becomes kSelNextParent.  The holes of this iteration's parents stay.
+struct MarkTally {
+  int stay, next;
+  uint32_t viable, dominated;
+  uint64_t mkey;
+};
+__device__ __forceinline__ void mark_tile(const SolverBufs& b, uint64_t tile, uint64_t n, uint32_t p, uint64_t gub,
+                                          const TargetView& A, const TargetView& B, bool pre, uint64_t (&base)[2],
+                                          MarkTally& m)
+{
+  const uint64_t t0 = tile_first(tile);
+  const uint64_t* __restrict__ lb = reinterpret_cast<const uint64_t*>(parity_buf(b.lb, p));
+  uint8_t* sel = parity_buf(b.sel, p);
+  uint64_t x[kScanItems];  // raw bits of the lower bounds
+  bool alive[kScanItems], eqA[kScanItems], eqB[kScanItems];
+#pragma unroll
+  for (int j = 0; j < kScanItems; ++j) {
+    const uint64_t i = tile_item(t0, j);
+    x[j] = i < n ? lb[i] : 0;
+    alive[j] = i < n && sel[i] == kSelAlive;
+  }
+#pragma unroll
+  for (int j = 0; j < kScanItems; ++j) {
+    const uint64_t key = bits_key(x[j]);
+    eqA[j] = A.active && alive[j] && (key & A.mask) == A.prefix;
+    eqB[j] = pre && B.active && alive[j] && (key & B.mask) == B.prefix;
+  }
+  int rankA[kScanItems] = {}, rankB[kScanItems] = {};
+  const uint64_t baseA = base[0], baseB = base[1];
+  if (A.ranked) base[0] += (uint64_t)tile_ranks<0>(eqA, rankA);  // the same for the whole grid
+  if (pre && B.ranked) base[1] += (uint64_t)tile_ranks<1>(eqB, rankB);
+#pragma unroll
+  for (int j = 0; j < kScanItems; ++j) {
+    if (!alive[j]) continue;
+    const uint64_t key = bits_key(x[j]);
+    const bool ta = A.take(key, eqA[j], baseA + (uint64_t)rankA[j]);
+    const bool tb = pre && ta && B.take(key, eqB[j], baseB + (uint64_t)rankB[j]);
+    const uint64_t i = tile_item(t0, j);
+    if (!ta) {
+      sel[i] = kSelEvicted;
+      if (bits_le(x[j], gub)) {
+        ++m.viable;
+        m.mkey = key < m.mkey ? key : m.mkey;
+      } else {
+        ++m.dominated;
+      }
+    } else if (tb) {
+      sel[i] = kSelNextParent;
+    }
+    m.stay += ta ? 1 : 0;
+    m.next += tb ? 1 : 0;
+  }
+}
+
+// Moves a tile's entries that stay, in order, to the other buffer (lower
+// bound, store slot and mark), lists the store slots of the next iteration's
+// parents among them in order, and pushes the store slots of the others (this
+// iteration's parents and the evicted) onto the free stack in position order.
+// `base`: stayers and next parents before the tile, advanced past it; `range`:
+// the smallest and largest key of this thread's stayers.
+__device__ __forceinline__ void copy_tile(const SolverCfg& cfg, const SolverBufs& b, uint64_t tile, uint64_t n,
+                                          uint32_t p, uint64_t free_base, uint64_t (&base)[2], uint64_t (&range)[2])
+{
+  const uint64_t t0 = tile_first(tile);
+  const uint64_t* __restrict__ slb = reinterpret_cast<const uint64_t*>(parity_buf(b.lb, p));
+  const uint32_t* __restrict__ sslot = parity_buf(b.slot, p);
+  const uint8_t* ssel = parity_buf(b.sel, p);
+  uint64_t* __restrict__ dlb = reinterpret_cast<uint64_t*>(parity_buf(b.lb, 1 - p));
+  uint32_t* __restrict__ dslot = parity_buf(b.slot, 1 - p);
+  uint8_t* __restrict__ dsel = parity_buf(b.sel, 1 - p);
+  bool f[kScanItems], g[kScanItems], in[kScanItems];
+  uint64_t x[kScanItems];  // raw bits of the lower bounds
+  uint32_t sl[kScanItems];
+#pragma unroll
+  for (int j = 0; j < kScanItems; ++j) {
+    const uint64_t i = tile_item(t0, j);
+    in[j] = i < n;
+    const uint8_t sv = in[j] ? ssel[i] : kSelParent;
+    x[j] = in[j] ? slb[i] : 0;
+    sl[j] = in[j] ? sslot[i] : 0u;
+    f[j] = sv == kSelAlive || sv == kSelNextParent;
+    g[j] = sv == kSelNextParent;
+  }
+#pragma unroll
+  for (int j = 0; j < kScanItems; ++j)
+    if (f[j]) {
+      const uint64_t k = bits_key(x[j]);
+      range[0] = k < range[0] ? k : range[0];
+      range[1] = k > range[1] ? k : range[1];
+    }
+  int rank[kScanItems], prank[kScanItems], total[2];  // stayers / next parents before each item
+  tile_ranks2(f, g, rank, prank, total);
+#pragma unroll
+  for (int j = 0; j < kScanItems; ++j) {
+    if (!in[j]) continue;
+    const uint64_t i = tile_item(t0, j);
+    const uint64_t stay_before = base[0] + (uint64_t)rank[j];
+    if (f[j]) {
+      dlb[stay_before] = x[j];
+      dslot[stay_before] = sl[j];
+      dsel[stay_before] = g[j] ? kSelParent : kSelAlive;
+      if (g[j]) {
+        const uint64_t pos = base[1] + (uint64_t)prank[j];
+        if (pos < cfg.e_max) b.pslot[pos] = sl[j];
+        else b.dev->error = 1;
+      }
+    } else {
+      b.free_slots[free_base + (i - stay_before)] = sl[j];
+    }
+  }
+  base[0] += (uint64_t)total[0];
+  base[1] += (uint64_t)total[1];
+}
+
+// Sizes, the radix passes, the marks, the move and the staging of the next
+// iteration's parents: each needs all of the one before, so the blocks meet at
+// a barrier between them, five and one per radix pass (a small pool's keys
+// differ in two or three digits).  Each block keeps the same consecutive
+// tiles throughout, so it needs only the counts of the blocks before it and no
+// scan of its own.  As twelve launches over a grid of every tile the pool
+// could have, an iteration of the n = 4 plain solve (a few hundred entries,
+// room for 2^24) spent 76 of its 178 us here.
+__global__ void __launch_bounds__(kScanBlock, 2) rebuild_kernel(const SolverCfg cfg, const SolverBufs b)
+{
+  SolverDev* d = b.dev;
+  if (d->done) return;
+  // (1) sizes, the select's start
+  if (!grid_barrier(d, [&] {
+        if (threadIdx.x == 0) size_pool(cfg, b);
+        __syncthreads();
+        radix_init(cfg, b);
+      }))
+    return;
+  const uint64_t n = d->extent, pre_k = d->pre_k, free_base = d->free_top;
+  const uint32_t p = d->parity;
+  // (2) digits of up to 11 bits from below the keys' common leading bits
+  for (int pass = 0; pass < (64 + kRadixBits - 1) / kRadixBits; ++pass) {
+    bool go[2];
+    if (!radix_hist(b, n, p, go)) break;  // the same for every block
+    if (!grid_barrier(d, [&] {
+          for (int t = 0; t < 2; ++t)
+            if (go[t]) radix_pick(b, b.radix + t);
+        }))
+      return;
+  }
+  const TargetView A(b.radix[0]), B(b.radix[1]);
+  const uint64_t tiles = (n + kScanTile - 1) / kScanTile, per = (tiles + gridDim.x - 1) / gridDim.x;
+  const uint64_t tile0 = (uint64_t)blockIdx.x * per < tiles ? (uint64_t)blockIdx.x * per : tiles;
+  const uint64_t tile1 = tile0 + per < tiles ? tile0 + per : tiles;
+  uint64_t base[2] = {0, 0}, all[2];
+  // (3) ranks inside the threshold buckets, where one is split
+  if (A.ranked || B.ranked) {
+    int c[2] = {0, 0};
+    for (uint64_t t = tile0; t < tile1; ++t) eq_count(b, t, n, p, A, B, c);
+    const int c0 = tile_count<0>(c[0]), c1 = tile_count<1>(c[1]);
+    if (threadIdx.x == 0) {
+      b.block_counts[blockIdx.x] = (uint32_t)c0;
+      b.block_counts2[blockIdx.x] = (uint32_t)c1;
+    }
+    if (!grid_barrier(d, [] {})) return;
+    blocks_before(b.block_counts, b.block_counts2, base, all);
+  }
+  // (4) the marks
+  MarkTally m = {0, 0, 0, 0, ~0ULL};
+  {
+    const uint64_t gub = dbits(d->gub);
+    for (uint64_t t = tile0; t < tile1; ++t) {
+      mark_tile(b, t, n, p, gub, A, B, pre_k > 0, base, m);
+      __syncthreads();  // the rank tables are reused
+    }
+    unsigned long long v[4] = {(unsigned)m.stay, (unsigned)m.next, m.viable, m.dominated};
+    block_sum(v);
+    const uint64_t mk = block_min(m.mkey);
+    if (threadIdx.x == 0) {
+      b.block_offsets[blockIdx.x] = (uint32_t)v[0];
+      b.block_offsets2[blockIdx.x] = (uint32_t)v[1];
+      if (v[2]) atomicAdd((unsigned long long*)&d->counters.dropped_viable, v[2]);
+      if (v[3]) atomicAdd((unsigned long long*)&d->counters.dropped_dominated, v[3]);
+      if (mk != ~0ULL) atomicMin((unsigned long long*)&d->dropped_min_key, (unsigned long long)mk);
+    }
+  }
+  if (!grid_barrier(d, [] {})) return;
+  // (5) the move, the key range of what stays
+  blocks_before(b.block_offsets, b.block_offsets2, base, all);
+  uint64_t range[2] = {~0ULL, 0};
+  for (uint64_t t = tile0; t < tile1; ++t) {
+    copy_tile(cfg, b, t, n, p, free_base, base, range);
+    __syncthreads();
+  }
+  range[0] = block_min(range[0]);
+  range[1] = block_max(range[1]);
+  if (threadIdx.x == 0) {
+    if (range[0] != ~0ULL) atomicMin((unsigned long long*)&d->pool_min_key, (unsigned long long)range[0]);
+    if (range[1] != 0) atomicMax((unsigned long long*)&d->pool_max_key, (unsigned long long)range[1]);
+  }
+  // (6) the next parents' boxes; one thread closes the iteration
+  if (!grid_barrier(d, [] {})) return;
+  const uint64_t next = all[1] < cfg.e_max ? all[1] : cfg.e_max;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    d->survivors = all[0];
+    d->pre_count = all[1];
+    finish_pool(cfg, b);
+  }
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < next; k += (uint64_t)gridDim.x * blockDim.x)
+    stage_parent(cfg, b, __ldcg(b.pslot + k), k);
+  if (threadIdx.x == 0) stamp_last(d->stamps + 4, (uint64_t)blockIdx.x * blockDim.x < next);
 }
 
 __global__ void pool_min_kernel(const SolverBufs b, uint64_t* viable_out)
@@ -1465,11 +1441,9 @@ __global__ void pool_min_reset_kernel(const SolverBufs b, uint64_t* viable_out)
 // ---------------------------------------------------------------------
 static int tiles(uint64_t max_items) { return (int)((max_items + kScanTile - 1) / kScanTile); }
 
-static void scan(const SolverBufs& b, const uint32_t* counts, uint32_t* offsets, const uint64_t* n_items_dev,
-                 uint64_t* total_dev, const uint32_t* active, const uint32_t* skip, cudaStream_t s)
+static void scan(const SolverBufs& b, const uint64_t* n_items_dev, uint64_t* total_dev, cudaStream_t s)
 {
-  const ScanArgs a = {counts, offsets, total_dev, active};
-  scan_kernel<<<1, 1024, 0, s>>>(a, a, n_items_dev, skip, &b.dev->done);
+  scan_kernel<<<1, 1024, 0, s>>>(b.block_counts, b.block_offsets, n_items_dev, total_dev, &b.dev->done);
 }
 
 template <class P>
@@ -1477,7 +1451,7 @@ static void compact(const P& pred, uint64_t max_items, const uint64_t* n_items_d
                     const SolverBufs& b, cudaStream_t s)
 {
   count_kernel<P><<<tiles(max_items), kScanBlock, 0, s>>>(pred, b.block_counts);
-  scan(b, b.block_counts, b.block_offsets, n_items_dev, total_dev, nullptr, nullptr, s);
+  scan(b, n_items_dev, total_dev, s);
 }
 
 template <class P, class Op>
@@ -1486,45 +1460,24 @@ static void scatter(const P& pred, const Op& op, uint64_t max_items, cudaStream_
   scatter_kernel<P, Op><<<tiles(max_items), kScanBlock, 0, s>>>(pred, op, b.block_offsets);
 }
 
-// which = 0: this iteration's parents (skipped when the previous iteration
-// staged them); which = 1: the cap and the next iteration's parents
-static void radix_select(const SolverCfg& cfg, const SolverBufs& b, int which, uint64_t max_items, cudaStream_t s)
+// The pool's rebuild: as many blocks as are resident at once (they wait for
+// one another), no more than its tiles.
+static cudaError_t rebuild(const SolverCfg& cfg, const SolverBufs& b, cudaStream_t s)
 {
-  const uint32_t* skip = which == 0 ? &b.dev->skip_select : nullptr;
-  if (which == 0) radix_init_kernel<<<1, 256, 0, s>>>(cfg, b, which);  // which = 1: size_kernel
-  const int grid = (int)std::min<uint64_t>((max_items + kHistThreads * kHistUnroll - 1) / (kHistThreads * kHistUnroll),
-                                           (uint64_t)sm_count() * 8);
-  // digits of up to 11 bits from below the keys' common leading bits;
-  // the passes after the buckets settle or the bits run out return at once
-  for (int p = 0; p < (64 + kRadixBits - 1) / kRadixBits; ++p) radix_hist_kernel<<<grid, kHistThreads, 0, s>>>(cfg, b, which);
-  // ranks among entries inside the threshold buckets, then the marks with
-  // the tile counts of the entries the next compactions move
-  const uint64_t* n_dev = which == 0 ? &b.dev->pool_size : &b.dev->extent;
-  const int scans = which == 0 ? 1 : 2;
-  eq_count_kernel<<<tiles(max_items), kScanBlock, 0, s>>>(cfg, b, which);
-  scan_kernel<<<scans, 1024, 0, s>>>(ScanArgs{b.block_counts, b.block_offsets, nullptr, &b.radix[0].rank},
-                                     ScanArgs{b.block_counts2, b.block_offsets2, nullptr, &b.radix[1].rank}, n_dev, skip,
-                                     &b.dev->done);
-  mark_kernel<<<tiles(max_items), kScanBlock, 0, s>>>(cfg, b, which);
-  scan_kernel<<<scans, 1024, 0, s>>>(
-      ScanArgs{b.block_counts, b.block_offsets, which == 0 ? nullptr : &b.dev->survivors, nullptr},
-      ScanArgs{b.block_counts2, b.block_offsets2, &b.dev->pre_count, nullptr}, n_dev, skip, &b.dev->done);
+  int occ = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rebuild_kernel, kScanBlock, 0);
+  if (e != cudaSuccess) return e;
+  const int grid = std::min(tiles(cfg.pstride), sm_count() * std::min(occ, 2));
+  void* args[] = {const_cast<SolverCfg*>(&cfg), const_cast<SolverBufs*>(&b)};
+  return cudaLaunchCooperativeKernel((const void*)rebuild_kernel, dim3((unsigned)grid), dim3(kScanBlock), args, 0, s);
 }
 
 cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval_grid, int sample_grid,
-                             cudaStream_t s, const SideStream& side, bool with_select)
+                             cudaStream_t s, const SideStream& side)
 {
   const bool lazy = cfg.precision == CMN_PRECISION_FP32_LAZY;
   const uint64_t max_children = cfg.e_max << cfg.log2C;
-  const uint64_t max_pool = cfg.pstride;
-  begin_kernel<<<1, 1, 0, s>>>(cfg, b, with_select ? 0 : 1);
-
-  // (1) select the E best parents and stage them (after the first
-  // iteration, the previous one staged them)
-  if (with_select) {
-    radix_select(cfg, b, 0, cfg.cap, s);
-    gather_parents_kernel<<<tiles(cfg.cap), kScanBlock, 0, s>>>(cfg, b, b.block_offsets);
-  }
+  begin_kernel<<<1, 1, 0, s>>>(cfg, b);
 
   // (1b) lazy form: the FP64 verdict of every staged parent -- its bound
   // has been an FP32 one (with its own parent's FP64 bound folded in) since
@@ -1728,7 +1681,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
   // the kept children go behind the pool in the current buffer; the
   // parents stay there as holes until the one compaction below
   KeptChild kept{b};
-  scan(b, b.block_counts, b.block_offsets, &b.dev->n_children, &b.dev->kept, nullptr, nullptr, s);
+  scan(b, &b.dev->n_children, &b.dev->kept, s);
   scatter(kept, ListChild{b}, max_children, s, b);
   {
     const int grid = (int)std::min<uint64_t>((max_children + 255) / 256, 4096);
@@ -1736,26 +1689,22 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
     else if (cfg.n_vars > 8) append_boxes_kernel<16><<<grid, 256, 0, s>>>(cfg, b);
     else append_children_kernel<<<grid, 256, 0, s>>>(cfg, b);
   }
-  size_kernel<<<1, 256, 0, s>>>(cfg, b);
 
   // (6) over the cap: keep the `cap` best alive entries, fold the rest into
-  // the floor; then move every alive entry to the other buffer in order
-  radix_select(cfg, b, 1, max_pool, s);
-  copy_pool_kernel<<<tiles(max_pool), kScanBlock, 0, s>>>(cfg, b);
-  {
-    const int grid = (int)std::min<uint64_t>((cfg.e_max + 255) / 256, 1024);
-    stage_next_kernel<<<grid, 256, 0, s>>>(cfg, b);
-  }
+  // the floor; select and stage the next iteration's parents; move every alive
+  // entry to the other buffer in order
+  e = rebuild(cfg, b, s);
+  if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
 
 cudaError_t solver_init(const SolverCfg& cfg, const SolverBufs& b, const double* root_lb_dev,
                         const double* root_ub_dev, double gub0, cudaStream_t s)
 {
-  init_kernel<<<1, 256, 0, s>>>(cfg, b, root_lb_dev, root_ub_dev, gub0);
   const int grid = (int)std::min<uint64_t>((cfg.pstride + 255) / 256, 4096);
   free_init_kernel<<<grid, 256, 0, s>>>(cfg, b);
   cudaMemsetAsync(b.sel[0], kSelAlive, cfg.pstride, s);
+  init_kernel<<<1, 256, 0, s>>>(cfg, b, root_lb_dev, root_ub_dev, gub0);
   cudaMemsetAsync(b.sel[1], kSelAlive, cfg.pstride, s);
   return cudaGetLastError();
 }
