@@ -970,66 +970,6 @@ __global__ void lazy_fold_kernel(const SolverCfg cfg, const SolverBufs b)
   }
 }
 
-// ---------------------------------------------------------------------
-// incumbent, prune accounting, pool finish
-// ---------------------------------------------------------------------
-// One tile of children: counts of their verdicts (search/driver.hpp:319-350),
-// of the evaluations the form counts per valid child, the key range of the
-// children the pool takes, and the tile's kept children for the compaction.
-__global__ void __launch_bounds__(kScanBlock) prune_count_kernel(const SolverCfg cfg, const SolverBufs b)
-{
-  const uint64_t t0 = tile_first();
-  SolverDev* d = b.dev;
-  if (d->done) return;
-  const uint64_t n = d->n_children;
-  if ((uint64_t)blockIdx.x * kScanTile >= n) return;
-  const uint64_t gub = dbits(d->gub);
-  uint32_t dup = 0, inf = 0, dom = 0, kept = 0, sampled = 0, valid = 0, entries = 0;
-  uint64_t mkey = ~0ULL, xkey = 0;
-#pragma unroll
-  for (int j = 0; j < kScanItems; ++j) {
-    const uint64_t g = tile_item(t0, j);
-    if (g >= n) continue;
-    const uint8_t s = b.cstate[g];
-    if (s == kChildNone) continue;
-    if (cfg.sample_all || s == kChildEligible) ++sampled;
-    if (s == kChildDuplicate) {
-      ++dup;
-      continue;
-    }
-    ++valid;
-    if (s == kChildInfeasible) {
-      ++inf;
-      continue;
-    }
-    const uint64_t lb = dbits(b.clb[g]);
-    const bool keep = s != kChildDominated && !bits_lt(gub, lb);
-    if (keep) ++kept;
-    else ++dom;
-    if (keep && s == kChildEligible) ++entries;  // KeptChild
-    if (s == kChildEligible) {  // a superset of the kept children
-      const uint64_t k = bits_key(lb);
-      mkey = k < mkey ? k : mkey;
-      xkey = k > xkey ? k : xkey;
-    }
-  }
-  const int mine = tile_count((int)entries);
-  unsigned long long c[6] = {dup, inf, dom, kept, sampled, valid};
-  block_sum(c);
-  mkey = block_min(mkey);
-  xkey = block_max(xkey);
-  if (threadIdx.x != 0) return;
-  b.block_counts[blockIdx.x] = (uint32_t)mine;
-  if (mkey != ~0ULL) atomicMin((unsigned long long*)&d->child_min_key, (unsigned long long)mkey);
-  if (xkey != 0) atomicMax((unsigned long long*)&d->child_max_key, (unsigned long long)xkey);
-  if (c[0]) atomicAdd((unsigned long long*)&d->counters.pruned_duplicate, c[0]);
-  if (c[1]) atomicAdd((unsigned long long*)&d->counters.pruned_infeasible, c[1]);
-  if (c[2]) atomicAdd((unsigned long long*)&d->counters.pruned_dominated, c[2]);
-  if (c[3]) atomicAdd((unsigned long long*)&d->counters.enqueued, c[3]);
-  if (c[4]) atomicAdd((unsigned long long*)&d->counters.sampled, c[4] * cfg.S);
-  if (c[5] && cfg.precision == CMN_PRECISION_FP64) atomicAdd((unsigned long long*)&d->counters.certified_fp64, c[5]);
-  if (c[5] && cfg.precision == CMN_PRECISION_FP32_LAZY) atomicAdd((unsigned long long*)&d->counters.screened_fp32, c[5]);
-}
 
 // The screen's tallies: children bounded, and excluded by the verdicts.
 __global__ void eval_count_kernel(const SolverCfg cfg, const SolverBufs b)
@@ -1176,6 +1116,95 @@ __device__ __forceinline__ void blocks_before(const uint32_t* c0, const uint32_t
   before[1] = acc[1];
   all[0] = acc[2];
   all[1] = acc[3];
+}
+
+// ---------------------------------------------------------------------
+// incumbent, prune accounting, pool finish
+// ---------------------------------------------------------------------
+// Counts of the children's verdicts (search/driver.hpp:319-350) and of the
+// evaluations the form counts per valid child, the key range of the children
+// the pool takes, and their list in order.  A count, a scan and a scatter in
+// three launches took 3.5 us more of the 119 of an iteration with a few
+// children.
+__global__ void __launch_bounds__(kScanBlock, 2) prune_kernel(const SolverCfg cfg, const SolverBufs b)
+{
+  SolverDev* d = b.dev;
+  if (d->done) return;
+  const uint64_t n = d->n_children;
+  const uint64_t tiles = (n + kScanTile - 1) / kScanTile, per = (tiles + gridDim.x - 1) / gridDim.x;
+  const uint64_t tile0 = (uint64_t)blockIdx.x * per < tiles ? (uint64_t)blockIdx.x * per : tiles;
+  const uint64_t tile1 = tile0 + per < tiles ? tile0 + per : tiles;
+  const uint64_t gub = dbits(d->gub);
+  uint32_t dup = 0, inf = 0, dom = 0, kept = 0, sampled = 0, valid = 0, entries = 0;
+  uint64_t mkey = ~0ULL, xkey = 0;
+  for (uint64_t t = tile0; t < tile1; ++t) {
+    const uint64_t t0 = tile_first(t);
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+      const uint64_t g = tile_item(t0, j);
+      if (g >= n) continue;
+      const uint8_t s = b.cstate[g];
+      if (s == kChildNone) continue;
+      if (cfg.sample_all || s == kChildEligible) ++sampled;
+      if (s == kChildDuplicate) {
+        ++dup;
+        continue;
+      }
+      ++valid;
+      if (s == kChildInfeasible) {
+        ++inf;
+        continue;
+      }
+      const uint64_t lb = dbits(b.clb[g]);
+      const bool keep = s != kChildDominated && !bits_lt(gub, lb);
+      if (keep) ++kept;
+      else ++dom;
+      if (keep && s == kChildEligible) ++entries;  // KeptChild
+      if (s == kChildEligible) {  // a superset of the kept children
+        const uint64_t k = bits_key(lb);
+        mkey = k < mkey ? k : mkey;
+        xkey = k > xkey ? k : xkey;
+      }
+    }
+  }
+  unsigned long long c[7] = {dup, inf, dom, kept, sampled, valid, entries};
+  block_sum(c);
+  mkey = block_min(mkey);
+  xkey = block_max(xkey);
+  if (threadIdx.x == 0) {
+    b.block_counts[blockIdx.x] = (uint32_t)c[6];
+    if (mkey != ~0ULL) atomicMin((unsigned long long*)&d->child_min_key, (unsigned long long)mkey);
+    if (xkey != 0) atomicMax((unsigned long long*)&d->child_max_key, (unsigned long long)xkey);
+    if (c[0]) atomicAdd((unsigned long long*)&d->counters.pruned_duplicate, c[0]);
+    if (c[1]) atomicAdd((unsigned long long*)&d->counters.pruned_infeasible, c[1]);
+    if (c[2]) atomicAdd((unsigned long long*)&d->counters.pruned_dominated, c[2]);
+    if (c[3]) atomicAdd((unsigned long long*)&d->counters.enqueued, c[3]);
+    if (c[4]) atomicAdd((unsigned long long*)&d->counters.sampled, c[4] * cfg.S);
+    if (c[5] && cfg.precision == CMN_PRECISION_FP64) atomicAdd((unsigned long long*)&d->counters.certified_fp64, c[5]);
+    if (c[5] && cfg.precision == CMN_PRECISION_FP32_LAZY) atomicAdd((unsigned long long*)&d->counters.screened_fp32, c[5]);
+  }
+  if (!grid_barrier(d, [] {})) return;
+  // the kept children's list, in order
+  uint64_t base[2], all[2];
+  blocks_before(b.block_counts, b.block_counts, base, all);
+  if (blockIdx.x == 0 && threadIdx.x == 0) d->kept = all[0];
+  const KeptChild is_kept{b};
+  for (uint64_t t = tile0; t < tile1; ++t) {
+    const uint64_t t0 = tile_first(t);
+    bool f[kScanItems];
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+      const uint64_t g = tile_item(t0, j);
+      f[j] = g < n && is_kept(g);
+    }
+    int rank[kScanItems];
+    const int total = tile_ranks(f, rank);
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j)
+      if (f[j]) b.list[base[0] + (uint64_t)rank[j]] = (uint32_t)tile_item(t0, j);
+    base[0] += (uint64_t)total;
+    __syncthreads();  // the rank table is reused
+  }
 }
 
 // Alive entries of tile `tile` inside each ranked target's threshold bucket.
@@ -1460,16 +1489,17 @@ static void scatter(const P& pred, const Op& op, uint64_t max_items, cudaStream_
   scatter_kernel<P, Op><<<tiles(max_items), kScanBlock, 0, s>>>(pred, op, b.block_offsets);
 }
 
-// The pool's rebuild: as many blocks as are resident at once (they wait for
-// one another), no more than its tiles.
-static cudaError_t rebuild(const SolverCfg& cfg, const SolverBufs& b, cudaStream_t s)
+// A kernel whose blocks meet at barriers, over the tiles of max_items: as many
+// blocks as are resident at once, no more than the tiles.
+static cudaError_t cooperative(void (*kernel)(SolverCfg, SolverBufs), uint64_t max_items, const SolverCfg& cfg,
+                               const SolverBufs& b, cudaStream_t s)
 {
   int occ = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rebuild_kernel, kScanBlock, 0);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kScanBlock, 0);
   if (e != cudaSuccess) return e;
-  const int grid = std::min(tiles(cfg.pstride), sm_count() * std::min(occ, 2));
+  const int grid = std::min(tiles(max_items), sm_count() * std::min(occ, 2));
   void* args[] = {const_cast<SolverCfg*>(&cfg), const_cast<SolverBufs*>(&b)};
-  return cudaLaunchCooperativeKernel((const void*)rebuild_kernel, dim3((unsigned)grid), dim3(kScanBlock), args, 0, s);
+  return cudaLaunchCooperativeKernel((const void*)kernel, dim3((unsigned)grid), dim3(kScanBlock), args, 0, s);
 }
 
 cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval_grid, int sample_grid,
@@ -1677,12 +1707,10 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
   if (e != cudaSuccess) return e;
 
   // (5) prune with the new incumbent and rebuild the pool
-  prune_count_kernel<<<tiles(max_children), kScanBlock, 0, s>>>(cfg, b);
-  // the kept children go behind the pool in the current buffer; the
-  // parents stay there as holes until the one compaction below
-  KeptChild kept{b};
-  scan(b, &b.dev->n_children, &b.dev->kept, s);
-  scatter(kept, ListChild{b}, max_children, s, b);
+  // (the kept children go behind the pool in the current buffer; the parents
+  // stay there as holes until the one compaction below)
+  e = cooperative(prune_kernel, max_children, cfg, b, s);
+  if (e != cudaSuccess) return e;
   {
     const int grid = (int)std::min<uint64_t>((max_children + 255) / 256, 4096);
     if (cfg.n_vars > 16) append_boxes_kernel<32><<<grid, 256, 0, s>>>(cfg, b);
@@ -1693,7 +1721,7 @@ cudaError_t solver_iteration(const SolverCfg& cfg, const SolverBufs& b, int eval
   // (6) over the cap: keep the `cap` best alive entries, fold the rest into
   // the floor; select and stage the next iteration's parents; move every alive
   // entry to the other buffer in order
-  e = rebuild(cfg, b, s);
+  e = cooperative(rebuild_kernel, cfg.pstride, cfg, b, s);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
