@@ -1,5 +1,6 @@
 // chain_kernels.cu -- the FP64 evaluator of programs that are sets of sum
 // chains, over the boxes of one instance: chain_tiles.cuh's two passes.
+#include <algorithm>
 #include <cfloat>
 #include <cstdint>
 
@@ -26,18 +27,13 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) chain_constraints_kernel(c
 // no chain decides feasibility and the children's states are found here.
 // 2^lg lanes share a box when few boxes are live.
 template <int kMode, bool kFused, bool kHi>
-__global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const EvalArgs a, int flags)
+__device__ __forceinline__ void objective_boxes(const EvalArgs& a, unsigned char* smem_raw, int flags, uint64_t total)
 {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int B = blockDim.x;
   const int ms = a.pinfo != nullptr ? a.max_slots : 0;
   double* olo = reinterpret_cast<double*>(smem_raw) + threadIdx.x;
   double* ohi = olo + (size_t)ms * B;
   int32_t* ovid = reinterpret_cast<int32_t*>(reinterpret_cast<double*>(smem_raw) + (size_t)2 * ms * B) + threadIdx.x;
-  if (a.done != nullptr && *a.done) return;
-  if constexpr (kFused)
-    if (!flags) stamp_first(a.t_first);
-  const uint64_t total = box_count(a, kMode == 3);
   const double gub = a.gub ? *a.gub : DBL_MAX;
   const ChainSeg s = a.chain.seg[0];
   const bool pure = s.kind == kChainObjective;
@@ -93,14 +89,41 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const E
     if ((threadIdx.x & 31) == 0) stamp_last(a.t_last, (uint64_t)blockIdx.x * per_block < total);
 }
 
+template <int kMode, bool kFused, bool kHi>
+__global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const EvalArgs a, int flags)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (a.done != nullptr && *a.done) return;
+  if constexpr (kFused)
+    if (!flags) stamp_first(a.t_first);
+  objective_boxes<kMode, kFused, kHi>(a, smem_raw, flags, box_count(a, kMode == 3));
+}
+
+// Most children the lane groups above take rather than the sharing kernel
+// below, for families of 2^lc consecutive siblings (all of them up to lc = 2).
+// With up to 32 lanes a child they cost little more for 1,024 children than for
+// 16; from there every SM's FP64 pipe is full, and sharing the terms' values
+// pays.  n = 32, lane groups against sharing: 16 siblings, 1,024 children 99 and
+// 145 us, 4,096 children 199 and 158, 65,536 children 727 and 396; 8 siblings,
+// 2,048 children 143 and 216, 8,192 children 251 and 235.  Two or four siblings
+// have few values in common and many families to tabulate: n = 12, four
+// siblings, 16,384 children 62 and 80 us, 262,144 children 234 and 317.
+static __host__ __device__ uint64_t objective_few(int lc) { return lc <= 2 ? ~0ULL : lc == 3 ? 2048 : 1024; }
+
 template <int kMode, bool kHi>
-__global__ void __launch_bounds__(kObjThreads, 5) chain_siblings_kernel(const EvalArgs a, int flags, int families)
+__global__ void __launch_bounds__(kObjThreads, 5) chain_siblings_kernel(const EvalArgs a, int flags, int families,
+                                                                           int few)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (a.done != nullptr && *a.done) return;
   const int wid = threadIdx.x >> 5, W = blockDim.x >> 5;
   unsigned char* smem = smem_raw + family_bytes(families, a.max_slots, kHi) * wid;
   const uint64_t total = box_count(a, false), tiles = (total + 31) >> 5;
+  if constexpr (!kHi)
+    if (total <= (uint64_t)few) {
+      objective_boxes<kMode, false, false>(a, smem_raw, flags, total);
+      return;
+    }
   for (uint64_t tile = (uint64_t)blockIdx.x * W + wid; tile < tiles; tile += (uint64_t)gridDim.x * W)
     siblings_tile<kMode, kHi>(a, smem, flags, families, tile, total);
 }
@@ -137,10 +160,13 @@ static cudaError_t launch_chain_t(const EvalArgs& a, cudaStream_t s)
     // children (of a role's box or of the solver's parents): siblings share
     const int lc = a.log2C < 0 || a.log2C > 5 ? 5 : a.log2C;
     const size_t fsmem = (kObjThreads / 32) * family_bytes(32 >> lc, ms, kHi);
-    if (a.pinfo != nullptr && lc > 0 && a.chain.pure_objective && fsmem + 1024 <= (size_t)max_dynamic_smem()) {
+    const uint64_t few = kHi ? 0 : objective_few(lc);  // (both bounds take one lane a box there)
+    if (a.pinfo != nullptr && lc > 0 && a.max_boxes > few && a.chain.pure_objective &&
+        fsmem + 1024 <= (size_t)max_dynamic_smem()) {
       auto siblings = chain_siblings_kernel<kMode, kHi>;
-      const uint64_t grid = resident(((a.max_boxes + 31) / 32 + 3) / 4, (const void*)siblings, kObjThreads, fsmem);
-      siblings<<<(unsigned)grid, kObjThreads, fsmem, s>>>(a, chains > 0 ? 1 : 0, 32 >> lc);
+      const uint64_t blocks = std::max<uint64_t>(((a.max_boxes + 31) / 32 + 3) / 4, 1024 * 32 / kObjThreads);
+      const uint64_t grid = resident(blocks, (const void*)siblings, kObjThreads, fsmem);
+      siblings<<<(unsigned)grid, kObjThreads, fsmem, s>>>(a, chains > 0 ? 1 : 0, 32 >> lc, (int)few);
       return cudaGetLastError();
     }
   }

@@ -253,7 +253,8 @@ __device__ void radix_pick(const SolverBufs& b, RadixState* rs)
 // histogram only when the bin changes: converging lower bounds share most
 // leading digits, so a pass makes few shared-memory atomics instead of one per
 // entry on one address.
-__device__ __forceinline__ bool radix_hist(const SolverBufs& b, uint64_t n, uint32_t parity, bool (&go)[2])
+__device__ __forceinline__ bool radix_hist(const SolverBufs& b, unsigned blocks, uint64_t n, uint32_t parity,
+                                           bool (&go)[2])
 {
   __shared__ uint32_t h[2][kRadixBins];
   int shift[2] = {0, 0}, nb[2] = {1, 1};
@@ -282,7 +283,7 @@ __device__ __forceinline__ bool radix_hist(const SolverBufs& b, uint64_t n, uint
   // each warp takes chunks of 32 x kHistUnroll consecutive entries and
   // issues all their loads before it bins them
   constexpr int kChunk = 32 * kHistUnroll;
-  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
+  const uint64_t warps = (uint64_t)blocks * (blockDim.x / 32);
   uint32_t run_bin[2] = {0, 0}, run[2] = {0, 0};
   for (uint64_t c = (uint64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); c * kChunk < n; c += warps) {
     uint64_t x[kHistUnroll];
@@ -1014,7 +1015,6 @@ __device__ void size_pool(const SolverCfg& cfg, const SolverBufs& b)
   if (cfg.precision == CMN_PRECISION_FP32_LAZY) d->counters.certified_fp64 += d->certify_count;
   d->remaining = d->pool_size - d->n_parents;
   d->new_size = d->remaining + d->kept;
-  d->extent = d->pool_size + d->kept;
   d->free_top -= d->kept;  // taken by the appended children
   d->evict = d->new_size > cfg.cap ? 1 : 0;
   // the next iteration's parents: its E (search/driver.hpp:221-233) over the
@@ -1049,14 +1049,14 @@ __device__ void finish_pool(const SolverCfg& cfg, const SolverBufs& b)
 // ---------------------------------------------------------------------
 // the pool's rebuild, one launch
 // ---------------------------------------------------------------------
-// A barrier of the launch's blocks: every block takes a ticket, the last one
-// runs `last` and opens it.  The launch is cooperative, so every block is
+// A barrier of the launch's first `blocks` blocks: each takes a ticket, the
+// last one runs `last` and opens it.  The launch is cooperative, so every block is
 // resident and the others wait no longer than a pass takes; the wait has a
 // limit (about a second) all the same, after which the device error is set and
 // false returned.
 constexpr uint32_t kBarrierSpins = 1u << 21;
 template <class F>
-__device__ __forceinline__ bool grid_barrier(SolverDev* d, F last)
+__device__ __forceinline__ bool grid_barrier(SolverDev* d, unsigned blocks, F last)
 {
   __shared__ int last_s, ok_s;
   __syncthreads();
@@ -1064,7 +1064,7 @@ __device__ __forceinline__ bool grid_barrier(SolverDev* d, F last)
   if (threadIdx.x == 0) {
     gen = *(volatile uint32_t*)&d->barrier;
     __threadfence();
-    last_s = atomicAdd(&d->ticket, 1u) == gridDim.x - 1;
+    last_s = atomicAdd(&d->ticket, 1u) == blocks - 1;
     __threadfence();
   }
   __syncthreads();
@@ -1088,16 +1088,25 @@ __device__ __forceinline__ bool grid_barrier(SolverDev* d, F last)
   return ok_s != 0;
 }
 
+// Blocks of a launch that take part: one per `items` of the n, so that few
+// entries do not wait for the tickets of a whole GPU (n does not change while
+// the kernel runs).
+__device__ __forceinline__ unsigned blocks_for(uint64_t n, uint64_t items)
+{
+  const uint64_t want = n < 1 ? 1 : (n + items - 1) / items;
+  return want < gridDim.x ? (unsigned)want : gridDim.x;
+}
+
 // Sums of two per-block counts over the blocks before this one, and over all.
-__device__ __forceinline__ void blocks_before(const uint32_t* c0, const uint32_t* c1, uint64_t (&before)[2],
-                                              uint64_t (&all)[2])
+__device__ __forceinline__ void blocks_before(const uint32_t* c0, const uint32_t* c1, unsigned blocks,
+                                              uint64_t (&before)[2], uint64_t (&all)[2])
 {
   __shared__ unsigned long long acc[4];
   __syncthreads();
   if (threadIdx.x < 4) acc[threadIdx.x] = 0;
   __syncthreads();
   unsigned long long v[4] = {};
-  for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+  for (uint32_t i = threadIdx.x; i < blocks; i += blockDim.x) {
     const uint32_t a = __ldcg(c0 + i), c = __ldcg(c1 + i);
     v[2] += a;
     v[3] += c;
@@ -1131,7 +1140,9 @@ __global__ void __launch_bounds__(kScanBlock, 2) prune_kernel(const SolverCfg cf
   SolverDev* d = b.dev;
   if (d->done) return;
   const uint64_t n = d->n_children;
-  const uint64_t tiles = (n + kScanTile - 1) / kScanTile, per = (tiles + gridDim.x - 1) / gridDim.x;
+  const unsigned blocks = blocks_for(n, kScanTile);
+  if (blockIdx.x >= blocks) return;
+  const uint64_t tiles = (n + kScanTile - 1) / kScanTile, per = (tiles + blocks - 1) / blocks;
   const uint64_t tile0 = (uint64_t)blockIdx.x * per < tiles ? (uint64_t)blockIdx.x * per : tiles;
   const uint64_t tile1 = tile0 + per < tiles ? tile0 + per : tiles;
   const uint64_t gub = dbits(d->gub);
@@ -1183,11 +1194,14 @@ __global__ void __launch_bounds__(kScanBlock, 2) prune_kernel(const SolverCfg cf
     if (c[5] && cfg.precision == CMN_PRECISION_FP64) atomicAdd((unsigned long long*)&d->counters.certified_fp64, c[5]);
     if (c[5] && cfg.precision == CMN_PRECISION_FP32_LAZY) atomicAdd((unsigned long long*)&d->counters.screened_fp32, c[5]);
   }
-  if (!grid_barrier(d, [] {})) return;
+  if (!grid_barrier(d, blocks, [] {})) return;
   // the kept children's list, in order
   uint64_t base[2], all[2];
-  blocks_before(b.block_counts, b.block_counts, base, all);
-  if (blockIdx.x == 0 && threadIdx.x == 0) d->kept = all[0];
+  blocks_before(b.block_counts, b.block_counts, blocks, base, all);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    d->kept = all[0];
+    d->extent = d->pool_size + all[0];
+  }
   const KeptChild is_kept{b};
   for (uint64_t t = tile0; t < tile1; ++t) {
     const uint64_t t0 = tile_first(t);
@@ -1355,27 +1369,30 @@ __global__ void __launch_bounds__(kScanBlock, 2) rebuild_kernel(const SolverCfg 
 {
   SolverDev* d = b.dev;
   if (d->done) return;
+  const uint64_t n = d->extent;
+  const unsigned blocks = blocks_for(n, kScanBlock);
+  if (blockIdx.x >= blocks) return;
   // (1) sizes, the select's start
-  if (!grid_barrier(d, [&] {
+  if (!grid_barrier(d, blocks, [&] {
         if (threadIdx.x == 0) size_pool(cfg, b);
         __syncthreads();
         radix_init(cfg, b);
       }))
     return;
-  const uint64_t n = d->extent, pre_k = d->pre_k, free_base = d->free_top;
+  const uint64_t pre_k = d->pre_k, free_base = d->free_top;
   const uint32_t p = d->parity;
   // (2) digits of up to 11 bits from below the keys' common leading bits
   for (int pass = 0; pass < (64 + kRadixBits - 1) / kRadixBits; ++pass) {
     bool go[2];
-    if (!radix_hist(b, n, p, go)) break;  // the same for every block
-    if (!grid_barrier(d, [&] {
+    if (!radix_hist(b, blocks, n, p, go)) break;  // the same for every block
+    if (!grid_barrier(d, blocks, [&] {
           for (int t = 0; t < 2; ++t)
             if (go[t]) radix_pick(b, b.radix + t);
         }))
       return;
   }
   const TargetView A(b.radix[0]), B(b.radix[1]);
-  const uint64_t tiles = (n + kScanTile - 1) / kScanTile, per = (tiles + gridDim.x - 1) / gridDim.x;
+  const uint64_t tiles = (n + kScanTile - 1) / kScanTile, per = (tiles + blocks - 1) / blocks;
   const uint64_t tile0 = (uint64_t)blockIdx.x * per < tiles ? (uint64_t)blockIdx.x * per : tiles;
   const uint64_t tile1 = tile0 + per < tiles ? tile0 + per : tiles;
   uint64_t base[2] = {0, 0}, all[2];
@@ -1388,8 +1405,8 @@ __global__ void __launch_bounds__(kScanBlock, 2) rebuild_kernel(const SolverCfg 
       b.block_counts[blockIdx.x] = (uint32_t)c0;
       b.block_counts2[blockIdx.x] = (uint32_t)c1;
     }
-    if (!grid_barrier(d, [] {})) return;
-    blocks_before(b.block_counts, b.block_counts2, base, all);
+    if (!grid_barrier(d, blocks, [] {})) return;
+    blocks_before(b.block_counts, b.block_counts2, blocks, base, all);
   }
   // (4) the marks
   MarkTally m = {0, 0, 0, 0, ~0ULL};
@@ -1410,9 +1427,9 @@ __global__ void __launch_bounds__(kScanBlock, 2) rebuild_kernel(const SolverCfg 
       if (mk != ~0ULL) atomicMin((unsigned long long*)&d->dropped_min_key, (unsigned long long)mk);
     }
   }
-  if (!grid_barrier(d, [] {})) return;
+  if (!grid_barrier(d, blocks, [] {})) return;
   // (5) the move, the key range of what stays
-  blocks_before(b.block_offsets, b.block_offsets2, base, all);
+  blocks_before(b.block_offsets, b.block_offsets2, blocks, base, all);
   uint64_t range[2] = {~0ULL, 0};
   for (uint64_t t = tile0; t < tile1; ++t) {
     copy_tile(cfg, b, t, n, p, free_base, base, range);
@@ -1425,14 +1442,14 @@ __global__ void __launch_bounds__(kScanBlock, 2) rebuild_kernel(const SolverCfg 
     if (range[1] != 0) atomicMax((unsigned long long*)&d->pool_max_key, (unsigned long long)range[1]);
   }
   // (6) the next parents' boxes; one thread closes the iteration
-  if (!grid_barrier(d, [] {})) return;
+  if (!grid_barrier(d, blocks, [] {})) return;
   const uint64_t next = all[1] < cfg.e_max ? all[1] : cfg.e_max;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     d->survivors = all[0];
     d->pre_count = all[1];
     finish_pool(cfg, b);
   }
-  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < next; k += (uint64_t)gridDim.x * blockDim.x)
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < next; k += (uint64_t)blocks * blockDim.x)
     stage_parent(cfg, b, __ldcg(b.pslot + k), k);
   if (threadIdx.x == 0) stamp_last(d->stamps + 4, (uint64_t)blockIdx.x * blockDim.x < next);
 }
