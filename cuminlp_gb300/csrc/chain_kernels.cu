@@ -101,14 +101,14 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const E
 
 // Most children the lane groups above take rather than the sharing kernel
 // below, for families of 2^lc consecutive siblings (all of them up to lc = 2).
-// With up to 32 lanes a child they cost little more for 1,024 children than for
-// 16; from there every SM's FP64 pipe is full, and sharing the terms' values
-// pays.  n = 32, lane groups against sharing: 16 siblings, 1,024 children 99 and
-// 145 us, 4,096 children 199 and 158, 65,536 children 727 and 396; 8 siblings,
-// 2,048 children 143 and 216, 8,192 children 251 and 235.  Two or four siblings
+// With up to 32 lanes a child they cost little more for 512 children than for
+// 16; from there the FP64 pipes fill, and sharing the terms' values pays.  The
+// bound phase at n = 32, lane groups against sharing: 16 siblings, 512 children
+// 73 and 84 us, 1,024 children 99 and 88, 4,096 children 199 and 99; 8 siblings,
+// 512 children 72 and 105 us, 2,048 children 144 and 112.  Two or four siblings
 // have few values in common and many families to tabulate: n = 12, four
 // siblings, 16,384 children 62 and 80 us, 262,144 children 234 and 317.
-static __host__ __device__ uint64_t objective_few(int lc) { return lc <= 2 ? ~0ULL : lc == 3 ? 2048 : 1024; }
+static __host__ __device__ uint64_t objective_few(int lc) { return lc <= 2 ? ~0ULL : 512; }
 
 template <int kMode, bool kHi>
 __global__ void __launch_bounds__(kObjThreads, 5) chain_siblings_kernel(const EvalArgs a, int flags, int families,
@@ -117,13 +117,17 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_siblings_kernel(const Ev
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (a.done != nullptr && *a.done) return;
   const int wid = threadIdx.x >> 5, W = blockDim.x >> 5;
-  unsigned char* smem = smem_raw + family_bytes(families, a.max_slots, kHi) * wid;
   const uint64_t total = box_count(a, false), tiles = (total + 31) >> 5;
   if constexpr (!kHi)
     if (total <= (uint64_t)few) {
       objective_boxes<kMode, false, false>(a, smem_raw, flags, total);
       return;
     }
+  if (tiles <= gridDim.x) {  // a block for every tile
+    if (blockIdx.x < tiles) siblings_tile<kMode, kHi, true>(a, smem_raw, flags, families, blockIdx.x, total);
+    return;
+  }
+  unsigned char* smem = smem_raw + family_bytes(families, a.max_slots, kHi) * wid;
   for (uint64_t tile = (uint64_t)blockIdx.x * W + wid; tile < tiles; tile += (uint64_t)gridDim.x * W)
     siblings_tile<kMode, kHi>(a, smem, flags, families, tile, total);
 }
@@ -164,8 +168,10 @@ static cudaError_t launch_chain_t(const EvalArgs& a, cudaStream_t s)
     if (a.pinfo != nullptr && lc > 0 && a.max_boxes > few && a.chain.pure_objective &&
         fsmem + 1024 <= (size_t)max_dynamic_smem()) {
       auto siblings = chain_siblings_kernel<kMode, kHi>;
-      const uint64_t blocks = std::max<uint64_t>(((a.max_boxes + 31) / 32 + 3) / 4, 1024 * 32 / kObjThreads);
-      const uint64_t grid = resident(blocks, (const void*)siblings, kObjThreads, fsmem);
+      // a block a tile while they are resident at once, else a warp a tile
+      const uint64_t tiles = (a.max_boxes + 31) / 32, most = 512 * 32 / kObjThreads;
+      uint64_t grid = resident(std::max(tiles, most), (const void*)siblings, kObjThreads, fsmem);
+      if (grid < tiles) grid = std::min(grid, std::max((tiles + 3) / 4, most));
       siblings<<<(unsigned)grid, kObjThreads, fsmem, s>>>(a, chains > 0 ? 1 : 0, 32 >> lc, (int)few);
       return cudaGetLastError();
     }
