@@ -756,7 +756,7 @@ def run_ours(args):
     hbm_peak = peaks.get("hbm_gbs", 6800.0)
 
     # live rooflines of the headline (lazy) form, per phase of the iteration
-    # (CUDA events inside the captured iteration): the FP64 verdict of the
+    # (times written by its kernels): the FP64 verdict of the
     # selected boxes (on its own stream) and the FP32 bound of the children,
     # which run at once, and the sampling; the dominant one is `roofline`
     launches = max(1, len(lazy["phases"]))
@@ -773,17 +773,19 @@ def run_ours(args):
 
     phase_rl = {
         "certify": dict(phase_line(0, ld["expansions"], fpb, peak64,
-                                   "eval_children_staged_kernel<0, 1> (FP64 verdict of each selected box, fused "
-                                   "terms, on its own stream beside the branching and the FP32 bound)",
+                                   "chain_constraints_kernel<0, 1> + chain_objective_kernel<0, 1, 0> (verdict of "
+                                   "each selected box: constraints decided in FP32 where its error bound allows, "
+                                   "else FP64; objective in FP64, fused terms; on its own stream beside the "
+                                   "branching and the FP32 bound)",
                                    VERDICT_DRAM_BYTES_PER_BOX, "selected box",
                                    "lazy_phases"), bound="fp64"),
         "bound": dict(phase_line(1, ld["bounded"], fpb, peak32,
-                                 "inc_common_kernel + inc_parts_kernel + eval_children_inc_kernel (FP32 child "
-                                 "bounds, incremental; beside the FP64 verdict)", INC32_DRAM_BYTES_PER_BOX, "child box", "lazy_phases"),
+                                 "lazy_children_kernel (FP32 child bounds, incremental; beside the FP64 "
+                                 "verdict)", INC32_DRAM_BYTES_PER_BOX, "child box", "lazy_phases"),
                       bound="fp32"),
         "sample": dict(phase_line(2, ld["sampled"], pfb, peak32,
-                                  "sample_screen_kernel (FP32 point ranking) + sample_children_kernel (FP64 "
-                                  "point of each chunk's best)", SCREEN32_DRAM_BYTES_PER_POINT, "sample point"),
+                                  "chain_screen_kernel (FP32 point ranking) + chain_sample_kernel (FP64 point of "
+                                  "each chunk's best)", SCREEN32_DRAM_BYTES_PER_POINT, "sample point"),
                        bound="fp32"),
     }
     dominant = max(phase_rl, key=lambda k: phase_rl[k]["ms_per_step"])
@@ -871,13 +873,16 @@ def run_ours(args):
                          peak_source="measured by cmn_measure_fma_peak (FMA loop, all SMs) in this run; FMA counted "
                                      "as 2 flops.  The interval operations round each product and sum on its own, so "
                                      "the instruction ceiling is half the peak, except the verdict's coefficient-and-"
-                                     "add pairs, which are one directed FMA each"),
+                                     "add pairs, which are one directed FMA each",
+                         work="flops_per_unit counts every operation of the DAG's interval evaluation.  The kernels "
+                              "give the same bits with fewer: constraints are decided in FP32 where its error bound "
+                              "allows and children share their parent's sums, so a fraction above 1 is work that "
+                              "was not needed, not a rate of the pipe"),
         "phase_rooflines": phase_rl,
         "roofline_plain_fp64": {
-            "bound": "fp64", "kernel": "eval_children_staged_kernel<1, 0> (plain FP64 form, program tiles in shared memory)",
+            "bound": "fp64", "kernel": "chain_constraints_kernel<1, 0> + chain_siblings_kernel<1, 0> (plain FP64 form)",
             "achieved": achieved64, "peak": peak64, "unit": "TFLOP/s", "frac": achieved64 / peak64,
             "frac_of_fp64_instruction_ceiling": achieved64 / (peak64 / 2),
-            "integer_pipe_ops": "interval multiply rounded up (csrc/fp64_emu.cuh)",
             "traffic": EVAL_DRAM_BYTES_PER_BOX * nb64 / max(1, len(plain["phases"])),
             "hbm": {"achieved": nb64 * bpb / (ev64_ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                     "bytes_per_box": bpb},
