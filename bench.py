@@ -59,18 +59,16 @@ from pathlib import Path
 ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
-EVAL_DRAM_BYTES_PER_BOX = (43186688 + 34048) / 1048576  # ncu, eval_children_kernel<double, 1>, n=32 MIQCQP
-# ncu, the n=64 MIQCQP at 2^14 parents x 2^4 children in a steady iteration
-# (profiles/lazy_form_kernels_miqcqp_n64.md): DRAM bytes per child box of the
-# FP32 bound (inc_common + inc_parts + eval_children_inc, reads and writes)
-# and per sample point of sample_screen_kernel, scaled by the units of a
-# launch
-INC32_DRAM_BYTES_PER_BOX = (10849280 + 11762688 + 2355968 + 59540224 + 154368) / 262144
-SCREEN32_DRAM_BYTES_PER_POINT = 20065792 / 262144
-# the same capture: the FP64 verdict of 2^14 selected boxes reads 17.8 MB
-# (their staged planes, 1,024 B a box, and the program); the 9 B a box it
-# writes (bound and state) are added as counted, not measured
-VERDICT_DRAM_BYTES_PER_BOX = 17.8e6 / 16384 + 9
+# ncu, steady iterations of the n=64 (plain bound: n=32) MIQCQP at 2^14 parents
+# x 2^4 children, scaled by the units of a launch: DRAM bytes per child box of the plain bound
+# (chain_constraints + chain_siblings), of the lazy form's FP32 bound
+# (lazy_children), per sample point of chain_screen_kernel, and per selected box
+# of the FP64 verdict (chain_constraints + chain_objective; the 9 B a box it
+# writes, bound and state, are added as counted, not measured)
+EVAL_DRAM_BYTES_PER_BOX = (11.7e6 + 11.4e6) / 262144
+INC32_DRAM_BYTES_PER_BOX = 12.0e6 / 262144
+SCREEN32_DRAM_BYTES_PER_POINT = 20.0e6 / 262144
+VERDICT_DRAM_BYTES_PER_BOX = (16.9e6 + 16.9e6) / 16384 + 9
 # time-to-gap on the n=4 QCQP: the cluster of boxes within 1e-6 of the optimum
 # holds tens of millions of boxes at n=4, so the frontier is capped at 2^25;
 # 2^21 parents x 2^2 children per iteration timed best (swept over
@@ -435,7 +433,7 @@ def batch_run(rt, precision, steps, warmup, n_inst=1024):
     b.sync()
     c0, _ = b.totals()
     phases = []
-    for _ in range(steps):  # device time of each captured iteration, from its own phase events
+    for _ in range(steps):  # device time of each captured iteration, from its own phase times
         b.launch(1)
         phases.append(b.phase_ms())
     ms = sum(p[4] for p in phases)

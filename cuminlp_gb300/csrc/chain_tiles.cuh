@@ -2,7 +2,7 @@
 // chains (every quadratic model), in two passes: the constraints, a tile of
 // boxes per block and a warp per chain; then the objective (chain_core.cuh).
 // The single-instance kernels are in chain_kernels.cu, the batch's in
-// batch_kernels.cu.
+// batch_chain_kernels.cu.
 //
 // What bounds it: FP64 instructions issue at 1/64 of the FP32 rate, and the
 // interpreter spends four of them per term on both bounds of every chain.

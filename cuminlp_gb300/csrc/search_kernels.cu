@@ -1364,7 +1364,7 @@ __device__ __forceinline__ void copy_tile(const SolverCfg& cfg, const SolverBufs
 // tiles throughout, so it needs only the counts of the blocks before it and no
 // scan of its own.  As twelve launches over a grid of every tile the pool
 // could have, an iteration of the n = 4 plain solve (a few hundred entries,
-// room for 2^24) spent 76 of its 178 us here.
+// room for 2^24) spent 76 of its 178 us here; the one launch takes 23.
 __global__ void __launch_bounds__(kScanBlock, 2) rebuild_kernel(const SolverCfg cfg, const SolverBufs b)
 {
   SolverDev* d = b.dev;
