@@ -27,7 +27,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) chain_constraints_kernel(c
 // no chain decides feasibility and the children's states are found here.
 // 2^lg lanes share a box when few boxes are live.
 template <int kMode, bool kFused, bool kHi>
-__device__ __forceinline__ void objective_boxes(const EvalArgs& a, unsigned char* smem_raw, int flags, uint64_t total)
+__device__ __forceinline__ void objective_boxes(const EvalArgs& a, unsigned char* smem_raw, int flags, uint64_t total,
+                                                unsigned block, unsigned blocks)
 {
   const int B = blockDim.x;
   const int ms = a.pinfo != nullptr ? a.max_slots : 0;
@@ -37,10 +38,10 @@ __device__ __forceinline__ void objective_boxes(const EvalArgs& a, unsigned char
   const double gub = a.gub ? *a.gub : DBL_MAX;
   const ChainSeg s = a.chain.seg[0];
   const bool pure = s.kind == kChainObjective;
-  const int lg = lanes_per_box(total, (uint64_t)gridDim.x * B, pure && !kHi ? 32 : 1);
+  const int lg = lanes_per_box(total, (uint64_t)blocks * B, pure && !kHi ? 32 : 1);
   const int G = 1 << lg;
   const uint64_t per_block = (uint64_t)(B >> lg);
-  for (uint64_t base = (uint64_t)blockIdx.x * per_block; base < total; base += (uint64_t)gridDim.x * per_block) {
+  for (uint64_t base = (uint64_t)block * per_block; base < total; base += (uint64_t)blocks * per_block) {
     const uint64_t idx = base + (threadIdx.x >> lg);
     const bool lead = (threadIdx.x & (G - 1)) == 0;
     bool live = idx < total;
@@ -86,7 +87,7 @@ __device__ __forceinline__ void objective_boxes(const EvalArgs& a, unsigned char
     }
   }
   if constexpr (kFused)
-    if ((threadIdx.x & 31) == 0) stamp_last(a.t_last, (uint64_t)blockIdx.x * per_block < total);
+    if ((threadIdx.x & 31) == 0) stamp_last(a.t_last, (uint64_t)block * per_block < total);
 }
 
 template <int kMode, bool kFused, bool kHi>
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const E
   if (a.done != nullptr && *a.done) return;
   if constexpr (kFused)
     if (!flags) stamp_first(a.t_first);
-  objective_boxes<kMode, kFused, kHi>(a, smem_raw, flags, box_count(a, kMode == 3));
+  objective_boxes<kMode, kFused, kHi>(a, smem_raw, flags, box_count(a, kMode == 3), blockIdx.x, gridDim.x);
 }
 
 // Most children the lane groups above take rather than the sharing kernel
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_siblings_kernel(const Ev
   const uint64_t total = box_count(a, false), tiles = (total + 31) >> 5;
   if constexpr (!kHi)
     if (total <= (uint64_t)few) {
-      objective_boxes<kMode, false, false>(a, smem_raw, flags, total);
+      objective_boxes<kMode, false, false>(a, smem_raw, flags, total, blockIdx.x, gridDim.x);
       return;
     }
   if (tiles <= gridDim.x) {  // a block for every tile
@@ -130,6 +131,29 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_siblings_kernel(const Ev
   unsigned char* smem = smem_raw + family_bytes(families, a.max_slots, kHi) * wid;
   for (uint64_t tile = (uint64_t)blockIdx.x * W + wid; tile < tiles; tile += (uint64_t)gridDim.x * W)
     siblings_tile<kMode, kHi>(a, smem, flags, families, tile, total);
+}
+
+// Both passes of a role's regions in one launch: a region's bound does not wait
+// for its feasibility, and with few regions each pass is latency on a part of
+// the GPU.  The first `objective` blocks take the objective, the others the
+// constraints; `oa` leaves out_flag to them.  A call's time in two launches and
+// in one: n = 4, 4 regions 40 and 29 us; n = 32, 4,096 regions 124 and 101;
+// n = 64, 8,192 regions 170 and 123.
+__global__ void __launch_bounds__(kObjThreads, 5) chain_role_kernel(const EvalArgs ca, const EvalArgs oa, int log_boxes,
+                                                                    unsigned objective, int share)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ TileShared sh;
+  if (blockIdx.x < objective) {
+    const uint64_t total = box_count(oa, false);
+    if (share) siblings_tile<0, false, true>(oa, smem_raw, 0, 1, blockIdx.x, total);
+    else objective_boxes<0, false, false>(oa, smem_raw, 0, total, blockIdx.x, objective);
+    return;
+  }
+  const uint64_t total = box_count(ca, false);
+  const uint64_t tiles = (total + (1ULL << log_boxes) - 1) >> log_boxes;
+  for (uint64_t tile = blockIdx.x - objective; tile < tiles; tile += gridDim.x - objective)
+    constraints_tile<0, false>(ca, smem_raw, sh, log_boxes, tile, total);
 }
 
 static uint64_t resident(uint64_t blocks, const void* kernel, int threads, size_t smem)
@@ -183,6 +207,41 @@ static cudaError_t launch_chain_t(const EvalArgs& a, cudaStream_t s)
   return cudaGetLastError();
 }
 
+// The role's one launch: regions of one box whose results go straight to the
+// host (EvalArgs::flags is then free for the objective's blocks).  8,192 at
+// most: with 16,384 the constraints fill the GPU by themselves, with their own
+// kernel's eight warps a tile (n = 64: 226 us in two launches, 255 in one).
+constexpr uint64_t kRoleMost = 8192;
+// Above this many of them the objective's values are shared (512 regions, n =
+// 32: 116 us by lane groups, 90 us for 1,024 shared).
+constexpr uint64_t kRoleFew = 256;
+static bool role_fits(const EvalArgs& a)
+{
+  return a.max_boxes <= kRoleMost && a.flags != nullptr && a.out_ub == nullptr && a.pinfo != nullptr && a.log2C < 0 && a.chain.pure_objective &&
+         a.chain.n_seg > 1 &&
+         (kObjThreads / 32) * family_bytes(1, a.max_slots, false) + 1024 <= (size_t)max_dynamic_smem();
+}
+
+static cudaError_t launch_role(const EvalArgs& a, cudaStream_t s)
+{
+  const bool share = a.max_boxes > kRoleFew;
+  int lb = 5;
+  while (lb > 0 && (a.max_boxes >> lb) < (uint64_t)sm_count() * 2) --lb;
+  const uint64_t most = (uint64_t)sm_count() * 4;
+  const uint64_t tiles = (a.max_boxes + 31) / 32, groups = (a.max_boxes * 32 + kObjThreads - 1) / kObjThreads;
+  const uint64_t objective = share ? tiles : std::min(groups, most);
+  const uint64_t constraints = std::min<uint64_t>((a.max_boxes + (1ull << lb) - 1) >> lb, most);
+  const size_t smem = std::max(tile_smem_bytes(a.n_vars, a.max_slots, 1 << lb),
+                               share ? (kObjThreads / 32) * family_bytes(1, a.max_slots, false) : objective_smem(a));
+  EvalArgs ca = a, oa = a;
+  ca.flags = nullptr;
+  oa.out_flag = a.flags;
+  oa.flags = nullptr;
+  chain_role_kernel<<<(unsigned)(objective + constraints), kObjThreads, smem, s>>>(ca, oa, lb, (unsigned)objective,
+                                                                                   share ? 1 : 0);
+  return cudaGetLastError();
+}
+
 bool chain_fits(const EvalArgs& a)
 {
   // the statics of the kernel take under 1 KiB beside the tile
@@ -192,6 +251,7 @@ bool chain_fits(const EvalArgs& a)
 
 cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s)
 {
+  if (mode == 0 && role_fits(a)) return launch_role(a, s);
   if (mode == 0) return a.out_ub != nullptr ? launch_chain_t<0, false, true>(a, s) : launch_chain_t<0, false, false>(a, s);
   if (mode == 6) return launch_chain_t<0, true, false>(a, s);
   if (mode == 1) return launch_chain_t<1, false, false>(a, s);
@@ -219,7 +279,8 @@ static cudaError_t allow_both(int max_smem)
 
 cudaError_t set_chain_kernel_attributes(int max_smem)
 {
-  cudaError_t e = allow_both<0, false, true>(max_smem);
+  cudaError_t e = allow(chain_role_kernel, max_smem);
+  if (e == cudaSuccess) e = allow_both<0, false, true>(max_smem);
   if (e == cudaSuccess) e = allow_both<0, false, false>(max_smem);
   if (e == cudaSuccess) e = allow_both<0, true, false>(max_smem);
   if (e == cudaSuccess) e = allow_both<1, false, false>(max_smem);

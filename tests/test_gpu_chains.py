@@ -156,6 +156,6 @@ def test_few_and_many_siblings(bits, parents):
     compare(G.miqcqp_n32(4), 7, bisection_budget=bits, batch_parents=parents, frontier_cap=6000)
 
 
-@pytest.mark.parametrize("bits", [10, 15])
+@pytest.mark.parametrize("bits", [8, 10, 13, 14, 15])
 def test_few_and_many_regions(bits):
     test_role_regions(bits)
