@@ -287,4 +287,47 @@ __device__ __forceinline__ double chain_lo_group(const Instr* __restrict__ prog,
   }
 }
 
+// The upper bound of a plain chain by a group of lanes: the mirror of
+// chain_lo_lanes.  A term past the end is -0, which adds nothing in this
+// rounding.
+template <int kLg, typename V>
+__device__ __noinline__ double chain_hi_lanes(const Instr* __restrict__ prog, int pc0, int pc1, const V& vars, bool active)
+{
+  constexpr int G = 1 << kLg;
+  const int gl = threadIdx.x & (G - 1);
+  double acc = 0.0;
+  const Instr first = load_instr(prog, pc0);
+  if (active) {
+    if ((first.head & 7) == kOpLoadAcc) acc = (first.modes & 3) == kModeVar ? vars.var(first.a).hi : first.c;
+    else acc = term_hi(first, vars);  // initialising TERM
+  }
+  auto form = [&](int pc) {
+    if (!active || pc >= pc1) return -0.0;
+    const Instr cur = load_instr(prog, pc);
+    const double h = term_hi(cur, vars);
+    return ((cur.head >> 3) & kTermSub) != 0 ? -h : h;
+  };
+  double p = form(pc0 + 1 + gl);
+  for (int base = pc0 + 1; base < pc1; base += G) {
+    const double pn = form(base + G + gl);
+#pragma unroll
+    for (int j = 0; j < G; ++j) acc = __dadd_ru(acc, __shfl_sync(0xffffffffu, p, j, G));
+    p = pn;
+  }
+  return acc;
+}
+
+template <typename V>
+__device__ __forceinline__ double chain_hi_group(const Instr* __restrict__ prog, int pc0, int pc1, const V& vars, int lg,
+                                                 bool active)
+{
+  switch (lg) {
+    case 1: return chain_hi_lanes<1>(prog, pc0, pc1, vars, active);
+    case 2: return chain_hi_lanes<2>(prog, pc0, pc1, vars, active);
+    case 3: return chain_hi_lanes<3>(prog, pc0, pc1, vars, active);
+    case 4: return chain_hi_lanes<4>(prog, pc0, pc1, vars, active);
+    default: return chain_hi_lanes<5>(prog, pc0, pc1, vars, active);
+  }
+}
+
 }  // namespace cmn

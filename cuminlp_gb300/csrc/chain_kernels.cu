@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 4) chain_constraints_kernel(c
 // `flags`: the constraint pass ran, out_flag holds its verdicts; otherwise
 // no chain decides feasibility and the children's states are found here.
 // 2^lg lanes share a box when few boxes are live.
-template <int kMode, bool kFused, bool kHi>
+template <int kMode, bool kFused, bool kHi, bool kLanes>
 __device__ __forceinline__ void objective_boxes(const EvalArgs& a, unsigned char* smem_raw, int flags, uint64_t total,
                                                 unsigned block, unsigned blocks)
 {
@@ -38,7 +38,7 @@ __device__ __forceinline__ void objective_boxes(const EvalArgs& a, unsigned char
   const double gub = a.gub ? *a.gub : DBL_MAX;
   const ChainSeg s = a.chain.seg[0];
   const bool pure = s.kind == kChainObjective;
-  const int lg = lanes_per_box(total, (uint64_t)blocks * B, pure && !kHi ? 32 : 1);
+  const int lg = lanes_per_box(total, (uint64_t)blocks * B, pure && (!kHi || kLanes) ? 32 : 1);
   const int G = 1 << lg;
   const uint64_t per_block = (uint64_t)(B >> lg);
   for (uint64_t base = (uint64_t)block * per_block; base < total; base += (uint64_t)blocks * per_block) {
@@ -73,10 +73,15 @@ __device__ __forceinline__ void objective_boxes(const EvalArgs& a, unsigned char
       }
     }
     Verdict<double> v = verdict_init<double>();
-    bool general = !pure || kHi;
+    // (both bounds: one lane a box forms them together in the interpreter)
+    bool general = !pure || (kHi && (!kLanes || lg == 0));
     if (!general) {
       v.obj.lo = chain_lo_group<kFused>(a.prog, s.pc0, s.pc1, cv, lg, live);
       general = v.obj.lo != v.obj.lo;
+      if constexpr (kHi && kLanes) {
+        v.obj.hi = chain_hi_group(a.prog, s.pc0, s.pc1, cv, lg, live);
+        general = general || v.obj.hi != v.obj.hi;
+      }
     }
     if (general && live) chain_general<kFused>(a.prog, s.pc0, s.pc2, cv, v);
     v.feasible = feasible;
@@ -90,14 +95,15 @@ __device__ __forceinline__ void objective_boxes(const EvalArgs& a, unsigned char
     if ((threadIdx.x & 31) == 0) stamp_last(a.t_last, (uint64_t)block * per_block < total);
 }
 
-template <int kMode, bool kFused, bool kHi>
+// kLanes: lane groups for both bounds too.
+template <int kMode, bool kFused, bool kHi, bool kLanes = false>
 __global__ void __launch_bounds__(kObjThreads, 5) chain_objective_kernel(const EvalArgs a, int flags)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (a.done != nullptr && *a.done) return;
   if constexpr (kFused)
     if (!flags) stamp_first(a.t_first);
-  objective_boxes<kMode, kFused, kHi>(a, smem_raw, flags, box_count(a, kMode == 3), blockIdx.x, gridDim.x);
+  objective_boxes<kMode, kFused, kHi, kLanes>(a, smem_raw, flags, box_count(a, kMode == 3), blockIdx.x, gridDim.x);
 }
 
 // Most children the lane groups above take rather than the sharing kernel
@@ -121,7 +127,7 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_siblings_kernel(const Ev
   const uint64_t total = box_count(a, false), tiles = (total + 31) >> 5;
   if constexpr (!kHi)
     if (total <= (uint64_t)few) {
-      objective_boxes<kMode, false, false>(a, smem_raw, flags, total, blockIdx.x, gridDim.x);
+      objective_boxes<kMode, false, false, false>(a, smem_raw, flags, total, blockIdx.x, gridDim.x);
       return;
     }
   if (tiles <= gridDim.x) {  // a block for every tile
@@ -147,7 +153,7 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_role_kernel(const EvalAr
   if (blockIdx.x < objective) {
     const uint64_t total = box_count(oa, false);
     if (share) siblings_tile<0, false, true>(oa, smem_raw, 0, 1, blockIdx.x, total);
-    else objective_boxes<0, false, false>(oa, smem_raw, 0, total, blockIdx.x, objective);
+    else objective_boxes<0, false, false, false>(oa, smem_raw, 0, total, blockIdx.x, objective);
     return;
   }
   const uint64_t total = box_count(ca, false);
@@ -200,7 +206,14 @@ static cudaError_t launch_chain_t(const EvalArgs& a, cudaStream_t s)
       return cudaGetLastError();
     }
   }
+  // few boxes of a program that is not tiny: lane groups for both bounds, in a
+  // kernel of its own (their registers cost 9 % at 50,001 boxes).  Host boxes,
+  // n = 64: 300 boxes 750 -> 190 us, 12,000 boxes 1,003 -> 849; 30,000 and 60,000
+  // as one lane a box; n = 4, 30 instructions: 3,000 boxes 87 us by one lane, 91
+  // by groups.
   auto kernel = chain_objective_kernel<kMode, kFused, kHi>;
+  if constexpr (kHi && kMode == 0)
+    if (a.max_boxes <= 16384 && a.prog_len > 64) kernel = chain_objective_kernel<kMode, kFused, kHi, true>;
   const size_t smem = objective_smem(a);
   const uint64_t grid = resident((a.max_boxes * 32 + kObjThreads - 1) / kObjThreads, (const void*)kernel, kObjThreads, smem);
   kernel<<<(unsigned)grid, kObjThreads, smem, s>>>(a, chains > 0 ? 1 : 0);
@@ -274,6 +287,8 @@ static cudaError_t allow_both(int max_smem)
   cudaError_t e = allow(chain_constraints_kernel<kMode, kFused>, max_smem);
   if constexpr (!kFused && kMode != 3)
     if (e == cudaSuccess) e = allow(chain_siblings_kernel<kMode, kHi>, max_smem);
+  if constexpr (kHi && kMode == 0)
+    if (e == cudaSuccess) e = allow(chain_objective_kernel<kMode, kFused, kHi, true>, max_smem);
   return e == cudaSuccess ? allow(chain_objective_kernel<kMode, kFused, kHi>, max_smem) : e;
 }
 
