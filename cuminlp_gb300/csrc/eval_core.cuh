@@ -225,9 +225,12 @@ __device__ Iv<T> iv_div(Iv<T> a, Iv<T> b)
   using A = Arith<T>;
   Iv<T> r;
   if (b.lo > T(0) || b.hi < T(0)) {
-    if (is_finite(a.lo) && is_finite(a.hi) && is_finite(b.lo) && is_finite(b.hi) && a.lo <= a.hi && b.lo <= b.hi) {
-      // the extreme quotients lie at corners the signs pick, so two directed
-      // divisions (a dozen FP64 instructions each) stand for eight
+    // the extreme quotients lie at corners the signs pick, so two directed
+    // divisions (a dozen FP64 instructions each) stand for eight; a dividend
+    // that ends in -0 takes all eight, whose order settles the zero's sign
+    const bool minus_zero = (A::sgn(a.lo) && A::is_zero(a.lo)) || (A::sgn(a.hi) && A::is_zero(a.hi));
+    if (is_finite(a.lo) && is_finite(a.hi) && is_finite(b.lo) && is_finite(b.hi) && a.lo <= a.hi && b.lo <= b.hi &&
+        !minus_zero) {
       if (b.lo > T(0)) {
         r.lo = A::div_rd(a.lo, a.lo >= T(0) ? b.hi : b.lo);
         r.hi = A::div_ru(a.hi, a.hi >= T(0) ? b.lo : b.hi);

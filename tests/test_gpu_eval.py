@@ -10,6 +10,7 @@ import pytest
 import oracle as O
 from cuminlp_gb300 import _abi as A
 from cuminlp_gb300 import generators as G
+from cuminlp_gb300.problem import Problem
 from cuminlp_gb300.solver import DeviceProblem, eval_boxes
 from tests.conftest import bits_equal
 from tests.gpu_common import ops_problem, random_boxes, with_objective
@@ -94,3 +95,28 @@ def test_enclosure_contains_sampled_points():
             x = rng.uniform(lo[:, b], hi[:, b])
             obj, _ = op.eval_point(x)
             assert lb[b] <= obj <= ub[b]
+
+
+@pytest.mark.parametrize("precision", [A.PRECISION_FP64, A.PRECISION_FP32_SCREEN])
+def test_quotients_of_signed_zeros(precision):
+    # every order of zeros, denormals and finite ends in the dividend, over
+    # positive and negative divisors: the bounds' zeros keep the oracle's sign
+    p = Problem()
+    x, y = p.var(-2.0, 2.0), p.var(0.5, 4.0)
+    p.set_objective(x / y)
+    ends = np.array([-2.0, -5e-324, -0.0, 0.0, 5e-324, 1e-300, 3.0])
+    divisors = np.array([-4.0, -0.5, -5e-324, 5e-324, 0.5, 4.0])
+    lo, hi = [], []
+    for a in ends:
+        for b in ends:
+            for c in divisors:
+                for d in divisors:
+                    if a <= b and c <= d and c * d > 0:
+                        lo.append((a, c))
+                        hi.append((b, d))
+    lo, hi = np.array(lo).T.copy(), np.array(hi).T.copy()
+    g = eval_boxes(DeviceProblem(p), lo, hi, precision)
+    o = O.OracleProblem(p).eval_boxes(lo, hi, precision)
+    for a, b in zip(g[:2], o[:2]):
+        nan = np.isnan(a) & np.isnan(b)
+        assert np.all(nan | (a.view(np.uint64) == b.view(np.uint64)))
