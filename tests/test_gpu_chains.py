@@ -159,3 +159,85 @@ def test_few_and_many_siblings(bits, parents):
 @pytest.mark.parametrize("bits", [8, 10, 13, 14, 15])
 def test_few_and_many_regions(bits):
     test_role_regions(bits)
+
+
+def long_problem(n: int = 12, readers: bool = False) -> Problem:
+    """An objective of more than 64 terms and <= chains of its length; with
+    `readers` an == chain and a root shared by the objective and a check."""
+    rng = np.random.default_rng(n)
+    p = Problem()
+    x = [p.int_var(-3.0, 6.0) if i % 5 == 4 else p.var(-4.0, 4.0) for i in range(n)]
+
+    def chain():
+        acc = float(rng.normal()) * x[0]
+        for i in range(n):
+            for j in range(i, n):
+                t = x[i] * x[j]
+                acc = acc - t if (i + j) % 7 == 3 else acc + float(rng.normal()) * t
+        return acc
+
+    obj = chain()
+    p.set_objective(obj)
+    p.add_constraint(chain(), A.CMP_LE, 20.0)
+    p.add_constraint(chain(), A.CMP_LE, 35.0)
+    if readers:
+        p.add_constraint(obj, A.CMP_LE, 300.0)
+        p.add_constraint(x[4] + 2.0 * x[9] - x[0] * x[1], A.CMP_EQ, 1.0)
+    return p
+
+
+OUTSIDE = [0.0, -0.0, 1e-300, 1e-20, 5e-324, 1e13, 1e30, 1e200, np.inf, -np.inf]
+
+
+def outside_boxes(p: Problem, value: float):
+    rng = np.random.default_rng(7)
+    lo, hi = random_boxes(p, 200, rng, 0.3)
+    at = rng.integers(0, lo.shape[0], 40), rng.integers(0, 200, 40)
+    lo[at] = np.minimum(value, hi[at])
+    both = rng.random(40) < 0.5
+    hi[at[0][both], at[1][both]] = np.maximum(value, lo[at[0][both], at[1][both]])
+    return lo, hi
+
+
+@pytest.mark.parametrize("value", OUTSIDE)
+def test_bounds_outside_the_filter_range_by_lane_groups(value):
+    # programs long enough for lane groups on both objective bounds
+    for p in (long_problem(), long_problem(readers=True)):
+        check(p, *outside_boxes(p, value))
+
+
+@pytest.mark.parametrize("value", OUTSIDE)
+def test_fp32_bounds_outside_the_fast_range(value):
+    for p in (mixed_problem(), near_problem(0.25), long_problem()):
+        lo, hi = outside_boxes(p, value)
+        g = eval_boxes(DeviceProblem(p), lo, hi, A.PRECISION_FP32_SCREEN)
+        o = O.OracleProblem(p).eval_boxes(lo, hi, A.PRECISION_FP32_SCREEN)
+        assert np.array_equal(g[2], o[2])
+        assert bits_equal(g[0], o[0]) and bits_equal(g[1], o[1])
+
+
+def outside_problem(n: int = 10) -> Problem:
+    """Variables whose bounds leave the fast ranges at either end beside
+    ordinary ones, so that parents inside and outside share a tile."""
+    p = Problem()
+    x = [p.var(-3e12, 3e12), p.var(-1e-14, 2e-14), p.int_var(0.0, 5.0)] + [p.var(-2.0, 3.0) for _ in range(n - 3)]
+    obj = 1e-12 * (x[0] * x[3]) + 3.0 * (x[1] * x[4]) - x[2] * x[5]
+    for i in range(3, n - 1):
+        obj = obj + 0.5 * (x[i] * x[i + 1])
+    p.set_objective(obj)
+    p.add_constraint(1e-12 * x[0] + x[3] * x[4] - 2.0 * x[2], A.CMP_LE, 4.0)
+    p.add_constraint(x[5] * x[5] + 1e11 * (x[1] * x[6]), A.CMP_LE, 6.0)
+    return p
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "lazy"])
+@pytest.mark.parametrize("bits,parents", [(2, 31), (4, 70)])
+def test_solver_outside_the_fast_range(precision, bits, parents):
+    compare(outside_problem(), 9, bisection_budget=bits, batch_parents=parents, frontier_cap=900, precision=precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "lazy"])
+@pytest.mark.parametrize("bits,parents", [(1, 40), (3, 65), (5, 33)])
+def test_solver_other_readers(precision, bits, parents):
+    compare(long_problem(readers=True), 8, bisection_budget=bits, batch_parents=parents, frontier_cap=2000,
+            precision=precision)
