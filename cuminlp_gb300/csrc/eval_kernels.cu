@@ -260,7 +260,6 @@ __device__ __forceinline__ void eval_children(const EvalArgs& a, const S* plo, c
   T* ohi = olo + (size_t)ms * B;
   int32_t* ovid = reinterpret_cast<int32_t*>(base + (size_t)2 * (a.n_slots + ms) * B) + threadIdx.x;
 
-  if (a.done != nullptr && *a.done) return;
   uint64_t total;
   if (kMode == 3) total = *a.list_count;
   else total = a.n_children_dev ? *a.n_children_dev : a.n_children;
@@ -498,9 +497,11 @@ __global__ void __launch_bounds__(kEvalThreads, CMN_EVAL_MIN_BLOCKS) eval_childr
   if ((threadIdx.x & 31) == 0) stamp_last(a.t_last, (uint64_t)blockIdx.x * B < total);
 }
 
+// (A launch after the search has stopped leaves the phase times as they are.)
 template <typename T, int kMode, bool kFused = false>
 __global__ void __launch_bounds__(kEvalThreads, CMN_EVAL_MIN_BLOCKS) eval_children_kernel(const EvalArgs a)
 {
+  if (a.done != nullptr && *a.done) return;
   if constexpr (sizeof(T) == 4) {
     if (a.plo32 != nullptr) {
       eval_children<T, kMode, float>(a, a.plo32, a.phi32);
@@ -518,6 +519,7 @@ __global__ void __launch_bounds__(kEvalThreads, CMN_EVAL_MIN_BLOCKS) eval_childr
 template <int kMode, bool kFused = false>
 __global__ void __launch_bounds__(kEvalThreads, CMN_EVAL_MIN_BLOCKS) eval_children_staged_kernel(const EvalArgs a)
 {
+  if (a.done != nullptr && *a.done) return;
   if constexpr (kFused) stamp_first(a.t_first);
   eval_children<double, kMode, double, true, kFused>(a, a.plo, a.phi);
   if constexpr (kFused)

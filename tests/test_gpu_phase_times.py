@@ -7,8 +7,10 @@ import time
 
 import pytest
 
+from cuminlp_gb300 import _abi as A
 from cuminlp_gb300 import generators as G
 from cuminlp_gb300._lib import CmnError
+from cuminlp_gb300.problem import Problem, sqr
 from cuminlp_gb300.solver import Batch, DeviceProblem, Solver
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +46,19 @@ def test_phase_times(precision, iterations):
     b = Batch(2, dp.n_vars, precision=s.options.precision, **SHARED)
     b.add(dp, iter_limit=1 << 30)
     check_phases(b, lambda: b.step(iterations))
+
+
+@pytest.mark.parametrize("bits", [1, 4])
+def test_lazy_times_after_the_stop(bits):
+    # a program with shared slots takes the interpreter; the iterations queued
+    # behind the last one that expanded boxes leave its times as they are
+    p = Problem()
+    x = [p.var(-2.0, 3.0) for _ in range(5)]
+    s = sqr(x[0]) + 1.0
+    p.set_objective(sqr(x[1] - x[2]) / s + 0.5 * s + x[3] * x[4])
+    p.add_constraint(s * x[3], A.CMP_LE, 4.0)
+    solver = Solver(DeviceProblem(p), precision="lazy", iter_limit=1 << 30, batch_iter_limit=5, bisection_budget=bits,
+                    batch_parents=64, frontier_cap=1024)
+    solver.step(0)
+    whole = solver.phase_ms()[4]
+    assert all(0 < t <= whole for t in solver.lazy_ms())
