@@ -791,6 +791,25 @@ extern "C" cmn_status cmn_enumerate(cmn_role* r, const double* box, const uint64
 // ----------------------------------------------------------------------
 // raw batched evaluation
 // ----------------------------------------------------------------------
+// n planes of n_boxes doubles, `stride` apart on the host, packed on the device.
+static cudaError_t copy_planes(double* dst, const double* src, int64_t n, uint64_t n_boxes, uint64_t stride, int device,
+                               cudaStream_t s)
+{
+  const size_t row = n_boxes * sizeof(double);
+  int max_pitch = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&max_pitch, cudaDevAttrMaxPitch, device);
+  if (e != cudaSuccess) return e;
+  switch (plane_copy((uint64_t)n, n_boxes, stride, (uint64_t)max_pitch)) {
+    case PlaneCopy::kPacked: return cudaMemcpyAsync(dst, src, (size_t)n * row, cudaMemcpyHostToDevice, s);
+    case PlaneCopy::kPitched:
+      return cudaMemcpy2DAsync(dst, row, src, stride * sizeof(double), row, (size_t)n, cudaMemcpyHostToDevice, s);
+    case PlaneCopy::kEach: break;
+  }
+  for (int64_t v = 0; v < n && e == cudaSuccess; ++v)
+    e = cudaMemcpyAsync(dst + (size_t)v * n_boxes, src + (size_t)v * stride, row, cudaMemcpyHostToDevice, s);
+  return e;
+}
+
 extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, const double* lo, const double* hi,
                                      uint64_t n_boxes, uint64_t stride, double* obj_lb, double* obj_ub,
                                      uint8_t* feasible, int32_t device_pointers, void* stream)
@@ -842,9 +861,8 @@ extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, co
       tmp = reinterpret_cast<double*>(own);
     }
     tmpf = reinterpret_cast<uint8_t*>(tmp + 2 * planes + 2 * n_boxes);
-    const size_t row = n_boxes * sizeof(double);
-    CK(cudaMemcpy2DAsync(tmp, row, lo, stride * sizeof(double), row, (size_t)n, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpy2DAsync(tmp + planes, row, hi, stride * sizeof(double), row, (size_t)n, cudaMemcpyHostToDevice, s));
+    CK(copy_planes(tmp, lo, n, n_boxes, stride, p->device, s));
+    CK(copy_planes(tmp + planes, hi, n, n_boxes, stride, p->device, s));
     dlo = tmp;
     dhi = tmp + planes;
     dlb = tmp + 2 * planes;

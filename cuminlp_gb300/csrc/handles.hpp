@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -93,6 +94,17 @@ struct cmn_problem {
 namespace cmn {
 
 constexpr size_t kEvalWorkspace = 64u << 20;
+
+// How `planes` planes of n_boxes doubles, `stride` apart, go to the device:
+// packed ones in one copy (33 boxes of two variables: 56 us a call, 73 by a
+// pitched copy), others in one pitched copy, or plane by plane where the
+// pitch is above the device's largest (documented as 2^31 - 1 bytes).
+enum class PlaneCopy { kPacked, kPitched, kEach };
+inline PlaneCopy plane_copy(uint64_t planes, uint64_t n_boxes, uint64_t stride, uint64_t max_pitch)
+{
+  if (stride == n_boxes || planes == 1) return PlaneCopy::kPacked;
+  return stride > max_pitch / sizeof(double) ? PlaneCopy::kEach : PlaneCopy::kPitched;
+}
 
 // Collects arrays and gives them places in one device allocation: a solver
 // has some forty, and each cudaMalloc / cudaFree of its own took 30-80 us.

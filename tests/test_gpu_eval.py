@@ -10,6 +10,7 @@ import pytest
 import oracle as O
 from cuminlp_gb300 import _abi as A
 from cuminlp_gb300 import generators as G
+from cuminlp_gb300._lib import check, lib
 from cuminlp_gb300.problem import Problem
 from cuminlp_gb300.solver import DeviceProblem, eval_boxes
 from tests.conftest import bits_equal
@@ -120,3 +121,22 @@ def test_quotients_of_signed_zeros(precision):
     for a, b in zip(g[:2], o[:2]):
         nan = np.isnan(a) & np.isnan(b)
         assert np.all(nan | (a.view(np.uint64) == b.view(np.uint64)))
+
+
+@pytest.mark.parametrize("stride", [5, 6, (1 << 28) - 1, 1 << 28])
+def test_host_planes_of_any_stride(stride):
+    # a few boxes of planes up to 2 GiB apart (untouched memory between them)
+    p = Problem()
+    x, y = p.var(-2.0, 2.0), p.var(-3.0, 4.0)
+    p.set_objective(x * y + 2.0 * x)
+    p.add_constraint(x + y, A.CMP_LE, 1.0)
+    lo, hi = random_boxes(p, 5, np.random.default_rng(1), 0.3)
+    far = [np.empty(stride + 5), np.empty(stride + 5)]
+    for f, b in zip(far, (lo, hi)):
+        f[:5], f[stride:stride + 5] = b[0], b[1]
+    lb, ub, fe = np.empty(5), np.empty(5), np.empty(5, dtype=np.uint8)
+    dp = DeviceProblem(p)
+    check(lib().cmn_eval_boxes(dp.handle, A.PRECISION_FP64, A.ptr(far[0]), A.ptr(far[1]), 5, stride, A.ptr(lb),
+                               A.ptr(ub), A.ptr(fe), 0, None))
+    o = O.OracleProblem(p).eval_boxes(lo, hi, A.PRECISION_FP64)
+    assert bits_equal(lb, o[0]) and bits_equal(ub, o[1]) and np.array_equal(fe, o[2])
