@@ -1319,6 +1319,7 @@ extern "C" cmn_status cmn_solver_step(cmn_solver* s, uint64_t max_iterations)
   const auto t0 = std::chrono::steady_clock::now();
   cmn_status st = pull_state(s);
   if (st != CMN_OK) return st;
+  if (s->h_dev->error) return fail(CMN_INTERNAL, "device-side error flag set");
   uint64_t done_iters = 0;
   uint64_t burst = 1;
   while (!s->h_dev->done && (max_iterations == 0 || done_iters < max_iterations)) {

@@ -88,6 +88,17 @@ struct SolverDev {
   uint64_t stamps[8];      // phase boundaries of the last iteration (ns); solver_iteration
 };
 
+// A device error ends the search: a barrier whose wait ran out leaves its
+// tickets part-counted and the lists behind it part-written.  What reads them
+// stops at once (halted), and no later iteration of a queued burst begins.
+inline __host__ __device__ bool halted(const SolverDev& d) { return d.done != 0 || d.error != 0; }
+inline __host__ __device__ bool begin_search(SolverDev& d)
+{
+  d.improved = 0;  // an iteration after the stop must not rewrite the witness
+  if (d.error) d.done = 1;
+  return !d.done;
+}
+
 // Static configuration baked into the captured iteration.
 struct SolverCfg {
   int n_vars;

@@ -88,8 +88,7 @@ __global__ void free_init_kernel(const SolverCfg cfg, const SolverBufs b)
 __global__ void begin_kernel(const SolverCfg cfg, const SolverBufs b)
 {
   SolverDev* d = b.dev;
-  d->improved = 0;  // an iteration after the stop must not rewrite the witness
-  if (d->done) return;
+  if (!begin_search(*d)) return;
   const uint64_t L = d->pool_size;
   if (L == 0) {
     d->done = 1;
@@ -740,7 +739,7 @@ __global__ void __launch_bounds__(kScanBlock) scatter_kernel(const P pred, const
 __global__ void append_children_kernel(const SolverCfg cfg, const SolverBufs b)
 {
   const SolverDev* d = b.dev;
-  if (d->done) return;
+  if (halted(*d)) return;
   const uint64_t n = d->kept;
   const AppendChild op{cfg, b};
   for (uint64_t pos = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; pos < n; pos += (uint64_t)gridDim.x * blockDim.x)
@@ -761,7 +760,7 @@ template <int G>
 __global__ void __launch_bounds__(256) append_boxes_kernel(const SolverCfg cfg, const SolverBufs b)
 {
   const SolverDev* d = b.dev;
-  if (d->done) return;
+  if (halted(*d)) return;
   const uint64_t kept = d->kept, free_top = d->free_top;
   const int n = cfg.n_vars;
   const int gl = threadIdx.x & (G - 1);
@@ -1053,7 +1052,7 @@ __device__ void finish_pool(const SolverCfg& cfg, const SolverBufs& b)
 // last one runs `last` and opens it.  The launch is cooperative, so every block is
 // resident and the others wait no longer than a pass takes; the wait has a
 // limit (about a second) all the same, after which the device error is set and
-// false returned.
+// false returned: the search ends there (halted).
 constexpr uint32_t kBarrierSpins = 1u << 21;
 template <class F>
 __device__ __forceinline__ bool grid_barrier(SolverDev* d, unsigned blocks, F last)
@@ -1368,7 +1367,7 @@ __device__ __forceinline__ void copy_tile(const SolverCfg& cfg, const SolverBufs
 __global__ void __launch_bounds__(kScanBlock, 2) rebuild_kernel(const SolverCfg cfg, const SolverBufs b)
 {
   SolverDev* d = b.dev;
-  if (d->done) return;
+  if (halted(*d)) return;
   const uint64_t n = d->extent;
   const unsigned blocks = blocks_for(n, kScanBlock);
   if (blockIdx.x >= blocks) return;

@@ -40,3 +40,25 @@ def test_planes_beyond_the_largest_pitch_go_one_by_one(tmp_path):
     CHECK(plane_copy(4, 1ull << 28, (1ull << 28) + 1, most) == PlaneCopy::kEach);
     CHECK(plane_copy(1, 100, 1ull << 40, most) == PlaneCopy::kPacked);
     """)
+
+
+def test_a_device_error_ends_the_search(tmp_path):
+    # a barrier's wait that ran out in one iteration: the kernels behind it
+    # stop, and the burst's other iterations begin nothing
+    run(tmp_path, "search.hpp", """
+    static SolverDev d;
+    d.pool_size = 5;
+    d.improved = 1;
+    CHECK(begin_search(d) && !halted(d) && d.improved == 0);
+    d.ticket = 3;
+    d.error = 1;
+    CHECK(halted(d));
+    for (int i = 0; i < 63; ++i) {
+      d.improved = 1;
+      CHECK(!begin_search(d) && halted(d) && d.done == 1 && d.improved == 0);
+    }
+    CHECK(d.pool_size == 5 && d.error == 1);
+    static SolverDev stopped;
+    stopped.done = 1;
+    CHECK(!begin_search(stopped) && halted(stopped) && stopped.error == 0);
+    """)
