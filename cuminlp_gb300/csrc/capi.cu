@@ -254,14 +254,6 @@ extern "C" cmn_status cmn_program_compile(const cmn_problem_desc* desc, int32_t 
   }
 }
 
-// Threads of an interpreter block over `boxes` boxes.  Below two full blocks
-// an SM, one-warp blocks: they spread over the SMs, and FP64 work is bound by
-// each SM's own pipe (3,001 boxes in blocks of 128 keep 24 of 152 SMs busy).
-static int eval_threads(uint64_t boxes)
-{
-  return boxes <= (uint64_t)sm_count() * 2 * kEvalThreads ? 32 : kEvalThreads;
-}
-
 static cmn_status check_interval(const cmn_problem* p)
 {
   if (!p->prog.interval_supported)
@@ -366,7 +358,6 @@ struct cmn_role {
   uint64_t S = 1;
   cudaStream_t stream = nullptr;
   int grid = 1;
-  int threads = kEvalThreads;  // of the bounder's interpreter blocks
   int lg_min = 0;  // sampler: lanes per point column (sample_lg_min)
   // one device block: [box lo planes n][box hi planes n][slots][pinfo]
   unsigned char* d_stage = nullptr;
@@ -495,8 +486,7 @@ extern "C" cmn_status cmn_role_build(const cmn_problem* p, int32_t role, const u
     cudaError_t e = cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = dalloc(&r->d_stage, r->stage_bytes);
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&r->h_stage), r->stage_bytes);
-    const int threads = role == CMN_ROLE_BOUNDER ? eval_threads(n_regions) : kEvalThreads;
-    r->threads = threads;
+    const int threads = kEvalThreads;
     const uint64_t blocks_needed = (n_regions * (uint64_t)p->prog.group_max + threads - 1) / threads;
     const int occ = std::max(
         1, eval_kernel_occupancy(0, false, eval_smem_bytes(p->prog.n_slots, (int)slot_count, false, threads), threads));
@@ -612,13 +602,13 @@ extern "C" cmn_status cmn_bound(cmn_role* r, const double* box, const uint64_t* 
   a.out_flag = r->d_feas;
   a.sched = r->p->d_sched;
   a.g_max = r->p->prog.group_max;
-  a.capacity = (uint64_t)r->grid * r->threads;
+  a.capacity = (uint64_t)r->grid * kEvalThreads;
   if (r->direct) {
     a.out_lb = r->h_lb;
     a.out_flag = r->h_feas;
     a.flags = r->d_feas;
   }
-  CK(launch_eval(a, 0, false, r->grid, r->threads, r->stream));
+  CK(launch_eval(a, 0, false, r->grid, kEvalThreads, r->stream));
   if (!r->direct) CK(cudaMemcpyAsync(r->h_lb, r->d_lb, r->n_regions * 9, cudaMemcpyDeviceToHost, r->stream));
   CK(cudaStreamSynchronize(r->stream));
   if (feasible) *feasible = r->h_feas;
@@ -696,12 +686,12 @@ extern "C" cmn_status cmn_bound_children(cmn_role* r, const double* box, const u
   a.max_boxes = r->n_regions;
   a.sched = r->p->d_sched;
   a.g_max = r->p->prog.group_max;
-  a.capacity = (uint64_t)r->grid * r->threads;
+  a.capacity = (uint64_t)r->grid * kEvalThreads;
   a.out_flag = r->d_feas;  // scratch: the regions' feasibility
   a.agg_keys = r->d_agg;
   a.agg_m = r->n_regions / k;
   a.agg_k = k;
-  CK(launch_eval(a, 4, false, r->grid, r->threads, r->stream));
+  CK(launch_eval(a, 4, false, r->grid, kEvalThreads, r->stream));
   CK(cudaMemcpyAsync(r->h_agg, r->d_agg, 2 * k * sizeof(unsigned long long), cudaMemcpyDeviceToHost, r->stream));
   CK(cudaStreamSynchronize(r->stream));
   for (uint64_t c = 0; c < k; ++c) {
@@ -886,7 +876,7 @@ extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, co
   a.out_lb = dlb;
   a.out_ub = dub;
   a.out_flag = dfe;
-  const int threads = eval_threads(n_boxes);
+  const int threads = kEvalThreads;
   const int occ =
       std::max(1, eval_kernel_occupancy(0, fp32, eval_smem_bytes(p->prog.n_slots, 0, fp32, threads), threads));
   const uint64_t need = (n_boxes * (uint64_t)p->prog.group_max + threads - 1) / threads;
