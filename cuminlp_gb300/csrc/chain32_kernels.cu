@@ -140,6 +140,20 @@ bool chain32_fits(const EvalArgs& a, int mode)
          eval32_smem(a.n_vars) + 1024 <= (size_t)max_dynamic_smem();
 }
 
+// Whether the tiles beat the interpreter over boxes (the screen always takes
+// them).  Staging a box costs about as much as a term a variable, so a chain
+// that reads each variable once or so does not pay where a tile is large: n =
+// 64, 65 instructions, 65,536 boxes 40 us by the interpreter and 67 in tiles; n
+// = 32, 33 instructions, 100,000 boxes 37 and 30.  Programs of less than 12
+// instructions take launch time either way (11 and 12 us) up to some 10^5
+// boxes (n = 2, 6 instructions, 524,288 boxes 26 and 22).
+bool chain32_pays(const EvalArgs& a, int mode)
+{
+  if (mode != 0) return true;
+  const int64_t len = a.prog_len, n = a.n_vars;
+  return (len >= 12 && (n <= 32 || len >= 2 * n)) || (len >= 6 && a.max_boxes >= 131072 && 5 * len >= 6 * n);
+}
+
 template <int kMode>
 static cudaError_t launch_chain32_t(const EvalArgs& a, cudaStream_t s)
 {

@@ -262,6 +262,68 @@ bool chain_fits(const EvalArgs& a)
          tile_smem_bytes(a.n_vars, a.pinfo != nullptr ? a.max_slots : 0, 32) + 1024 <= (size_t)max_dynamic_smem();
 }
 
+// Whether the passes here beat the interpreter's one launch.  They save three
+// quarters of the <= chains' time, for a second launch and the staging of every
+// box, worth about 3/4 of a term a variable and 3/2 a chain; `saved` is what is
+// left, in quarters of a term a box.  Boxes, both bounds, interpreter against
+// here: n = 4, one constraint (30 instructions), 20,000 boxes 26 and 39 us,
+// 65,536 boxes 49 and 47, 524,288 boxes 220 and 148; n = 8, three constraints
+// (145), 2,000 boxes 56 and 46, 131,072 boxes 359 and 126; n = 2, one
+// constraint (6), 524,288 boxes 32 and 44.  Few boxes of a long program: here
+// lane groups form the objective faster (64 terms, 300 boxes 48 and 19 us).
+// Chains with other readers keep the interpreter's arithmetic here, a warp
+// each, so they need many boxes, and <= chains beside them to pay: sixteen ==
+// chains of n = 24, 1,000 boxes 291 and 760 us; two chains of n = 24, one ==,
+// 8,192 boxes 247 and 316, 131,072 boxes 1,427 and 986.
+static bool general_pays(const EvalArgs& a, int mode, int64_t boxes, int64_t saved)
+{
+  const ChainTab& t = a.chain;
+  const bool pure = t.pure_objective != 0;
+  // the solver's children and parents: with many of them the chains fill the
+  // GPU (256 parents x 4 children, sixteen == chains, n = 24: 8.6 and 10.8 ms)
+  if (mode == 1 || mode == 3 || mode == 6) return boxes >= 8192 || (pure && t.general <= 4);
+  // a role's one launch (n = 12, 1,024 regions, four == chains 134 and 103 us,
+  // eight 146 and 168)
+  if (mode == 0 && role_fits(a)) return t.general <= 4;
+  if (boxes < 8192) return false;
+  const int64_t terms = t.general_terms;
+  if (t.constraint_terms >= 2 * terms && saved >= 160 && saved * boxes >= 12000000) return true;
+  if (!pure) return false;
+  // 180 boxes a term of an average such chain keep the other warps busy
+  if (4 * t.constraint_terms >= 3 * terms && saved * boxes >= 2000000 && boxes >= 16384 &&
+      boxes * t.general >= 180 * terms)
+    return true;
+  // between one wave and many, several chains spread over the warps (n = 12,
+  // four == chains, 16,384 boxes 178 and 132 us; 524,288 boxes 2,014 and 2,030)
+  return (t.general >= 2 && a.prog_len >= 140 && boxes >= 32768 && boxes <= 262144) ||
+         (t.general >= 4 && a.prog_len >= 86 && boxes >= 16384 && boxes < 98304);
+}
+
+bool chain_pays(const EvalArgs& a, int mode)
+{
+  const ChainTab& t = a.chain;
+  const int64_t boxes = (int64_t)a.max_boxes, len = a.prog_len;
+  const int64_t saved = 4ll * t.constraint_terms - 3ll * a.n_vars - 6ll * t.constraints;
+  if (t.general > 0) return general_pays(a, mode, boxes, saved);
+  if (mode == 1 || mode == 3 || mode == 6) return true;  // in the solver no form or size lost
+  const bool region = a.pinfo != nullptr, both = mode == 4 || a.out_ub != nullptr;
+  if (t.constraints == 0) {
+    // the objective alone: the same work on either side, the program staged
+    // there, lane groups or half the bounds here
+    if (mode == 4) return len >= 45;
+    if (region) return true;
+    if (both) return (len > 64 && boxes <= 10240) || (len >= 5 && boxes >= 98304);
+    return len >= 12 || (len > 3 && boxes >= 65536);
+  }
+  if (mode == 4)  // 8 of n = 4's 30 instructions a child: 65,536 regions 74 and 66 us, 16,384 50 and 65
+    return len >= 20 && (len >= 72 || saved * boxes >= 3200000) && (len >= 40 || 2 * t.constraint_terms >= len);
+  if (region) return role_fits(a) || saved * boxes >= 1600000;
+  if (both)
+    return saved * boxes >= (boxes <= 16384 ? 4200000 : 3200000) ||
+           (boxes <= 16384 && len >= 78 + boxes / 140 && (saved >= 64 || boxes <= 2048));
+  return len >= 64 || saved * boxes >= 2800000 || (len >= 30 && boxes <= 512);
+}
+
 cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s)
 {
   if (mode == 0 && role_fits(a)) return launch_role(a, s);

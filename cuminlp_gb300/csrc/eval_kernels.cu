@@ -1096,12 +1096,12 @@ cudaError_t launch_eval(const EvalArgs& a, int mode, bool fp32, int grid, int th
 {
   if (mode == 0 && level_fits(a, fp32)) return launch_level(a, fp32, s);
   if (fp32) {
-    if (chain32_fits(a, mode)) return launch_chain32(a, mode, s);
+    if (chain32_fits(a, mode) && chain32_pays(a, mode)) return launch_chain32(a, mode, s);
     if (mode == 0) return launch_eval_t<float, 0>(a, grid, threads, s);
     if (mode == 5) return launch_eval_t<float, 5>(a, grid, threads, s);
     return launch_eval_t<float, 2>(a, grid, threads, s);
   }
-  if (chain_fits(a)) return launch_chain(a, mode, s);
+  if (chain_fits(a) && chain_pays(a, mode)) return launch_chain(a, mode, s);
   if (mode == 0) return launch_eval_t<double, 0>(a, grid, threads, s);
   if (mode == 6) return launch_eval_t<double, 0, true>(a, grid, threads, s);
   if (mode == 1) return launch_eval_t<double, 1>(a, grid, threads, s);

@@ -69,6 +69,13 @@ struct cmn_problem {
       const int64_t len = s.pc1 - s.pc0;
       all += len;
       if (len > most) most = len;
+      if (s.kind == cmn::kChainLe) {
+        t.constraints += 1;
+        t.constraint_terms += (int32_t)len;
+      } else if (s.kind == cmn::kChainGeneral) {
+        t.general += 1;
+        t.general_terms += (int32_t)len;
+      }
     }
     const int64_t w = (all + most - 1) / most;
     t.warps32 = (int32_t)(w < 1 ? 1 : w > 8 ? 8 : w);

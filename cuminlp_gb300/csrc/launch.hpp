@@ -40,8 +40,10 @@ int sample_screen_lg_min(int n_vars, int n_slots, bool has_sched, int threads);
 // each term's coefficient and chain add fused into __fma_rd / __fma_ru)
 cudaError_t launch_eval(const EvalArgs& a, int mode, bool fp32, int grid, int threads, cudaStream_t s);
 // The FP64 modes over a program of sum chains (EvalArgs::chain):
-// chain_kernels.cu.  chain_fits: whether the launch takes that path.
+// chain_kernels.cu.  chain_fits: whether the launch can take that path;
+// chain_pays: whether it is the faster one.
 bool chain_fits(const EvalArgs& a);
+bool chain_pays(const EvalArgs& a, int mode);
 cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s);
 cudaError_t set_chain_kernel_attributes(int max_smem);
 // mode 0 over few boxes of a program in levels (level_kernels.cu)
@@ -51,6 +53,7 @@ cudaError_t set_level_kernel_attributes(int max_smem);
 // FP32 modes 0 (boxes) and 2 (screen) over such a program, and the lazy
 // form's child bounds (chain32_kernels.cu)
 bool chain32_fits(const EvalArgs& a, int mode);
+bool chain32_pays(const EvalArgs& a, int mode);
 cudaError_t launch_chain32(const EvalArgs& a, int mode, cudaStream_t s);
 bool lazy_children_fits(const ChainTab& t, int n_vars, int max_slots, int log2C);
 cudaError_t launch_lazy_children(const EvalArgs& a, uint64_t max_parents, cudaStream_t s);

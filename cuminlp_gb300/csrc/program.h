@@ -171,6 +171,10 @@ struct ChainTab {
   const ChainTerm* term_pt;
   int32_t n_vars;
   int32_t warps32;  // warps of a tile that keep its chains' lengths balanced
+  // what the choice of a path goes by: the <= chains and their terms, the
+  // kChainGeneral ones and theirs
+  int32_t constraints, constraint_terms;
+  int32_t general, general_terms;
 };
 
 // A program laid out in levels (Program::level_*), on the device.

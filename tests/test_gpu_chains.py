@@ -12,6 +12,7 @@ import pytest
 import oracle as O
 from cuminlp_gb300 import _abi as A
 from cuminlp_gb300 import generators as G
+from cuminlp_gb300._lib import check as status, lib
 from cuminlp_gb300.problem import Expr, Problem
 from cuminlp_gb300.solver import Bounder, DeviceProblem, Sampler, eval_boxes
 from tests.conftest import bits_equal
@@ -241,3 +242,66 @@ def test_solver_outside_the_fast_range(precision, bits, parents):
 def test_solver_other_readers(precision, bits, parents):
     compare(long_problem(readers=True), 8, bisection_budget=bits, batch_parents=parents, frontier_cap=2000,
             precision=precision)
+
+
+def chain_problem(n: int, terms: int, constraints: int, equalities: int = 0, shared: bool = False) -> Problem:
+    """Chains of about `terms` products each."""
+    rng = np.random.default_rng(100 * n + terms)
+    p = Problem()
+    x = [p.var(-4.0, 4.0) for _ in range(n)]
+
+    def chain():
+        acc = float(rng.normal()) * x[0]
+        for _ in range(terms):
+            i, j = rng.integers(0, n, 2)
+            acc = acc + float(rng.normal()) * (x[i] * x[j])
+        return acc
+
+    obj = chain()
+    p.set_objective(obj)
+    for k in range(constraints):
+        p.add_constraint(chain(), A.CMP_EQ if k < equalities else A.CMP_LE, 3.0 + k)
+    if shared:
+        p.add_constraint(obj, A.CMP_LE, 5.0)
+    return p
+
+
+# shapes that change the path with the number of boxes: no constraint, short
+# and long ones, equalities, a root with two readers
+PATHS = [(2, 2, 0), (3, 12, 0), (6, 70, 0), (2, 2, 1), (4, 12, 1), (6, 25, 3), (9, 60, 2), (4, 10, 2, 1),
+         (6, 30, 6, 5), (5, 60, 3, 1), (6, 25, 4, 0, True), (40, 20, 1), (40, 70, 0)]
+
+
+@pytest.mark.parametrize("boxes", [511, 2049, 8191, 10240, 16385, 40000, 98304, 131072])
+def test_either_path(boxes):
+    for shape in PATHS:
+        p = chain_problem(*shape)
+        if boxes > 20000 and p.n_vars > 6:
+            continue
+        rng = np.random.default_rng(boxes)
+        lo, hi = random_boxes(p, boxes, rng, 0.3)
+        dp, op = DeviceProblem(p), O.OracleProblem(p)
+        for precision in (A.PRECISION_FP64, A.PRECISION_FP32_SCREEN):
+            g, o = eval_boxes(dp, lo, hi, precision), op.eval_boxes(lo, hi, precision)
+            assert np.array_equal(g[2], o[2])
+            assert bits_equal(g[0], o[0]) and bits_equal(g[1], o[1])
+            # the lower bound alone
+            lb, fe = np.empty(boxes), np.empty(boxes, dtype=np.uint8)
+            status(lib().cmn_eval_boxes(dp.handle, precision, A.ptr(lo), A.ptr(hi), boxes, boxes, A.ptr(lb), None,
+                                        A.ptr(fe), 0, None))
+            assert np.array_equal(fe, o[2]) and bits_equal(lb, o[0])
+
+
+@pytest.mark.parametrize("bits", [6, 13, 14, 16])
+def test_either_path_of_regions(bits):
+    for shape in PATHS:
+        p = chain_problem(*shape)
+        kinds, vids, widths, _ = O.bisection_choose(p.root_box(), p.var_kinds, bits)
+        n = int(np.prod(widths))
+        b, op = Bounder(DeviceProblem(p), kinds, n), O.OracleProblem(p)
+        fe, lb = b.bound(p.root_box(), vids, widths)
+        ofe, olb = op.bound(p.root_box(), kinds, vids, widths, n)
+        assert np.array_equal(fe, ofe) and bits_equal(lb, olb)
+        clb, cub, cfe = b.bound_children(p.root_box(), vids, widths, 4)
+        olb, oub, ofe = op.aggregate_bound(p.root_box(), kinds, vids, widths, n, 4)
+        assert np.array_equal(cfe, ofe) and bits_equal(clb, olb) and bits_equal(cub, oub)
