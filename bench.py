@@ -822,10 +822,11 @@ def run_ours(args):
                 "time_to_gap_run": serving_ttg_run()}
 
     def autotune_leg():
-        # cmn_autotune on the headline problem: launch shapes timed over
-        # 2^18 random boxes, FP64 and FP32 evaluator
+        # cmn_autotune on the headline problem over 2^18 random boxes, FP64 and
+        # FP32: a set of sum chains, whose kernels size their own grids
         return {"fp64": dp.autotune(0, 1 << 18), "fp32": dp.autotune(1, 1 << 18),
-                "candidates": "blocks per SM 1..residency x lanes per box 1, 2, 4 .. program maximum"}
+                "candidates": "one (sum chains); otherwise blocks per SM 1..residency x lanes per box 1, 2, 4 .. "
+                              "program maximum"}
 
     ref_gpu = None if args.no_reference_gpu else extra_leg(reference_gpu_run)
     tune = extra_leg(autotune_leg)

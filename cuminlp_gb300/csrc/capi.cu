@@ -900,6 +900,16 @@ extern "C" cmn_status cmn_eval_boxes(const cmn_problem* p, int32_t precision, co
 // ----------------------------------------------------------------------
 // solver
 // ----------------------------------------------------------------------
+// Whether a solver's bounds run kernels that size their own grids (sum chains
+// in tiles): the interpreter's shape is then not theirs to tune.
+static bool shape_fixed(const cmn_problem* p, bool fp32)
+{
+  EvalArgs a = {};
+  a.n_vars = (int)p->host.n_vars();
+  a.chain = p->chain();
+  return fp32 ? chain32_fits(a, 0) : chain_fits(a);
+}
+
 extern "C" cmn_status cmn_autotune(cmn_problem* p, int32_t precision, uint64_t n_boxes, cmn_tune_result* out)
 {
   if (!p || !out) return fail(CMN_INVALID_CONFIGURATION, "null argument");
@@ -962,6 +972,11 @@ extern "C" cmn_status cmn_autotune(cmn_problem* p, int32_t precision, uint64_t n
   a.out_lb = d + 2 * planes;
   a.out_flag = f;
   a.sched = p->d_sched;
+  const bool fixed = shape_fixed(p, fp32);
+  if (fixed) {  // one candidate: the path evaluation takes
+    a.chain = p->chain();
+    a.max_boxes = n_boxes;
+  }
   const int threads = kEvalThreads;
   const int occ =
       std::max(1, eval_kernel_occupancy(0, fp32, eval_smem_bytes(p->prog.n_slots, 0, fp32, threads), threads));
@@ -988,7 +1003,7 @@ extern "C" cmn_status cmn_autotune(cmn_problem* p, int32_t precision, uint64_t n
   out->ms_best = out->ms_default;
   out->blocks_per_sm = occ;
   out->lanes_cap = lanes_max;
-  for (int bps = 1; bps <= occ && e == cudaSuccess; ++bps) {
+  for (int bps = 1; bps <= occ && e == cudaSuccess && !fixed; ++bps) {
     for (int lanes = 1; lanes <= lanes_max && e == cudaSuccess; lanes <<= 1) {
       if (bps == occ && lanes == lanes_max) continue;
       double ms;
@@ -1147,7 +1162,7 @@ extern "C" cmn_status cmn_solver_create(const cmn_problem* p, const cmn_solve_op
     const int occ_s =
         std::max(1, sample_kernel_occupancy(sample_smem_bytes(n, p->prog.n_slots, threads, lg_min), threads));
     const int tp = fp32 ? 1 : 0;
-    if (o.autotune && p->tuned_bps[tp] == 0) {
+    if (o.autotune && p->tuned_bps[tp] == 0 && !shape_fixed(p, fp32)) {
       cmn_tune_result tr{};
       cmn_status ts =
           cmn_autotune(const_cast<cmn_problem*>(p), tp, std::min<uint64_t>(maxc, 1ull << 18), &tr);

@@ -315,7 +315,7 @@ bool chain_pays(const EvalArgs& a, int mode)
     if (both) return (len > 64 && boxes <= 10240) || (len >= 5 && boxes >= 98304);
     return len >= 12 || (len > 3 && boxes >= 65536);
   }
-  if (mode == 4)  // 8 of n = 4's 30 instructions a child: 65,536 regions 74 and 66 us, 16,384 50 and 65
+  if (mode == 4)  // n = 4, 30 instructions: 16,384 regions 50 and 65 us, 65,536 74 and 66
     return len >= 20 && (len >= 72 || saved * boxes >= 3200000) && (len >= 40 || 2 * t.constraint_terms >= len);
   if (region) return role_fits(a) || saved * boxes >= 1600000;
   if (both)

@@ -111,8 +111,9 @@ class DeviceProblem:
         return buf
 
     def autotune(self, precision: int = 0, n_boxes: int = 1 << 16) -> dict:
-        """cmn_autotune: times the evaluator's launch shapes on this problem
-        and records the fastest for solvers created with autotune=1."""
+        """cmn_autotune: times the interpreter's launch shapes on this problem
+        and records the fastest for solvers created with autotune=1.  A
+        program of sum chains has one: its kernels size their own grids."""
         r = A.TuneResult()
         check(lib().cmn_autotune(self.handle, precision, n_boxes, C.byref(r)))
         return {f: getattr(r, f) for f, _ in A.TuneResult._fields_ if f != "reserved"}

@@ -356,8 +356,9 @@ typedef struct cmn_solve_options {
   uint64_t max_cycle_size;    /* slot cap (SearchCalibration) 0 = 64 */
   uint64_t enumerate_cap;     /* SearchCalibration::enumerate_cap */
   int32_t has_known_primal;   /* seeds GUB (known_primal_bound) */
-  int32_t autotune;           /* 1: the evaluator's launch shape from
-                                 cmn_autotune (run on first use) */
+  int32_t autotune;           /* 1: the interpreter's launch shape from
+                                 cmn_autotune (run on first use; not for
+                                 a program of sum chains) */
   double known_primal_bound;
   uint64_t time_limit_ms;     /* 0 = none */
 } cmn_solve_options;
@@ -501,7 +502,7 @@ cmn_status cmn_fp64_emu_check_host(uint64_t n, uint64_t seed, int32_t family, ui
  * or a sum cancels exactly (those take the FP64 instruction). */
 cmn_status cmn_fp64_emu_op_host(int32_t op, double a, double b, double* out, int32_t* handled);
 
-/* Timed autotuning of the fused evaluator's launch shape for one problem.
+/* Timed autotuning of the interpreter's launch shape for one problem.
  * No counterpart in the reference (its graph backend launches one kernel
  * per DAG node with a fixed shape).  Candidates: blocks per SM from 1 to
  * the kernel's residency, and caps on the lanes that share one box (boxes
@@ -510,7 +511,11 @@ cmn_status cmn_fp64_emu_op_host(int32_t op, double a, double b, double* out, int
  * inside the root box, best of three launches.  The fastest is recorded on
  * the problem (for `precision` 0, FP64, or 1, FP32) and used by every
  * solver created for it with cmn_solve_options.autotune = 1; results never
- * depend on the choice.  Synchronous; allocates its test boxes. */
+ * depend on the choice.  A program that is a set of sum chains (any
+ * quadratic model; in FP32, one of <= constraints) is bounded by kernels
+ * that size their own grids: its evaluation is timed once, as one
+ * candidate, and a solver skips the search.  Synchronous; allocates its
+ * test boxes. */
 typedef struct cmn_tune_result {
   int32_t blocks_per_sm;   /* chosen */
   int32_t lanes_cap;       /* chosen: most lanes per box */

@@ -282,3 +282,38 @@ def test_autotuned_launch_shape_changes_no_result(precision):
     assert a["lower_bound"] == b["lower_bound"] and a["upper_bound"] == b["upper_bound"]
     assert a["counters"] == b["counters"]
     assert bits_equal(fa[1], fb[1]) and bits_equal(fa[0], fb[0])
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_autotune_times_what_evaluation_runs(precision):
+    # a quadratic model's bounds run kernels with grids of their own: one
+    # candidate, at the time of the evaluation itself; a model with shared
+    # slots has the interpreter's shapes
+    import torch
+    from cuminlp_gb300.problem import Problem, sqr
+    from cuminlp_gb300.solver import eval_boxes_device
+    p = G.miqcqp_n32(1)
+    dp = DeviceProblem(p)
+    n = 1 << 15
+    t = dp.autotune(precision, n)
+    assert t["candidates"] == 1 and t["ms_best"] == t["ms_default"]
+    box = p.root_box().reshape(-1, 2)
+    lo = torch.tensor(box[:, :1]).repeat(1, n).contiguous().cuda()
+    hi = torch.tensor(box[:, 1:]).repeat(1, n).contiguous().cuda()
+    lb = torch.empty(n, dtype=torch.float64, device="cuda")
+    fe = torch.empty(n, dtype=torch.uint8, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    best = float("inf")
+    for _ in range(6):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        eval_boxes_device(dp, lo.data_ptr(), hi.data_ptr(), n, n, lb.data_ptr(), None, fe.data_ptr(), precision, s)
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b))
+    assert best / 2 < t["ms_best"] < best * 2
+    q = Problem()
+    x = [q.var(-2.0, 3.0) for _ in range(4)]
+    r = sqr(x[0]) + 1.0
+    q.set_objective(sqr(x[1] - x[2]) / r + r * x[3])
+    assert DeviceProblem(q).autotune(precision, 1 << 12)["candidates"] > 1
