@@ -568,7 +568,7 @@ extern "C" cmn_status cmn_batch_frontier(cmn_batch* s, uint64_t slot, double* bo
   std::vector<uint32_t> idx(m);
   BCK(cudaMemcpyAsync(idx.data(), s->b.idx + (size_t)slot * c.P, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
   BCK(cudaStreamSynchronize(s->stream));
-  const uint64_t top = m == 0 ? 0 : *std::max_element(idx.begin(), idx.end()) + 1;
+  const uint64_t top = *std::max_element(idx.begin(), idx.end()) + 1;
   if (boxes) {
     const size_t base = (size_t)slot * c.P * c.n_max;
     std::vector<double> lo(top * c.n_max), hi(top * c.n_max);

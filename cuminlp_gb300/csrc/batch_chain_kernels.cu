@@ -270,30 +270,19 @@ bool batch_tile_takes(const BatchCfg& c, const ChainTab& t)
   return c.precision == CMN_PRECISION_FP32_LAZY ? t.term32 != nullptr && t.term_pt != nullptr : t.points != 0;
 }
 
-template <typename K>
-static int resident(K kernel, int threads, size_t smem)
-{
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess) {
-    (void)cudaGetLastError();
-    n = 1;
-  }
-  return sm_count() * std::max(1, n);
-}
-
 BatchTileGrids batch_tile_grids(const BatchCfg& c)
 {
   BatchTileGrids g;
   if (!c.tiles) return g;
   if (c.precision == CMN_PRECISION_FP32_LAZY) {
-    g.constraints = resident(batch_constraints_kernel<0, true>, kTileWarps * 32, constraints_smem(c));
-    g.lazy = resident(batch_lazy_kernel, kLazyThreads, lazy_bytes(c));
-    g.points = resident(batch_points_kernel<true>, kPointThreads, points_smem(c, true));
-    g.picks = resident(batch_picks_kernel, kPointThreads, picks_smem(c));
+    g.constraints = (int)resident_blocks(~0ULL, batch_constraints_kernel<0, true>, kTileWarps * 32, constraints_smem(c));
+    g.lazy = (int)resident_blocks(~0ULL, batch_lazy_kernel, kLazyThreads, lazy_bytes(c));
+    g.points = (int)resident_blocks(~0ULL, batch_points_kernel<true>, kPointThreads, points_smem(c, true));
+    g.picks = (int)resident_blocks(~0ULL, batch_picks_kernel, kPointThreads, picks_smem(c));
   } else {
-    g.children = resident(batch_constraints_kernel<1, false>, kTileWarps * 32, constraints_smem(c));
-    g.objective = resident(batch_siblings_kernel, kObjThreads, siblings_smem(c));
-    g.points = resident(batch_points_kernel<false>, kPointThreads, points_smem(c, false));
+    g.children = (int)resident_blocks(~0ULL, batch_constraints_kernel<1, false>, kTileWarps * 32, constraints_smem(c));
+    g.objective = (int)resident_blocks(~0ULL, batch_siblings_kernel, kObjThreads, siblings_smem(c));
+    g.points = (int)resident_blocks(~0ULL, batch_points_kernel<false>, kPointThreads, points_smem(c, false));
   }
   return g;
 }
@@ -335,24 +324,15 @@ cudaError_t batch_tile_points(const BatchCfg& c, const BatchBufs& b, const Batch
   return cudaGetLastError();
 }
 
-template <typename K>
-static cudaError_t allow(K kernel, int max_smem)
-{
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
-}
-
 cudaError_t set_batch_tile_attributes(int max_smem)
 {
-  cudaError_t e = allow(batch_constraints_kernel<0, true>, max_smem);
-  if (e == cudaSuccess) e = allow(batch_constraints_kernel<1, false>, max_smem);
-  if (e == cudaSuccess) e = allow(batch_siblings_kernel, max_smem);
-  if (e == cudaSuccess) e = allow(batch_lazy_kernel, max_smem);
-  if (e == cudaSuccess) e = allow(batch_points_kernel<true>, max_smem);
-  if (e == cudaSuccess) e = allow(batch_points_kernel<false>, max_smem);
-  if (e == cudaSuccess) e = allow(batch_picks_kernel, max_smem);
+  cudaError_t e = allow_dynamic_smem(batch_constraints_kernel<0, true>, max_smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(batch_constraints_kernel<1, false>, max_smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(batch_siblings_kernel, max_smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(batch_lazy_kernel, max_smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(batch_points_kernel<true>, max_smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(batch_points_kernel<false>, max_smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(batch_picks_kernel, max_smem);
   return e;
 }
 

@@ -124,14 +124,6 @@ __global__ void __launch_bounds__(kLazyThreads, 2) lazy_children_kernel(const Ev
 }
 
 // ---- launchers ----
-static uint64_t resident(uint64_t blocks, const void* kernel, int threads, size_t smem)
-{
-  int occ = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) occ = 1;
-  const uint64_t room = (uint64_t)sm_count() * (uint64_t)occ;
-  return blocks < 1 ? 1 : blocks < room ? blocks : room;
-}
-
 static size_t eval32_smem(int n) { return (size_t)(n + 1) * 32 * 8; }
 
 bool chain32_fits(const EvalArgs& a, int mode)
@@ -159,7 +151,7 @@ static cudaError_t launch_chain32_t(const EvalArgs& a, cudaStream_t s)
 {
   const size_t smem = eval32_smem(a.n_vars);
   const int threads = 32 * a.chain.warps32;
-  const uint64_t grid = resident((a.max_boxes + 31) >> 5, (const void*)chain32_eval_kernel<kMode>, threads, smem);
+  const uint64_t grid = resident_blocks((a.max_boxes + 31) >> 5, chain32_eval_kernel<kMode>, threads, smem);
   chain32_eval_kernel<kMode><<<(unsigned)grid, threads, smem, s>>>(a);
   return cudaGetLastError();
 }
@@ -191,25 +183,16 @@ cudaError_t launch_lazy_children(const EvalArgs& a, uint64_t max_parents, cudaSt
 {
   const LazyShape h = lazy_shape(a.n_vars, a.max_slots, a.log2C, a.chain.n_seg);
   const size_t smem = lazy_smem(a.n_vars, a.max_slots, h, 1 << a.log2C);
-  const uint64_t grid = resident((max_parents + 31) >> 5, (const void*)lazy_children_kernel, kLazyThreads, smem);
+  const uint64_t grid = resident_blocks((max_parents + 31) >> 5, lazy_children_kernel, kLazyThreads, smem);
   lazy_children_kernel<<<(unsigned)grid, kLazyThreads, smem, s>>>(a, h);
   return cudaGetLastError();
 }
 
-template <typename K>
-static cudaError_t allow(K kernel, int max_smem)
-{
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
-}
-
 cudaError_t set_chain32_kernel_attributes(int max_smem)
 {
-  cudaError_t e = allow(chain32_eval_kernel<0>, max_smem);
-  if (e == cudaSuccess) e = allow(chain32_eval_kernel<2>, max_smem);
-  if (e == cudaSuccess) e = allow(lazy_children_kernel, max_smem);
+  cudaError_t e = allow_dynamic_smem(chain32_eval_kernel<0>, max_smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(chain32_eval_kernel<2>, max_smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(lazy_children_kernel, max_smem);
   return e;
 }
 

@@ -162,14 +162,6 @@ __global__ void __launch_bounds__(kObjThreads, 5) chain_role_kernel(const EvalAr
     constraints_tile<0, false>(ca, smem_raw, sh, log_boxes, tile, total);
 }
 
-static uint64_t resident(uint64_t blocks, const void* kernel, int threads, size_t smem)
-{
-  int occ = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) occ = 1;
-  const uint64_t room = (uint64_t)sm_count() * (uint64_t)occ;
-  return blocks < 1 ? 1 : blocks < room ? blocks : room;
-}
-
 static size_t objective_smem(const EvalArgs& a)
 {
   return (size_t)(a.pinfo != nullptr ? a.max_slots : 0) * 20 * kObjThreads;
@@ -187,7 +179,7 @@ static cudaError_t launch_chain_t(const EvalArgs& a, cudaStream_t s)
     auto kernel = chain_constraints_kernel<kMode, kFused>;
     const int threads = 32 * (chains < kTileWarps ? chains : kTileWarps);
     const size_t smem = tile_smem_bytes(a.n_vars, ms, 1 << lb);
-    const uint64_t grid = resident((a.max_boxes + (1ull << lb) - 1) >> lb, (const void*)kernel, threads, smem);
+    const uint64_t grid = resident_blocks((a.max_boxes + (1ull << lb) - 1) >> lb, kernel, threads, smem);
     kernel<<<(unsigned)grid, threads, smem, s>>>(a, lb);
   }
   if constexpr (!kFused && kMode != 3) {
@@ -200,7 +192,7 @@ static cudaError_t launch_chain_t(const EvalArgs& a, cudaStream_t s)
       auto siblings = chain_siblings_kernel<kMode, kHi>;
       // a block a tile while they are resident at once, else a warp a tile
       const uint64_t tiles = (a.max_boxes + 31) / 32, most = 512 * 32 / kObjThreads;
-      uint64_t grid = resident(std::max(tiles, most), (const void*)siblings, kObjThreads, fsmem);
+      uint64_t grid = resident_blocks(std::max(tiles, most), siblings, kObjThreads, fsmem);
       if (grid < tiles) grid = std::min(grid, std::max((tiles + 3) / 4, most));
       siblings<<<(unsigned)grid, kObjThreads, fsmem, s>>>(a, chains > 0 ? 1 : 0, 32 >> lc, (int)few);
       return cudaGetLastError();
@@ -215,7 +207,7 @@ static cudaError_t launch_chain_t(const EvalArgs& a, cudaStream_t s)
   if constexpr (kHi && kMode == 0)
     if (a.max_boxes <= 16384 && a.prog_len > 64) kernel = chain_objective_kernel<kMode, kFused, kHi, true>;
   const size_t smem = objective_smem(a);
-  const uint64_t grid = resident((a.max_boxes * 32 + kObjThreads - 1) / kObjThreads, (const void*)kernel, kObjThreads, smem);
+  const uint64_t grid = resident_blocks((a.max_boxes * 32 + kObjThreads - 1) / kObjThreads, kernel, kObjThreads, smem);
   kernel<<<(unsigned)grid, kObjThreads, smem, s>>>(a, chains > 0 ? 1 : 0);
   return cudaGetLastError();
 }
@@ -334,29 +326,20 @@ cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s)
   return launch_chain_t<3, false, false>(a, s);
 }
 
-template <typename K>
-static cudaError_t allow(K kernel, int max_smem)
-{
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
-}
-
 template <int kMode, bool kFused, bool kHi>
 static cudaError_t allow_both(int max_smem)
 {
-  cudaError_t e = allow(chain_constraints_kernel<kMode, kFused>, max_smem);
+  cudaError_t e = allow_dynamic_smem(chain_constraints_kernel<kMode, kFused>, max_smem);
   if constexpr (!kFused && kMode != 3)
-    if (e == cudaSuccess) e = allow(chain_siblings_kernel<kMode, kHi>, max_smem);
+    if (e == cudaSuccess) e = allow_dynamic_smem(chain_siblings_kernel<kMode, kHi>, max_smem);
   if constexpr (kHi && kMode == 0)
-    if (e == cudaSuccess) e = allow(chain_objective_kernel<kMode, kFused, kHi, true>, max_smem);
-  return e == cudaSuccess ? allow(chain_objective_kernel<kMode, kFused, kHi>, max_smem) : e;
+    if (e == cudaSuccess) e = allow_dynamic_smem(chain_objective_kernel<kMode, kFused, kHi, true>, max_smem);
+  return e == cudaSuccess ? allow_dynamic_smem(chain_objective_kernel<kMode, kFused, kHi>, max_smem) : e;
 }
 
 cudaError_t set_chain_kernel_attributes(int max_smem)
 {
-  cudaError_t e = allow(chain_role_kernel, max_smem);
+  cudaError_t e = allow_dynamic_smem(chain_role_kernel, max_smem);
   if (e == cudaSuccess) e = allow_both<0, false, true>(max_smem);
   if (e == cudaSuccess) e = allow_both<0, false, false>(max_smem);
   if (e == cudaSuccess) e = allow_both<0, true, false>(max_smem);

@@ -129,20 +129,11 @@ cudaError_t launch_chain_screen(const SampleArgs& a, uint64_t max_children, cuda
   return cudaGetLastError();
 }
 
-template <typename K>
-static cudaError_t allow(K kernel, int max_smem)
-{
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
-}
-
 cudaError_t set_chain_points_attributes(int max_smem)
 {
-  cudaError_t e = allow(chain_sample_kernel<false>, max_smem);
-  if (e == cudaSuccess) e = allow(chain_sample_kernel<true>, max_smem);
-  return e == cudaSuccess ? allow(chain_screen_kernel, max_smem) : e;
+  cudaError_t e = allow_dynamic_smem(chain_sample_kernel<false>, max_smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(chain_sample_kernel<true>, max_smem);
+  return e == cudaSuccess ? allow_dynamic_smem(chain_screen_kernel, max_smem) : e;
 }
 
 }  // namespace cmn

@@ -186,7 +186,7 @@ __device__ void constraints_tile(const EvalArgs& a, unsigned char* smem, TileSha
   __syncthreads();
   if (alive != 0u) {
     const bool in_range = !((sh.bad >> box) & 1u);
-    // (2) the chains, drawn from a ticket until every box is excluded
+    // (2) the chains, drawn from a ticket
     for (;;) {
       int q = 0;
       if (lane == 0) q = atomicAdd(&sh.next, 1);

@@ -995,20 +995,6 @@ int sample_lg_min(int n_vars, int n_slots, bool has_sched, int threads)
   return lg;
 }
 
-// Kernel attributes are set once per device, before any launch, so that
-// launches stay legal inside stream capture.
-// The dynamic allowance is the opt-in maximum less the kernel's own static
-// shared memory (the reduction scratch of the sampler).
-template <typename K>
-static cudaError_t allow_dynamic_smem(K kernel, int max_smem)
-{
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              max_smem - (int)fa.sharedSizeBytes);
-}
-
 cudaError_t set_eval_kernel_attributes(int max_smem)
 {
   cudaError_t e = allow_dynamic_smem(eval_children_kernel<double, 0>, max_smem);

@@ -79,9 +79,33 @@ cudaError_t launch_candidate(const Cand* block_best, int n, Cand* out, const Wit
 
 // Largest dynamic shared memory a block may use on this device.
 int max_dynamic_smem();
+
+// Kernel attributes are set once per device, before any launch, so that
+// launches stay legal inside stream capture.  The dynamic allowance is the
+// opt-in maximum less the kernel's own static shared memory.
+template <typename K>
+cudaError_t allow_dynamic_smem(K kernel, int max_smem)
+{
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
+}
+
 // Resident blocks per SM of the sampler at this shared-memory size.
 int sample_kernel_occupancy(size_t smem, int threads);
 int sample_screen_occupancy(size_t smem, int threads);
 int sm_count();
+
+// Blocks of a launch whose kernel strides over `blocks` blocks' work: as many
+// as are resident at once, no more than that.
+template <typename K>
+uint64_t resident_blocks(uint64_t blocks, K kernel, int threads, size_t smem)
+{
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess) (void)cudaGetLastError();
+  const uint64_t room = (uint64_t)sm_count() * (uint64_t)(occ < 1 ? 1 : occ);
+  return blocks < 1 ? 1 : blocks < room ? blocks : room;
+}
 
 }  // namespace cmn

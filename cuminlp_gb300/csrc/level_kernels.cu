@@ -106,19 +106,10 @@ cudaError_t launch_level(const EvalArgs& a, bool fp32, cudaStream_t s)
   return cudaGetLastError();
 }
 
-template <typename K>
-static cudaError_t allow(K kernel, int max_smem)
-{
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes);
-}
-
 cudaError_t set_level_kernel_attributes(int max_smem)
 {
-  cudaError_t e = allow(level_eval_kernel<double>, max_smem);
-  return e == cudaSuccess ? allow(level_eval_kernel<float>, max_smem) : e;
+  cudaError_t e = allow_dynamic_smem(level_eval_kernel<double>, max_smem);
+  return e == cudaSuccess ? allow_dynamic_smem(level_eval_kernel<float>, max_smem) : e;
 }
 
 }  // namespace cmn

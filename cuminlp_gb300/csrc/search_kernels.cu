@@ -561,12 +561,10 @@ __global__ void __launch_bounds__(1024) scan_kernel(const uint32_t* __restrict__
 // ---- predicates / operations -----------------------------------------
 struct KeptChild {
   SolverBufs b;
-  __device__ uint64_t size() const { return b.dev->n_children; }
   __device__ bool operator()(uint64_t g) const
   {
     return b.cstate[g] == kChildEligible && !bits_lt(dbits(b.dev->gub), dbits(b.clb[g]));
   }
-  __device__ bool skip() const { return b.dev->done != 0; }
 };
 
 struct ScreenedChild {
