@@ -199,3 +199,26 @@ def test_batch_slot_errors():
     b.close()
     with pytest.raises(CmnError):
         Batch(1, 4, bisection_budget=4, batch_parents=512, frontier_cap=1024)
+
+
+def fallback_problems():
+    """Sum chains the tiles leave in part or whole to their general paths."""
+    from tests.test_gpu_chains import chain_problem, equality_problem, long_problem, mixed_problem, outside_problem
+    return {"mixed": mixed_problem(), "equality": equality_problem(), "outside": outside_problem(),
+            "readers": long_problem(readers=True), "long": long_problem(), "short": chain_problem(2, 2, 1),
+            "all_equal": chain_problem(6, 12, 4, 4), "shared": chain_problem(5, 12, 2, 0, True),
+            "free": chain_problem(7, 20, 0)}
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "lazy"])
+@pytest.mark.parametrize("bits,parents", [(1, 5), (3, 40), (5, 33)])
+def test_batch_fallbacks_match_single_instance_solver(precision, bits, parents):
+    shared = dict(bisection_budget=bits, batch_parents=parents, frontier_cap=700, sample_points=2, precision=precision)
+    named = fallback_problems()
+    got = run_batch(named, shared, dict(batch_iter_limit=7))
+    for k, p in named.items():
+        s = Solver(DeviceProblem(p), batch_iter_limit=7, **shared)
+        s.step(0)
+        same_outcome(got[k][0], s.outcome(), k)
+        same_frontier(got[k][1], s.frontier(), k)
+        s.close()
