@@ -684,7 +684,7 @@ class Compiler {
   {
     const size_t n = p_.var_lb.size(), S = out_.chain_seg.size();
     if (n + 1 > 0xffff) return;
-    std::vector<std::vector<ChainTerm32>> by_var(n * S);
+    std::vector<std::pair<size_t, ChainTerm32>> by_var;  // (variable, chain) of each term read, in program order
     std::vector<ChainTerm32> all;
     for (size_t q = 0; q < S; ++q) {
       ChainSeg& cs = out_.chain_seg[q];
@@ -717,20 +717,22 @@ class Compiler {
         else if (!has_c) t.flags |= kT32Raw;
         t.ab = a | (b << 16);
         all.push_back(t);
-        by_var[a * S + q].push_back(t);
+        by_var.push_back({a * S + q, t});
         if (b != a && b < n) {
           t.ab = b | (a << 16);
-          by_var[b * S + q].push_back(t);
+          by_var.push_back({b * S + q, t});
         }
       }
       cs.t32_end = (int32_t)all.size();
     }
     out_.chain_term32 = all;
-    out_.chain_var_off.push_back(0);
-    for (const auto& l : by_var) {
-      out_.chain_var32.insert(out_.chain_var32.end(), l.begin(), l.end());
-      out_.chain_var_off.push_back((int32_t)out_.chain_var32.size());
-    }
+    std::vector<int32_t>& off = out_.chain_var_off;  // by counting: a list per pair took 13 % of 1,500 x 1,500
+    off.assign(n * S + 1, 0);
+    for (const auto& e : by_var) ++off[e.first + 1];
+    for (size_t i = 0; i < n * S; ++i) off[i + 1] += off[i];
+    std::vector<int32_t> at(off.begin(), off.end() - 1);
+    out_.chain_var32.resize(by_var.size());
+    for (const auto& e : by_var) out_.chain_var32[at[e.first]++] = e.second;
   }
 
   // The FP32 filter's terms of a chain; leaves eps 0 (no filter) when a
