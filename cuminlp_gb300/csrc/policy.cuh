@@ -29,7 +29,7 @@ namespace cmn {
 #define CMN_POLICY_D2U(x) ((unsigned long long)(x))
 #endif
 
-// Most variables whose policy scratch (88 bytes each) a device thread keeps in
+// Most variables whose policy scratch (80 bytes each) a device thread keeps in
 // local memory.
 constexpr int kPolicyLocal = 64;
 
