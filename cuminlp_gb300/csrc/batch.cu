@@ -88,6 +88,8 @@ struct cmn_batch {
   std::vector<Clock::time_point> t_add;
   std::vector<double> elapsed_ms;  // add -> first step that saw it stopped
   void* slab = nullptr;  // every device array
+  unsigned char* h_front = nullptr;  // pinned: where a frontier is gathered, as large as the largest so far
+  size_t front_bytes = 0;
   uint64_t alloc_bytes = 0;
   bool fresh = false;  // h_st matches the device: nothing enqueued since pull()
   int eval_grid = 1;
@@ -103,6 +105,7 @@ struct cmn_batch {
     if (graph) cudaGraphDestroy(graph);
     if (slab) cudaFree(slab);
     if (h_st) cudaFreeHost(h_st);
+    if (h_front) cudaFreeHost(h_front);
     if (stream) cudaStreamDestroy(stream);
     if (cur != device) cudaSetDevice(cur);
   }
@@ -564,34 +567,25 @@ extern "C" cmn_status cmn_batch_frontier(cmn_batch* s, uint64_t slot, double* bo
   if (m == 0) return CMN_OK;
   const BatchCfg& c = s->cfg;
   const int n = s->h_desc[slot].n_vars;
-  // the pool's store slots, then the boxes and depths they name
-  std::vector<uint32_t> idx(m);
-  BCK(cudaMemcpyAsync(idx.data(), s->b.idx + (size_t)slot * c.P, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
-  BCK(cudaStreamSynchronize(s->stream));
-  const uint64_t top = *std::max_element(idx.begin(), idx.end()) + 1;
-  if (boxes) {
-    const size_t base = (size_t)slot * c.P * c.n_max;
-    std::vector<double> lo(top * c.n_max), hi(top * c.n_max);
-    BCK(cudaMemcpyAsync(lo.data(), s->b.lo + base, lo.size() * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-    BCK(cudaMemcpyAsync(hi.data(), s->b.hi + base, hi.size() * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-    BCK(cudaStreamSynchronize(s->stream));
-    for (uint64_t i = 0; i < m; ++i)
-      for (int v = 0; v < n; ++v) {
-        boxes[2 * (i * n + v)] = lo[(size_t)idx[i] * c.n_max + v];
-        boxes[2 * (i * n + v) + 1] = hi[(size_t)idx[i] * c.n_max + v];
-      }
+  // gathered by a kernel straight into pinned memory, then copied out
+  const size_t box_bytes = boxes ? m * 2 * (size_t)n * sizeof(double) : 0;
+  const size_t bytes = box_bytes + m * (sizeof(double) + sizeof(uint32_t));
+  if (s->front_bytes < bytes) {
+    const size_t room_bytes = std::max(bytes, 2 * s->front_bytes);
+    if (s->h_front) cudaFreeHost(s->h_front);
+    s->h_front = nullptr;
+    s->front_bytes = 0;
+    BCK(cudaMallocHost(reinterpret_cast<void**>(&s->h_front), room_bytes));
+    s->front_bytes = room_bytes;
   }
-  if (lower_bounds)
-    BCK(cudaMemcpyAsync(lower_bounds, s->b.lb + (size_t)slot * c.P, m * sizeof(double), cudaMemcpyDeviceToHost,
-                        s->stream));
-  if (depths) {
-    std::vector<uint32_t> dep(top);
-    BCK(cudaMemcpyAsync(dep.data(), s->b.depth + (size_t)slot * c.P, top * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                        s->stream));
-    BCK(cudaStreamSynchronize(s->stream));
-    for (uint64_t i = 0; i < m; ++i) depths[i] = dep[idx[i]];
-  }
+  double* fb = reinterpret_cast<double*>(s->h_front);
+  double* fl = reinterpret_cast<double*>(s->h_front + box_bytes);
+  uint32_t* fd = reinterpret_cast<uint32_t*>(fl + m);
+  BCK(batch_frontier(c, s->b, slot, m, boxes ? fb : nullptr, fl, fd, s->stream));
   BCK(cudaStreamSynchronize(s->stream));
+  if (boxes) std::memcpy(boxes, fb, box_bytes);
+  if (lower_bounds) std::memcpy(lower_bounds, fl, m * sizeof(double));
+  if (depths) std::memcpy(depths, fd, m * sizeof(uint32_t));
   return CMN_OK;
 }
 

@@ -217,6 +217,10 @@ BatchGrids batch_grids(const BatchCfg& cfg, int eval_grid);
 // The kernels write BatchBufs::stamps (ns) at the phase boundaries: start,
 // after select + branch, after bound, after sample, after finish.
 cudaError_t batch_iteration(const BatchCfg& cfg, const BatchBufs& b, const BatchGrids& grids, cudaStream_t s);
+// The first m pool entries of `slot` in position order: boxes as (lower,
+// upper) pairs (or null), lower bounds and depths.
+cudaError_t batch_frontier(const BatchCfg& cfg, const BatchBufs& b, uint64_t slot, uint64_t m, double* boxes,
+                           double* lower_bounds, uint32_t* depths, cudaStream_t s);
 size_t batch_eval_smem(const BatchCfg& cfg, bool fp32);
 size_t batch_sample_smem(const BatchCfg& cfg);
 // resident blocks per SM of the bound (fp32: screen) and sample kernels

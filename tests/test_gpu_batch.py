@@ -222,3 +222,19 @@ def test_batch_fallbacks_match_single_instance_solver(precision, bits, parents):
         same_outcome(got[k][0], s.outcome(), k)
         same_frontier(got[k][1], s.frontier(), k)
         s.close()
+
+
+@pytest.mark.parametrize("room", [1, 7, 8, 33, 200, 1 << 12])
+def test_part_of_a_frontier(room):
+    # the first entries of the whole, of each instance of the batch
+    named = {k: mixed_problems()[k] for k in ("contract", "qcqp_n4", "uneven_1", "uneven_4")}
+    n_max = max(p.n_vars for p in named.values())
+    dps = {k: DeviceProblem(p) for k, p in named.items()}
+    b = Batch(len(named), n_max, max(dp.info()["program_slots"] for dp in dps.values()), **SHARED)
+    slots = {k: b.add(dp, batch_iter_limit=9) for k, dp in dps.items()}
+    assert b.step(0) == 0
+    for k, s in slots.items():
+        whole, part = b.frontier(s), b.frontier(s, room)
+        assert len(part[1]) == min(room, len(whole[1]))
+        same_frontier(part, tuple(a[:room] for a in whole), k)
+    b.close()
