@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 #include <chrono>
 #include <cmath>
@@ -62,20 +63,29 @@ std::mutex g_attr_mu;
 // ----------------------------------------------------------------------
 namespace cmn {
 
-int sm_count()
+// An attribute of the current device, asked for once per device: choosing a
+// path reads some several times, of a call that takes 10 us in all.
+static int device_attribute(cudaDeviceAttr attr, std::atomic<int> (&known)[32])
 {
   int dev = 0, n = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  if (dev < 32 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, attr, dev) != cudaSuccess) return 0;
+  if (dev < 32) known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+int sm_count()
+{
+  static std::atomic<int> known[32];
+  const int n = device_attribute(cudaDevAttrMultiProcessorCount, known);
   return n > 0 ? n : 1;
 }
 
 int max_dynamic_smem()
 {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return n;
+  static std::atomic<int> known[32];
+  return device_attribute(cudaDevAttrMaxSharedMemoryPerBlockOptin, known);
 }
 
 }  // namespace cmn
