@@ -1,5 +1,6 @@
 // chain32_kernels.cu -- the FP32 passes over programs of sum chains for one
 // instance (chain32_tiles.cuh).
+#include <algorithm>
 #include <cfloat>
 #include <cstdint>
 
@@ -133,17 +134,22 @@ bool chain32_fits(const EvalArgs& a, int mode)
 }
 
 // Whether the tiles beat the interpreter over boxes (the screen always takes
-// them).  Staging a box costs about as much as a term a variable, so a chain
-// that reads each variable once or so does not pay where a tile is large: n =
-// 64, 65 instructions, 65,536 boxes 40 us by the interpreter and 67 in tiles; n
-// = 32, 33 instructions, 100,000 boxes 37 and 30.  Programs of less than 12
-// instructions take launch time either way (11 and 12 us) up to some 10^5
-// boxes (n = 2, 6 instructions, 524,288 boxes 26 and 22).
+// them).  Up to one wave they do.  Beyond, a tile waits for its variables with
+// the few warps that its shared memory leaves an SM, so the terms have to
+// outweigh that (a product counts 2.4: the interpreter takes that much longer
+// for it): a linear objective, n = 64, 12 warps, 65,536 boxes 40 us by the
+// interpreter and 67 in tiles; n = 150, 301 terms, 5 warps, 200,000 boxes 985
+// and 1,231; n = 300 with two linear constraints, 6 warps, 20,000 boxes 201 and
+// 283; n = 100, 201 terms, 8 warps, 200,000 boxes 608 and 565.  Programs of
+// less than 12 instructions take launch time either way (11 and 12 us) up to
+// some 10^5 boxes (n = 2, 6 instructions, 524,288 boxes 26 and 22).
 bool chain32_pays(const EvalArgs& a, int mode)
 {
   if (mode != 0) return true;
-  const int64_t len = a.prog_len, n = a.n_vars;
-  return (len >= 12 && (n <= 32 || len >= 2 * n)) || (len >= 6 && a.max_boxes >= 131072 && 5 * len >= 6 * n);
+  const int64_t len = a.prog_len, n = a.n_vars, boxes = (int64_t)a.max_boxes;
+  if (len < 12) return len >= 6 && boxes >= 131072 && 5 * len >= 6 * n;
+  const int64_t tiles = std::min<int64_t>(32, max_dynamic_smem() / (int64_t)(eval32_smem(a.n_vars) + 1024));
+  return boxes <= 32 * tiles * sm_count() || (10 * len + 14ll * a.chain.products) * tiles * a.chain.warps32 >= 250 * n;
 }
 
 template <int kMode>

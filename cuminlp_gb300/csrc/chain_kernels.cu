@@ -256,12 +256,14 @@ bool chain_fits(const EvalArgs& a)
 
 // Whether the passes here beat the interpreter's one launch.  They save three
 // quarters of the <= chains' time, for a second launch and the staging of every
-// box, worth about 3/4 of a term a variable and 3/2 a chain; `saved` is what is
-// left, in quarters of a term a box.  Boxes, both bounds, interpreter against
+// box, worth about 3/4 of a term a variable (more where many boxes meet tiles so
+// large that fewer than 16 warps of them fit an SM) and 3/2 a chain; `saved` is
+// what is left, in quarters of a term a box.  Boxes, both bounds, interpreter against
 // here: n = 4, one constraint (30 instructions), 20,000 boxes 26 and 39 us,
 // 65,536 boxes 49 and 47, 524,288 boxes 220 and 148; n = 8, three constraints
 // (145), 2,000 boxes 56 and 46, 131,072 boxes 359 and 126; n = 2, one
-// constraint (6), 524,288 boxes 32 and 44.  Few boxes of a long program: here
+// constraint (6), 524,288 boxes 32 and 44; n = 200, one linear constraint, 4 warps,
+// 20,000 boxes 177 and 335.  Few boxes of a long program: here
 // lane groups form the objective faster (64 terms, 300 boxes 48 and 19 us).
 // Chains with other readers keep the interpreter's arithmetic here, a warp
 // each, so they need many boxes, and <= chains beside them to pay: sixteen ==
@@ -295,7 +297,10 @@ bool chain_pays(const EvalArgs& a, int mode)
 {
   const ChainTab& t = a.chain;
   const int64_t boxes = (int64_t)a.max_boxes, len = a.prog_len;
-  const int64_t saved = 4ll * t.constraint_terms - 3ll * a.n_vars - 6ll * t.constraints;
+  const int64_t tiles = max_dynamic_smem() / (int64_t)(tile_smem_bytes(a.n_vars, a.pinfo ? a.max_slots : 0, 32) + 1024);
+  const int64_t warps = tiles * std::max(1, std::min(t.constraints + t.general, kTileWarps));
+  const bool waits = boxes > 32 * tiles * sm_count() && warps < 16;
+  const int64_t saved = 4ll * t.constraint_terms - (waits ? 48ll * a.n_vars / warps : 3ll * a.n_vars) - 6ll * t.constraints;
   if (t.general > 0) return general_pays(a, mode, boxes, saved);
   if (mode == 1 || mode == 3 || mode == 6) return true;  // in the solver no form or size lost
   const bool region = a.pinfo != nullptr, both = mode == 4 || a.out_ub != nullptr;
@@ -308,12 +313,12 @@ bool chain_pays(const EvalArgs& a, int mode)
     return len >= 12 || (len > 3 && boxes >= 65536);
   }
   if (mode == 4)  // n = 4, 30 instructions: 16,384 regions 50 and 65 us, 65,536 74 and 66
-    return len >= 20 && (len >= 72 || saved * boxes >= 3200000) && (len >= 40 || 2 * t.constraint_terms >= len);
+    return len >= 20 && ((len >= 72 && !waits) || saved * boxes >= 3200000) && (len >= 40 || 2 * t.constraint_terms >= len);
   if (region) return role_fits(a) || saved * boxes >= 1600000;
   if (both)
-    return saved * boxes >= (boxes <= 16384 ? 4200000 : 3200000) ||
+    return saved * boxes >= (boxes <= 24576 ? 4200000 : 3200000) ||
            (boxes <= 16384 && len >= 78 + boxes / 140 && (saved >= 64 || boxes <= 2048));
-  return len >= 64 || saved * boxes >= 2800000 || (len >= 30 && boxes <= 512);
+  return (len >= 64 && !waits) || saved * boxes >= 2800000 || (len >= 30 && boxes <= 512);
 }
 
 cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s)

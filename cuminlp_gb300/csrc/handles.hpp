@@ -63,6 +63,7 @@ struct cmn_problem {
     t.var_off = d_chain_var_off;
     t.term_pt = d_chain_term_pt;
     t.n_vars = (int32_t)host.n_vars();
+    t.products = prog.chain_products;
     // no more warps than the terms over the longest chain, at most eight
     int64_t most = 1, all = 0;
     for (const cmn::ChainSeg& s : prog.chain_seg) {

@@ -641,6 +641,8 @@ class Compiler {
       return ra != rb ? ra < rb : a.pc1 - a.pc0 > b.pc1 - b.pc0;
     });
     out_.chain_seg = segs;
+    for (const Instr& in : code)
+      if ((in.head & 7) == kOpTerm && ((in.head >> 3) & kTermPMask) != kTermVar) ++out_.chain_products;
     build_chains32();
     build_point_chains();
     out_.chain_points = !segs.empty() && segs[0].kind == kChainObjective;

@@ -175,6 +175,7 @@ struct ChainTab {
   // kChainGeneral ones and theirs
   int32_t constraints, constraint_terms;
   int32_t general, general_terms;
+  int32_t products;  // terms of all chains that are products or squares
 };
 
 // A program laid out in levels (Program::level_*), on the device.

@@ -85,6 +85,7 @@ struct Program {
   std::vector<int32_t> level_off, level_run;
   std::vector<Instr> code64l, code32l;
   int level_slots = 0;
+  int32_t chain_products = 0;  // chain terms that are products or squares
   bool chain_points = false;  // every chain has a filter and the root box is in its range
 };
 

@@ -305,3 +305,29 @@ def test_either_path_of_regions(bits):
         clb, cub, cfe = b.bound_children(p.root_box(), vids, widths, 4)
         olb, oub, ofe = op.aggregate_bound(p.root_box(), kinds, vids, widths, n, 4)
         assert np.array_equal(cfe, ofe) and bits_equal(clb, olb) and bits_equal(cub, oub)
+
+
+@pytest.mark.parametrize("n,constraints", [(150, 1), (150, 4), (400, 0), (400, 2)])
+def test_tiles_of_many_variables(n, constraints):
+    # few tiles fit an SM: boxes of one wave and of several, on either path
+    rng = np.random.default_rng(n)
+    p = Problem()
+    x = [p.var(-4.0, 4.0) for _ in range(n)]
+
+    def chain(products):
+        acc = float(rng.normal()) * x[0]
+        for i in range(n):
+            t = x[i] * x[int(rng.integers(0, n))] if products else x[i]
+            acc = acc + float(rng.normal()) * t
+        return acc
+
+    p.set_objective(chain(True))
+    for k in range(constraints):
+        p.add_constraint(chain(k % 2 == 1), A.CMP_LE, 4.0)
+    dp, op = DeviceProblem(p), O.OracleProblem(p)
+    for boxes in (700, 24000):
+        lo, hi = random_boxes(p, boxes, rng, 0.2)
+        for precision in (A.PRECISION_FP64, A.PRECISION_FP32_SCREEN):
+            g, o = eval_boxes(dp, lo, hi, precision), op.eval_boxes(lo, hi, precision)
+            assert np.array_equal(g[2], o[2])
+            assert bits_equal(g[0], o[0]) and bits_equal(g[1], o[1])
