@@ -279,13 +279,20 @@ static bool general_pays(const EvalArgs& a, int mode, int64_t boxes, int64_t sav
   // a role's one launch (n = 12, 1,024 regions, four == chains 134 and 103 us,
   // eight 146 and 168)
   if (mode == 0 && role_fits(a)) return t.general <= 4;
-  if (boxes < 8192) return false;
   const int64_t terms = t.general_terms;
+  // few boxes: the objective by lane groups, or most of the chains <= ones
+  // (n = 24, two constraints, one ==, 300 boxes 223 and 191 us; twelve, two ==,
+  // 1,024 regions of an aggregate 433 and 337)
+  if (pure && a.prog_len >= 200 && boxes < 8192)
+    return mode == 4 ? 2 * t.constraint_terms >= 5 * terms : boxes <= 512 && t.general <= 2;
+  if (boxes < 8192) return false;
   if (t.constraint_terms >= 2 * terms && saved >= 160 && saved * boxes >= 12000000) return true;
   if (!pure) return false;
-  // 180 boxes a term of an average such chain keep the other warps busy
-  if (4 * t.constraint_terms >= 3 * terms && saved * boxes >= 2000000 && boxes >= 16384 &&
-      boxes * t.general >= 180 * terms)
+  // 180 boxes a term of an average such chain keep the other warps busy, 80
+  // regions, whose variables come from the cache (n = 24, two constraints, one
+  // ==, 16,384 regions 434 and 327 us, 16,384 boxes 314 and 370)
+  if (2 * t.constraint_terms >= terms && saved * boxes >= 2000000 && boxes >= 16384 &&
+      boxes * t.general >= (a.pinfo != nullptr ? 80 : 180) * terms)
     return true;
   // between one wave and many, several chains spread over the warps (n = 12,
   // four == chains, 16,384 boxes 178 and 132 us; 524,288 boxes 2,014 and 2,030)
@@ -299,7 +306,8 @@ bool chain_pays(const EvalArgs& a, int mode)
   const int64_t boxes = (int64_t)a.max_boxes, len = a.prog_len;
   const int64_t tiles = max_dynamic_smem() / (int64_t)(tile_smem_bytes(a.n_vars, a.pinfo ? a.max_slots : 0, 32) + 1024);
   const int64_t warps = tiles * std::max(1, std::min(t.constraints + t.general, kTileWarps));
-  const bool waits = boxes > 32 * tiles * sm_count() && warps < 16;
+  // (regions read one parent's variables, from the cache)
+  const bool waits = boxes > 32 * tiles * sm_count() && warps < (a.pinfo != nullptr ? 6 : 16);
   const int64_t saved = 4ll * t.constraint_terms - (waits ? 48ll * a.n_vars / warps : 3ll * a.n_vars) - 6ll * t.constraints;
   if (t.general > 0) return general_pays(a, mode, boxes, saved);
   if (mode == 1 || mode == 3 || mode == 6) return true;  // in the solver no form or size lost
@@ -307,18 +315,26 @@ bool chain_pays(const EvalArgs& a, int mode)
   if (t.constraints == 0) {
     // the objective alone: the same work on either side, the program staged
     // there, lane groups or half the bounds here
-    if (mode == 4) return len >= 45;
+    if (mode == 4) return len >= 45 || (len >= 15 && boxes <= 8);
     if (region) return true;
     if (both) return (len > 64 && boxes <= 10240) || (len >= 5 && boxes >= 98304);
     return len >= 12 || (len > 3 && boxes >= 65536);
   }
+  const bool warped = t.constraints >= 2;  // a tile has a warp a chain
   if (mode == 4)  // n = 4, 30 instructions: 16,384 regions 50 and 65 us, 65,536 74 and 66
-    return len >= 20 && ((len >= 72 && !waits) || saved * boxes >= 3200000) && (len >= 40 || 2 * t.constraint_terms >= len);
-  if (region) return role_fits(a) || saved * boxes >= 1600000;
+    return len >= 20 && ((len >= 72 && !waits) || saved * boxes >= (warped ? 2500000 : 3200000)) &&
+           (len >= 40 || 2 * t.constraint_terms >= len);
+  // n = 5, two constraints, 36 instructions, 32,768 regions 52 and 43 us; n = 4,
+  // one, 30 instructions 49 and 63
+  if (region)
+    return role_fits(a) || (len >= 64 && !waits) || saved * boxes >= (warped && boxes >= 24576 ? 1000000 : 1600000);
+  // the second launch weighs less the longer the first is
+  const int64_t need = boxes >= 90000                                    ? 1600000
+                       : boxes >= 50000 || (boxes >= 28000 && warped) ? 2000000
+                                                                         : 4200000;
   if (both)
-    return saved * boxes >= (boxes <= 24576 ? 4200000 : 3200000) ||
-           (boxes <= 16384 && len >= 78 + boxes / 140 && (saved >= 64 || boxes <= 2048));
-  return (len >= 64 && !waits) || saved * boxes >= 2800000 || (len >= 30 && boxes <= 512);
+    return saved * boxes >= need || (boxes <= 16384 && len >= 72 + boxes / 140 && (saved >= 64 || boxes <= 2048));
+  return (len >= 64 && !waits) || saved * boxes >= need * 7 / 10 || (len >= 30 && boxes <= 512);
 }
 
 cudaError_t launch_chain(const EvalArgs& a, int mode, cudaStream_t s)
