@@ -324,10 +324,10 @@ bool chain_pays(const EvalArgs& a, int mode)
   if (mode == 4)  // n = 4, 30 instructions: 16,384 regions 50 and 65 us, 65,536 74 and 66
     return len >= 20 && ((len >= 72 && !waits) || saved * boxes >= (warped ? 2500000 : 3200000)) &&
            (len >= 40 || 2 * t.constraint_terms >= len);
-  // n = 5, two constraints, 36 instructions, 32,768 regions 52 and 43 us; n = 4,
+  // n = 8, two constraints, 60 instructions, 32,768 regions 98 and 64 us; n = 4,
   // one, 30 instructions 49 and 63
   if (region)
-    return role_fits(a) || (len >= 64 && !waits) || saved * boxes >= (warped && boxes >= 24576 ? 1000000 : 1600000);
+    return role_fits(a) || (len >= 64 && !waits) || saved * boxes >= (warped && boxes >= 24576 ? 600000 : 1600000);
   // the second launch weighs less the longer the first is
   const int64_t need = boxes >= 90000                                    ? 1600000
                        : boxes >= 50000 || (boxes >= 28000 && warped) ? 2000000
