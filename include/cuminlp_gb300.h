@@ -621,7 +621,9 @@ cmn_status cmn_batch_poll(const cmn_batch* batch, uint64_t slot,
  * `slot` (`best_point`: n_vars doubles, NaN when none; may be NULL). */
 cmn_status cmn_batch_outcome(cmn_batch* batch, uint64_t slot,
                              cmn_outcome* out, double* best_point);
-/* Copies `slot`'s frontier (pool order) as cmn_solver_frontier does. */
+/* Copies `slot`'s frontier (pool order) as cmn_solver_frontier does, through
+ * pinned host memory that the batch keeps, as large as its largest call took
+ * (at most twice that). */
 cmn_status cmn_batch_frontier(cmn_batch* batch, uint64_t slot, double* boxes,
                               double* lower_bounds, uint32_t* depths,
                               uint64_t room, uint64_t* count);
